@@ -217,9 +217,9 @@ static void FN(gemm)(int ta, int tb, int64_t M, int64_t N, int64_t K, const T *A
       }
     } else {
       for (int64_t j = 0; j < N; j++) {
-        T s = (T)0;
-        for (int64_t k = 0; k < K; k++) s += (ta ? A[k * M + i] : A[i * K + k]) * Bm[j * K + k];
-        crow[j] += s;
+        double s = 0;   /* (K is a whole image here: in float the sum itself would be off by more than the tests allow) */
+        for (int64_t k = 0; k < K; k++) s += (double)(ta ? A[k * M + i] : A[i * K + k]) * Bm[j * K + k];
+        crow[j] += (T)s;
       }
     }
   }
