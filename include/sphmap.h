@@ -100,6 +100,36 @@ int sph_resample_from_map(const void *x, const void *map, const void *iw, void *
                           void *stream);
 
 /* ------------------------------------------------------------------------
+ * Scratch for resampling and pooling (optional).  The *_ws entry points are
+ * the operators of this header with caller scratch: with at least
+ * sph_staging_bytes() bytes (32-byte aligned, contents irrelevant) float32
+ * tensors are processed in groups of 8 or 4 planes, transposed chunk by chunk
+ * into the scratch, so that one load per tap serves a whole group; without
+ * (NULL, or too small) they run the kernels of the entry points that take no
+ * scratch.  Results are bit-identical either way.  sph_staging_bytes()
+ * returns 0 where the transposition does not pay.
+ *   planes  B*C;  n_src  pixels of a plane that is read (GATHER, POOL: H*W;
+ *   SCATTER: MH*MW, ARGMAX: OH*OW);  reads  taps GATHER and POOL read per plane (positions x
+ *   slots x points x 1 or 4), else ignored.
+ * No counterpart in the reference.
+ * ---------------------------------------------------------------------- */
+enum sph_stage_op { SPH_STAGE_GATHER = 0, SPH_STAGE_POOL = 1, SPH_STAGE_ARGMAX = 2, SPH_STAGE_SCATTER = 3 };
+size_t sph_staging_bytes(int op, int64_t planes, int64_t n_src, int64_t reads, int dtype);
+int sph_resample_from_map_ws(const void *x, const void *map, const void *iw, void *y, int64_t B, int64_t C, int64_t H,
+                             int64_t W, int64_t MH, int64_t MW, int64_t P, int dtype, int interp, void *ws,
+                             size_t ws_bytes, void *stream);
+/* normalize != 0: sph_resample_to_map_normalized */
+int sph_resample_to_map_ws(const void *x, const void *plan, void *out, int64_t B, int64_t C, int64_t MH, int64_t MW,
+                           int64_t OH, int64_t OW, int normalize, int dtype, void *ws, size_t ws_bytes, void *stream);
+/* max pooling, or (average != 0, idx ignored) average pooling */
+int sph_mapped_pool_ws(const void *x, const void *map, const void *iw, void *out, int64_t *idx, int64_t B, int64_t C,
+                       int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P, int average, int dtype,
+                       int interp, void *ws, size_t ws_bytes, void *stream);
+int sph_mapped_max_unpool_ws(const void *g, const int64_t *idx, const void *plan, void *grad_in, int64_t B, int64_t C,
+                             int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, void *ws,
+                             size_t ws_bytes, void *stream);
+
+/* ------------------------------------------------------------------------
  * Scatter plan.  Every adjoint ("scatter") operator of the reference adds
  * through float atomics.  This library instead inverts the sample map once
  * into a CSR table keyed by (destination pixel, kernel slot) and every

@@ -244,6 +244,21 @@ inline int launch_status(int n = 1) {
   return cudaGetLastError() == cudaSuccess ? SPH_OK : SPH_ERR_CUDA;
 }
 
+// Division by a runtime constant as multiply-high + shift (exact for 0 <= x < 2^31 and 1 <= d < 2^31).
+struct FastDiv {
+  unsigned mul, shift, d;
+  __host__ __device__ static FastDiv make(unsigned d) {
+    FastDiv f;
+    f.d = d;
+    unsigned l = 0;
+    while ((1ull << l) < d) l++;
+    f.shift = l;
+    f.mul = (unsigned)((((1ull << l) - d) << 32) / d + 1);
+    return f;
+  }
+  __device__ __forceinline__ unsigned div(unsigned x) const { return (__umulhi(x, mul) + x) >> shift; }
+};
+
 inline int cdiv(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
 // Dispatch a runtime interpolation code to a template parameter.

@@ -24,21 +24,6 @@ constexpr int kWalkWindow = 32 * kWalkUnroll;       // entries per window
 template <typename T, int PL, bool NORM>
 __host__ __device__ constexpr int walk_smem_per_warp() { return (PL + (NORM ? 1 : 0)) * kWalkWindow * (int)sizeof(T); }
 
-// Division by a runtime constant as multiply-high + shift (exact for 0 <= x < 2^31 and 1 <= d < 2^31).
-struct FastDiv {
-  unsigned mul, shift, d;
-  __host__ __device__ static FastDiv make(unsigned d) {
-    FastDiv f;
-    f.d = d;
-    unsigned l = 0;
-    while ((1ull << l) < d) l++;
-    f.shift = l;
-    f.mul = (unsigned)((((1ull << l) - d) << 32) / d + 1);
-    return f;
-  }
-  __device__ __forceinline__ unsigned div(unsigned x) const { return (__umulhi(x, mul) + x) >> shift; }
-};
-
 // prepare(s) -> per-entry value shared by all planes (source offset, decoded slot ...); contrib(pre, w, j) ->
 // contribution of that entry to plane j of this CTA's plane group.  Pixels [q_begin, q_end) are walked by the calling
 // CTA's warps; out_plane0 points at plane 0 of the group and planes are n_dst apart; np <= PL planes are written.

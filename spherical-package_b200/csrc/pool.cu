@@ -3,6 +3,7 @@
 
 #include "common.cuh"
 #include "plan_walk.cuh"
+#include "plane_groups.cuh"
 
 namespace sph {
 
@@ -193,6 +194,235 @@ max_unpool_plan_kernel(const T *__restrict__ g, const int64_t *__restrict__ idx,
                           gin + (size_t)p0 * n_dst, np);
 }
 
+// ---- over plane groups (plane_groups.cuh) ----------------------------------------------------------------------
+// Max / average pooling.  TABLE: the taps of the tile's outputs are decoded once into shared memory for the PG / 4 threads
+// of every output (groups of 16 or 32 planes); else every thread decodes its own.
+template <int PG, int INTERP, bool WEIGHTED, bool AVG>
+struct PoolOp {
+  static constexpr int VP = Split<PG>::VP, LP = Split<PG>::LP, TO = Split<PG>::TO;
+  static constexpr bool TABLE = LP > 1 && !WEIGHTED;
+  PlaneChunks c;
+  const float *x, *map, *iw;
+  float *out;
+  int64_t *idx;
+  int n, H, W, K, P;
+  TileGrid grid;
+  FastDiv stage_tiles, use_tiles;
+
+  bool table;  // the tap table fits the shared memory a block has without opting in
+
+  static size_t table_bytes(int64_t K) {
+    const size_t b = TABLE ? (size_t)K * TO * (INTERP == SPH_NEAREST ? 4 : 32) : 0;
+    return b <= 48 * 1024 ? b : 0;
+  }
+
+  __device__ __forceinline__ void stage(int p0, char *rows, int tile) const { stage_quad<PG>(x, c.planes, c.n_src, p0, tile, rows); }
+  __device__ __forceinline__ void use(int p0, const char *rows, int tile) const {
+    extern __shared__ __align__(16) unsigned char pool_table[];
+    unsigned *near_off = (unsigned *)pool_table;                       // nearest: [K][TO] offsets
+    uint4 *tab_off = (uint4 *)pool_table;                              // else [K][TO] offsets, then [K][TO] weights
+    float4 *tab_w = (float4 *)pool_table + (size_t)K * TO;
+    const int ol = threadIdx.x / LP, o = grid.output<PG>(tile, ol);
+    if (TABLE && table) {
+      for (int e = threadIdx.x; e < K * TO; e += kStageThreads) {
+        const int k = e / TO, oo = grid.output<PG>(tile, e % TO);
+        const float *m = map + 2 * ((size_t)max(oo, 0) * K + k);
+        const RowTaps t = row_taps<INTERP>(__ldg(m), __ldg(m + 1), H, W, PG * 4);
+        if (INTERP == SPH_NEAREST) {
+          near_off[e] = t.off.x;
+        } else {
+          tab_off[e] = t.off;
+          tab_w[e] = t.w;
+        }
+      }
+      __syncthreads();
+    }
+    if (o < 0) return;
+    const int PP = WEIGHTED ? P : 1;
+    const float *m = map + 2 * (size_t)o * K * PP;
+    const float *wgt = WEIGHTED ? iw + (size_t)o * K * PP : nullptr;
+    rows += threadIdx.x % LP * (VP * 4);
+    p0 += threadIdx.x % LP * VP;
+    Vec<VP> best = vec_fill<VP>(AVG ? 0.0f : -FLT_MAX);
+    int bk[VP];
+#pragma unroll
+    for (int j = 0; j < VP; j++) bk[j] = -1;
+    constexpr int UNROLL = INTERP == SPH_NEAREST && !WEIGHTED ? 3 : 1;
+#pragma unroll UNROLL
+    for (int k = 0; k < K; k++) {
+      Vec<VP> v;
+      if (WEIGHTED) {
+        v = vec_fill<VP>(0.0f);
+        for (int q = 0; q < P; q++) {
+          const int e = k * P + q;
+          const RowTaps t = row_taps<INTERP>(__ldg(m + 2 * e), __ldg(m + 2 * e + 1), H, W, PG * 4);
+          v = vec_add<VP>(v, vec_scale<VP>(__ldg(wgt + e), row_gather<VP, INTERP>(rows, t)));
+        }
+      } else {
+        RowTaps t;
+        if (!TABLE || !table) {
+          t = row_taps<INTERP>(__ldg(m + 2 * k), __ldg(m + 2 * k + 1), H, W, PG * 4);
+        } else if (INTERP == SPH_NEAREST) {
+          t.off.x = near_off[k * TO + ol];
+        } else {
+          t.off = tab_off[k * TO + ol];
+          t.w = tab_w[k * TO + ol];
+        }
+        v = row_gather<VP, INTERP>(rows, t);
+      }
+      if (AVG) {
+        best = vec_add<VP>(best, v);
+      } else {
+#pragma unroll
+        for (int j = 0; j < VP; j++)
+          if (v.f[j] > best.f[j]) { best.f[j] = v.f[j]; bk[j] = k; }
+      }
+    }
+    if (AVG) {
+#pragma unroll
+      for (int j = 0; j < VP; j++) best.f[j] = best.f[j] / (float)K;
+    }
+    store_planes<VP>(out, n, o, p0, c.planes, best);
+    if (!AVG) {
+      const long long first = (long long)o * K;
+      long long *ip = (long long *)idx + (size_t)p0 * n + o;
+#pragma unroll
+      for (int j = 0; j < VP; j++)
+        if (p0 + j < c.planes) __stcs(ip + (size_t)j * n, bk[j] < 0 ? -1ll : (first + bk[j]) * (2 * PP));
+    }
+  }
+};
+
+// Deterministic argmax backward.  Behind a group's gradient rows lie the PG winning slots of every output as bytes
+// (kNoSlot: none).  With all slots below 128, a byte b of (winners ^ slot in every byte) + 0x7f.. keeps its top bit clear
+// exactly where the slots are equal: two instructions test four planes, and only threads with a winner read the gradient.
+constexpr unsigned kNoSlot = 127u;
+template <int PG>
+struct UnpoolOp {
+  PlaneChunks c;
+  const float *g;
+  const int64_t *idx;
+  const void *plan;
+  float *gin;
+  int n_dst, K, PP;
+  TileGrid grid;
+  FastDiv divK, div2P, stage_tiles, use_tiles;
+
+  __device__ __forceinline__ size_t winners_at() const { return (size_t)(c.n_src + 1) * PG * 4; }
+  __device__ __forceinline__ void stage(int p0, char *rows, int tile) const {
+    constexpr int LP = PG / 4;
+    stage_quad<PG>(g, c.planes, c.n_src, p0, tile, rows);
+    const int q = threadIdx.x % LP, o = tile * kStagePixels<PG> + threadIdx.x / LP * 4;
+    const int slots = K * 2 * PP;
+    p0 += q * 4;
+    const long long *ip = (const long long *)idx + (size_t)p0 * c.n_src + o;
+    unsigned *w = (unsigned *)(rows + winners_at()) + (size_t)o * LP + q;
+    const bool vec = (c.n_src & 3) == 0 && (((uintptr_t)idx) & 15) == 0;
+    unsigned win[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      long long s[4] = {-1, -1, -1, -1};
+      if (p0 + j < c.planes && o < c.n_src) {
+        if (vec) {
+          const longlong2 a = __ldcs((const longlong2 *)(ip + (size_t)j * c.n_src)), b = __ldcs((const longlong2 *)(ip + (size_t)j * c.n_src) + 1);
+          s[0] = a.x; s[1] = a.y; s[2] = b.x; s[3] = b.y;
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+            if (o + i < c.n_src) s[i] = __ldcs(ip + (size_t)j * c.n_src + i);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const long long d = s[i] - (long long)(o + i) * slots;  // from this output's slot 0
+        unsigned k = kNoSlot;
+        if (s[i] >= 0 && d >= 0 && d < slots) {
+          const unsigned slot = div2P.div((unsigned)d);
+          if (slot * (2 * PP) == (unsigned)d) k = slot;
+        }
+        win[i] |= k << (8 * j);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (o + i < c.n_src) w[(size_t)i * LP] = win[i];
+  }
+  __device__ __forceinline__ void use(int p0, const char *rows, int tile) const {
+    constexpr int VP = Split<PG>::VP, LP = Split<PG>::LP, W4 = VP / 4;
+    const int q = grid.output<PG>(tile, threadIdx.x / LP);
+    if (q < 0) return;
+    bool ok;
+    const PlanView<float> pv = plan_view<float>(plan, n_dst, ok, c.n_src * K);
+    const char *wins = rows + winners_at() + threadIdx.x % LP * VP;
+    rows += threadIdx.x % LP * (VP * 4);
+    const int e0 = ok ? __ldg(pv.offsets + q) : 0, e1 = ok ? __ldg(pv.offsets + q + 1) : 0;
+    Vec<VP> acc = vec_fill<VP>(0.0f);
+#pragma unroll 2
+    for (int e = e0; e < e1; e++) {
+      const int s = __ldg(pv.src + e);
+      if (!index_ok(s, pv.n_src)) continue;
+      const unsigned o = divK.div((unsigned)s), k4 = ((unsigned)s - o * K) * 0x01010101u;
+      unsigned miss[W4], all = 0x80808080u;
+      if constexpr (W4 == 2) {
+        const uint2 w2 = __ldg((const uint2 *)(wins + o * PG));
+        miss[0] = w2.x;
+        miss[1] = w2.y;
+      } else {
+        miss[0] = __ldg((const unsigned *)(wins + o * PG));
+      }
+#pragma unroll
+      for (int i = 0; i < W4; i++) {
+        miss[i] = (miss[i] ^ k4) + 0x7f7f7f7fu;
+        all &= miss[i];
+      }
+      if (all != 0x80808080u) {
+        const float w = __ldg(pv.w + e);
+        const Vec<VP> v = vec_scale<VP>(w, row_load<VP>(rows, o * (PG * 4u)));
+#pragma unroll
+        for (int j = 0; j < VP; j++)
+          if (!(miss[j >> 2] & (0x80u << (8 * (j & 3))))) acc.f[j] = __fadd_rn(acc.f[j], v.f[j]);
+      }
+    }
+    store_planes<VP>(gin, n_dst, q, p0 + threadIdx.x % LP * VP, c.planes, acc);
+  }
+};
+
+template <int PG>
+static int pool_groups(const PlaneChunks &c, const void *x, const void *map, const void *iw, void *out, int64_t *idx, int64_t H, int64_t W,
+                       int64_t OH, int64_t OW, int64_t K, int64_t P, int interp, cudaStream_t st, bool avg) {
+  const int64_t n = OH * OW;
+  const TileGrid grid = TileGrid::make<PG>(OH, OW);
+  const FastDiv ts = FastDiv::make(stage_tiles<PG>(H * W)), tu = FastDiv::make(grid.tiles<PG>());
+#define SPH_POOL_GROUPS(WEIGHTED, AVG)                                                                                                     \
+  do {                                                                                                                                  \
+    using Op = PoolOp<PG, INTERP, WEIGHTED, AVG>;                                                                                       \
+    const size_t tb = Op::table_bytes(K);                                                                                               \
+    return launch_plane_groups(Op{c, (const float *)x, (const float *)map, (const float *)iw, (float *)out, idx, (int)n, (int)H, (int)W, \
+                                  (int)K, (int)P, grid, ts, tu, tb > 0}, tb, st);                                                             \
+  } while (0)
+  SPH_DISPATCH_INTERP(interp, {
+    if (P > 0) {
+      if (avg) SPH_POOL_GROUPS(true, true);
+      SPH_POOL_GROUPS(true, false);
+    }
+    if (avg) SPH_POOL_GROUPS(false, true);
+    SPH_POOL_GROUPS(false, false);
+  });
+#undef SPH_POOL_GROUPS
+  return SPH_ERR_INVALID_ARGUMENT;
+}
+
+template <int PG>
+static int unpool_groups(const PlaneChunks &c, const void *g, const int64_t *idx, const void *plan, void *gin, int64_t IH, int64_t IW,
+                         int64_t K, int64_t P, cudaStream_t st) {
+  const int64_t n_dst = IH * IW;
+  const TileGrid grid = TileGrid::make<PG>(IH, IW);
+  const int PP = (int)(P > 0 ? P : 1);
+  return launch_plane_groups(UnpoolOp<PG>{c, (const float *)g, idx, plan, (float *)gin, (int)n_dst, (int)K, PP, grid, FastDiv::make((unsigned)K),
+                                          FastDiv::make((unsigned)(2 * PP)), FastDiv::make(stage_tiles<PG>(c.n_src)),
+                                          FastDiv::make(grid.tiles<PG>())}, 0, st);
+}
+
 template <typename T>
 static int unpool_planned(const void *g, const int64_t *idx, const void *plan, void *gin, int64_t planes, int64_t n_dst,
                           int64_t n, int64_t K, int64_t P, cudaStream_t st) {
@@ -293,16 +523,29 @@ using namespace sph;
 
 SPH_TU_STATUS(pool)
 
-extern "C" int sph_mapped_max_pool(const void *x, const void *map, const void *iw, void *out, int64_t *idx, int64_t B,
-                                   int64_t C, int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P,
-                                   int dtype, int interp, void *stream) {
-  SPH_RANGE("sph_mapped_max_pool");
-  const int rc = check(x, map, out, idx, iw, B, C, IH, IW, OH, OW, K, P, dtype, interp);
+extern "C" int sph_mapped_pool_ws(const void *x, const void *map, const void *iw, void *out, int64_t *idx, int64_t B, int64_t C,
+                                  int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P, int average, int dtype,
+                                  int interp, void *ws, size_t ws_bytes, void *stream) {
+  SPH_RANGE(average ? "sph_mapped_avg_pool" : "sph_mapped_max_pool");
+  const int rc = check(x, map, out, average ? out : (const void *)idx, iw, B, C, IH, IW, OH, OW, K, P, dtype, interp);
   if (rc != SPH_OK) return rc;
   if (B * C == 0 || OH * OW == 0) return SPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  return dtype == SPH_F32 ? pool<float>(x, map, iw, out, idx, B * C, IH, IW, OH * OW, K, P, interp, st)
-                          : pool<double>(x, map, iw, out, idx, B * C, IH, IW, OH * OW, K, P, interp, st);
+  if (dtype == SPH_F32 && B * C >= 3 && scratch_ok(ws)) {
+    PlaneChunks c = stage_chunks(B * C, IH * IW, 4);
+    if (ws_bytes >= stage_bytes(c) && stage_fits(c)) {
+      c.buf = (char *)ws;
+      SPH_DISPATCH_GROUP(c.group_planes, return pool_groups<PG>(c, x, map, iw, out, idx, IH, IW, OH, OW, K, P, interp, st, average != 0));
+    }
+  }
+  return dtype == SPH_F32 ? pool<float>(x, map, iw, out, idx, B * C, IH, IW, OH * OW, K, P, interp, st, average != 0)
+                          : pool<double>(x, map, iw, out, idx, B * C, IH, IW, OH * OW, K, P, interp, st, average != 0);
+}
+
+extern "C" int sph_mapped_max_pool(const void *x, const void *map, const void *iw, void *out, int64_t *idx, int64_t B,
+                                   int64_t C, int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P,
+                                   int dtype, int interp, void *stream) {
+  return sph_mapped_pool_ws(x, map, iw, out, idx, B, C, IH, IW, OH, OW, K, P, 0, dtype, interp, nullptr, 0, stream);
 }
 
 extern "C" int sph_mapped_max_unpool(const void *g, const int64_t *idx, const void *map, const void *iw, void *grad_in,
@@ -323,6 +566,12 @@ extern "C" int sph_mapped_max_unpool(const void *g, const int64_t *idx, const vo
 extern "C" int sph_mapped_max_unpool_planned(const void *g, const int64_t *idx, const void *plan, void *grad_in, int64_t B,
                                              int64_t C, int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P,
                                              int dtype, void *stream) {
+  return sph_mapped_max_unpool_ws(g, idx, plan, grad_in, B, C, IH, IW, OH, OW, K, P, dtype, nullptr, 0, stream);
+}
+
+extern "C" int sph_mapped_max_unpool_ws(const void *g, const int64_t *idx, const void *plan, void *grad_in, int64_t B, int64_t C,
+                                        int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, void *ws,
+                                        size_t ws_bytes, void *stream) {
   SPH_RANGE("sph_mapped_max_unpool_planned");
   const int rc = check(g, plan, grad_in, idx, nullptr, B, C, IH, IW, OH, OW, K, 0, dtype, 0);
   if (rc != SPH_OK) return rc;
@@ -332,6 +581,13 @@ extern "C" int sph_mapped_max_unpool_planned(const void *g, const int64_t *idx, 
   if (OH * OW == 0)
     return cudaMemsetAsync(grad_in, 0, (dtype == SPH_F64 ? 8 : 4) * (size_t)(B * C * IH * IW), st) == cudaSuccess
                ? SPH_OK : SPH_ERR_CUDA;
+  if (dtype == SPH_F32 && B * C >= 3 && K < kNoSlot && scratch_ok(ws)) {
+    PlaneChunks c = stage_chunks(B * C, OH * OW, 5);
+    if (ws_bytes >= stage_bytes(c) && stage_fits(c)) {
+      c.buf = (char *)ws;
+      SPH_DISPATCH_GROUP(c.group_planes, return unpool_groups<PG>(c, g, idx, plan, grad_in, IH, IW, K, P, st));
+    }
+  }
   return dtype == SPH_F32 ? unpool_planned<float>(g, idx, plan, grad_in, B * C, IH * IW, OH * OW, K, P, st)
                           : unpool_planned<double>(g, idx, plan, grad_in, B * C, IH * IW, OH * OW, K, P, st);
 }
@@ -339,11 +595,5 @@ extern "C" int sph_mapped_max_unpool_planned(const void *g, const int64_t *idx, 
 extern "C" int sph_mapped_avg_pool(const void *x, const void *map, const void *iw, void *out, int64_t B, int64_t C, int64_t IH,
                                    int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp,
                                    void *stream) {
-  SPH_RANGE("sph_mapped_avg_pool");
-  const int rc = check(x, map, out, out, iw, B, C, IH, IW, OH, OW, K, P, dtype, interp);
-  if (rc != SPH_OK) return rc;
-  if (B * C == 0 || OH * OW == 0) return SPH_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  return dtype == SPH_F32 ? pool<float>(x, map, iw, out, nullptr, B * C, IH, IW, OH * OW, K, P, interp, st, true)
-                          : pool<double>(x, map, iw, out, nullptr, B * C, IH, IW, OH * OW, K, P, interp, st, true);
+  return sph_mapped_pool_ws(x, map, iw, out, nullptr, B, C, IH, IW, OH, OW, K, P, 1, dtype, interp, nullptr, 0, stream);
 }

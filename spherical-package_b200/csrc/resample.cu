@@ -2,7 +2,7 @@
 #include <algorithm>
 
 #include "common.cuh"
-#include "plan_walk.cuh"
+#include "plane_groups.cuh"
 
 namespace sph {
 
@@ -60,37 +60,61 @@ resample_from_map_kernel(const T *__restrict__ x, const T *__restrict__ map, con
   }
 }
 
-// How a plan entry's source id s turns into the value it contributes.
-//   div == 1   x[s]                       resample_to_map
-//   div  > 1   x[s / div] / div           mapped average unpooling: the plan runs over the flattened map slots
-//                                         s = o * K + k and every slot carries grad[o] / K
-//                                         (common/mapped_avg_pool.h:41-69, 109-143)
-template <typename T, bool DIV>
-struct SrcValue {
-  int div;
-  FastDiv fd;
-  __device__ __forceinline__ int index(int s) const { return DIV ? (int)fd.div((unsigned)s) : s; }
-  __device__ __forceinline__ T value(T v) const { return DIV ? v / (T)div : v; }
-};
-
-// Adjoint as a gather through the plan (plan_walk.cuh): a CTA takes a chunk of destination pixels and PL planes.
-// NORM: the sum is divided by (sum of the segment's weights + 1e-12), i.e. scatter(x) / (scatter(1) + 1e-12), the
-// weight-sum normalisation the reference composes in Python (layers/functional/sphere_ops.py:74-80).
+// Adjoint as a gather through the plan.  A thread owns one destination pixel of PL planes and walks the pixel's segment:
+// an entry's source and weight are read once (the next entry's while this one's values are on their way) and serve PL
+// independent loads, products and sums.  Sums run in plan order whatever the scheduling: deterministic, with no zero-fill
+// pass and no atomics (the reference's scatter kernels use atomicAdd: ext_modules/include/cuda/resample.cuh:14-47).
+//   DIV   x[s / div] / div instead of x[s]: mapped average unpooling, whose plan runs over the flattened map slots
+//         s = o * K + k and whose slots all carry grad[o] / K (common/mapped_avg_pool.h:41-69, 109-143)
+//   NORM  the sum is divided by (sum of the segment's weights + 1e-12), i.e. scatter(x) / (scatter(1) + 1e-12), the
+//         weight-sum normalisation the reference composes in Python (layers/functional/sphere_ops.py:74-80)
 template <typename T, int PL, bool NORM, bool DIV>
 __global__ void __launch_bounds__(256)
-resample_to_map_kernel(const T *__restrict__ x, const void *__restrict__ plan_blob, T *__restrict__ out, int n_dst,
-                       int n_src, int planes, int chunk, SrcValue<T, DIV> sv) {
-  extern __shared__ unsigned char walk_smem[];
+resample_to_map_kernel(const T *__restrict__ x, const void *__restrict__ plan_blob, T *__restrict__ out, int n_dst, int n_src,
+                       int planes, int div, FastDiv fd) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n_dst) return;
   bool ok;
-  const PlanView<T> plan = plan_view<T>(plan_blob, n_dst, ok, DIV ? n_src * sv.div : n_src);
-  const int p0 = blockIdx.y * PL;
-  const int np = min(PL, planes - p0);
+  const PlanView<T> pv = plan_view<T>(plan_blob, n_dst, ok, DIV ? n_src * div : n_src);
+  const int e0 = ok ? __ldg(pv.offsets + q) : 0, e1 = ok ? __ldg(pv.offsets + q + 1) : 0;
+  const int p0 = blockIdx.y * PL, np = min(PL, planes - p0);
   const T *xp = x + (size_t)p0 * n_src;
-  const int q_begin = blockIdx.x * chunk, q_end = min(q_begin + chunk, n_dst);
-  plan_walk<T, PL, NORM>(plan, ok, n_dst, q_begin, q_end, (T *)walk_smem,
-                         [&](int s) { return xp + sv.index(s); },
-                         [&](const T *src, T w, int j) { return w * sv.value(__ldg(src + (size_t)j * n_src)); },
-                         out + (size_t)p0 * n_dst, np);
+  T acc[PL], wsum = T(0);
+#pragma unroll
+  for (int j = 0; j < PL; j++) acc[j] = T(0);
+  int s = e0 < e1 ? __ldg(pv.src + e0) : 0;
+  T w = e0 < e1 ? __ldg(pv.w + e0) : T(0);
+  for (int e = e0; e < e1; e++) {
+    const unsigned o = DIV ? fd.div((unsigned)s) : (unsigned)s;
+    const bool fine = index_ok(s, pv.n_src);
+    const T we = w;
+    if (e + 1 < e1) {
+      s = __ldg(pv.src + e + 1);
+      w = __ldg(pv.w + e + 1);
+    }
+    if (!fine) continue;
+    T v[PL];
+    const T *src = xp + o;
+    if (np == PL) {  // (the usual block: no predicates)
+#pragma unroll
+      for (int j = 0; j < PL; j++, src += n_src) v[j] = __ldg(src);
+    } else {
+#pragma unroll
+      for (int j = 0; j < PL; j++, src += n_src) v[j] = j < np ? __ldg(src) : T(0);
+    }
+#pragma unroll
+    for (int j = 0; j < PL; j++) acc[j] = RN<T>::add(acc[j], RN<T>::mul(we, DIV ? v[j] / (T)div : v[j]));
+    if (NORM) wsum += we;
+  }
+  if (NORM && e1 > e0) {  // (an empty sum is zero already: dividing a zero takes the slow way through the divide)
+    const T den = wsum + T(1e-12);
+#pragma unroll
+    for (int j = 0; j < PL; j++) acc[j] = acc[j] / den;
+  }
+  T *op = out + (size_t)p0 * n_dst + q;
+#pragma unroll
+  for (int j = 0; j < PL; j++)
+    if (j < np) __stcs(op + (size_t)j * n_dst, acc[j]);
 }
 
 // Planes walked per thread: 8 amortises the tap decode best; small problems use 2 so that enough threads are
@@ -121,39 +145,135 @@ static int from_map(const void *x, const void *map, const void *iw, void *y, int
   return launch_status();
 }
 
-// n_src: elements per source plane; src_div: see SrcValue.
-template <typename T, int PL, bool NORM, bool DIV>
-static void to_map_launch(const void *x, const void *plan, void *out, int64_t planes, int64_t n_src, int64_t n_dst, int src_div,
-                          cudaStream_t st) {
-  const int groups = cdiv(planes, PL);
-  // CTAs of 8 warps; enough CTAs for a few waves of the SMs, each warp walking several 32-pixel blocks so that the
-  // segment bounds of the next block are in flight while the current one is summed
-  int64_t chunks = ((int64_t)148 * 16 + groups - 1) / groups;
-  const int64_t max_chunks = (n_dst + 255) / 256;
-  if (chunks > max_chunks) chunks = max_chunks;
-  if (chunks < 1) chunks = 1;
-  const int chunk = (int)(((n_dst + chunks - 1) / chunks + 255) / 256 * 256);
-  const size_t smem = 8 * (size_t)walk_smem_per_warp<T, PL, NORM>();
-  resample_to_map_kernel<T, PL, NORM, DIV><<<dim3(cdiv(n_dst, chunk), groups), 256, smem, st>>>(
-      (const T *)x, plan, (T *)out, (int)n_dst, (int)n_src, (int)planes, chunk, SrcValue<T, DIV>{src_div, FastDiv::make((unsigned)src_div)});
-}
-
-template <typename T, bool NORM, bool DIV>
-static int to_map_n(const void *x, const void *plan, void *out, int64_t planes, int64_t n_src, int64_t n_dst, int src_div,
-                    cudaStream_t st) {
-  // planes per CTA: more planes amortise the plan reads and put more stores in flight per warp
-  if (sizeof(T) == 4 && planes >= 128) to_map_launch<T, 16, NORM, DIV>(x, plan, out, planes, n_src, n_dst, src_div, st);
-  else if (planes >= 8) to_map_launch<T, 8, NORM, DIV>(x, plan, out, planes, n_src, n_dst, src_div, st);
-  else to_map_launch<T, 4, NORM, DIV>(x, plan, out, planes, n_src, n_dst, src_div, st);
-  return launch_status();
-}
-
 template <typename T>
 static int to_map(const void *x, const void *plan, void *out, int64_t planes, int64_t n_src, int64_t n_dst, cudaStream_t st,
                   int src_div = 1, bool normalize = false) {
-  if (src_div > 1) return to_map_n<T, false, true>(x, plan, out, planes, n_src, n_dst, src_div, st);  // never normalised
-  return normalize ? to_map_n<T, true, false>(x, plan, out, planes, n_src, n_dst, 1, st)
-                   : to_map_n<T, false, false>(x, plan, out, planes, n_src, n_dst, 1, st);
+  constexpr int PL = 8;
+  const dim3 grid(cdiv(n_dst, 256), cdiv(planes, PL));
+  const FastDiv fd = FastDiv::make((unsigned)src_div);
+#define SPH_SCATTER(NORM, DIV)                                                                                                       \
+  resample_to_map_kernel<T, PL, NORM, DIV><<<grid, 256, 0, st>>>((const T *)x, plan, (T *)out, (int)n_dst, (int)n_src, (int)planes, \
+                                                                 src_div, fd)
+  if (src_div > 1) SPH_SCATTER(false, true);  // (never normalised)
+  else if (normalize) SPH_SCATTER(true, false);
+  else SPH_SCATTER(false, false);
+#undef SPH_SCATTER
+  return launch_status();
+}
+
+// ---- over plane groups (plane_groups.cuh) ----------------------------------------------------------------------
+// The scatter: a thread owns one destination pixel of all PG planes of a group; an entry is one row.  Groups of at most 16
+// (96 planes of 20 x 256 x 256 positions onto 1024 x 2048 pixels, transposition apart: 8 planes 0.55 ms, 16 0.48 ms, 32 0.54 ms;
+// two entries in flight 0.61 ms; the kernel above 0.74 ms).
+template <int PG, bool NORM>
+struct ScatterOp {
+  PlaneChunks c;
+  const float *x;
+  const void *plan;
+  float *out;
+  int n_dst;
+  FastDiv stage_tiles, use_tiles;
+
+  __device__ __forceinline__ void stage(int p0, char *rows, int tile) const { stage_quad<PG>(x, c.planes, c.n_src, p0, tile, rows); }
+  __device__ __forceinline__ void use(int p0, const char *rows, int tile) const {
+    constexpr int VP = PG < 8 ? PG : 8, NV = PG / VP;
+    const int q = tile * kStageThreads + threadIdx.x;
+    if (q >= n_dst) return;
+    bool ok;
+    const PlanView<float> pv = plan_view<float>(plan, n_dst, ok, c.n_src);
+    const int e0 = __ldg(pv.offsets + q), e1 = __ldg(pv.offsets + q + 1);
+    Vec<VP> acc[NV];
+#pragma unroll
+    for (int i = 0; i < NV; i++) acc[i] = vec_fill<VP>(0.0f);
+    float wsum = 0.0f;
+    if (ok && e0 < e1) {
+      const int *sp = pv.src + e0, *end = pv.src + e1;
+      const float *wp = pv.w + e0;
+      int s = __ldg(sp);
+      float w = __ldg(wp);
+      for (;;) {
+        const char *row = rows + (size_t)(unsigned)s * (PG * 4);
+        const bool fine = index_ok(s, pv.n_src);
+        const float we = w;
+        sp++;
+        wp++;
+        const bool more = sp < end;
+        if (more) {  // the next entry's source and weight travel with this one's row
+          s = __ldg(sp);
+          w = __ldg(wp);
+        }
+        if (fine) {
+          Vec<VP> v[NV];
+#pragma unroll
+          for (int i = 0; i < NV; i++) v[i] = row_load<VP>(row, i * (VP * 4));
+#pragma unroll
+          for (int i = 0; i < NV; i++) acc[i] = vec_add<VP>(acc[i], vec_scale<VP>(we, v[i]));
+          if (NORM) wsum += we;
+        }
+        if (!more) break;
+      }
+      if (NORM) {  // (an empty sum is zero already: dividing a zero takes the slow way through the divide)
+        const float den = wsum + 1e-12f;
+#pragma unroll
+        for (int i = 0; i < NV; i++)
+#pragma unroll
+          for (int j = 0; j < VP; j++) acc[i].f[j] = acc[i].f[j] / den;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NV; i++) store_planes<VP>(out, n_dst, q, p0 + i * VP, c.planes, acc[i]);
+  }
+};
+
+template <int PG>
+static int to_map_groups(const PlaneChunks &c, const void *x, const void *plan, void *out, int64_t n_src, int64_t n_dst, bool normalize,
+                         cudaStream_t st) {
+  const FastDiv ts = FastDiv::make(stage_tiles<PG>(n_src)), tu = FastDiv::make(cdiv(n_dst, kStageThreads));
+  if (normalize)
+    return launch_plane_groups(ScatterOp<PG, true>{c, (const float *)x, plan, (float *)out, (int)n_dst, ts, tu}, 0, st);
+  return launch_plane_groups(ScatterOp<PG, false>{c, (const float *)x, plan, (float *)out, (int)n_dst, ts, tu}, 0, st);
+}
+
+template <int PG, int INTERP, bool WEIGHTED>
+struct GatherOp {
+  PlaneChunks c;
+  const float *x, *map, *iw;
+  float *y;
+  int n, H, W, P;
+  TileGrid grid;
+  FastDiv stage_tiles, use_tiles;
+
+  __device__ __forceinline__ void stage(int p0, char *rows, int tile) const { stage_quad<PG>(x, c.planes, c.n_src, p0, tile, rows); }
+  __device__ __forceinline__ void use(int p0, const char *rows, int tile) const {
+    constexpr int VP = Split<PG>::VP, LP = Split<PG>::LP;
+    const int i = grid.output<PG>(tile, threadIdx.x / LP);
+    if (i < 0) return;
+    rows += threadIdx.x % LP * (VP * 4);
+    Vec<VP> acc = vec_fill<VP>(0.0f);
+    for (int q = 0; q < (WEIGHTED ? P : 1); q++) {
+      const size_t e = (size_t)i * (WEIGHTED ? P : 1) + q;
+      const RowTaps t = row_taps<INTERP>(__ldg(map + 2 * e), __ldg(map + 2 * e + 1), H, W, PG * 4);
+      const Vec<VP> v = row_gather<VP, INTERP>(rows, t);
+      acc = WEIGHTED ? vec_add<VP>(acc, vec_scale<VP>(__ldg(iw + e), v)) : v;
+    }
+    store_planes<VP>(y, n, i, p0 + threadIdx.x % LP * VP, c.planes, acc);
+  }
+};
+
+template <int PG>
+static int from_map_groups(const PlaneChunks &c, const void *x, const void *map, const void *iw, void *y, int64_t H, int64_t W,
+                           int64_t MH, int64_t MW, int64_t P, int interp, cudaStream_t st) {
+  const int64_t n = MH * MW;
+  const TileGrid grid = TileGrid::make<PG>(MH, MW);
+  const FastDiv ts = FastDiv::make(stage_tiles<PG>(H * W)), tu = FastDiv::make(grid.tiles<PG>());
+  SPH_DISPATCH_INTERP(interp, {
+    if (P > 0)
+      return launch_plane_groups(GatherOp<PG, INTERP, true>{c, (const float *)x, (const float *)map, (const float *)iw, (float *)y, (int)n,
+                                                            (int)H, (int)W, (int)P, grid, ts, tu}, 0, st);
+    return launch_plane_groups(GatherOp<PG, INTERP, false>{c, (const float *)x, (const float *)map, nullptr, (float *)y, (int)n, (int)H,
+                                                           (int)W, 0, grid, ts, tu}, 0, st);
+  });
+  return SPH_ERR_INVALID_ARGUMENT;
 }
 
 // Voting resample of integer labels through a nearest-neighbour plan: destination pixel o takes the label that most
@@ -198,9 +318,31 @@ using namespace sph;
 
 SPH_TU_STATUS(resample)
 
+extern "C" size_t sph_staging_bytes(int op, int64_t planes, int64_t n_src, int64_t reads, int dtype) {
+  if (dtype != SPH_F32 || planes < 3 || n_src <= 0 || n_src >= ((int64_t)1 << 31)) return 0;
+  switch (op) {
+    // A gather that reads a pixel less than once on average leaves whole sectors of the source untouched, which the
+    // transposition would fetch; and the few taps per position of a resampling map do not pay for rows that go through HBM.
+    case SPH_STAGE_GATHER: {
+      const PlaneChunks c = stage_chunks(planes, n_src, 4);
+      return reads < n_src || c.group_bytes > kStageGroup ? 0 : stage_bytes(c);
+    }
+    case SPH_STAGE_SCATTER: return stage_bytes(stage_chunks(planes, n_src, 4, kScatterGroup));
+    case SPH_STAGE_POOL: return reads < n_src ? 0 : stage_bytes(stage_chunks(planes, n_src, 4));
+    case SPH_STAGE_ARGMAX: return stage_bytes(stage_chunks(planes, n_src, 5));
+    default: return 0;
+  }
+}
+
 extern "C" int sph_resample_from_map(const void *x, const void *map, const void *iw, void *y, int64_t B, int64_t C,
                                      int64_t H, int64_t W, int64_t MH, int64_t MW, int64_t P, int dtype, int interp,
                                      void *stream) {
+  return sph_resample_from_map_ws(x, map, iw, y, B, C, H, W, MH, MW, P, dtype, interp, nullptr, 0, stream);
+}
+
+extern "C" int sph_resample_from_map_ws(const void *x, const void *map, const void *iw, void *y, int64_t B, int64_t C,
+                                        int64_t H, int64_t W, int64_t MH, int64_t MW, int64_t P, int dtype, int interp,
+                                        void *ws, size_t ws_bytes, void *stream) {
   SPH_RANGE("sph_resample_from_map");
   if (!x || !map || !y || B < 0 || C < 0 || H <= 0 || W <= 0 || MH < 0 || MW < 0 || P < 0 || (P > 0 && !iw))
     return SPH_ERR_INVALID_ARGUMENT;
@@ -210,48 +352,60 @@ extern "C" int sph_resample_from_map(const void *x, const void *map, const void 
   if (H * W >= lim || n * (P > 0 ? P : 1) * 2 >= lim || planes / 2 >= 65535) return SPH_ERR_TOO_LARGE;
   if (n == 0 || planes == 0) return SPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  if (dtype == SPH_F32 && planes >= 3 && scratch_ok(ws)) {
+    PlaneChunks c = stage_chunks(planes, H * W, 4);
+    if (ws_bytes >= stage_bytes(c) && stage_fits(c)) {
+      c.buf = (char *)ws;
+      SPH_DISPATCH_GROUP(c.group_planes, return from_map_groups<PG>(c, x, map, iw, y, H, W, MH, MW, P, interp, st));
+    }
+  }
   return dtype == SPH_F32 ? from_map<float>(x, map, iw, y, planes, H, W, n, P, interp, st)
                           : from_map<double>(x, map, iw, y, planes, H, W, n, P, interp, st);
+}
+
+namespace {
+int resample_to_map(const void *x, const void *plan, void *out, int64_t B, int64_t C, int64_t MH, int64_t MW, int64_t OH, int64_t OW,
+                    int64_t K, bool normalize, int dtype, void *ws, size_t ws_bytes, void *stream) {
+  if (!x || !plan || !out || B < 0 || C < 0 || MH <= 0 || MW <= 0 || OH <= 0 || OW <= 0 || K <= 0) return SPH_ERR_INVALID_ARGUMENT;
+  if (dtype != SPH_F32 && dtype != SPH_F64) return SPH_ERR_UNSUPPORTED;
+  const int64_t planes = B * C, lim = (int64_t)1 << 31;
+  if (OH * OW >= lim || MH * MW * K >= lim || planes / 2 >= 65535) return SPH_ERR_TOO_LARGE;
+  if (planes == 0) return SPH_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (dtype == SPH_F32 && planes >= 3 && K == 1 && scratch_ok(ws)) {
+    PlaneChunks c = stage_chunks(planes, MH * MW, 4, kScatterGroup);
+    if (ws_bytes >= stage_bytes(c) && stage_fits(c)) {
+      c.buf = (char *)ws;
+      SPH_DISPATCH_GROUP(c.group_planes, return to_map_groups<PG>(c, x, plan, out, MH * MW, OH * OW, normalize, st));
+    }
+  }
+  return dtype == SPH_F32 ? to_map<float>(x, plan, out, planes, MH * MW, OH * OW, st, (int)K, normalize)
+                          : to_map<double>(x, plan, out, planes, MH * MW, OH * OW, st, (int)K, normalize);
+}
+}  // namespace
+
+extern "C" int sph_resample_to_map_ws(const void *x, const void *plan, void *out, int64_t B, int64_t C, int64_t MH, int64_t MW,
+                                      int64_t OH, int64_t OW, int normalize, int dtype, void *ws, size_t ws_bytes, void *stream) {
+  SPH_RANGE("sph_resample_to_map");
+  return resample_to_map(x, plan, out, B, C, MH, MW, OH, OW, 1, normalize != 0, dtype, ws, ws_bytes, stream);
 }
 
 extern "C" int sph_resample_to_map(const void *x, const void *plan, void *out, int64_t B, int64_t C, int64_t MH,
                                    int64_t MW, int64_t OH, int64_t OW, int dtype, void *stream) {
   SPH_RANGE("sph_resample_to_map");
-  if (!x || !plan || !out || B < 0 || C < 0 || MH <= 0 || MW <= 0 || OH <= 0 || OW <= 0) return SPH_ERR_INVALID_ARGUMENT;
-  if (dtype != SPH_F32 && dtype != SPH_F64) return SPH_ERR_UNSUPPORTED;
-  const int64_t planes = B * C, lim = (int64_t)1 << 31;
-  if (OH * OW >= lim || MH * MW >= lim || planes / 2 >= 65535) return SPH_ERR_TOO_LARGE;
-  if (planes == 0) return SPH_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  return dtype == SPH_F32 ? to_map<float>(x, plan, out, planes, MH * MW, OH * OW, st)
-                          : to_map<double>(x, plan, out, planes, MH * MW, OH * OW, st);
+  return resample_to_map(x, plan, out, B, C, MH, MW, OH, OW, 1, false, dtype, nullptr, 0, stream);
 }
 
 extern "C" int sph_resample_to_map_normalized(const void *x, const void *plan, void *out, int64_t B, int64_t C, int64_t MH,
                                               int64_t MW, int64_t OH, int64_t OW, int dtype, void *stream) {
   SPH_RANGE("sph_resample_to_map_normalized");
-  if (!x || !plan || !out || B < 0 || C < 0 || MH <= 0 || MW <= 0 || OH <= 0 || OW <= 0) return SPH_ERR_INVALID_ARGUMENT;
-  if (dtype != SPH_F32 && dtype != SPH_F64) return SPH_ERR_UNSUPPORTED;
-  const int64_t planes = B * C, lim = (int64_t)1 << 31;
-  if (OH * OW >= lim || MH * MW >= lim || planes / 2 >= 65535) return SPH_ERR_TOO_LARGE;
-  if (planes == 0) return SPH_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  return dtype == SPH_F32 ? to_map<float>(x, plan, out, planes, MH * MW, OH * OW, st, 1, true)
-                          : to_map<double>(x, plan, out, planes, MH * MW, OH * OW, st, 1, true);
+  return resample_to_map(x, plan, out, B, C, MH, MW, OH, OW, 1, true, dtype, nullptr, 0, stream);
 }
 
 extern "C" int sph_mapped_avg_unpool(const void *g, const void *plan, void *grad_in, int64_t B, int64_t C, int64_t IH,
                                      int64_t IW, int64_t OH, int64_t OW, int64_t K, int dtype, void *stream) {
   SPH_RANGE("sph_mapped_avg_unpool");
-  if (!g || !plan || !grad_in || B < 0 || C < 0 || IH <= 0 || IW <= 0 || OH <= 0 || OW <= 0 || K <= 0)
-    return SPH_ERR_INVALID_ARGUMENT;
-  if (dtype != SPH_F32 && dtype != SPH_F64) return SPH_ERR_UNSUPPORTED;
-  const int64_t planes = B * C, lim = (int64_t)1 << 31;
-  if (OH * OW * K >= lim || IH * IW >= lim || planes / 2 >= 65535) return SPH_ERR_TOO_LARGE;
-  if (planes == 0) return SPH_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  return dtype == SPH_F32 ? to_map<float>(g, plan, grad_in, planes, OH * OW, IH * IW, st, (int)K)
-                          : to_map<double>(g, plan, grad_in, planes, OH * OW, IH * IW, st, (int)K);
+  return resample_to_map(g, plan, grad_in, B, C, OH, OW, IH, IW, K, false, dtype, nullptr, 0, stream);
 }
 
 extern "C" int sph_resample_from_uv_maps(const void *tex, const int64_t *quad_idx, const void *tex_uv, void *out, int64_t B,

@@ -11,6 +11,7 @@
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <list>
 #include <memory>
@@ -258,6 +259,18 @@ torch::Tensor workspace(size_t bytes, const torch::Tensor &like) {
   return torch::empty({(int64_t)(bytes ? bytes : 1)}, like.options().dtype(torch::kUInt8));
 }
 
+// Scratch of the plane-group kernels of resampling and pooling; undefined where they would not pay.
+struct Staging {
+  torch::Tensor buf;
+  size_t bytes = 0;
+  Staging(int op, int64_t planes, int64_t n_src, int64_t reads, const torch::Tensor &like) {
+    bytes = sph_staging_bytes(op, planes, n_src, reads, dtype_of(like));
+    if (bytes) buf = workspace(bytes, like);
+  }
+  void *ptr() const { return bytes ? buf.data_ptr() : nullptr; }
+};
+int64_t taps_of(InterpolationType it) { return it == InterpolationType::NEAREST ? 1 : 4; }
+
 cudaStream_t stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 // ---- resample (include/layers/resample_layer.h:40-82, weighted_resample_layer.h:49-105) ----
@@ -269,8 +282,9 @@ torch::Tensor resample_from_map_impl(torch::Tensor x, torch::Tensor map, const t
   const MapInfo m = map_info(map, iw, false, 1);
   c10::cuda::CUDAGuard guard(x.device());
   torch::Tensor y = torch::empty({x.size(0), x.size(1), m.H, m.W}, x.options());
-  ok(sph_resample_from_map(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, y.data_ptr(), x.size(0), x.size(1),
-                           x.size(2), x.size(3), m.H, m.W, m.P, dtype_of(x), (int)it, stream()),
+  const Staging sg(SPH_STAGE_GATHER, x.size(0) * x.size(1), x.size(2) * x.size(3), m.H * m.W * std::max<int64_t>(m.P, 1) * taps_of(it), x);
+  ok(sph_resample_from_map_ws(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, y.data_ptr(), x.size(0), x.size(1),
+                              x.size(2), x.size(3), m.H, m.W, m.P, dtype_of(x), (int)it, sg.ptr(), sg.bytes, stream()),
      "sph_resample_from_map");
   return y;
 }
@@ -287,8 +301,9 @@ torch::Tensor resample_to_map_impl(torch::Tensor x, torch::Tensor map, const tor
   c10::cuda::CUDAGuard guard(x.device());
   torch::Tensor plan = get_plan(map, iw, m.H * m.W, 1, m.P, (int)it, oh, ow);
   torch::Tensor out = torch::empty({x.size(0), x.size(1), oh, ow}, x.options());
-  ok(sph_resample_to_map(x.data_ptr(), plan.data_ptr(), out.data_ptr(), x.size(0), x.size(1), m.H, m.W, oh, ow, dtype_of(x),
-                         stream()),
+  const Staging sg(SPH_STAGE_SCATTER, x.size(0) * x.size(1), m.H * m.W, 0, x);
+  ok(sph_resample_to_map_ws(x.data_ptr(), plan.data_ptr(), out.data_ptr(), x.size(0), x.size(1), m.H, m.W, oh, ow, 0, dtype_of(x),
+                            sg.ptr(), sg.bytes, stream()),
      "sph_resample_to_map");
   return out;
 }
@@ -320,8 +335,9 @@ torch::Tensor resample_to_map_normalized(torch::Tensor x, torch::Tensor map, c10
   c10::cuda::CUDAGuard guard(x.device());
   torch::Tensor plan = get_plan(map, iw ? &*iw : nullptr, m.H * m.W, 1, m.P, (int)it, oh, ow);
   torch::Tensor out = torch::empty({x.size(0), x.size(1), oh, ow}, x.options());
-  ok(sph_resample_to_map_normalized(x.data_ptr(), plan.data_ptr(), out.data_ptr(), x.size(0), x.size(1), m.H, m.W, oh, ow,
-                                    dtype_of(x), stream()),
+  const Staging sg(SPH_STAGE_SCATTER, x.size(0) * x.size(1), m.H * m.W, 0, x);
+  ok(sph_resample_to_map_ws(x.data_ptr(), plan.data_ptr(), out.data_ptr(), x.size(0), x.size(1), m.H, m.W, oh, ow, 1, dtype_of(x),
+                            sg.ptr(), sg.bytes, stream()),
      "sph_resample_to_map_normalized");
   return out;
 }
@@ -359,8 +375,9 @@ torch::Tensor resample_to_uv_maps(torch::Tensor x, torch::Tensor quad, torch::Te
   c10::cuda::CUDAGuard guard(x.device());
   torch::Tensor plan = get_plan(uv, &quad, quad.size(0) * quad.size(1), 1, 0, (int)it, nt * th, tw, nt);
   torch::Tensor out = torch::empty({x.size(0), x.size(1), nt, th, tw}, x.options());
-  ok(sph_resample_to_map(x.data_ptr(), plan.data_ptr(), out.data_ptr(), x.size(0), x.size(1), x.size(2), x.size(3), nt * th, tw,
-                         dtype_of(x), stream()),
+  const Staging sg(SPH_STAGE_SCATTER, x.size(0) * x.size(1), x.size(2) * x.size(3), 0, x);
+  ok(sph_resample_to_map_ws(x.data_ptr(), plan.data_ptr(), out.data_ptr(), x.size(0), x.size(1), x.size(2), x.size(3), nt * th, tw, 0,
+                            dtype_of(x), sg.ptr(), sg.bytes, stream()),
      "sph_resample_to_map (uv)");
   return out;
 }
@@ -441,9 +458,11 @@ std::vector<torch::Tensor> max_pool_impl(torch::Tensor x, torch::Tensor map, con
   c10::cuda::CUDAGuard guard(x.device());
   torch::Tensor out = torch::empty({x.size(0), x.size(1), m.H, m.W}, x.options());
   torch::Tensor idx = torch::empty({x.size(0), x.size(1), m.H, m.W}, x.options().dtype(torch::kLong));
-  ok(sph_mapped_max_pool(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, out.data_ptr(),
-                         idx.data_ptr<int64_t>(), x.size(0), x.size(1), x.size(2), x.size(3), m.H, m.W, m.K, m.P,
-                         dtype_of(x), (int)it, stream()),
+  const Staging sg(SPH_STAGE_POOL, x.size(0) * x.size(1), x.size(2) * x.size(3),
+                   m.H * m.W * m.K * std::max<int64_t>(m.P, 1) * taps_of(it), x);
+  ok(sph_mapped_pool_ws(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, out.data_ptr(), idx.data_ptr<int64_t>(),
+                        x.size(0), x.size(1), x.size(2), x.size(3), m.H, m.W, m.K, m.P, 0, dtype_of(x), (int)it, sg.ptr(), sg.bytes,
+                        stream()),
      "sph_mapped_max_pool");
   return {out, idx};
 }
@@ -465,8 +484,9 @@ torch::Tensor max_unpool_impl(torch::Tensor g, torch::Tensor idx, torch::Tensor 
   if (g_deterministic_unpool) {
     // plan over the flattened map slots: every input pixel sums the winners that touch it in a fixed order
     torch::Tensor plan = get_plan(map, iw, m.H * m.W * m.K, 1, m.P, (int)it, ih, iwidth);
-    ok(sph_mapped_max_unpool_planned(g.data_ptr(), idx.data_ptr<int64_t>(), plan.data_ptr(), gin.data_ptr(), g.size(0),
-                                     g.size(1), ih, iwidth, m.H, m.W, m.K, m.P, dtype_of(g), stream()),
+    const Staging sg(SPH_STAGE_ARGMAX, g.size(0) * g.size(1), m.H * m.W, 0, g);
+    ok(sph_mapped_max_unpool_ws(g.data_ptr(), idx.data_ptr<int64_t>(), plan.data_ptr(), gin.data_ptr(), g.size(0), g.size(1), ih,
+                                iwidth, m.H, m.W, m.K, m.P, dtype_of(g), sg.ptr(), sg.bytes, stream()),
        "sph_mapped_max_unpool_planned");
     return gin;
   }
@@ -486,8 +506,10 @@ torch::Tensor avg_pool_impl(torch::Tensor x, torch::Tensor map, const torch::Ten
   const MapInfo m = map_info(map, iw, true, K);
   c10::cuda::CUDAGuard guard(x.device());
   torch::Tensor out = torch::empty({x.size(0), x.size(1), m.H, m.W}, x.options());
-  ok(sph_mapped_avg_pool(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, out.data_ptr(), x.size(0), x.size(1),
-                         x.size(2), x.size(3), m.H, m.W, m.K, m.P, dtype_of(x), (int)it, stream()),
+  const Staging sg(SPH_STAGE_POOL, x.size(0) * x.size(1), x.size(2) * x.size(3),
+                   m.H * m.W * m.K * std::max<int64_t>(m.P, 1) * taps_of(it), x);
+  ok(sph_mapped_pool_ws(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, out.data_ptr(), nullptr, x.size(0), x.size(1),
+                        x.size(2), x.size(3), m.H, m.W, m.K, m.P, 1, dtype_of(x), (int)it, sg.ptr(), sg.bytes, stream()),
      "sph_mapped_avg_pool");
   return out;
 }

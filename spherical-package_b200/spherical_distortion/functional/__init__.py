@@ -101,12 +101,15 @@ class _MappedMaxPool(torch.autograd.Function):
         else:
             pooled, idx_mask = _wpool.weighted_mapped_max_pool(x, sample_map, interp_weights, kernel_size, interp)
         ctx.mark_non_differentiable(idx_mask)
+        ctx.set_materialize_grads(False)  # no zero tensor of the indices' size in every backward pass
         ctx.save_for_backward(torch.tensor([x.shape[2], x.shape[3]]), idx_mask, sample_map,
                               *_scalars(kernel_size, interp), interp_weights)
         return pooled, idx_mask
 
     @staticmethod
     def backward(ctx, grad_output, _idx_grad=None):
+        if grad_output is None:
+            return None, None, None, None, None
         in_shape, idx_mask, sample_map, kernel_size, interp, interp_weights = ctx.saved_tensors
         interp = InterpolationType(interp)
         if interp_weights is None:
