@@ -321,6 +321,12 @@ enum sph_conv_op {
 size_t sph_conv_workspace_bytes(int op, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW,
                                 int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp,
                                 int precision);
+/* Scratch with which the float32 operators of precision 0 run on the tensor cores (operands split into three bf16 parts
+ * each, float32-accurate: csrc/conv_x3.cu); with less, down to sph_conv_workspace_bytes(), they run on the CUDA cores.
+ * For everything else the two are equal. */
+size_t sph_conv_workspace_preferred_bytes(int op, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW,
+                                          int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp,
+                                          int precision);
 int sph_mapped_conv_forward(const void *x, const void *map, const void *iw, const void *weight,
                             const void *bias, void *out, int64_t B, int64_t Cin, int64_t Cout, int64_t IH,
                             int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp,

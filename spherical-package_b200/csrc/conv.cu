@@ -98,6 +98,38 @@ extern "C" size_t sph_conv_workspace_bytes(int op, int64_t B, int64_t Cin, int64
   return thin > base ? thin : base;
 }
 
+// The exact precision's float32 operators run on the tensor cores through three-way split operands (conv_x3.cu) when the
+// caller brings the scratch for it, which sph_conv_workspace_preferred_bytes reports; with the smaller scratch of
+// sph_conv_workspace_bytes, in float64 and for the shapes x3 does not cover they run on the SIMT kernels.
+namespace {
+bool split_fits(int dtype, const void *ws, size_t ws_bytes, size_t need) {
+  return dtype == SPH_F32 && need > 0 && ws != nullptr && ws_bytes >= need && ((uintptr_t)ws & 255) == 0;
+}
+}  // namespace
+
+extern "C" size_t sph_conv_workspace_preferred_bytes(int op, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH,
+                                                     int64_t OW, int64_t K, int64_t P, int dtype, int interp, int precision) {
+  const size_t base = sph_conv_workspace_bytes(op, B, Cin, Cout, IH, IW, OH, OW, K, P, dtype, interp, precision);
+  const Dims d{B, Cin, Cout, IH, IW, OH, OW, K, P};
+  if (check_dims(d, dtype, interp, precision) != SPH_OK || precision != SPH_PRECISION_EXACT || dtype != SPH_F32 || B == 0) return base;
+  const bool transposed = op == SPH_TCONV_FORWARD || op == SPH_TCONV_BACKWARD_INPUT || op == SPH_TCONV_BACKWARD_WEIGHT;
+  if (transposed ? small_ok(Cout, K, Cin, 4) : small_ok(Cin, K, Cout, 4)) return base;
+  size_t x3 = 0;
+  switch (op) {
+    case SPH_CONV_FORWARD: x3 = x3_gemm_workspace(false, B, Cin, IH * IW, K, P, interp, Cout, 0); break;
+    case SPH_CONV_BACKWARD_INPUT: x3 = x3_gemm_workspace(true, B, Cout, OH * OW, K, 0, 0, Cin, IH * IW); break;
+    case SPH_CONV_BACKWARD_WEIGHT: x3 = x3_dw_workspace(B, Cin, IH * IW, K, P, interp, Cout, OH, OW); break;
+    case SPH_TCONV_FORWARD: x3 = x3_gemm_workspace(true, B, Cin, IH * IW, K, 0, 0, Cout, OH * OW); break;
+    case SPH_TCONV_BACKWARD_INPUT: x3 = x3_gemm_workspace(false, B, Cout, OH * OW, K, P, interp, Cin, 0); break;
+    case SPH_TCONV_BACKWARD_WEIGHT:
+      x3 = x3_dw_workspace(B, Cout, OH * OW, K, P, interp, Cin, IH, IW);
+      if (x3 > 0) x3 += simt_bias_workspace(Cout, 4);
+      break;
+    default: break;
+  }
+  return x3 > base ? x3 : base;
+}
+
 #define SPH_BY_DTYPE(fn, ...) (dtype == SPH_F32 ? fn<float>(__VA_ARGS__) : fn<double>(__VA_ARGS__))
 
 namespace {
@@ -123,6 +155,8 @@ int conv_forward(const void *x, const void *map, const void *iw, const void *wei
   if (precision == SPH_PRECISION_BF16)
     return tc_conv_forward(x, map, iw, weight, bias, out, B, Cin, Cout, IH, IW, OH, OW, K, P, interp, ws, ws_bytes, st, fz);
   if (fz.active() || fz.out_cl != nullptr) return SPH_ERR_UNSUPPORTED;
+  if (split_fits(dtype, ws, ws_bytes, x3_gemm_workspace(false, B, Cin, IH * IW, K, P, interp, Cout, 0)))
+    return x3_gemm(false, x, map, iw, nullptr, Cin, IH, IW, K, P, OH, OW, interp, weight, Cin * K, K, 1, bias, out, Cout, B, ws, st);
   return SPH_BY_DTYPE(simt_gemm, false, x, map, iw, nullptr, Cin, IH, IW, K, P, OH * OW, interp, weight, Cin * K, K, 1,
                       bias, out, Cout, B, st, ws, ws_bytes);
 }
@@ -150,6 +184,8 @@ int conv_backward_input(const void *gout, const void *plan, const void *weight, 
   if (precision == SPH_PRECISION_BF16)
     return tc_conv_backward_input(gout, plan, weight, gx, B, Cin, Cout, IH, IW, OH, OW, K, ws, ws_bytes, st, fz);
   if (fz.active()) return SPH_ERR_UNSUPPORTED;
+  if (split_fits(dtype, ws, ws_bytes, x3_gemm_workspace(true, B, Cout, OH * OW, K, 0, 0, Cin, IH * IW)))
+    return x3_gemm(true, gout, nullptr, nullptr, plan, Cout, OH, OW, K, 0, IH, IW, 0, weight, K, Cin * K, 1, nullptr, gx, Cin, B, ws, st);
   return SPH_BY_DTYPE(simt_gemm, true, gout, nullptr, nullptr, plan, Cout, OH, OW, K, 0, IH * IW, 0, weight, K, Cin * K, 1,
                       nullptr, gx, Cin, B, st, ws, ws_bytes);
 }
@@ -179,6 +215,8 @@ int conv_backward_weight(const void *gout, const void *x, const void *map, const
   if (precision == SPH_PRECISION_BF16)
     return tc_conv_backward_weight(gout, x, map, iw, gw, gb, B, Cin, Cout, IH, IW, OH, OW, K, P, interp, ws, ws_bytes, st, fz);
   if (fz.active()) return SPH_ERR_UNSUPPORTED;
+  if (split_fits(dtype, ws, ws_bytes, x3_dw_workspace(B, Cin, IH * IW, K, P, interp, Cout, OH, OW)))
+    return x3_dw(gout, x, map, iw, Cin, IH, IW, K, P, OH, OW, interp, Cout, B, gw, Cin * K, K, 1, gb, ws, st);
   return SPH_BY_DTYPE(simt_dw, gout, x, map, iw, Cin, IH, IW, K, P, OH * OW, interp, Cout, B, gw, Cin * K, K, 1, gout, Cout,
                       OH * OW, gb, ws, ws_bytes, st);
 }
@@ -316,6 +354,8 @@ extern "C" int sph_mapped_tconv_forward(const void *x, const void *plan, const v
                         st);
   if (precision == SPH_PRECISION_BF16)
     return tc_tconv_forward(x, plan, weight, bias, out, B, Cin, Cout, IH, IW, OH, OW, K, ws, ws_bytes, st);
+  if (split_fits(dtype, ws, ws_bytes, x3_gemm_workspace(true, B, Cin, IH * IW, K, 0, 0, Cout, OH * OW)))
+    return x3_gemm(true, x, nullptr, nullptr, plan, Cin, IH, IW, K, 0, OH, OW, 0, weight, K, Cout * K, 1, bias, out, Cout, B, ws, st);
   return SPH_BY_DTYPE(simt_gemm, true, x, nullptr, nullptr, plan, Cin, IH, IW, K, 0, OH * OW, 0, weight, K, Cout * K, 1,
                       bias, out, Cout, B, st, ws, ws_bytes);
 }
@@ -336,6 +376,8 @@ extern "C" int sph_mapped_tconv_backward_input(const void *gout, const void *map
                         st);
   if (precision == SPH_PRECISION_BF16)
     return tc_tconv_backward_input(gout, map, iw, weight, gx, B, Cin, Cout, IH, IW, OH, OW, K, P, interp, ws, ws_bytes, st);
+  if (split_fits(dtype, ws, ws_bytes, x3_gemm_workspace(false, B, Cout, OH * OW, K, P, interp, Cin, 0)))
+    return x3_gemm(false, gout, map, iw, nullptr, Cout, OH, OW, K, P, IH, IW, interp, weight, Cout * K, K, 1, nullptr, gx, Cin, B, ws, st);
   return SPH_BY_DTYPE(simt_gemm, false, gout, map, iw, nullptr, Cout, OH, OW, K, P, IH * IW, interp, weight, Cout * K, K, 1,
                       nullptr, gx, Cin, B, st, ws, ws_bytes);
 }
@@ -360,6 +402,11 @@ extern "C" int sph_mapped_tconv_backward_weight(const void *gout, const void *x,
                         OH * OW, gb, ws, ws_bytes, st);
   if (precision == SPH_PRECISION_BF16)
     return tc_tconv_backward_weight(gout, x, map, iw, gw, gb, B, Cin, Cout, IH, IW, OH, OW, K, P, interp, ws, ws_bytes, st);
+  const size_t wx = x3_dw_workspace(B, Cout, OH * OW, K, P, interp, Cin, IH, IW), wb = simt_bias_workspace(Cout, 4);
+  if (wx > 0 && split_fits(dtype, ws, ws_bytes, wx + wb)) {  // (the bias gradient sums grad_output, the gathered side)
+    const int rx = x3_dw(x, gout, map, iw, Cout, OH, OW, K, P, IH, IW, interp, Cin, B, gw, Cout * K, K, 1, nullptr, ws, st);
+    return rx == SPH_OK ? simt_bias_grad<float>(gout, B, Cout, OH * OW, gb, (char *)ws + wx, st) : rx;
+  }
   return SPH_BY_DTYPE(simt_dw, x, gout, map, iw, Cout, OH, OW, K, P, IH * IW, interp, Cin, B, gw, Cout * K, K, 1, gout, Cout,
                       OH * OW, gb, ws, ws_bytes, st);
 }

@@ -2064,6 +2064,7 @@ int sph_tu_status_plan(int);
 int sph_tu_status_pool(int);
 int sph_tu_status_conv_simt(int);
 int sph_tu_status_conv_small(int);
+int sph_tu_status_conv_x3(int);
 }
 #endif
 
@@ -2075,11 +2076,13 @@ extern "C" int sph_device_status(int *status, int reset) {
     const int zero = 0;
     if (cudaMemcpyToSymbol(sph::g_wait_status, &zero, sizeof(int)) != cudaSuccess) return SPH_ERR_CUDA;
   }
-  v = v ? 1 : 0;
+  const int v3 = sph::x3_wait_status(reset);
+  if (v3 < 0) return SPH_ERR_CUDA;
+  v = v || v3 ? 1 : 0;
 #ifdef SPH_BOUNDS_CHECK
   // checked build: bit 1 = some kernel met an index outside its range (and skipped the access)
   int (*const parts[])(int) = {sph_tu_status_resample, sph_tu_status_plan, sph_tu_status_pool, sph_tu_status_conv_simt,
-                               sph_tu_status_conv_small, sph_tu_status_conv_tc};
+                               sph_tu_status_conv_small, sph_tu_status_conv_tc, sph_tu_status_conv_x3};
   for (auto f : parts) {
     const int r = f(reset);
     if (r < 0) return SPH_ERR_CUDA;

@@ -1,0 +1,981 @@
+// float32 mapped convolutions on the tensor cores, without giving up float32.
+//
+// A float32 operand is the exact sum of three bf16 parts, x = h + m + l (8 + 8 + 8 significand bits, by truncation), so a
+// float32 product is nine bf16 products, of which l*l, m*l and l*m lie below 2^-23 of it.  The other six run on tcgen05
+// with float32 accumulation in tensor memory.  What remains to be guarded is the accumulation: the tensor core cuts
+// every addition off toward zero (measured on B200: 144 additions of one sign lose 6.6e-6 of the sum, where a chain of
+// float32 multiply-adds is off by 7e-7).  So
+//   - the large products h*h go to an accumulator of their own, which takes at most kSeg chunks (64 columns, four additions)
+//     before warps of the epilogue add it, round to nearest, to float32 registers; two such accumulators alternate;
+//   - the five small ones share a second accumulator for the whole tile: its losses are 2^-8 of the large one's.
+// The result is at least as close to the exact sum as the SIMT kernels' (conv_simt.cu; tests/test_conv_x3_gpu.py compares
+// both with float64).  An infinite operand gives NaN where float32 arithmetic could have kept an infinity.
+//
+// The two kernels mirror conv_tc.cu (tiles of 128 pixels, producer warps that gather, weights or gradient tile images by
+// bulk copies, one MMA thread, epilogue warps), but gather float32 values from a channels-last float32 copy of the source
+// and interpolate in float32 with the roundings of the SIMT kernels before the values are split:
+//   x3_gemm_kernel   Out[b, n, pix] = sum_j Col[b, pix, j] * Wt[n, j]  (+ bias[n])     through a map, a plan, or the identity
+//   x3_dw_kernel     dW[n, j] = sum_{b, pix} G[b, n, pix] * Col[b, pix, j]
+//
+// Why the tiles are what they are: per chunk of 128 pixels x 32 columns the six products take 768 tensor cycles (N = 128) and
+// the SM's 128-byte data path carries 512 wavefronts of gathered taps, 192 + 192 of operand stores and 768 of operand
+// reads; 32-column chunks (64-byte swizzled rows, 48 KB a stage for both operands in three parts) leave the L1 room for
+// the tile's neighbourhood, which 64-column chunks (96 KB a stage) do not.
+#include <string.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "conv_internal.h"
+#include "tc_common.cuh"
+
+namespace sph {
+namespace {
+
+using namespace tc;
+
+constexpr int kCols = 32;                               // GEMM columns per chunk
+constexpr int kPix = 128, kTileW = 16, kTileH = 8;      // pixels of a tile: 8 rows of 16
+constexpr int kEpi = 8, kProd = 8;                      // epilogue and producer warps
+constexpr int kThreads3 = 32 * (kEpi + 1 + kProd);
+constexpr int kProd0 = 32 * (kEpi + 1);                 // first producer thread
+constexpr int kSeg = 2;                                 // chunks per large-product segment
+constexpr int kPartA = kPix * 64;                       // bytes of one part of a 128-row x 32-column operand tile
+constexpr int kNMax = 128;
+constexpr size_t kSmemMax = 227 * 1024;
+constexpr uint32_t kHh = 0, kCorr = 256;                // tensor memory columns: large products (2 x 128), small ones (2 x 128)
+
+enum { SRC_MAP1 = 0, SRC_MAP4 = 1, SRC_PLAN = 2, SRC_SELF = 3 };
+
+__device__ int g_wait_status3;
+
+int padded3(int64_t CH) {
+  if (CH <= 8) return 8;
+  if (CH <= 16) return 16;
+  return (int)align_up((size_t)CH, 32);
+}
+
+// Descriptor of a K-major operand tile stored as rows of 64 bytes (32 bf16) with the 64-byte swizzle (16-byte unit index XOR
+// (row >> 1) & 3): 8-row groups 512 bytes apart, layout code 4.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(512 >> 4) << 32) | (1ull << 46) | (4ull << 61);
+}
+
+struct Src3 {
+  const char *xl;            // (B, SH*SW + 1, Cp) channels-last float32; the last pixel of every image is zero
+  const float *map, *iw;
+  const void *plan;
+  int Cp, SH, SW, K, P, GH, GW, interp;
+};
+
+struct Ring3 {
+  int s = 0;
+  uint32_t ph = 0;
+  __device__ __forceinline__ void next(int stages) {
+    if (++s == stages) { s = 0; ph ^= 1u; }
+  }
+};
+
+// ---- taps of a tile in shared memory, for slots [s0, s0 + ns): offsets [slot][pixel] (4 or 1), weights [slot][pixel] (4), and in
+// plan mode the range of entries beyond the fourth
+template <int SRC> struct TapTable {
+  static constexpr int NT = SRC == SRC_MAP1 || SRC == SRC_SELF ? 1 : 4;
+  static size_t bytes(int ns) { return SRC == SRC_SELF ? 0 : (size_t)ns * kPix * (NT == 1 ? 4 : SRC == SRC_PLAN ? 40 : 32); }
+  uint32_t off, w, rest;  // shared-space addresses
+  __device__ __forceinline__ TapTable(uint32_t base, int ns) {
+    off = base;
+    w = off + ns * kPix * (NT * 4);
+    rest = w + ns * kPix * 16;
+  }
+};
+
+__device__ __forceinline__ int tile_pixel3(int l, int ty, int tx, int GH, int GW) {
+  const int y = ty * kTileH + (l >> 4), x = tx * kTileW + (l & 15);
+  return (y < GH && x < GW) ? y * GW + x : -1;
+}
+
+template <int SRC>
+__device__ __forceinline__ void fill_taps3(const Src3 &g, const TapTable<SRC> &t, const PlanView<float> &pv, bool plan_ok, int s0, int ns,
+                                           int ty, int tx, int pt) {
+  if (SRC == SRC_SELF) return;
+  const uint32_t pitch = (uint32_t)g.Cp * 4u, zero = (uint32_t)(g.SH * g.SW) * pitch;
+  for (int idx = pt; idx < ns * kPix; idx += 32 * kProd) {
+    const int slot = s0 + idx / kPix, pix = tile_pixel3(idx % kPix, ty, tx, g.GH, g.GW);
+    const bool in = pix >= 0 && slot < g.K;
+    if constexpr (SRC == SRC_MAP1) {
+      uint32_t o = zero;
+      if (in) {
+        const float *m = g.map + 2 * ((size_t)pix * g.K + slot);
+        Taps<float> q;
+        decode<float, SPH_NEAREST>(__ldg(m), __ldg(m + 1), g.SH, g.SW, q);
+        if (q.off[0] >= 0 && index_ok(q.off[0], q.limit)) o = (uint32_t)q.off[0] * pitch;
+      }
+      sts32(t.off + idx * 4, o);
+    } else {
+      uint32_t o[4] = {zero, zero, zero, zero};
+      float w[4] = {0.f, 0.f, 0.f, 0.f};
+      if constexpr (SRC == SRC_MAP4) {
+        if (in) {
+          const size_t e = ((size_t)pix * g.K + slot) * (g.P > 0 ? g.P : 1);
+          Taps<float> q;
+          if (g.P > 0) {  // weighted nearest, at most four points: the points take the taps' places
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+              if (i < g.P) {
+                decode<float, SPH_NEAREST>(__ldg(g.map + 2 * (e + i)), __ldg(g.map + 2 * (e + i) + 1), g.SH, g.SW, q);
+                if (q.off[0] >= 0 && index_ok(q.off[0], q.limit)) o[i] = (uint32_t)q.off[0] * pitch;
+                w[i] = __ldg(g.iw + e + i);
+              }
+          } else {
+            const float x = __ldg(g.map + 2 * e), y = __ldg(g.map + 2 * e + 1);
+            if (g.interp == SPH_BISPHERICAL) decode<float, SPH_BISPHERICAL>(x, y, g.SH, g.SW, q);
+            else decode<float, SPH_BILINEAR>(x, y, g.SH, g.SW, q);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              if (q.off[i] >= 0 && index_ok(q.off[i], q.limit)) o[i] = (uint32_t)q.off[i] * pitch;
+              w[i] = q.w[i];
+            }
+          }
+        }
+      } else {
+        int e0 = 0, e1 = 0;
+        if (plan_ok && in) {
+          e0 = __ldg(pv.offsets + (size_t)pix * g.K + slot);
+          e1 = __ldg(pv.offsets + (size_t)pix * g.K + slot + 1);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          if (e0 + i < e1) {
+            const int s = __ldg(pv.src + e0 + i);
+            if (index_ok(s, pv.n_src)) {
+              o[i] = (uint32_t)s * pitch;
+              w[i] = __ldg(pv.w + e0 + i);
+            }
+          }
+        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(t.rest + idx * 8), "r"(min(e0 + 4, e1)), "r"(e1) : "memory");
+      }
+      sts128(t.off + idx * 16, make_uint4(o[0], o[1], o[2], o[3]));
+      sts128(t.w + idx * 16, make_uint4(__float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), __float_as_uint(w[3])));
+    }
+  }
+}
+
+// Eight channels of one source pixel.
+struct V8 {
+  float f[8];
+};
+__device__ __forceinline__ V8 load8(const char *p) {
+  V8 v;
+  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(v.f[0]), "=f"(v.f[1]), "=f"(v.f[2]), "=f"(v.f[3]), "=f"(v.f[4]), "=f"(v.f[5]), "=f"(v.f[6]), "=f"(v.f[7])
+               : "l"(p));
+  return v;
+}
+
+// The loads of one (pixel, slot, 8 channels) item, issued ahead of their use.
+template <int SRC> struct Item {
+  static constexpr int NT = TapTable<SRC>::NT;
+  V8 q[NT];
+  float w[NT];
+};
+template <int SRC>
+__device__ __forceinline__ void item_load(Item<SRC> &it, const TapTable<SRC> &t, const char *img, int entry, uint32_t self_off) {
+  if constexpr (SRC == SRC_SELF) {
+    it.q[0] = load8(img + self_off);
+  } else if constexpr (SRC == SRC_MAP1) {
+    uint32_t o;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(o) : "r"(t.off + entry * 4));
+    it.q[0] = load8(img + o);
+  } else {
+    const uint4 o = lds128(t.off + entry * 16), w = lds128(t.w + entry * 16);
+    it.q[0] = load8(img + o.x);
+    it.q[1] = load8(img + o.y);
+    it.q[2] = load8(img + o.z);
+    it.q[3] = load8(img + o.w);
+    it.w[0] = __uint_as_float(w.x);
+    it.w[1] = __uint_as_float(w.y);
+    it.w[2] = __uint_as_float(w.z);
+    it.w[3] = __uint_as_float(w.w);
+  }
+}
+template <int SRC>
+__device__ __forceinline__ V8 item_value(const Item<SRC> &it, const TapTable<SRC> &t, const PlanView<float> &pv, const char *img, int entry,
+                                         uint32_t pitch) {
+  V8 v;
+  if constexpr (Item<SRC>::NT == 1) {
+    v = it.q[0];
+  } else if constexpr (SRC == SRC_MAP4) {
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      v.f[j] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(it.w[0], it.q[0].f[j]), __fmul_rn(it.w[1], it.q[1].f[j])),
+                                   __fmul_rn(it.w[2], it.q[2].f[j])), __fmul_rn(it.w[3], it.q[3].f[j]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      v.f[j] = it.w[0] * it.q[0].f[j];
+#pragma unroll
+      for (int i = 1; i < 4; i++) v.f[j] = fmaf(it.w[i], it.q[i].f[j], v.f[j]);
+    }
+    const uint2 r = lds64(t.rest + entry * 8);
+    for (int e = (int)r.x; e < (int)r.y; e++) {  // segments longer than the table
+      const int s = __ldg(pv.src + e);
+      if (!index_ok(s, pv.n_src)) continue;
+      const float w = __ldg(pv.w + e);
+      const V8 x = load8(img + (size_t)s * pitch);
+#pragma unroll
+      for (int j = 0; j < 8; j++) v.f[j] = fmaf(w, x.f[j], v.f[j]);
+    }
+  }
+  return v;
+}
+
+// x = h + m + l by truncation; the parts of eight values as three 16-byte vectors, stored `part` bytes apart.
+__device__ __forceinline__ void store_parts(uint32_t dst, uint32_t part, const V8 &v) {
+  uint32_t h[4], m[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float a = v.f[2 * i], b = v.f[2 * i + 1];
+    const float ra = a - __uint_as_float(__float_as_uint(a) & 0xffff0000u), rb = b - __uint_as_float(__float_as_uint(b) & 0xffff0000u);
+    const float la = ra - __uint_as_float(__float_as_uint(ra) & 0xffff0000u), lb = rb - __uint_as_float(__float_as_uint(rb) & 0xffff0000u);
+    h[i] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+    m[i] = __byte_perm(__float_as_uint(ra), __float_as_uint(rb), 0x7632);
+    l[i] = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
+  }
+  sts128(dst, make_uint4(h[0], h[1], h[2], h[3]));
+  sts128(dst + part, make_uint4(m[0], m[1], m[2], m[3]));
+  sts128(dst + 2 * part, make_uint4(l[0], l[1], l[2], l[3]));
+}
+
+__device__ __forceinline__ void producer_bar3() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kProd) : "memory"); }
+
+struct Bars {
+  uint64_t *full, *empty, *seg_full, *seg_empty, *corr_empty;
+  uint32_t *tmem_ptr;
+  volatile int *abort_flag;
+};
+inline size_t bars_bytes(int stages) { return 8 * (2 * stages + 6) + 16; }
+__device__ __forceinline__ Bars carve_bars(uint8_t *q, int stages) {
+  Bars b;
+  b.full = (uint64_t *)q;
+  b.empty = b.full + stages;
+  b.seg_full = b.empty + stages;
+  b.seg_empty = b.seg_full + 2;
+  b.corr_empty = b.seg_empty + 2;
+  b.tmem_ptr = (uint32_t *)(b.corr_empty + 2);
+  b.abort_flag = (volatile int *)(b.tmem_ptr + 1);
+  return b;
+}
+__device__ __forceinline__ uint32_t start_block(const Bars &b, int stages, int tid) {
+  if (tid == 0) {
+    for (int s = 0; s < stages; s++) {
+      mbar_init(b.full + s, kProd + 1);
+      mbar_init(b.empty + s, 1);
+    }
+    for (int i = 0; i < 2; i++) {
+      mbar_init(b.seg_full + i, 1);
+      mbar_init(b.seg_empty + i, kEpi);
+      mbar_init(b.corr_empty + i, kEpi);
+    }
+    *b.abort_flag = 0;
+    fence_barrier_init();
+  }
+  if ((tid >> 5) == kEpi) {
+    tmem_alloc(b.tmem_ptr, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  return *b.tmem_ptr;
+}
+
+// The twelve MMAs of one 32-deep step: h*h into `hh`, the five smaller products into `corr`.  Descriptors of part 0; `pa` / `pb` =
+// distance between parts, `ka` / `kb` = advance per 16 of depth, all in 16-byte units.
+__device__ __forceinline__ void issue_step(uint32_t hh, uint32_t corr, uint64_t a, uint64_t b, uint32_t pa, uint32_t pb, uint32_t ka,
+                                           uint32_t kb, uint32_t idesc, bool first_hh, bool first_corr) {
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const uint64_t a0 = a + k * ka, b0 = b + k * kb;
+    umma_bf16(hh, a0, b0, idesc, !(first_hh && k == 0));
+    umma_bf16(corr, a0, b0 + pb, idesc, !(first_corr && k == 0));  // h * m
+    umma_bf16(corr, a0 + pa, b0, idesc, 1);                        // m * h
+    umma_bf16(corr, a0 + pa, b0 + pb, idesc, 1);                   // m * m
+    umma_bf16(corr, a0, b0 + 2 * pb, idesc, 1);                    // h * l
+    umma_bf16(corr, a0 + 2 * pa, b0, idesc, 1);                    // l * h
+  }
+}
+
+// An epilogue warp's share of the accumulators: lanes 32 * (warp & 3) .., columns [col0, col0 + 16 * nb16) of at most 64.
+struct EpiSlice {
+  uint32_t lane_addr;
+  int col0, nb16;
+  __device__ __forceinline__ EpiSlice(uint32_t tmem_base, int warp, int ncols) {
+    const int per = (ncols + 31) / 32 * 16;  // columns of the first half
+    const int half = warp >> 2;
+    col0 = half * per;
+    nb16 = half == 0 ? per / 16 : (ncols - per + 15) / 16;
+    lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + col0;
+  }
+  __device__ __forceinline__ void add(float (&acc)[64], uint32_t col) const {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (i < nb16) {
+        uint32_t r[16];
+        tmem_ld_32x16(lane_addr + col + i * 16, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; j++) acc[i * 16 + j] = __fadd_rn(acc[i * 16 + j], __uint_as_float(r[j]));
+      }
+    }
+  }
+};
+
+// Sums of one tile: `nseg` segments, then the small products.  False if a wait gave up.
+__device__ __forceinline__ bool drain_tile(const Bars &b, const EpiSlice &e, float (&acc)[64], int nseg, int &sg, int tl, int lane) {
+#pragma unroll
+  for (int j = 0; j < 64; j++) acc[j] = 0.0f;
+  for (int s = 0; s < nseg; s++, sg++) {
+    const int buf = sg & 1;
+    if (!mbar_wait(b.seg_full + buf, (sg >> 1) & 1, b.abort_flag)) return false;
+    tc_fence_after();
+    e.add(acc, kHh + buf * 128);
+    if (s + 1 == nseg) e.add(acc, kCorr + (tl & 1) * 128);  // (its last product was committed with this segment)
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) {
+      mbar_arrive(b.seg_empty + buf);
+      if (s + 1 == nseg) mbar_arrive(b.corr_empty + (tl & 1));
+    }
+  }
+  return true;
+}
+
+struct Gemm3 {
+  Src3 g;
+  const __nv_bfloat16 *wp;  // weight tile images [nblk][chunk][part][Npb rows][32 columns], 64-byte swizzled
+  const float *bias;        // (Nout) or null
+  float *out;               // (B, Nout, GH*GW)
+  int *status;
+  int B, Nout, Npb, nblk, nchunks, tiles_x, tiles_y, stages;
+};
+
+__host__ __device__ inline int chunks3(int Cp, int K) { return Cp >= kCols ? Cp / kCols * K : (K * Cp + kCols - 1) / kCols; }
+// (slot, first channel) of vector v (8 columns) of a chunk: channel blocks outermost, so that consecutive chunks read the same
+// neighbourhood; slots packed into a chunk where a slot has fewer than 32 channels (slot >= K: padding)
+__host__ __device__ inline void chunk_item3(int Cp, int K, int chunk, int v, int &slot, int &c0) {
+  if (Cp >= kCols) {
+    const int cc = chunk / K;
+    slot = chunk - cc * K;
+    c0 = cc * kCols + v * 8;
+  } else {
+    const int q = chunk * kCols + v * 8;
+    slot = q / Cp;
+    c0 = q - slot * Cp;
+  }
+}
+
+template <int SRC> inline size_t gemm3_smem(int stages, int Npb, int K) {
+  return 1024 + (size_t)stages * (3 * kPartA + 3 * Npb * 64) + align_up(TapTable<SRC>::bytes(K), 16) + bars_bytes(stages);
+}
+
+template <int SRC>
+__global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, S = p.stages;
+  const Src3 &g = p.g;
+  const uint32_t bbytes = 3u * (uint32_t)p.Npb * 64u, stage_bytes = 3u * kPartA + bbytes;
+  const uint32_t stage0 = smem_u32(base);
+  const TapTable<SRC> taps(stage0 + S * stage_bytes, g.K);
+  const Bars bars = carve_bars(base + (size_t)S * stage_bytes + ((TapTable<SRC>::NT == 1 ? (SRC == SRC_SELF ? 0 : g.K * kPix * 4)
+                                                                                     : g.K * kPix * (SRC == SRC_PLAN ? 40 : 32)) + 15) / 16 * 16, S);
+  const uint32_t tmem = start_block(bars, S, tid);
+  const int tiles_per_image = p.tiles_x * p.tiles_y, total = p.B * tiles_per_image * p.nblk, npix = g.GH * g.GW;
+  const int nseg = (p.nchunks + kSeg - 1) / kSeg;
+
+  if (warp < kEpi) {
+    const EpiSlice e(tmem, warp, p.Npb);
+    int sg = 0, tl = 0;
+    for (int tile = blockIdx.x; tile < total; tile += gridDim.x, tl++) {
+      const int nb = tile % p.nblk, rest = tile / p.nblk, b = rest / tiles_per_image, t2 = rest % tiles_per_image;
+      const int pix = tile_pixel3((warp & 3) * 32 + lane, t2 / p.tiles_x, t2 % p.tiles_x, g.GH, g.GW);
+      float acc[64];
+      if (!drain_tile(bars, e, acc, nseg, sg, tl, lane)) break;
+      if (pix < 0) continue;
+      const int n0 = nb * p.Npb + e.col0;
+      float *o = p.out + ((size_t)b * p.Nout + n0) * npix + pix;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (i < e.nb16) {
+#pragma unroll
+          for (int j = 0; j < 16; j++, o += npix) {
+            const int n = n0 + i * 16 + j;
+            if (n < p.Nout && e.col0 + i * 16 + j < p.Npb) *o = acc[i * 16 + j] + (p.bias ? __ldg(p.bias + n) : 0.0f);
+          }
+        }
+      }
+    }
+  } else if (warp == kEpi) {
+    if (lane == 0) {
+      const uint32_t idesc = idesc_bf16(kPix, p.Npb, 0, 0);
+      int tl = 0, sg = 0;
+      Ring3 ring;
+      bool alive = true;
+      for (int tile = blockIdx.x; alive && tile < total; tile += gridDim.x, tl++) {
+        const int cb = tl & 1;
+        if (!mbar_wait(bars.corr_empty + cb, ((tl >> 1) & 1) ^ 1, bars.abort_flag)) break;
+        for (int chunk = 0; chunk < p.nchunks; chunk++, ring.next(S)) {
+          const bool first = chunk % kSeg == 0;
+          const int buf = sg & 1;
+          if (first && !mbar_wait(bars.seg_empty + buf, ((sg >> 1) & 1) ^ 1, bars.abort_flag)) { alive = false; break; }
+          if (!mbar_wait(bars.full + ring.s, ring.ph, bars.abort_flag)) { alive = false; break; }
+          tc_fence_after();
+          const uint32_t a = stage0 + ring.s * stage_bytes, bw = a + 3 * kPartA;
+          issue_step(tmem + kHh + buf * 128, tmem + kCorr + cb * 128, smem_desc_sw64(a), smem_desc_sw64(bw), kPartA >> 4,
+                     (uint32_t)p.Npb * 4u, 2, 2, idesc, first, chunk == 0);
+          umma_commit(bars.empty + ring.s);
+          if (chunk % kSeg == kSeg - 1 || chunk + 1 == p.nchunks) {
+            umma_commit(bars.seg_full + buf);
+            sg++;
+          }
+        }
+      }
+    }
+  } else {
+    // producers: thread = vector v (8 columns) of pixels px and px + 64
+    const int pt = tid - kProd0, v = pt & 3, px = pt >> 2;
+    const uint32_t pitch = (uint32_t)g.Cp * 4u;
+    const size_t image = (size_t)(g.SH * g.SW + 1) * pitch;
+    uint32_t dst[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) dst[i] = stage0 + (px + 64 * i) * 64 + ((v ^ (((px + 64 * i) >> 1) & 3)) << 4);
+    PlanView<float> pv{};
+    bool plan_ok = true;
+    if (SRC == SRC_PLAN) pv = plan_view<float>(g.plan, npix * g.K, plan_ok);
+    Ring3 ring;
+    bool alive = true;
+    for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
+      const int nb = tile % p.nblk, rest = tile / p.nblk, b = rest / tiles_per_image, t2 = rest % tiles_per_image;
+      const int ty = t2 / p.tiles_x, tx = t2 % p.tiles_x;
+      const char *img = g.xl + (size_t)b * image;
+      producer_bar3();  // the previous tile's taps have been read
+      fill_taps3<SRC>(g, taps, pv, plan_ok, 0, g.K, ty, tx, pt);
+      producer_bar3();
+      if (!alive) continue;
+      uint32_t self[2] = {0u, 0u};
+      if (SRC == SRC_SELF) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const int q = tile_pixel3(px + 64 * i, ty, tx, g.GH, g.GW);
+          self[i] = (uint32_t)(q >= 0 ? q : g.SH * g.SW) * pitch;
+        }
+      }
+      Item<SRC> it[2];
+      int slot, c0;
+      chunk_item3(g.Cp, g.K, 0, v, slot, c0);
+      const auto load = [&]() {
+        if (slot < g.K) {
+#pragma unroll
+          for (int i = 0; i < 2; i++) item_load<SRC>(it[i], taps, img + c0 * 4, slot * kPix + px + 64 * i, self[i]);
+        }
+      };
+      load();
+      for (int chunk = 0; chunk < p.nchunks; chunk++, ring.next(S)) {
+        V8 val[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          if (slot < g.K) {
+            val[i] = item_value<SRC>(it[i], taps, pv, img + c0 * 4, slot * kPix + px + 64 * i, pitch);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++) val[i].f[j] = 0.0f;
+          }
+        }
+        if (chunk + 1 < p.nchunks) {  // the next chunk's loads are in flight while this one is split, stored and handed over
+          chunk_item3(g.Cp, g.K, chunk + 1, v, slot, c0);
+          load();
+        }
+        if (!mbar_wait(bars.empty + ring.s, ring.ph ^ 1u, bars.abort_flag)) { alive = false; break; }
+        if (pt == 0) {
+          mbar_arrive_expect_tx(bars.full + ring.s, bbytes);
+          bulk_copy_g2s(base + (size_t)ring.s * stage_bytes + 3 * kPartA, (const char *)p.wp + ((size_t)nb * p.nchunks + chunk) * bbytes,
+                        bbytes, bars.full + ring.s);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) store_parts(dst[i] + ring.s * stage_bytes, kPartA, val[i]);
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bars.full + ring.s);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kEpi) tmem_dealloc(tmem, 512);
+  if (tid == 0 && *bars.abort_flag) {
+    *p.status = 1;
+    g_wait_status3 = 1;
+  }
+}
+
+// ---- weight gradient ---------------------------------------------------------------------------------------------------
+// A block owns 128 gradient rows x 128 columns (a column group) and a range of pixel tiles; a tile is four steps of 32 pixels.
+// A operand: the gradient's tile image, K-major (64-byte rows); B operand: gathered columns, MN-major (rows of 64 columns of one
+// pixel, 128-byte swizzle).  The tap table is double buffered: the next tile's taps are decoded while this one is gathered.
+constexpr int kDwN = 128, kDwPix3 = 32;
+constexpr int kPartB3 = 2 * kDwPix3 * 128;  // one part of a step's columns: two groups of 64 columns
+constexpr int kStepA = 3 * kPartA, kStepB = 3 * kPartB3;
+
+struct Dw3 {
+  Src3 g;
+  const __nv_bfloat16 *gt;  // gradient tile images [tile][row block][step][part][128 rows][32 pixels]
+  float *partial;           // [split][mbs * 128][groups * 128]
+  int *status;
+  int B, mbs, groups, slots, tiles_x, tiles_y, splits, stages;  // slots: most slots of a column group
+};
+
+template <int SRC> inline size_t dw3_smem(int stages, int slots) {
+  return 1024 + (size_t)stages * (kStepA + kStepB) + 2 * align_up(TapTable<SRC>::bytes(slots), 16) + bars_bytes(stages);
+}
+
+template <int SRC>
+__global__ void __launch_bounds__(kThreads3, 1) x3_dw_kernel(const Dw3 p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, S = p.stages;
+  const Src3 &g = p.g;
+  constexpr uint32_t stage_bytes = kStepA + kStepB;
+  const uint32_t stage0 = smem_u32(base), table_bytes = (uint32_t)p.slots * kPix * (TapTable<SRC>::NT == 1 ? 4 : 32);
+  const Bars bars = carve_bars(base + (size_t)S * stage_bytes + 2 * ((table_bytes + 15) / 16 * 16), S);
+  const uint32_t tmem = start_block(bars, S, tid);
+  const int grp = blockIdx.x, split = blockIdx.y, mb = blockIdx.z;
+  const int tiles_per_image = p.tiles_x * p.tiles_y;
+  const int64_t total = (int64_t)p.B * tiles_per_image;
+  const int lo = (int)(total * split / p.splits), hi = (int)(total * (split + 1) / p.splits);
+  const int nseg = (hi - lo) * 4 / kSeg;
+
+  if (warp < kEpi) {
+    const EpiSlice e(tmem, warp, kDwN);
+    int sg = 0;
+    float acc[64];
+    drain_tile(bars, e, acc, nseg, sg, 0, lane);
+    const int row = mb * 128 + (warp & 3) * 32 + lane;
+    float *o = p.partial + ((size_t)split * p.mbs * 128 + row) * (p.groups * kDwN) + grp * kDwN + e.col0;
+#pragma unroll
+    for (int j = 0; j < 64; j += 4) *(float4 *)(o + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+  } else if (warp == kEpi) {
+    if (lane == 0) {
+      const uint32_t idesc = idesc_bf16(128, kDwN, 0, 1);
+      Ring3 ring;
+      const int steps = (hi - lo) * 4;
+      for (int st = 0; st < steps; st++, ring.next(S)) {
+        const int sg = st / kSeg, buf = sg & 1;
+        const bool first = st % kSeg == 0;
+        if (first && !mbar_wait(bars.seg_empty + buf, ((sg >> 1) & 1) ^ 1, bars.abort_flag)) break;
+        if (!mbar_wait(bars.full + ring.s, ring.ph, bars.abort_flag)) break;
+        tc_fence_after();
+        const uint32_t a = stage0 + ring.s * stage_bytes;
+        issue_step(tmem + kHh + buf * 128, tmem + kCorr, smem_desc_sw64(a), smem_desc_sw128(a + kStepA, kDwPix3 * 128, 1024), kPartA >> 4,
+                   kPartB3 >> 4, 2, 16 * 128 >> 4, idesc, first, st == 0);
+        umma_commit(bars.empty + ring.s);
+        if (st % kSeg == kSeg - 1) umma_commit(bars.seg_full + buf);
+      }
+    }
+  } else {
+    // producers: thread = vector v (8 of the group's 128 columns) of pixels px and px + 16 of the step
+    const int pt = tid - kProd0, v = pt & 15, px = pt >> 4;
+    const uint32_t pitch = (uint32_t)g.Cp * 4u;
+    const size_t image = (size_t)(g.SH * g.SW + 1) * pitch;
+    const int s0 = grp * kDwN / g.Cp, col = grp * kDwN + v * 8, slot = col / g.Cp, c0 = col - slot * g.Cp;
+    const bool have = slot < g.K;
+    const int row0 = have ? (slot - s0) * kPix : 0;
+    uint32_t dst[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const int q = px + 16 * i;
+      dst[i] = stage0 + kStepA + (v >> 3) * (kDwPix3 * 128) + q * 128 + (((v & 7) ^ (q & 7)) << 4);
+    }
+    const uint32_t table0 = stage0 + S * stage_bytes, table_pitch = (table_bytes + 15) / 16 * 16;
+    const PlanView<float> none{};
+    const auto fill = [&](int tile, int buf) {
+      const int t2 = tile % tiles_per_image;
+      fill_taps3<SRC>(g, TapTable<SRC>(table0 + buf * table_pitch, p.slots), none, true, s0, p.slots, t2 / p.tiles_x, t2 % p.tiles_x, pt);
+    };
+    if (lo < hi) fill(lo, 0);
+    Ring3 ring;
+    bool alive = true;
+    for (int tile = lo; tile < hi; tile++) {
+      const TapTable<SRC> taps(table0 + ((tile - lo) & 1) * table_pitch, p.slots);
+      const char *img = g.xl + (size_t)(tile / tiles_per_image) * image + c0 * 4;
+      producer_bar3();  // this tile's table is complete, the other one no longer read
+      Item<SRC> it[2];
+      const auto load = [&](int q) {
+        if (have) {
+#pragma unroll
+          for (int i = 0; i < 2; i++) item_load<SRC>(it[i], taps, img, row0 + q * kDwPix3 + px + 16 * i, 0u);
+        }
+      };
+      if (alive) load(0);
+      if (tile + 1 < hi) fill(tile + 1, (tile + 1 - lo) & 1);
+      for (int q = 0; alive && q < 4; q++, ring.next(S)) {
+        V8 val[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          if (have) {
+            val[i] = item_value<SRC>(it[i], taps, none, img, 0, pitch);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; j++) val[i].f[j] = 0.0f;
+          }
+        }
+        if (q < 3) load(q + 1);
+        if (!mbar_wait(bars.empty + ring.s, ring.ph ^ 1u, bars.abort_flag)) { alive = false; break; }
+        if (pt == 0) {
+          mbar_arrive_expect_tx(bars.full + ring.s, kStepA);
+          bulk_copy_g2s(base + (size_t)ring.s * stage_bytes, (const char *)p.gt + (((size_t)tile * p.mbs + mb) * 4 + q) * kStepA, kStepA,
+                        bars.full + ring.s);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; i++) store_parts(dst[i] + ring.s * stage_bytes, kPartB3, val[i]);
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bars.full + ring.s);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kEpi) tmem_dealloc(tmem, 512);
+  if (tid == 0 && *bars.abort_flag) {
+    *p.status = 1;
+    g_wait_status3 = 1;
+  }
+}
+
+// ---- layout pre-passes ---------------------------------------------------------------------------------------------------
+// (B, C, HW) -> (B, HW + 1, Cp) float32; padding channels and the extra pixel are zero.  32 pixels x 32 channels per block,
+// through shared memory.
+__global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const float *__restrict__ x, float *__restrict__ y, int C, int Cp, int HW) {
+  __shared__ float tile[32][33];
+  const int b = blockIdx.z, c0 = blockIdx.y * 32, p0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int c = c0 + ty + 8 * i, p = p0 + tx;
+    tile[ty + 8 * i][tx] = c < C && p < HW ? __ldg(x + ((size_t)b * C + c) * HW + p) : 0.0f;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int p = p0 + ty + 8 * i, c = c0 + tx;
+    if (p <= HW && c < Cp) y[((size_t)b * (HW + 1) + p) * Cp + c] = tile[tx][ty + 8 * i];
+  }
+}
+
+__device__ __forceinline__ void split3(float x, uint16_t &h, uint16_t &m, uint16_t &l) {
+  const float r = x - __uint_as_float(__float_as_uint(x) & 0xffff0000u), s = r - __uint_as_float(__float_as_uint(r) & 0xffff0000u);
+  h = (uint16_t)(__float_as_uint(x) >> 16);
+  m = (uint16_t)(__float_as_uint(r) >> 16);
+  l = (uint16_t)(__float_as_uint(s) >> 16);
+}
+
+// Weights -> three-part tile images.  Rows n = nb * Npb + row; `premul`: rows are n = k * M + m of the multiply-first adjoint
+// (columns: source channels), else rows are output channels and columns (slot, channel) items.  W[m * sm + ch * sc + k * sk].
+__global__ void weight_image3_kernel(const float *__restrict__ w, uint16_t *__restrict__ wp, int M, int CH, int Cp, int K, int Npb, int nblk,
+                                     int nchunks, int64_t sm, int64_t sc, int64_t sk, int premul) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (int64_t)nblk * nchunks * Npb * kCols) return;
+  const int col = (int)(i % kCols), r = (int)((i / kCols) % Npb), chunk = (int)((i / ((int64_t)kCols * Npb)) % nchunks);
+  const int nb = (int)(i / ((int64_t)kCols * Npb * nchunks)), n = nb * Npb + r;
+  int slot, c0;
+  float v = 0.0f;
+  if (premul) {
+    const int k = n / M, ch = chunk * kCols + col;
+    if (k < K && ch < CH) v = __ldg(w + (n - k * M) * sm + ch * sc + k * sk);
+  } else {
+    chunk_item3(Cp, K, chunk, col >> 3, slot, c0);
+    const int ch = c0 + (col & 7);
+    if (n < M && slot < K && ch < CH) v = __ldg(w + n * sm + ch * sc + slot * sk);
+  }
+  uint16_t h, m, l;
+  split3(v, h, m, l);
+  uint16_t *t = wp + ((int64_t)nb * nchunks + chunk) * 3 * Npb * kCols + r * kCols + ((((col >> 3) ^ ((r >> 1) & 3)) << 3) | (col & 7));
+  t[0] = h;
+  t[(int64_t)Npb * kCols] = m;
+  t[(int64_t)2 * Npb * kCols] = l;
+}
+
+// Gradient (B, N, GH*GW) -> tile images [tile][row block][step][part][128 rows][32 pixels] and, with `sums`, the sum of every
+// row over the tile's pixels: sums[(tile * mbs + row block) * 128 + row].  One block = one tile and row block.
+__global__ void __launch_bounds__(256) grad_image3_kernel(const float *__restrict__ gsrc, uint8_t *__restrict__ gt, int N, int GH, int GW,
+                                                          int tiles_x, int tiles_y, int mbs, float *__restrict__ sums) {
+  const int t2 = blockIdx.x, mb = blockIdx.y, b = blockIdx.z, ty = t2 / tiles_x, tx = t2 % tiles_x;
+  const size_t npix = (size_t)GH * GW, tile = (size_t)b * tiles_x * tiles_y + t2;
+  uint8_t *dst = gt + (tile * mbs + mb) * 4 * kStepA;
+  const bool vec = (GW & 3) == 0 && (((uintptr_t)gsrc) & 15) == 0;
+  for (int i = threadIdx.x; i < 128 * 16; i += 256) {
+    const int r = i >> 4, u = i & 15, n = mb * 128 + r;  // u: 8 pixels of the tile, row u >> 1, columns (u & 1) * 8 ..
+    const int y = ty * kTileH + (u >> 1), x0 = tx * kTileW + (u & 1) * 8;
+    const float *src = gsrc + ((size_t)b * N + n) * npix + (size_t)y * GW + x0;
+    V8 v;
+    if (n < N && y < GH && x0 + 8 <= GW && vec) {
+      const float4 a = __ldg((const float4 *)src), c = __ldg((const float4 *)src + 1);
+      v.f[0] = a.x; v.f[1] = a.y; v.f[2] = a.z; v.f[3] = a.w;
+      v.f[4] = c.x; v.f[5] = c.y; v.f[6] = c.z; v.f[7] = c.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; e++) v.f[e] = n < N && y < GH && x0 + e < GW ? __ldg(src + e) : 0.0f;
+    }
+    uint16_t h[8], m[8], l[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) split3(v.f[e], h[e], m[e], l[e]);
+    const auto pack = [](const uint16_t (&q)[8]) {
+      return make_uint4(q[0] | (uint32_t)q[1] << 16, q[2] | (uint32_t)q[3] << 16, q[4] | (uint32_t)q[5] << 16, q[6] | (uint32_t)q[7] << 16);
+    };
+    uint8_t *d = dst + (size_t)(u >> 2) * kStepA + r * 64 + (((u & 3) ^ ((r >> 1) & 3)) << 4);
+    *(uint4 *)d = pack(h);
+    *(uint4 *)(d + kPartA) = pack(m);
+    *(uint4 *)(d + 2 * kPartA) = pack(l);
+    if (sums) {
+      float s = ((v.f[0] + v.f[1]) + (v.f[2] + v.f[3])) + ((v.f[4] + v.f[5]) + (v.f[6] + v.f[7]));
+#pragma unroll
+      for (int d2 = 1; d2 < 16; d2 <<= 1) s += __shfl_xor_sync(0xffffffffu, s, d2);
+      if (u == 0) sums[(tile * mbs + mb) * 128 + r] = s;
+    }
+  }
+}
+
+// gw[m, ch, k] = sum over splits, in order, of the partial sums.
+__global__ void dw3_reduce_kernel(const float *__restrict__ partial, int splits, int rows, int cols, int M, int CH, int Cp, int K, int64_t sm,
+                                  int64_t sc, int64_t sk, float *__restrict__ gw) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= M * CH * K) return;
+  const int ch = i % CH, k = (i / CH) % K, m = i / (CH * K);
+  const float *s = partial + (size_t)m * cols + k * Cp + ch;
+  float a = 0.0f;
+  for (int z = 0; z < splits; z++) a += __ldg(s + (size_t)z * rows * cols);
+  gw[m * sm + ch * sc + k * sk] = a;
+}
+
+// gb[c] = sum over tiles of the row sums: one block per channel, fixed order.
+__global__ void __launch_bounds__(256) bias_sum3_kernel(const float *__restrict__ sums, int64_t tiles, int rows, float *__restrict__ gb) {
+  __shared__ float red[256];
+  const int c = blockIdx.x;
+  float s = 0.0f;
+  for (int64_t t = threadIdx.x; t < tiles; t += 256) s += __ldg(sums + t * rows + c);
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int d = 128; d > 0; d >>= 1) {
+    if (threadIdx.x < d) red[threadIdx.x] += red[threadIdx.x + d];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) gb[c] = red[0];
+}
+
+// ---- host side -------------------------------------------------------------------------------------------------------------
+constexpr int kMaxDev3 = 64;
+int device3() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev3) dev = 0;
+  return dev;
+}
+int sms3() {
+  static int n[kMaxDev3];
+  const int dev = device3();
+  int v = __atomic_load_n(&n[dev], __ATOMIC_RELAXED);
+  if (v == 0) {
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0) v = 148;
+    __atomic_store_n(&n[dev], v, __ATOMIC_RELAXED);
+  }
+  return v;
+}
+template <typename Kernel> void allow_smem3(Kernel kernel, int *granted, size_t smem) {
+  const int dev = device3();
+  if (__atomic_load_n(&granted[dev], __ATOMIC_RELAXED) >= (int)smem) return;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  __atomic_store_n(&granted[dev], (int)smem, __ATOMIC_RELAXED);
+}
+
+// Source kind of a gather, or -1 where the kernels here do not cover it (more than four taps per slot).
+int source3(bool use_plan, int64_t P, int interp) {
+  if (use_plan) return SRC_PLAN;
+  if (P == 0) return interp == SPH_NEAREST ? SRC_MAP1 : SRC_MAP4;
+  return P <= 4 && interp == SPH_NEAREST ? SRC_MAP4 : -1;
+}
+size_t table3(int src, int ns) {
+  return src == SRC_SELF ? 0 : (size_t)ns * kPix * (src == SRC_MAP1 ? 4 : src == SRC_PLAN ? 40 : 32);
+}
+// Three stages where they leave the L1 about 90 KB, else two.
+constexpr size_t kSmemSoft = 140 * 1024;
+
+struct GemmPlan3 {
+  int Cp, nchunks, Npb, nblk, stages;
+  size_t xl_bytes, wp_bytes, smem;
+  bool ok;
+};
+GemmPlan3 gemm_plan3(int src, int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t Nout) {
+  GemmPlan3 q{};
+  q.Cp = padded3(CH);
+  q.nchunks = chunks3(q.Cp, (int)K);
+  const int np = (int)align_up((size_t)Nout, 16);
+  q.nblk = (np + kNMax - 1) / kNMax;
+  q.Npb = (int)align_up((size_t)((np + q.nblk - 1) / q.nblk), 16);  // blocks of equal width
+  q.xl_bytes = align_up((size_t)(B * (SHW + 1)) * q.Cp * 4, 256);
+  q.wp_bytes = align_up((size_t)q.nblk * q.nchunks * 3 * q.Npb * kCols * 2, 256);
+  const auto smem = [&](int s) { return 1024 + (size_t)s * (3 * kPartA + 3 * q.Npb * 64) + align_up(table3(src, (int)K), 16) + bars_bytes(s); };
+  q.stages = smem(3) <= kSmemSoft ? 3 : 2;
+  q.smem = smem(q.stages);
+  q.ok = src >= 0 && q.smem <= kSmemMax && (SHW + 1) * q.Cp * 4 < ((int64_t)1 << 32) &&
+         (int64_t)q.nblk * q.nchunks * q.Npb * kCols < ((int64_t)1 << 31);
+  return q;
+}
+
+// Multiply first (conv_simt.cu says when and why): a dense product over the source grid with N = K * M rows.
+struct Premul3 {
+  GemmPlan3 q;
+  size_t t_bytes;
+  bool use;
+};
+Premul3 premul3(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t M, int64_t n_dst) {
+  Premul3 r{};
+  r.q = gemm_plan3(SRC_SELF, B, CH, SHW, 1, K * M);
+  r.t_bytes = align_up((size_t)(B * K * M * SHW) * 4, 256);
+  r.use = r.q.ok && n_dst >= 3 * SHW && CH >= 16 && r.t_bytes <= ((size_t)8 << 30);
+  return r;
+}
+
+struct DwPlan3 {
+  int Cp, groups, mbs, slots, splits, stages, tiles_x, tiles_y;
+  size_t xl_bytes, gt_bytes, partial_bytes, sums_bytes, smem;
+  bool ok;
+};
+DwPlan3 dw_plan3(int src, int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t M, int64_t GH, int64_t GW) {
+  DwPlan3 d{};
+  d.Cp = padded3(CH);
+  d.groups = (int)((K * d.Cp + kDwN - 1) / kDwN);
+  d.mbs = (int)((M + 127) / 128);
+  for (int g = 0; g < d.groups && g < 64; g++)
+    d.slots = std::max(d.slots, (g * kDwN + kDwN - 1) / d.Cp - g * kDwN / d.Cp + 1);
+  d.tiles_x = cdiv(GW, kTileW);
+  d.tiles_y = cdiv(GH, kTileH);
+  const int64_t tiles = B * d.tiles_x * d.tiles_y;
+  int64_t s = sms3() / ((int64_t)d.groups * d.mbs);
+  d.splits = (int)(s < 1 ? 1 : s > tiles ? tiles : s);
+  d.stages = 2;
+  d.smem = 1024 + (size_t)d.stages * (kStepA + kStepB) + 2 * align_up(table3(src, d.slots), 16) + bars_bytes(d.stages);
+  d.xl_bytes = align_up((size_t)(B * (SHW + 1)) * d.Cp * 4, 256);
+  d.gt_bytes = align_up((size_t)tiles * d.mbs * 4 * kStepA, 256);
+  d.partial_bytes = align_up((size_t)d.splits * d.mbs * 128 * d.groups * kDwN * 4, 256);
+  d.sums_bytes = align_up((size_t)tiles * d.mbs * 128 * 4, 256);
+  d.ok = src >= 0 && src != SRC_PLAN && d.smem <= kSmemMax && (SHW + 1) * d.Cp * 4 < ((int64_t)1 << 32) && tiles < ((int64_t)1 << 28);
+  return d;
+}
+
+void to_nhwc3(const void *x, float *y, int64_t B, int64_t C, int Cp, int64_t HW, cudaStream_t st) {
+  nchw_to_nhwc_kernel<<<dim3(cdiv(HW + 1, 32), cdiv(Cp, 32), (unsigned)B), 256, 0, st>>>((const float *)x, y, (int)C, Cp, (int)HW);
+}
+
+template <int SRC> void launch_gemm3(const Gemm3 &p, int64_t tiles, size_t smem, cudaStream_t st) {
+  static int granted[kMaxDev3];
+  allow_smem3(x3_gemm_kernel<SRC>, granted, smem);
+  x3_gemm_kernel<SRC><<<(unsigned)std::min<int64_t>(tiles, sms3()), kThreads3, smem, st>>>(p);
+}
+template <int SRC> void launch_dw3(const Dw3 &p, size_t smem, cudaStream_t st) {
+  static int granted[kMaxDev3];
+  allow_smem3(x3_dw_kernel<SRC>, granted, smem);
+  x3_dw_kernel<SRC><<<dim3(p.groups, p.splits, p.mbs), kThreads3, smem, st>>>(p);
+}
+
+}  // namespace
+
+// Scratch of x3_gemm; 0: not covered.
+size_t x3_gemm_workspace(bool use_plan, int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int interp, int64_t Nout, int64_t n_dst) {
+  if (use_plan) {
+    const Premul3 r = premul3(B, CH, SHW, K, Nout, n_dst);
+    if (r.use) return 256 + r.q.xl_bytes + r.q.wp_bytes + r.t_bytes;
+  }
+  const GemmPlan3 q = gemm_plan3(source3(use_plan, P, interp), B, CH, SHW, K, Nout);
+  return q.ok ? 256 + q.xl_bytes + q.wp_bytes : 0;
+}
+
+int x3_gemm(bool use_plan, const void *src, const void *map, const void *iw, const void *plan, int64_t CH, int64_t SH, int64_t SW, int64_t K,
+            int64_t P, int64_t GH, int64_t GW, int interp, const void *wgt, int64_t sm, int64_t sc, int64_t sk, const void *bias, void *out,
+            int64_t Nout, int64_t B, void *ws, cudaStream_t st) {
+  const Premul3 r = use_plan ? premul3(B, CH, SH * SW, K, Nout, GH * GW) : Premul3{};
+  const int kind = r.use ? (int)SRC_SELF : source3(use_plan, P, interp);
+  const GemmPlan3 q = r.use ? r.q : gemm_plan3(kind, B, CH, SH * SW, K, Nout);
+  char *w = (char *)ws;
+  int *status = (int *)w;
+  float *xl = (float *)(w + 256);
+  uint16_t *wp = (uint16_t *)(w + 256 + q.xl_bytes);
+  float *T = (float *)(w + 256 + q.xl_bytes + q.wp_bytes);
+  if (cudaMemsetAsync(status, 0, 4, st) != cudaSuccess) return SPH_ERR_CUDA;
+  to_nhwc3(src, xl, B, CH, q.Cp, SH * SW, st);
+  const int64_t wtotal = (int64_t)q.nblk * q.nchunks * q.Npb * kCols;
+  weight_image3_kernel<<<cdiv(wtotal, 256), 256, 0, st>>>((const float *)wgt, wp, (int)Nout, (int)CH, q.Cp, (int)K, q.Npb, q.nblk, q.nchunks,
+                                                          sm, sc, sk, r.use ? 1 : 0);
+  Gemm3 p{};
+  p.g = Src3{(const char *)xl, (const float *)map, (const float *)iw, plan, q.Cp, (int)SH, (int)SW, r.use ? 1 : (int)K, (int)P,
+             (int)(r.use ? SH : GH), (int)(r.use ? SW : GW), interp};
+  p.wp = (const __nv_bfloat16 *)wp;
+  p.bias = r.use ? nullptr : (const float *)bias;
+  p.out = r.use ? T : (float *)out;
+  p.status = status;
+  p.B = (int)B; p.Nout = (int)(r.use ? K * Nout : Nout); p.Npb = q.Npb; p.nblk = q.nblk; p.nchunks = q.nchunks;
+  p.tiles_x = cdiv(p.g.GW, kTileW); p.tiles_y = cdiv(p.g.GH, kTileH); p.stages = q.stages;
+  const int64_t tiles = B * p.tiles_x * p.tiles_y * q.nblk;
+  switch (kind) {
+    case SRC_MAP1: launch_gemm3<SRC_MAP1>(p, tiles, q.smem, st); break;
+    case SRC_MAP4: launch_gemm3<SRC_MAP4>(p, tiles, q.smem, st); break;
+    case SRC_PLAN: launch_gemm3<SRC_PLAN>(p, tiles, q.smem, st); break;
+    default: launch_gemm3<SRC_SELF>(p, tiles, q.smem, st); break;
+  }
+  const int rc = launch_status(3);
+  return rc == SPH_OK && r.use ? simt_plan_gather_planes(T, plan, bias, out, K, Nout, SH * SW, GH * GW, B, st) : rc;
+}
+
+size_t x3_dw_workspace(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int interp, int64_t M, int64_t GH, int64_t GW) {
+  const DwPlan3 d = dw_plan3(source3(false, P, interp), B, CH, SHW, K, M, GH, GW);
+  return d.ok ? 256 + d.xl_bytes + d.gt_bytes + d.partial_bytes + d.sums_bytes : 0;
+}
+
+// gw[m, ch, k] = sum A[b, m, pix] * Col[b, pix, (ch, k)];  with gb, also gb[m] = sum A[b, m, :].
+int x3_dw(const void *A, const void *src, const void *map, const void *iw, int64_t CH, int64_t SH, int64_t SW, int64_t K, int64_t P,
+          int64_t GH, int64_t GW, int interp, int64_t M, int64_t B, void *gw, int64_t sm, int64_t sc, int64_t sk, void *gb, void *ws,
+          cudaStream_t st) {
+  const int kind = source3(false, P, interp);
+  const DwPlan3 d = dw_plan3(kind, B, CH, SH * SW, K, M, GH, GW);
+  char *w = (char *)ws;
+  int *status = (int *)w;
+  float *xl = (float *)(w + 256);
+  uint8_t *gt = (uint8_t *)(w + 256 + d.xl_bytes);
+  float *partial = (float *)(w + 256 + d.xl_bytes + d.gt_bytes), *sums = (float *)((char *)partial + d.partial_bytes);
+  if (cudaMemsetAsync(status, 0, 4, st) != cudaSuccess) return SPH_ERR_CUDA;
+  to_nhwc3(src, xl, B, CH, d.Cp, SH * SW, st);
+  grad_image3_kernel<<<dim3(d.tiles_x * d.tiles_y, d.mbs, (unsigned)B), 256, 0, st>>>((const float *)A, gt, (int)M, (int)GH, (int)GW, d.tiles_x,
+                                                                                     d.tiles_y, d.mbs, gb ? sums : nullptr);
+  Dw3 p{};
+  p.g = Src3{(const char *)xl, (const float *)map, (const float *)iw, nullptr, d.Cp, (int)SH, (int)SW, (int)K, (int)P, (int)GH, (int)GW, interp};
+  p.gt = (const __nv_bfloat16 *)gt; p.partial = partial; p.status = status;
+  p.B = (int)B; p.mbs = d.mbs; p.groups = d.groups; p.slots = d.slots; p.tiles_x = d.tiles_x; p.tiles_y = d.tiles_y;
+  p.splits = d.splits; p.stages = d.stages;
+  if (kind == SRC_MAP1) launch_dw3<SRC_MAP1>(p, d.smem, st);
+  else launch_dw3<SRC_MAP4>(p, d.smem, st);
+  dw3_reduce_kernel<<<cdiv(M * CH * K, 256), 256, 0, st>>>(partial, d.splits, d.mbs * 128, d.groups * kDwN, (int)M, (int)CH, d.Cp, (int)K, sm,
+                                                           sc, sk, (float *)gw);
+  if (gb) bias_sum3_kernel<<<(unsigned)M, 256, 0, st>>>(sums, B * d.tiles_x * d.tiles_y, d.mbs * 128, (float *)gb);
+  return launch_status(gb ? 5 : 4);
+}
+
+int x3_wait_status(int reset) {
+  int v = 0;
+  if (cudaMemcpyFromSymbol(&v, g_wait_status3, sizeof(int)) != cudaSuccess) return -1;
+  if (reset && v) {
+    const int zero = 0;
+    if (cudaMemcpyToSymbol(g_wait_status3, &zero, sizeof(int)) != cudaSuccess) return -1;
+  }
+  return v;
+}
+
+}  // namespace sph
+
+SPH_TU_STATUS(conv_x3)

@@ -586,7 +586,7 @@ torch::Tensor conv_forward_impl(torch::Tensor x, torch::Tensor map, const torch:
   const ConvArgs a{x.size(0), x.size(1), weight.size(0), x.size(2), x.size(3), m.H, m.W, K, m.P, dtype_of(x), (int)it,
                    dtype_of(x) == SPH_F32 ? precision() : SPH_PRECISION_EXACT};
   torch::Tensor out = torch::empty({a.B, a.Cout, a.OH, a.OW}, x.options());
-  const size_t wb = sph_conv_workspace_bytes(SPH_CONV_FORWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
+  const size_t wb = sph_conv_workspace_preferred_bytes(SPH_CONV_FORWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
                                              a.interp, a.prec);
   torch::Tensor ws = workspace(wb, x);
   if (a.prec == SPH_PRECISION_BF16 && g_use_companions) {
@@ -670,7 +670,7 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
   if (a.prec == SPH_PRECISION_BF16) {
     // all three gradients in one call: grad_output is converted (and masked) once for both of its consumers, and the
     // input's channels-last copy is used if a previous layer left one
-    const size_t wbc = sph_conv_workspace_bytes(SPH_CONV_BACKWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
+    const size_t wbc = sph_conv_workspace_preferred_bytes(SPH_CONV_BACKWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
                                                 a.interp, a.prec);
     if (wbc > 0) {
       torch::Tensor wsc = workspace(wbc, x);
@@ -686,10 +686,10 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
       }
     }
   }
-  size_t wb = sph_conv_workspace_bytes(SPH_CONV_BACKWARD_INPUT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
+  size_t wb = sph_conv_workspace_preferred_bytes(SPH_CONV_BACKWARD_INPUT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
                                        a.dtype, a.interp, a.prec);
   torch::Tensor ws = workspace(wb, x);
-  size_t wb2 = sph_conv_workspace_bytes(SPH_CONV_BACKWARD_WEIGHT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
+  size_t wb2 = sph_conv_workspace_preferred_bytes(SPH_CONV_BACKWARD_WEIGHT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
                                         a.interp, a.prec);
   torch::Tensor ws2 = workspace(wb2, x);
   if (act_out) {  // gradient of the fused ReLU: the kernels read grad_output * (act_out > 0)
@@ -781,7 +781,7 @@ torch::Tensor tconv_forward_impl(torch::Tensor x, torch::Tensor map, const torch
                    dtype_of(x) == SPH_F32 ? precision() : SPH_PRECISION_EXACT};
   torch::Tensor plan = get_plan(map, iw, a.IH * a.IW, a.K, a.P, a.interp, a.OH, a.OW);
   torch::Tensor out = torch::empty({a.B, a.Cout, a.OH, a.OW}, x.options());
-  const size_t wb = sph_conv_workspace_bytes(SPH_TCONV_FORWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
+  const size_t wb = sph_conv_workspace_preferred_bytes(SPH_TCONV_FORWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
                                              a.interp, a.prec);
   torch::Tensor ws = workspace(wb, x);
   ok(sph_mapped_tconv_forward(x.data_ptr(), plan.data_ptr(), weight.data_ptr(), bias.data_ptr(), out.data_ptr(), a.B, a.Cin,
@@ -809,14 +809,14 @@ std::vector<torch::Tensor> tconv_backward_impl(torch::Tensor go, torch::Tensor m
   const ConvArgs a{x.size(0), x.size(1), weight.size(1), x.size(2), x.size(3), go.size(2), go.size(3), K, m.P, dtype_of(x),
                    (int)it, dtype_of(x) == SPH_F32 ? precision() : SPH_PRECISION_EXACT};
   torch::Tensor gx = torch::empty_like(x), gw = torch::empty_like(weight), gb = torch::empty({a.Cout}, x.options());
-  size_t wb = sph_conv_workspace_bytes(SPH_TCONV_BACKWARD_INPUT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
+  size_t wb = sph_conv_workspace_preferred_bytes(SPH_TCONV_BACKWARD_INPUT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
                                        a.dtype, a.interp, a.prec);
   torch::Tensor ws = workspace(wb, x);
   ok(sph_mapped_tconv_backward_input(go.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, weight.data_ptr(),
                                      gx.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp,
                                      a.prec, ws.data_ptr(), wb, stream()),
      "sph_mapped_tconv_backward_input");
-  wb = sph_conv_workspace_bytes(SPH_TCONV_BACKWARD_WEIGHT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
+  wb = sph_conv_workspace_preferred_bytes(SPH_TCONV_BACKWARD_WEIGHT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
                                 a.interp, a.prec);
   torch::Tensor ws2 = workspace(wb, x);
   ok(sph_mapped_tconv_backward_weight(go.data_ptr(), x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr,

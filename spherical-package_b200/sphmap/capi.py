@@ -31,7 +31,7 @@ SYMBOLS = [
     "sph_device_status", "sph_debug_bounded_wait", "sph_mapped_max_unpool_planned", "sph_mapped_avg_pool",
     "sph_mapped_avg_unpool", "sph_resample_to_map_normalized", "sph_resample_from_uv_maps", "sph_plan_build_uv",
     "sph_voting_resample_to_map", "sph_build_kernel_map", "sph_build_is_checked", "sph_conv_companion_bytes",
-    "sph_staging_bytes", "sph_resample_from_map_ws", "sph_resample_to_map_ws", "sph_mapped_pool_ws", "sph_mapped_max_unpool_ws",
+    "sph_staging_bytes", "sph_conv_workspace_preferred_bytes", "sph_resample_from_map_ws", "sph_resample_to_map_ws", "sph_mapped_pool_ws", "sph_mapped_max_unpool_ws",
     "sph_conv_companion_channels", "sph_conv_companion_fill", "sph_trace_phases", "sph_mapped_conv_forward_cl", "sph_mapped_conv_backward_cl",
 ]
 ERR_UNSUPPORTED = 2
@@ -45,6 +45,7 @@ lib.sph_plan_bytes.restype = ctypes.c_size_t
 lib.sph_staging_bytes.restype = ctypes.c_size_t
 lib.sph_launch_count.restype = ctypes.c_ulonglong
 lib.sph_conv_workspace_bytes.restype = ctypes.c_size_t
+lib.sph_conv_workspace_preferred_bytes.restype = ctypes.c_size_t
 lib.sph_conv_companion_bytes.restype = ctypes.c_size_t
 
 _vp, _i64, _int, _sz = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_size_t

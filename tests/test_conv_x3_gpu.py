@@ -1,0 +1,78 @@
+"""float32 convolutions through three-way split operands on the tensor cores (what the host extension runs in the exact
+precision) against the library's float64 kernels, beside the float32 SIMT kernels (what the C ABI runs with the smaller
+scratch): no less accurate than those, at channel counts around the padding steps, row counts around the 128-row blocks,
+ragged grids, every kind of map, and adjoints over down-sampling maps (multiply first)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+#        B, Cin, Cout, (H, W), (OH, OW), K, interpolation, points
+CASES = [(2, 16, 32, (16, 32), (16, 32), 9, 1, 0),
+         (3, 20, 37, (45, 91), (45, 91), 9, 2, 0),
+         (1, 5, 33, (8, 16), (8, 16), 9, 1, 0),
+         (1, 64, 129, (9, 17), (8, 15), 9, 0, 0),
+         (2, 40, 200, (20, 30), (7, 11), 9, 1, 0),
+         (1, 100, 50, (20, 33), (20, 33), 5, 0, 3),
+         (1, 96, 16, (24, 40), (24, 40), 25, 1, 0),
+         (1, 260, 256, (16, 32), (16, 32), 9, 1, 0)]
+
+
+def _rel(a, ref):
+    return ((a.double() - ref).norm() / ref.norm()).item()
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_split_products_are_float32_accurate(case):
+    import _spherical_distortion_ext._C as C
+    from sphmap import capi
+    B, ci, co, (H, W), (OH, OW), K, interp, P = case
+    g = torch.Generator().manual_seed(ci)
+    r = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    x, w, b, go = r(B, ci, H, W), r(co, ci, K) / 30, r(co), r(B, co, OH, OW)
+    m = torch.rand(*((OH, OW, K, P, 2) if P else (OH, OW, K, 2)), generator=g) * torch.tensor([W + 1.0, H + 1.0]) - 1.0
+    iw = torch.rand(OH, OW, K, P, generator=g) if P else None
+    wt, bt, xt, got = r(ci, co, K) / 30, r(co), r(B, ci, OH, OW), r(B, co, H, W)
+    dev = lambda *t: [None if v is None else v.cuda() for v in t]  # noqa: E731
+    dbl = lambda *t: [None if v is None else v.double() for v in t]  # noqa: E731
+
+    def simt(x, w, b, go, m, iw, wt, bt, xt, got):
+        plan = capi.plan_build(m, iw, OH * OW, K, interp, H, W)
+        return [capi.conv_forward(x, m, w, b, K, interp, iw), capi.conv_backward_input(go, plan, w, H, W, K),
+                *capi.conv_backward_weight(go, x, m, K, interp, iw), capi.tconv_forward(xt, plan, wt, bt, H, W, K),
+                capi.tconv_backward_input(got, m, wt, K, interp, iw), *capi.tconv_backward_weight(got, xt, m, K, interp, iw)]
+
+    a = dev(x, w, b, go, m, iw, wt, bt, xt, got)
+    ref, old = simt(*dbl(*a)), simt(*a)
+    x, w, b, go, m, iw, wt, bt, xt, got = a
+    it, ws = C.InterpolationType(interp), (m, iw) if P else (m,)
+    name = "weighted_" if P else ""
+    new = [getattr(C, name + "mapped_conv_forward")(x, *ws, w, b, K, it), *getattr(C, name + "mapped_conv_backward")(go, *ws, x, w, b, K, it),
+           getattr(C, name + "mapped_transposed_conv_forward")(xt, *ws, wt, bt, H, W, K, it),
+           *getattr(C, name + "mapped_transposed_conv_backward")(got, *ws, xt, wt, bt, K, it)]
+    for what, n, o, f in zip(("forward", "dInput", "dW", "dBias", "t forward", "t dInput", "t dW", "t dBias"), new, old, ref):
+        assert _rel(n, f) <= 1.25 * _rel(o, f) + 5e-8, (what, _rel(n, f), _rel(o, f))
+    assert capi.device_status() == 0
+
+
+def test_cancellation_and_one_sided_sums():
+    """Sums of one sign (where truncating accumulation would drift) and sums that cancel."""
+    import _spherical_distortion_ext._C as C
+    from sphmap import capi
+    g = torch.Generator().manual_seed(7)
+    B, ci, co, H, W, K = 2, 256, 64, 16, 64, 9
+    m = (torch.rand(H, W, K, 2, generator=g) * torch.tensor([W - 1.0, H - 1.0])).cuda()
+    for sign in ("positive", "alternating"):
+        x, w, go = (torch.rand(*s, generator=g).cuda() + 0.5 for s in ((B, ci, H, W), (co, ci, K), (B, co, H, W)))
+        if sign == "alternating":
+            w[:, ::2] *= -1
+            go[..., ::2] *= -1
+        b = torch.zeros(co, device="cuda")
+        it = C.InterpolationType(1)
+        new = [C.mapped_conv_forward(x, m, w, b, K, it), *C.mapped_conv_backward(go, m, x, w, b, K, it)]
+        def simt(x, m, w, b, go):
+            plan = capi.plan_build(m, None, H * W, K, 1, H, W)
+            return [capi.conv_forward(x, m, w, b, K, 1), capi.conv_backward_input(go, plan, w, H, W, K), *capi.conv_backward_weight(go, x, m, K, 1)]
+        old, ref = simt(x, m, w, b, go), simt(*(t.double() for t in (x, m, w, b, go)))
+        for what, n, o, f in zip(("forward", "dInput", "dW"), new, old, ref):
+            assert _rel(n, f) <= 1.25 * _rel(o, f) + 5e-8, (sign, what, _rel(n, f), _rel(o, f))
