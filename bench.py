@@ -267,6 +267,7 @@ def run_encoder(args, rank, local, world):
             torch.cuda.current_stream().wait_event(staged["ev"])
             xb = staged["x"]
             xb.record_stream(torch.cuda.current_stream())
+            xb.requires_grad_(True)   # the step counts dInput of every layer, the first one's included
             stage_next()
             h = xb
             for m, sm in zip(mods, maps):

@@ -391,7 +391,8 @@ int sph_mapped_conv_relu_backward_weight(const void *gout, const void *act_out, 
  *       (ext_modules/include/layers/mapped_convolution_layer.h:89-134):
  *       grad_output is read once and converted for both consumers; act_out
  *       (or NULL) is the fused ReLU's output whose sign masks it; x_cl (or
- *       NULL) the companion of x.  Workspace: op SPH_CONV_BACKWARD.  Returns
+ *       NULL) the companion of x; gx (and plan) NULL: an input that takes no
+ *       gradient.  Workspace: op SPH_CONV_BACKWARD.  Returns
  *       SPH_ERR_UNSUPPORTED before launching anything for shapes that do not
  *       run on tensor-core kernels (exact precision; thin layers whose
  *       tensor-core form does not apply): use the separate entry points

@@ -323,7 +323,7 @@ extern "C" int sph_mapped_conv_backward_cl(const void *gout, const void *act_out
   const Dims d{B, Cin, Cout, IH, IW, OH, OW, K, P};
   const int rc = check_dims(d, dtype, interp, precision);
   if (rc != SPH_OK) return rc;
-  if (!gout || !x || !plan || !map || !weight || !gx || !gw || !gb || (P > 0 && !iw)) return SPH_ERR_INVALID_ARGUMENT;
+  if (!gout || !x || (gx && !plan) || !map || !weight || !gw || !gb || (P > 0 && !iw)) return SPH_ERR_INVALID_ARGUMENT;
   if (precision != SPH_PRECISION_BF16 || B == 0) return SPH_ERR_UNSUPPORTED;
   if (tc_thin_backward_ok(Cin, K, Cout, OH * OW)) {
     const int rt = tc_thin_conv_backward(gout, act_out, x, plan, map, iw, weight, gx, gw, gb, B, Cin, Cout, IH, IW, OH, OW, K, P, interp, ws,

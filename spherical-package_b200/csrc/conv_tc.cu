@@ -1974,18 +1974,20 @@ int tc_conv_backward(const void *gout, const void *x, const void *plan, const vo
   } phase_scope;
   mark_phase(0, st);
   // the zero pixel behind every image of the channels-last copy (unused taps point there)
-  if (cudaMemset2DAsync((char *)go_cl + npix * cp_go * 2, (npix + 1) * cp_go * 2, 0, (size_t)cp_go * 2, (size_t)B, st) != cudaSuccess)
+  if (gx && cudaMemset2DAsync((char *)go_cl + npix * cp_go * 2, (npix + 1) * cp_go * 2, 0, (size_t)cp_go * 2, (size_t)B, st) != cudaSuccess)
     return SPH_ERR_CUDA;
   grad_image_kernel<<<dim3(d.tiles_x * d.tiles_y, d.mbs_total, (unsigned)B), 256, 0, st>>>(
       (const float *)gout, gt, (int)Cout, (int)OH, (int)OW, d.tiles_x, d.tiles_y, d.mbs_total, row_part, (const float *)fz.mask,
-      go_cl, cp_go);
+      gx ? go_cl : nullptr, cp_go);  // (the copy serves the input gradient only)
   note_launches(1);
   mark_phase(1, st);
   // channels between mbs_total * 128 and cp_go do not exist (cp_go <= mbs_total * 128), so the copy is complete
   Fusion fx;
   fx.src_cl = go_cl;  // already masked
-  int rc = tc_gemm(true, gout, nullptr, nullptr, plan, Cout, OH, OW, K, 0, IH, IW, 0, weight, K, Cin * K, 1, nullptr, gx, Cin, B,
-                   ws_dx, dx_bytes, st, fx);
+  int rc = SPH_OK;
+  if (gx)
+    rc = tc_gemm(true, gout, nullptr, nullptr, plan, Cout, OH, OW, K, 0, IH, IW, 0, weight, K, Cin * K, 1, nullptr, gx, Cin, B, ws_dx,
+                 dx_bytes, st, fx);
   if (rc != SPH_OK) return rc;
   mark_phase(2, st);
   Fusion fw;

@@ -6,8 +6,11 @@
 // every addition off toward zero (measured on B200: 144 additions of one sign lose 6.6e-6 of the sum, where a chain of
 // float32 multiply-adds is off by 7e-7).  So
 //   - the large products h*h go to an accumulator of their own, which takes at most kSeg chunks (64 columns, four additions)
-//     before warps of the epilogue add it, round to nearest, to float32 registers; two such accumulators alternate;
+//     before the epilogue warps add it, round to nearest, to float32 sums (kept in tensor memory); two such accumulators
+//     alternate;
 //   - the five small ones share a second accumulator for the whole tile: its losses are 2^-8 of the large one's.
+// (Tiles of one segment need no sums: their columns are the small products' second buffer, and the next tile's products run
+// while this one's results are stored.)
 // The result is at least as close to the exact sum as the SIMT kernels' (conv_simt.cu; tests/test_conv_x3_gpu.py compares
 // both with float64).  An infinite operand gives NaN where float32 arithmetic could have kept an infinity.
 //
@@ -36,14 +39,16 @@ using namespace tc;
 
 constexpr int kCols = 32;                               // GEMM columns per chunk
 constexpr int kPix = 128, kTileW = 16, kTileH = 8;      // pixels of a tile: 8 rows of 16
-constexpr int kEpi = 8, kProd = 8;                      // epilogue and producer warps
+constexpr int kEpi = 4, kProd = 16;                     // epilogue and producer warps
 constexpr int kThreads3 = 32 * (kEpi + 1 + kProd);
 constexpr int kProd0 = 32 * (kEpi + 1);                 // first producer thread
-constexpr int kSeg = 2;                                 // chunks per large-product segment
+constexpr int kSeg = 2;                                 // chunks per segment of large products; tiles of at most kOneSeg chunks
+constexpr int kOneSeg = 4;                              // (the multiply-first product) are one segment
 constexpr int kPartA = kPix * 64;                       // bytes of one part of a 128-row x 32-column operand tile
 constexpr int kNMax = 128;
 constexpr size_t kSmemMax = 227 * 1024;
-constexpr uint32_t kHh = 0, kCorr = 256;                // tensor memory columns: large products (2 x 128), small ones (2 x 128)
+// tensor memory columns: large products of a segment (two buffers of 128), small products, float32 sums of finished segments
+constexpr uint32_t kHh = 0, kCorr = 256, kSum = 384;
 
 enum { SRC_MAP1 = 0, SRC_MAP4 = 1, SRC_PLAN = 2, SRC_SELF = 3 };
 
@@ -305,46 +310,41 @@ __device__ __forceinline__ void issue_step(uint32_t hh, uint32_t corr, uint64_t 
   }
 }
 
-// An epilogue warp's share of the accumulators: lanes 32 * (warp & 3) .., columns [col0, col0 + 16 * nb16) of at most 64.
-struct EpiSlice {
-  uint32_t lane_addr;
-  int col0, nb16;
-  __device__ __forceinline__ EpiSlice(uint32_t tmem_base, int warp, int ncols) {
-    const int per = (ncols + 31) / 32 * 16;  // columns of the first half
-    const int half = warp >> 2;
-    col0 = half * per;
-    nb16 = half == 0 ? per / 16 : (ncols - per + 15) / 16;
-    lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + col0;
-  }
-  __device__ __forceinline__ void add(float (&acc)[64], uint32_t col) const {
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      if (i < nb16) {
-        uint32_t r[16];
-        tmem_ld_32x16(lane_addr + col + i * 16, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 16; j++) acc[i * 16 + j] = __fadd_rn(acc[i * 16 + j], __uint_as_float(r[j]));
-      }
-    }
-  }
-};
-
-// Sums of one tile: `nseg` segments, then the small products.  False if a wait gave up.
-__device__ __forceinline__ bool drain_tile(const Bars &b, const EpiSlice &e, float (&acc)[64], int nseg, int &sg, int tl, int lane) {
-#pragma unroll
-  for (int j = 0; j < 64; j++) acc[j] = 0.0f;
+// One tile's sums in an epilogue warp (lanes 32 * warp ..): every finished segment of large products is added to the running
+// sums in tensor memory; with the last one the small products join and the 16-column blocks go to `put(first column, values)`.
+// `sg` counts segments over all tiles; `cb`: the small products' buffer.  False if a wait gave up.
+template <class Put>
+__device__ __forceinline__ bool drain_tile(const Bars &b, uint32_t lane_addr, int ncols, int nseg, int &sg, int lane, int cb, Put put) {
   for (int s = 0; s < nseg; s++, sg++) {
     const int buf = sg & 1;
     if (!mbar_wait(b.seg_full + buf, (sg >> 1) & 1, b.abort_flag)) return false;
     tc_fence_after();
-    e.add(acc, kHh + buf * 128);
-    if (s + 1 == nseg) e.add(acc, kCorr + (tl & 1) * 128);  // (its last product was committed with this segment)
+    const bool last = s + 1 == nseg;
+    for (int c = 0; c < ncols; c += 16) {
+      uint32_t r[16], t[16], u[16];
+      tmem_ld_32x16(lane_addr + kHh + buf * 128 + c, r);
+      if (s > 0) tmem_ld_32x16(lane_addr + kSum + c, t);
+      if (last) tmem_ld_32x16(lane_addr + kCorr + cb * 128 + c, u);
+      tmem_ld_wait();
+      if (s > 0) {
+#pragma unroll
+        for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(t[j]), __uint_as_float(r[j])));
+      }
+      if (last) {  // (the small products' last one was committed with this segment)
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; j++) v[j] = __fadd_rn(__uint_as_float(r[j]), __uint_as_float(u[j]));
+        put(c, v);
+      } else {
+        tmem_st_32x16(lane_addr + kSum + c, r);
+      }
+    }
+    if (!last) tmem_st_wait();
     tc_fence_before();
     __syncwarp();
     if (lane == 0) {
       mbar_arrive(b.seg_empty + buf);
-      if (s + 1 == nseg) mbar_arrive(b.corr_empty + (tl & 1));
+      if (last) mbar_arrive(b.corr_empty + cb);
     }
   }
   return true;
@@ -391,29 +391,36 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
                                                                                      : g.K * kPix * (SRC == SRC_PLAN ? 40 : 32)) + 15) / 16 * 16, S);
   const uint32_t tmem = start_block(bars, S, tid);
   const int tiles_per_image = p.tiles_x * p.tiles_y, total = p.B * tiles_per_image * p.nblk, npix = g.GH * g.GW;
-  const int nseg = (p.nchunks + kSeg - 1) / kSeg;
+  const int seg = p.nchunks <= kOneSeg ? kOneSeg : kSeg, nseg = (p.nchunks + seg - 1) / seg;
+  const int nc = nseg == 1 ? 2 : 1;  // buffers of the small products
 
   if (warp < kEpi) {
-    const EpiSlice e(tmem, warp, p.Npb);
     int sg = 0, tl = 0;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x, tl++) {
       const int nb = tile % p.nblk, rest = tile / p.nblk, b = rest / tiles_per_image, t2 = rest % tiles_per_image;
-      const int pix = tile_pixel3((warp & 3) * 32 + lane, t2 / p.tiles_x, t2 % p.tiles_x, g.GH, g.GW);
-      float acc[64];
-      if (!drain_tile(bars, e, acc, nseg, sg, tl, lane)) break;
-      if (pix < 0) continue;
-      const int n0 = nb * p.Npb + e.col0;
-      float *o = p.out + ((size_t)b * p.Nout + n0) * npix + pix;
+      const int pix = tile_pixel3(warp * 32 + lane, t2 / p.tiles_x, t2 % p.tiles_x, g.GH, g.GW);
+      const int n0 = nb * p.Npb;
+      float *out = p.out + ((size_t)b * p.Nout + n0) * npix + pix;
+      const bool ok = drain_tile(bars, tmem + ((uint32_t)(warp * 32) << 16), p.Npb, nseg, sg, lane, nc == 2 ? tl & 1 : 0,
+                                 [&](int c, float (&v)[16]) {
+        if (pix < 0) return;
+        const int left = p.Nout - n0 - c;
+        if (p.bias) {
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        if (i < e.nb16) {
-#pragma unroll
-          for (int j = 0; j < 16; j++, o += npix) {
-            const int n = n0 + i * 16 + j;
-            if (n < p.Nout && e.col0 + i * 16 + j < p.Npb) *o = acc[i * 16 + j] + (p.bias ? __ldg(p.bias + n) : 0.0f);
-          }
+          for (int j = 0; j < 16; j++)
+            if (j < left) v[j] += __ldg(p.bias + n0 + c + j);
         }
-      }
+        float *o = out + (size_t)c * npix;
+        if (left >= 16) {
+#pragma unroll
+          for (int j = 0; j < 16; j++, o += npix) *o = v[j];
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; j++, o += npix)
+            if (j < left) *o = v[j];
+        }
+      });
+      if (!ok) break;
     }
   } else if (warp == kEpi) {
     if (lane == 0) {
@@ -422,10 +429,10 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
       Ring3 ring;
       bool alive = true;
       for (int tile = blockIdx.x; alive && tile < total; tile += gridDim.x, tl++) {
-        const int cb = tl & 1;
-        if (!mbar_wait(bars.corr_empty + cb, ((tl >> 1) & 1) ^ 1, bars.abort_flag)) break;
+        const int cb = nc == 2 ? tl & 1 : 0, use = nc == 2 ? tl >> 1 : tl;  // this buffer's use count
+        if (!mbar_wait(bars.corr_empty + cb, (use & 1) ^ 1, bars.abort_flag)) break;
         for (int chunk = 0; chunk < p.nchunks; chunk++, ring.next(S)) {
-          const bool first = chunk % kSeg == 0;
+          const bool first = chunk % seg == 0;
           const int buf = sg & 1;
           if (first && !mbar_wait(bars.seg_empty + buf, ((sg >> 1) & 1) ^ 1, bars.abort_flag)) { alive = false; break; }
           if (!mbar_wait(bars.full + ring.s, ring.ph, bars.abort_flag)) { alive = false; break; }
@@ -434,7 +441,7 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
           issue_step(tmem + kHh + buf * 128, tmem + kCorr + cb * 128, smem_desc_sw64(a), smem_desc_sw64(bw), kPartA >> 4,
                      (uint32_t)p.Npb * 4u, 2, 2, idesc, first, chunk == 0);
           umma_commit(bars.empty + ring.s);
-          if (chunk % kSeg == kSeg - 1 || chunk + 1 == p.nchunks) {
+          if (chunk % seg == seg - 1 || chunk + 1 == p.nchunks) {
             umma_commit(bars.seg_full + buf);
             sg++;
           }
@@ -442,13 +449,11 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
       }
     }
   } else {
-    // producers: thread = vector v (8 columns) of pixels px and px + 64
+    // producers: thread = vector v (8 columns) of pixel px
     const int pt = tid - kProd0, v = pt & 3, px = pt >> 2;
     const uint32_t pitch = (uint32_t)g.Cp * 4u;
     const size_t image = (size_t)(g.SH * g.SW + 1) * pitch;
-    uint32_t dst[2];
-#pragma unroll
-    for (int i = 0; i < 2; i++) dst[i] = stage0 + (px + 64 * i) * 64 + ((v ^ (((px + 64 * i) >> 1) & 3)) << 4);
+    const uint32_t dst = stage0 + px * 64 + ((v ^ ((px >> 1) & 3)) << 4);
     PlanView<float> pv{};
     bool plan_ok = true;
     if (SRC == SRC_PLAN) pv = plan_view<float>(g.plan, npix * g.K, plan_ok);
@@ -462,38 +467,33 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
       fill_taps3<SRC>(g, taps, pv, plan_ok, 0, g.K, ty, tx, pt);
       producer_bar3();
       if (!alive) continue;
-      uint32_t self[2] = {0u, 0u};
+      uint32_t self = 0u;
       if (SRC == SRC_SELF) {
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-          const int q = tile_pixel3(px + 64 * i, ty, tx, g.GH, g.GW);
-          self[i] = (uint32_t)(q >= 0 ? q : g.SH * g.SW) * pitch;
-        }
+        const int q = tile_pixel3(px, ty, tx, g.GH, g.GW);
+        self = (uint32_t)(q >= 0 ? q : g.SH * g.SW) * pitch;
       }
-      Item<SRC> it[2];
+      Item<SRC> it;
       int slot, c0;
       chunk_item3(g.Cp, g.K, 0, v, slot, c0);
-      const auto load = [&]() {
-        if (slot < g.K) {
-#pragma unroll
-          for (int i = 0; i < 2; i++) item_load<SRC>(it[i], taps, img + c0 * 4, slot * kPix + px + 64 * i, self[i]);
-        }
-      };
-      load();
+      if (slot < g.K) item_load<SRC>(it, taps, img + c0 * 4, slot * kPix + px, self);
       for (int chunk = 0; chunk < p.nchunks; chunk++, ring.next(S)) {
-        V8 val[2];
+        V8 val;
+        if (slot < g.K) {
+          val = item_value<SRC>(it, taps, pv, img + c0 * 4, slot * kPix + px, pitch);
+        } else {
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-          if (slot < g.K) {
-            val[i] = item_value<SRC>(it[i], taps, pv, img + c0 * 4, slot * kPix + px + 64 * i, pitch);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; j++) val[i].f[j] = 0.0f;
-          }
+          for (int j = 0; j < 8; j++) val.f[j] = 0.0f;
         }
         if (chunk + 1 < p.nchunks) {  // the next chunk's loads are in flight while this one is split, stored and handed over
-          chunk_item3(g.Cp, g.K, chunk + 1, v, slot, c0);
-          load();
+          if (g.Cp >= kCols) {        // (chunk_item3 without its division)
+            if (++slot == g.K) {
+              slot = 0;
+              c0 += kCols;
+            }
+          } else {
+            chunk_item3(g.Cp, g.K, chunk + 1, v, slot, c0);
+          }
+          if (slot < g.K) item_load<SRC>(it, taps, img + c0 * 4, slot * kPix + px, self);
         }
         if (!mbar_wait(bars.empty + ring.s, ring.ph ^ 1u, bars.abort_flag)) { alive = false; break; }
         if (pt == 0) {
@@ -501,8 +501,7 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
           bulk_copy_g2s(base + (size_t)ring.s * stage_bytes + 3 * kPartA, (const char *)p.wp + ((size_t)nb * p.nchunks + chunk) * bbytes,
                         bbytes, bars.full + ring.s);
         }
-#pragma unroll
-        for (int i = 0; i < 2; i++) store_parts(dst[i] + ring.s * stage_bytes, kPartA, val[i]);
+        store_parts(dst + ring.s * stage_bytes, kPartA, val);
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(bars.full + ring.s);
@@ -555,14 +554,13 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_dw_kernel(const Dw3 p) {
   const int nseg = (hi - lo) * 4 / kSeg;
 
   if (warp < kEpi) {
-    const EpiSlice e(tmem, warp, kDwN);
     int sg = 0;
-    float acc[64];
-    drain_tile(bars, e, acc, nseg, sg, 0, lane);
-    const int row = mb * 128 + (warp & 3) * 32 + lane;
-    float *o = p.partial + ((size_t)split * p.mbs * 128 + row) * (p.groups * kDwN) + grp * kDwN + e.col0;
+    float *o = p.partial + ((size_t)split * p.mbs * 128 + mb * 128 + warp * 32 + lane) * (p.groups * kDwN) + grp * kDwN;
+    const auto put = [&](int c, const float (&v)[16]) {
 #pragma unroll
-    for (int j = 0; j < 64; j += 4) *(float4 *)(o + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+      for (int j = 0; j < 16; j += 4) *(float4 *)(o + c + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    };
+    drain_tile(bars, tmem + ((uint32_t)(warp * 32) << 16), kDwN, nseg, sg, lane, 0, put);
   } else if (warp == kEpi) {
     if (lane == 0) {
       const uint32_t idesc = idesc_bf16(128, kDwN, 0, 1);
@@ -582,61 +580,50 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_dw_kernel(const Dw3 p) {
       }
     }
   } else {
-    // producers: thread = vector v (8 of the group's 128 columns) of pixels px and px + 16 of the step
+    // producers: thread = vector v (8 of the group's 128 columns) of pixel px of the step
     const int pt = tid - kProd0, v = pt & 15, px = pt >> 4;
     const uint32_t pitch = (uint32_t)g.Cp * 4u;
     const size_t image = (size_t)(g.SH * g.SW + 1) * pitch;
     const int s0 = grp * kDwN / g.Cp, col = grp * kDwN + v * 8, slot = col / g.Cp, c0 = col - slot * g.Cp;
     const bool have = slot < g.K;
-    const int row0 = have ? (slot - s0) * kPix : 0;
-    uint32_t dst[2];
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const int q = px + 16 * i;
-      dst[i] = stage0 + kStepA + (v >> 3) * (kDwPix3 * 128) + q * 128 + (((v & 7) ^ (q & 7)) << 4);
-    }
+    const int row0 = have ? (slot - s0) * kPix + px : 0;
+    const uint32_t dst = stage0 + kStepA + (v >> 3) * (kDwPix3 * 128) + px * 128 + (((v & 7) ^ (px & 7)) << 4);
     const uint32_t table0 = stage0 + S * stage_bytes, table_pitch = (table_bytes + 15) / 16 * 16;
     const PlanView<float> none{};
-    const auto fill = [&](int tile, int buf) {
-      const int t2 = tile % tiles_per_image;
+    const auto fill = [&](int t2, int buf) {
       fill_taps3<SRC>(g, TapTable<SRC>(table0 + buf * table_pitch, p.slots), none, true, s0, p.slots, t2 / p.tiles_x, t2 % p.tiles_x, pt);
     };
-    if (lo < hi) fill(lo, 0);
+    int image_of = lo / tiles_per_image, t2 = lo - image_of * tiles_per_image;  // image and tile of `tile`
+    if (lo < hi) fill(t2, 0);
     Ring3 ring;
     bool alive = true;
     for (int tile = lo; tile < hi; tile++) {
       const TapTable<SRC> taps(table0 + ((tile - lo) & 1) * table_pitch, p.slots);
-      const char *img = g.xl + (size_t)(tile / tiles_per_image) * image + c0 * 4;
+      const char *img = g.xl + (size_t)image_of * image + c0 * 4;
+      if (++t2 == tiles_per_image) {
+        t2 = 0;
+        image_of++;
+      }
       producer_bar3();  // this tile's table is complete, the other one no longer read
-      Item<SRC> it[2];
-      const auto load = [&](int q) {
-        if (have) {
-#pragma unroll
-          for (int i = 0; i < 2; i++) item_load<SRC>(it[i], taps, img, row0 + q * kDwPix3 + px + 16 * i, 0u);
-        }
-      };
-      if (alive) load(0);
-      if (tile + 1 < hi) fill(tile + 1, (tile + 1 - lo) & 1);
+      Item<SRC> it;
+      if (alive && have) item_load<SRC>(it, taps, img, row0, 0u);
+      if (tile + 1 < hi) fill(t2, (tile + 1 - lo) & 1);
       for (int q = 0; alive && q < 4; q++, ring.next(S)) {
-        V8 val[2];
+        V8 val;
+        if (have) {
+          val = item_value<SRC>(it, taps, none, img, 0, pitch);
+        } else {
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-          if (have) {
-            val[i] = item_value<SRC>(it[i], taps, none, img, 0, pitch);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; j++) val[i].f[j] = 0.0f;
-          }
+          for (int j = 0; j < 8; j++) val.f[j] = 0.0f;
         }
-        if (q < 3) load(q + 1);
+        if (q < 3 && have) item_load<SRC>(it, taps, img, row0 + (q + 1) * kDwPix3, 0u);
         if (!mbar_wait(bars.empty + ring.s, ring.ph ^ 1u, bars.abort_flag)) { alive = false; break; }
         if (pt == 0) {
           mbar_arrive_expect_tx(bars.full + ring.s, kStepA);
           bulk_copy_g2s(base + (size_t)ring.s * stage_bytes, (const char *)p.gt + (((size_t)tile * p.mbs + mb) * 4 + q) * kStepA, kStepA,
                         bars.full + ring.s);
         }
-#pragma unroll
-        for (int i = 0; i < 2; i++) store_parts(dst[i] + ring.s * stage_bytes, kPartB3, val[i]);
+        store_parts(dst + ring.s * stage_bytes, kPartB3, val);
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(bars.full + ring.s);
@@ -804,8 +791,10 @@ int source3(bool use_plan, int64_t P, int interp) {
 size_t table3(int src, int ns) {
   return src == SRC_SELF ? 0 : (size_t)ns * kPix * (src == SRC_MAP1 ? 4 : src == SRC_PLAN ? 40 : 32);
 }
-// Three stages where they leave the L1 about 90 KB, else two.
-constexpr size_t kSmemSoft = 140 * 1024;
+// Three stages where they leave the L1 about 70 KB, else two (64 -> 128 channels, 8 x 128 x 256: bilinear forward 348 us with two
+// stages of 48 KB and 36 KB of taps, 355 with three; its input gradient, 36 KB stages, 681 with two, 662 with three).  The
+// weight gradient, whose tap tables are small, takes three (350 -> 310 us).
+constexpr size_t kSmemSoft = 160 * 1024;
 
 struct GemmPlan3 {
   int Cp, nchunks, Npb, nblk, stages;
@@ -860,7 +849,7 @@ DwPlan3 dw_plan3(int src, int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t
   const int64_t tiles = B * d.tiles_x * d.tiles_y;
   int64_t s = sms3() / ((int64_t)d.groups * d.mbs);
   d.splits = (int)(s < 1 ? 1 : s > tiles ? tiles : s);
-  d.stages = 2;
+  d.stages = 3;
   d.smem = 1024 + (size_t)d.stages * (kStepA + kStepB) + 2 * align_up(table3(src, d.slots), 16) + bars_bytes(d.stages);
   d.xl_bytes = align_up((size_t)(B * (SHW + 1)) * d.Cp * 4, 256);
   d.gt_bytes = align_up((size_t)tiles * d.mbs * 4 * kStepA, 256);

@@ -10,6 +10,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/functions/utils.h>
 
 #include <algorithm>
 #include <cstdlib>
@@ -645,7 +646,7 @@ torch::Tensor conv_forward_impl(torch::Tensor x, torch::Tensor map, const torch:
 
 std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor map, const torch::Tensor *iw, torch::Tensor x,
                                               torch::Tensor weight, torch::Tensor bias, int64_t K, InterpolationType it,
-                                              const torch::Tensor *act_out = nullptr) {
+                                              const torch::Tensor *act_out = nullptr, bool need_gx = true) {
   TORCH_CHECK(x.dim() == 4 && go.dim() == 4 && weight.dim() == 3, "input/grad_output (B,C,H,W), weight (Cout,Cin,K)");
   go = go.contiguous();  // the reference never checks grad_output; make it dense here
   check(x, "input", x);
@@ -661,8 +662,11 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
   c10::cuda::CUDAGuard guard(x.device());
   const ConvArgs a{x.size(0), x.size(1), weight.size(0), x.size(2), x.size(3), m.H, m.W, K, m.P, dtype_of(x), (int)it,
                    dtype_of(x) == SPH_F32 ? precision() : SPH_PRECISION_EXACT};
-  torch::Tensor gx = torch::empty_like(x), gw = torch::empty_like(weight), gb = torch::empty({a.Cout}, x.options());
-  torch::Tensor plan = get_plan(map, iw, a.OH * a.OW, a.K, a.P, a.interp, a.IH, a.IW);
+  torch::Tensor gw = torch::empty_like(weight), gb = torch::empty({a.Cout}, x.options()), gx, plan;
+  if (need_gx) {  // (an input that takes no gradient, a batch of images, leaves its share out)
+    gx = torch::empty_like(x);
+    plan = get_plan(map, iw, a.OH * a.OW, a.K, a.P, a.interp, a.IH, a.IW);
+  }
   if (act_out)
     TORCH_CHECK(act_out->is_contiguous() && act_out->sizes() == go.sizes() && act_out->dtype() == go.dtype() &&
                     act_out->device() == go.device(),
@@ -675,9 +679,9 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
     if (wbc > 0) {
       torch::Tensor wsc = workspace(wbc, x);
       const int rc = sph_mapped_conv_backward_cl(go.data_ptr(), act_out ? act_out->data_ptr() : nullptr, x.data_ptr(),
-                                                 find_companion(x), plan.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr,
-                                                 weight.data_ptr(), gx.data_ptr(), gw.data_ptr(), gb.data_ptr(), a.B, a.Cin, a.Cout,
-                                                 a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec, wsc.data_ptr(), wbc,
+                                                 find_companion(x), need_gx ? plan.data_ptr() : nullptr, map.data_ptr(), iw ? iw->data_ptr() : nullptr,
+                                                 weight.data_ptr(), need_gx ? gx.data_ptr() : nullptr, gw.data_ptr(), gb.data_ptr(), a.B,
+                                                 a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec, wsc.data_ptr(), wbc,
                                                  stream());
       if (rc != SPH_ERR_UNSUPPORTED) {
         ok(rc, "sph_mapped_conv_backward_cl");
@@ -686,14 +690,14 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
       }
     }
   }
-  size_t wb = sph_conv_workspace_preferred_bytes(SPH_CONV_BACKWARD_INPUT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
+  size_t wb = !need_gx ? 0 : sph_conv_workspace_preferred_bytes(SPH_CONV_BACKWARD_INPUT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
                                        a.dtype, a.interp, a.prec);
   torch::Tensor ws = workspace(wb, x);
   size_t wb2 = sph_conv_workspace_preferred_bytes(SPH_CONV_BACKWARD_WEIGHT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
                                         a.interp, a.prec);
   torch::Tensor ws2 = workspace(wb2, x);
   if (act_out) {  // gradient of the fused ReLU: the kernels read grad_output * (act_out > 0)
-    const int rc = sph_mapped_conv_relu_backward_input(go.data_ptr(), act_out->data_ptr(), plan.data_ptr(), weight.data_ptr(),
+    const int rc = !need_gx ? SPH_OK : sph_mapped_conv_relu_backward_input(go.data_ptr(), act_out->data_ptr(), plan.data_ptr(), weight.data_ptr(),
                                                        gx.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.dtype,
                                                        a.prec, ws.data_ptr(), wb, stream());
     // The two fused operators are eligible independently (the weight-gradient kernel's tap table is smaller than the
@@ -722,9 +726,10 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
       return {gx, gw, gb};
     }
   }
-  ok(sph_mapped_conv_backward_input(go.data_ptr(), plan.data_ptr(), weight.data_ptr(), gx.data_ptr(), a.B, a.Cin, a.Cout,
-                                    a.IH, a.IW, a.OH, a.OW, a.K, a.dtype, a.prec, ws.data_ptr(), wb, stream()),
-     "sph_mapped_conv_backward_input");
+  if (need_gx)
+    ok(sph_mapped_conv_backward_input(go.data_ptr(), plan.data_ptr(), weight.data_ptr(), gx.data_ptr(), a.B, a.Cin, a.Cout,
+                                      a.IH, a.IW, a.OH, a.OW, a.K, a.dtype, a.prec, ws.data_ptr(), wb, stream()),
+       "sph_mapped_conv_backward_input");
   wb = wb2;
   ok(sph_mapped_conv_backward_weight(go.data_ptr(), x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr,
                                      gw.data_ptr(), gb.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
@@ -846,6 +851,184 @@ std::vector<torch::Tensor> weighted_mapped_transposed_conv_backward(torch::Tenso
   return tconv_backward_impl(go, map, &iw, x, w, b, K, it);
 }
 
+// ---- differentiable operators -----------------------------------------------------------------------------------------
+// The functional interface's operators with their autograd nodes on this side of the language boundary: one call from
+// Python per operator, none in backward.  The argument checks of the Python layer are repeated here as a yes or no; a
+// call that fails them returns nothing, and the Python layer then raises its own assertion.
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+using OptTensor = c10::optional<torch::Tensor>;
+
+// spherical_distortion.layer_utils.check_args; in_channels / kernel_size < 0: not checked
+bool args_ok(const torch::Tensor &x, const torch::Tensor &map, const OptTensor &iw, int64_t in_channels, int64_t kernel_size) {
+  const bool k = kernel_size >= 0;
+  const int64_t want = 3 + (k ? 1 : 0) + (iw ? 1 : 0);
+  if (x.dim() != 4 || map.dim() != want || map.size(-1) != 2 || x.scalar_type() != map.scalar_type()) return false;
+  if (iw && (iw->dim() != want - 1 || x.scalar_type() != iw->scalar_type() || map.size(-2) != iw->size(-1))) return false;
+  return (in_channels < 0 || x.size(1) == in_channels) && (!k || map.size(2) == kernel_size);
+}
+bool map_covers(const torch::Tensor &x, const torch::Tensor &map) { return x.size(2) == map.size(0) && x.size(3) == map.size(1); }
+
+// A node's saved tensors (an absent one stays undefined) and the operator's plain arguments.
+struct MapNode : public Node {
+  SavedVariable x, weight, bias, map, iw, out;
+  InterpolationType it = InterpolationType::NEAREST;
+  int64_t K = 0, h = 0, w = 0;
+  bool weighted = false;
+  std::mutex mu;
+
+  void save_map(const torch::Tensor &m, const OptTensor &weights) {
+    map = SavedVariable(m, false);
+    weighted = weights.has_value();
+    if (weighted) iw = SavedVariable(*weights, false);
+  }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mu);
+    for (SavedVariable *v : {&x, &weight, &bias, &map, &iw, &out}) v->reset_data();
+  }
+  variable_list apply(variable_list &&g) override {
+    std::lock_guard<std::mutex> lock(mu);
+    variable_list r(num_outputs());
+    if (!g[0].defined()) return r;
+    at::NoGradGuard no_grad;
+    const torch::Tensor m = map.unpack(), q = weighted ? iw.unpack() : torch::Tensor();
+    gradients(r, g[0], m, weighted ? &q : nullptr);
+    return r;
+  }
+  virtual void gradients(variable_list &r, torch::Tensor go, const torch::Tensor &m, const torch::Tensor *q) = 0;
+};
+
+bool wants_grad(std::initializer_list<const torch::Tensor *> ts) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const torch::Tensor *t : ts)
+    if (t->requires_grad()) return true;
+  return false;
+}
+template <class N> std::shared_ptr<N> new_node(const torch::autograd::edge_list &edges) {
+  std::shared_ptr<N> n(new N(), torch::autograd::deleteNode);
+  n->set_next_edges(torch::autograd::edge_list(edges));
+  return n;
+}
+
+struct MappedConvNode : public MapNode {
+  bool relu = false;
+  std::string name() const override { return "MappedConvolutionBackward"; }
+  void gradients(variable_list &r, torch::Tensor go, const torch::Tensor &m, const torch::Tensor *q) override {
+    const torch::Tensor o = relu ? out.unpack(shared_from_this()) : torch::Tensor();
+    const auto g = conv_backward_impl(go, m, q, x.unpack(), weight.unpack(), bias.unpack(), K, it, relu ? &o : nullptr,
+                                      task_should_compute_output(0));
+    for (int i = 0; i < 3; i++) r[i] = g[i];
+  }
+};
+OptTensor mapped_convolution(const torch::Tensor &x, const torch::Tensor &weight, const torch::Tensor &bias, const torch::Tensor &map,
+                             int64_t K, InterpolationType it, const OptTensor &iw, bool relu) {
+  if (weight.dim() != 3 || !args_ok(x, map, iw, weight.size(1), weight.size(2))) return c10::nullopt;
+  torch::Tensor out;
+  {
+    at::NoGradGuard no_grad;
+    out = conv_forward_impl(x, map, iw ? &*iw : nullptr, weight, bias, K, it, relu);
+  }
+  if (wants_grad({&x, &weight, &bias})) {
+    auto n = new_node<MappedConvNode>(torch::autograd::collect_next_edges(x, weight, bias));
+    n->x = SavedVariable(x, false);
+    n->weight = SavedVariable(weight, false);
+    n->bias = SavedVariable(bias, false);
+    n->save_map(map, iw);
+    n->K = K;
+    n->it = it;
+    n->relu = relu;
+    torch::autograd::set_history(out, n);
+    if (relu) n->out = SavedVariable(out, true);
+  }
+  return out;
+}
+
+struct MappedTransposedConvNode : public MapNode {
+  std::string name() const override { return "MappedTransposedConvolutionBackward"; }
+  void gradients(variable_list &r, torch::Tensor go, const torch::Tensor &m, const torch::Tensor *q) override {
+    const auto g = tconv_backward_impl(go, m, q, x.unpack(), weight.unpack(), bias.unpack(), K, it);
+    for (int i = 0; i < 3; i++) r[i] = g[i];
+  }
+};
+OptTensor mapped_transposed_convolution(const torch::Tensor &x, const torch::Tensor &weight, const torch::Tensor &bias,
+                                        const torch::Tensor &map, int64_t oh, int64_t ow, int64_t K, InterpolationType it,
+                                        const OptTensor &iw) {
+  if (weight.dim() != 3 || !args_ok(x, map, iw, weight.size(0), weight.size(2)) || !map_covers(x, map)) return c10::nullopt;
+  torch::Tensor out;
+  {
+    at::NoGradGuard no_grad;
+    out = tconv_forward_impl(x, map, iw ? &*iw : nullptr, weight, bias, oh, ow, K, it);
+  }
+  if (wants_grad({&x, &weight, &bias})) {
+    auto n = new_node<MappedTransposedConvNode>(torch::autograd::collect_next_edges(x, weight, bias));
+    n->x = SavedVariable(x, false);
+    n->weight = SavedVariable(weight, false);
+    n->bias = SavedVariable(bias, false);
+    n->save_map(map, iw);
+    n->K = K;
+    n->it = it;
+    torch::autograd::set_history(out, n);
+  }
+  return out;
+}
+
+struct MappedMaxPoolNode : public MapNode {
+  std::string name() const override { return "MappedMaxPoolBackward"; }
+  void gradients(variable_list &r, torch::Tensor go, const torch::Tensor &m, const torch::Tensor *q) override {
+    r[0] = max_unpool_impl(go, x.unpack(), m, q, h, w, K, it);   // (x holds the indices)
+  }
+};
+c10::optional<std::tuple<torch::Tensor, torch::Tensor>> max_pool_op(const torch::Tensor &x, const torch::Tensor &map, int64_t K,
+                                                                   InterpolationType it, const OptTensor &iw) {
+  if (!args_ok(x, map, iw, -1, K)) return c10::nullopt;
+  std::vector<torch::Tensor> r;
+  {
+    at::NoGradGuard no_grad;
+    r = max_pool_impl(x, map, iw ? &*iw : nullptr, K, it);
+  }
+  if (wants_grad({&x})) {
+    auto n = new_node<MappedMaxPoolNode>(torch::autograd::collect_next_edges(x));
+    n->x = SavedVariable(r[1], false);
+    n->save_map(map, iw);
+    n->K = K;
+    n->it = it;
+    n->h = x.size(2);
+    n->w = x.size(3);
+    torch::autograd::set_history(r[0], n);
+  }
+  return std::make_tuple(r[0], r[1]);
+}
+
+// Scatter forward, gather backward (Resample), or the other way round (Unresample).
+struct ResampleNode : public MapNode {
+  bool scatter = false;
+  std::string name() const override { return scatter ? "ResampleBackward" : "UnresampleBackward"; }
+  void gradients(variable_list &r, torch::Tensor go, const torch::Tensor &m, const torch::Tensor *q) override {
+    go = go.contiguous();
+    r[0] = scatter ? resample_from_map_impl(go, m, q, it) : resample_to_map_impl(go, m, q, h, w, it);
+  }
+};
+OptTensor resample_op(const torch::Tensor &x, const torch::Tensor &map, InterpolationType it, const OptTensor &iw, bool scatter, int64_t oh,
+                      int64_t ow) {
+  if (!args_ok(x, map, iw, -1, -1) || (scatter && !map_covers(x, map))) return c10::nullopt;
+  torch::Tensor out;
+  {
+    at::NoGradGuard no_grad;
+    out = scatter ? resample_to_map_impl(x, map, iw ? &*iw : nullptr, oh, ow, it) : resample_from_map_impl(x, map, iw ? &*iw : nullptr, it);
+  }
+  if (wants_grad({&x})) {
+    auto n = new_node<ResampleNode>(torch::autograd::collect_next_edges(x));
+    n->save_map(map, iw);
+    n->it = it;
+    n->scatter = scatter;
+    n->h = x.size(2);
+    n->w = x.size(3);
+    torch::autograd::set_history(out, n);
+  }
+  return out;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -859,6 +1042,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .value("BROWN", DistortionType::BROWN)
       .value("FISHEYE", DistortionType::FISHEYE);
 
+  m.def("mapped_convolution_op", &mapped_convolution);
+  m.def("mapped_transposed_convolution_op", &mapped_transposed_convolution);
+  m.def("mapped_max_pool_op", &max_pool_op);
+  m.def("resample_op", &resample_op);
   m.def("resample_to_map", &resample_to_map);
   m.def("resample_from_map", &resample_from_map);
   m.def("weighted_resample_to_map", &weighted_resample_to_map);

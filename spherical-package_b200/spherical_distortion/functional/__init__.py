@@ -4,28 +4,17 @@ Mirrors layers/functional/mapped_convolution.py:121-148,
 layers/functional/mapped_pooling.py:203-245, layers/functional/resample.py:113-219,
 layers/functional/convolution.py:62-71 and the map-driven halves of
 layers/functional/tangent_images.py:6-55 of the reference: the same call
-signatures and assertions, autograd Functions that hand the same positional
-arguments to ``_spherical_distortion_ext`` (integers saved for backward travel
-as 0-d tensors, the interpolation type as an int that is cast back to the
-enum).
+signatures and assertions, on top of ``_spherical_distortion_ext``.
 """
 import torch
 
 import _spherical_distortion_ext._C as _C
 import _spherical_distortion_ext._convolution as _std_conv
 import _spherical_distortion_ext._mapped_avg_pooling as _avgpool
-import _spherical_distortion_ext._mapped_convolution as _conv
-import _spherical_distortion_ext._mapped_max_pooling as _pool
-import _spherical_distortion_ext._mapped_transposed_convolution as _tconv
-import _spherical_distortion_ext._resample as _res
 import _spherical_distortion_ext._transposed_convolution as _std_tconv
 import _spherical_distortion_ext._uv_resample as _uv
 import _spherical_distortion_ext._voting_resample as _vote
 import _spherical_distortion_ext._weighted_mapped_avg_pooling as _wavgpool
-import _spherical_distortion_ext._weighted_mapped_convolution as _wconv
-import _spherical_distortion_ext._weighted_mapped_max_pooling as _wpool
-import _spherical_distortion_ext._weighted_mapped_transposed_convolution as _wtconv
-import _spherical_distortion_ext._weighted_resample as _wres
 
 from ..layer_utils import InterpolationType, check_args, check_input_map_shape
 
@@ -34,154 +23,39 @@ def _scalars(kernel_size, interp):
     return torch.tensor(kernel_size), torch.tensor(int(interp))
 
 
-class _MappedConv(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias, sample_map, kernel_size, interp, interp_weights):
-        ctx.save_for_backward(x, weight, bias, sample_map, *_scalars(kernel_size, interp), interp_weights)
-        if interp_weights is None:
-            return _conv.mapped_conv_forward(x, sample_map, weight, bias, kernel_size, interp)
-        return _wconv.weighted_mapped_conv_forward(x, sample_map, interp_weights, weight, bias, kernel_size, interp)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        x, weight, bias, sample_map, kernel_size, interp, interp_weights = ctx.saved_tensors
-        interp = InterpolationType(interp)
-        if interp_weights is None:
-            gx, gw, gb = _conv.mapped_conv_backward(grad_output, sample_map, x, weight, bias, kernel_size, interp)
-        else:
-            gx, gw, gb = _wconv.weighted_mapped_conv_backward(grad_output, sample_map, interp_weights, x, weight, bias,
-                                                              kernel_size, interp)
-        return gx, gw, gb, None, None, None, None
+def _failed(*check):
+    """The native operator returned nothing: its arguments fail the checks, whose assertions are raised here."""
+    for fn, *args in check:
+        fn(*args)
+    raise AssertionError("arguments do not fit the operator")
 
 
-class _MappedConvReLU(torch.autograd.Function):
-    """relu(mapped_convolution(...)) with the activation fused into the kernels; not in the reference."""
-
-    @staticmethod
-    def forward(ctx, x, weight, bias, sample_map, kernel_size, interp, interp_weights):
-        out = _conv.mapped_conv_relu_forward(x, sample_map, interp_weights, weight, bias, kernel_size, interp)
-        ctx.save_for_backward(x, weight, bias, sample_map, *_scalars(kernel_size, interp), interp_weights, out)
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        x, weight, bias, sample_map, kernel_size, interp, interp_weights, out = ctx.saved_tensors
-        gx, gw, gb = _conv.mapped_conv_relu_backward(grad_output, out, sample_map, interp_weights, x, weight, bias,
-                                                     kernel_size, InterpolationType(interp))
-        return gx, gw, gb, None, None, None, None
-
-
-class _MappedTransposedConv(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias, sample_map, oh, ow, kernel_size, interp, interp_weights):
-        ctx.save_for_backward(x, sample_map, weight, bias, *_scalars(kernel_size, interp), interp_weights)
-        if interp_weights is None:
-            return _tconv.mapped_transposed_conv_forward(x, sample_map, weight, bias, oh, ow, kernel_size, interp)
-        return _wtconv.weighted_mapped_transposed_conv_forward(x, sample_map, interp_weights, weight, bias, oh, ow,
-                                                               kernel_size, interp)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        x, sample_map, weight, bias, kernel_size, interp, interp_weights = ctx.saved_tensors
-        interp = InterpolationType(interp)
-        if interp_weights is None:
-            gx, gw, gb = _tconv.mapped_transposed_conv_backward(grad_output, sample_map, x, weight, bias, kernel_size,
-                                                                interp)
-        else:
-            gx, gw, gb = _wtconv.weighted_mapped_transposed_conv_backward(grad_output, sample_map, interp_weights, x,
-                                                                          weight, bias, kernel_size, interp)
-        return gx, gw, gb, None, None, None, None, None, None
-
-
-class _MappedMaxPool(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, sample_map, kernel_size, interp, interp_weights):
-        if interp_weights is None:
-            pooled, idx_mask = _pool.mapped_max_pool(x, sample_map, kernel_size, interp)
-        else:
-            pooled, idx_mask = _wpool.weighted_mapped_max_pool(x, sample_map, interp_weights, kernel_size, interp)
-        ctx.mark_non_differentiable(idx_mask)
-        ctx.set_materialize_grads(False)  # no zero tensor of the indices' size in every backward pass
-        ctx.save_for_backward(torch.tensor([x.shape[2], x.shape[3]]), idx_mask, sample_map,
-                              *_scalars(kernel_size, interp), interp_weights)
-        return pooled, idx_mask
-
-    @staticmethod
-    def backward(ctx, grad_output, _idx_grad=None):
-        if grad_output is None:
-            return None, None, None, None, None
-        in_shape, idx_mask, sample_map, kernel_size, interp, interp_weights = ctx.saved_tensors
-        interp = InterpolationType(interp)
-        if interp_weights is None:
-            gx = _pool.mapped_max_unpool(grad_output, idx_mask, sample_map, in_shape[0], in_shape[1], kernel_size, interp)
-        else:
-            gx = _wpool.weighted_mapped_max_unpool(grad_output, idx_mask, sample_map, interp_weights, in_shape[0],
-                                                   in_shape[1], kernel_size, interp)
-        return gx, None, None, None, None
-
-
-class _Resample(torch.autograd.Function):
-    """Scatter forward, gather backward (layers/functional/resample.py:11-48)."""
-
-    @staticmethod
-    def forward(ctx, x, sample_map, output_shape, interp, interp_weights):
-        ctx.save_for_backward(sample_map, torch.tensor(int(interp)), interp_weights)
-        if interp_weights is None:
-            return _res.resample_to_map(x, sample_map, output_shape[0], output_shape[1], interp)
-        return _wres.weighted_resample_to_map(x, sample_map, interp_weights, output_shape[0], output_shape[1], interp)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        sample_map, interp, interp_weights = ctx.saved_tensors
-        interp = InterpolationType(interp)
-        grad_output = grad_output.contiguous()
-        if interp_weights is None:
-            return _res.resample_from_map(grad_output, sample_map, interp), None, None, None, None
-        return _wres.weighted_resample_from_map(grad_output, sample_map, interp_weights, interp), None, None, None, None
-
-
-class _Unresample(torch.autograd.Function):
-    """Gather forward, scatter backward (layers/functional/resample.py:51-83)."""
-
-    @staticmethod
-    def forward(ctx, x, sample_map, interp, interp_weights):
-        ctx.save_for_backward(sample_map, torch.tensor(int(interp)), interp_weights)
-        ctx.in_hw = (x.shape[2], x.shape[3])
-        if interp_weights is None:
-            return _res.resample_from_map(x, sample_map, interp)
-        return _wres.weighted_resample_from_map(x, sample_map, interp_weights, interp)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        sample_map, interp, interp_weights = ctx.saved_tensors
-        interp = InterpolationType(interp)
-        grad_output = grad_output.contiguous()
-        h, w = ctx.in_hw
-        if interp_weights is None:
-            return _res.resample_to_map(grad_output, sample_map, h, w, interp), None, None, None
-        return _wres.weighted_resample_to_map(grad_output, sample_map, interp_weights, h, w, interp), None, None, None
-
-
+# The operators' autograd nodes are part of the native extension: one call per operator.
 def mapped_convolution(input, weight, bias, sample_map, kernel_size, interp, interp_weights=None, activation=None):
     """`activation` (None or "relu") is an extension of this library: the ReLU runs inside the convolution kernels
     instead of as separate passes over the output and its gradient."""
-    check_args(input, sample_map, interp_weights, weight.shape[1], weight.shape[2])
     assert activation in (None, "relu"), "activation must be None or 'relu'"
-    fn = _MappedConvReLU if activation == "relu" else _MappedConv
-    return fn.apply(input, weight, bias, sample_map, kernel_size, interp, interp_weights)
+    out = _C.mapped_convolution_op(input, weight, bias, sample_map, kernel_size, interp, interp_weights, activation is not None)
+    if out is None:
+        _failed((check_args, input, sample_map, interp_weights, weight.shape[1], weight.shape[2]))
+    return out
 
 
 def mapped_transposed_convolution(input, weight, bias, sample_map, output_height, output_width, kernel_size, interp,
                                   interp_weights=None):
-    check_args(input, sample_map, interp_weights, weight.shape[0], weight.shape[2])
-    check_input_map_shape(input, sample_map)
-    return _MappedTransposedConv.apply(input, weight, bias, sample_map, output_height, output_width, kernel_size,
-                                       interp, interp_weights)
+    out = _C.mapped_transposed_convolution_op(input, weight, bias, sample_map, output_height, output_width, kernel_size,
+                                              interp, interp_weights)
+    if out is None:
+        _failed((check_args, input, sample_map, interp_weights, weight.shape[0], weight.shape[2]),
+                (check_input_map_shape, input, sample_map))
+    return out
 
 
 def mapped_max_pool(input, sample_map, kernel_size, interp, interp_weights=None):
-    check_args(input, sample_map, interp_weights, None, kernel_size)
-    return _MappedMaxPool.apply(input, sample_map, kernel_size, interp, interp_weights)
+    out = _C.mapped_max_pool_op(input, sample_map, kernel_size, interp, interp_weights)
+    if out is None:
+        _failed((check_args, input, sample_map, interp_weights, None, kernel_size))
+    return out
 
 
 def _with_batch(fn, input, *args):
@@ -192,17 +66,22 @@ def _with_batch(fn, input, *args):
 
 
 def resample(input, sample_map, output_shape, interp, interp_weights=None):
+    """Scatter forward, gather backward (layers/functional/resample.py:11-48)."""
     def run(x):
-        check_args(x, sample_map, interp_weights, None, None)
-        check_input_map_shape(x, sample_map)
-        return _Resample.apply(x, sample_map, output_shape, interp, interp_weights)
+        out = _C.resample_op(x, sample_map, interp, interp_weights, True, output_shape[0], output_shape[1])
+        if out is None:
+            _failed((check_args, x, sample_map, interp_weights, None, None), (check_input_map_shape, x, sample_map))
+        return out
     return _with_batch(run, input)
 
 
 def unresample(input, sample_map, interp, interp_weights=None):
+    """Gather forward, scatter backward (layers/functional/resample.py:51-83)."""
     def run(x):
-        check_args(x, sample_map, interp_weights, None, None)
-        return _Unresample.apply(x, sample_map, interp, interp_weights)
+        out = _C.resample_op(x, sample_map, interp, interp_weights, False, 0, 0)
+        if out is None:
+            _failed((check_args, x, sample_map, interp_weights, None, None))
+        return out
     return _with_batch(run, input)
 
 
