@@ -121,10 +121,7 @@ extern "C" size_t sph_conv_workspace_preferred_bytes(int op, int64_t B, int64_t 
     case SPH_CONV_BACKWARD_WEIGHT: x3 = x3_dw_workspace(B, Cin, IH * IW, K, P, interp, Cout, OH, OW); break;
     case SPH_TCONV_FORWARD: x3 = x3_gemm_workspace(true, B, Cin, IH * IW, K, 0, 0, Cout, OH * OW); break;
     case SPH_TCONV_BACKWARD_INPUT: x3 = x3_gemm_workspace(false, B, Cout, OH * OW, K, P, interp, Cin, 0); break;
-    case SPH_TCONV_BACKWARD_WEIGHT:
-      x3 = x3_dw_workspace(B, Cout, OH * OW, K, P, interp, Cin, IH, IW);
-      if (x3 > 0) x3 += simt_bias_workspace(Cout, 4);
-      break;
+    case SPH_TCONV_BACKWARD_WEIGHT: x3 = x3_dw_workspace(B, Cout, OH * OW, K, P, interp, Cin, IH, IW); break;
     default: break;
   }
   return x3 > base ? x3 : base;
@@ -216,7 +213,7 @@ int conv_backward_weight(const void *gout, const void *x, const void *map, const
     return tc_conv_backward_weight(gout, x, map, iw, gw, gb, B, Cin, Cout, IH, IW, OH, OW, K, P, interp, ws, ws_bytes, st, fz);
   if (fz.active()) return SPH_ERR_UNSUPPORTED;
   if (split_fits(dtype, ws, ws_bytes, x3_dw_workspace(B, Cin, IH * IW, K, P, interp, Cout, OH, OW)))
-    return x3_dw(gout, x, map, iw, Cin, IH, IW, K, P, OH, OW, interp, Cout, B, gw, Cin * K, K, 1, gb, ws, st);
+    return x3_dw(gout, x, map, iw, Cin, IH, IW, K, P, OH, OW, interp, Cout, B, gw, Cin * K, K, 1, gb, false, ws, st);
   return SPH_BY_DTYPE(simt_dw, gout, x, map, iw, Cin, IH, IW, K, P, OH * OW, interp, Cout, B, gw, Cin * K, K, 1, gout, Cout,
                       OH * OW, gb, ws, ws_bytes, st);
 }
@@ -402,11 +399,8 @@ extern "C" int sph_mapped_tconv_backward_weight(const void *gout, const void *x,
                         OH * OW, gb, ws, ws_bytes, st);
   if (precision == SPH_PRECISION_BF16)
     return tc_tconv_backward_weight(gout, x, map, iw, gw, gb, B, Cin, Cout, IH, IW, OH, OW, K, P, interp, ws, ws_bytes, st);
-  const size_t wx = x3_dw_workspace(B, Cout, OH * OW, K, P, interp, Cin, IH, IW), wb = simt_bias_workspace(Cout, 4);
-  if (wx > 0 && split_fits(dtype, ws, ws_bytes, wx + wb)) {  // (the bias gradient sums grad_output, the gathered side)
-    const int rx = x3_dw(x, gout, map, iw, Cout, OH, OW, K, P, IH, IW, interp, Cin, B, gw, Cout * K, K, 1, nullptr, ws, st);
-    return rx == SPH_OK ? simt_bias_grad<float>(gout, B, Cout, OH * OW, gb, (char *)ws + wx, st) : rx;
-  }
+  if (split_fits(dtype, ws, ws_bytes, x3_dw_workspace(B, Cout, OH * OW, K, P, interp, Cin, IH, IW)))
+    return x3_dw(x, gout, map, iw, Cout, OH, OW, K, P, IH, IW, interp, Cin, B, gw, Cout * K, K, 1, gb, true, ws, st);
   return SPH_BY_DTYPE(simt_dw, x, gout, map, iw, Cout, OH, OW, K, P, IH * IW, interp, Cin, B, gw, Cout * K, K, 1, gout, Cout,
                       OH * OW, gb, ws, ws_bytes, st);
 }

@@ -46,10 +46,6 @@ size_t simt_bias_workspace(int64_t C, size_t ts);
 template <typename T>
 int simt_bias_grad(const void *g, int64_t B, int64_t C, int64_t n, void *gb, void *ws, cudaStream_t st);
 
-// out[b][m][q] (+bias) = sum over the plan entries of q of w * T[b][k*M + m][source]
-int simt_plan_gather_planes(const float *T, const void *plan, const void *bias, void *out, int64_t K, int64_t M, int64_t n_src, int64_t n_dst,
-                            int64_t B, cudaStream_t st);
-
 // ---- float32 through three bf16 parts on the tensor cores (conv_x3.cu) ---------------------------------------------
 // The workspace queries return 0 for shapes the kernels do not cover; operands as simt_gemm / simt_dw.
 size_t x3_gemm_workspace(bool use_plan, int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int interp, int64_t Nout, int64_t n_dst);
@@ -58,8 +54,8 @@ int x3_gemm(bool use_plan, const void *src, const void *map, const void *iw, con
             int64_t Nout, int64_t B, void *ws, cudaStream_t st);
 size_t x3_dw_workspace(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int interp, int64_t M, int64_t GH, int64_t GW);
 int x3_dw(const void *A, const void *src, const void *map, const void *iw, int64_t CH, int64_t SH, int64_t SW, int64_t K, int64_t P,
-          int64_t GH, int64_t GW, int interp, int64_t M, int64_t B, void *gw, int64_t sm, int64_t sc, int64_t sk, void *gb, void *ws,
-          cudaStream_t st);
+          int64_t GH, int64_t GW, int interp, int64_t M, int64_t B, void *gw, int64_t sm, int64_t sc, int64_t sk, void *gb, bool bias_of_src,
+          void *ws, cudaStream_t st);
 int x3_wait_status(int reset);  // sticky word of a bounded wait that gave up; < 0: CUDA error
 
 template <typename T>

@@ -751,13 +751,6 @@ __global__ void __launch_bounds__(128) plan_gather_planes_kernel(const float *__
     if (m0 + j < M) out[((size_t)b * M + m0 + j) * n_dst + q] = acc[j] + (bias ? __ldg(bias + m0 + j) : 0.0f);
 }
 
-int simt_plan_gather_planes(const float *T, const void *plan, const void *bias, void *out, int64_t K, int64_t M, int64_t n_src, int64_t n_dst,
-                            int64_t B, cudaStream_t st) {
-  plan_gather_planes_kernel<<<dim3(cdiv(n_dst, 128), cdiv(M, 8), (unsigned)B), 128, 0, st>>>(T, plan, (const float *)bias, (float *)out, (int)K,
-                                                                                           (int)M, (int)n_src, (int)n_dst);
-  return launch_status();
-}
-
 static bool premul_applies(int64_t M, int64_t CH, int64_t K, int64_t n_src, int64_t n_dst, int64_t B) {
   return n_dst >= 3 * n_src && K * M >= 48 && CH >= 16 && (size_t)(B * K * M * n_src) * 4 <= ((size_t)8 << 30);
 }
@@ -816,8 +809,9 @@ int simt_gemm(bool use_plan, const void *src, const void *map, const void *iw, c
       } else {
         conv_gemm128_kernel<COL_IDENT, false, 8><<<dim3(cdiv(n_src, GN), cdiv(MM, GM), (unsigned)B), 256, 0, st>>>(ci, nullptr, 0, 0, 0, nullptr, Tb, MM, wt);
       }
-      const int rc = launch_status(2);
-      return rc == SPH_OK ? simt_plan_gather_planes(Tb, plan, bias, out, K, M, n_src, npix, B, st) : rc;
+      plan_gather_planes_kernel<<<dim3(cdiv(npix, 128), cdiv(M, 8), (unsigned)B), 128, 0, st>>>(Tb, plan, (const float *)bias, (float *)out,
+                                                                                              (int)K, (int)M, (int)n_src, (int)npix);
+      return launch_status(3);
     }
   }
   if (use_plan) {

@@ -354,7 +354,7 @@ struct Gemm3 {
   Src3 g;
   const __nv_bfloat16 *wp;  // weight tile images [nblk][chunk][part][Npb rows][32 columns], 64-byte swizzled
   const float *bias;        // (Nout) or null
-  float *out;               // (B, Nout, GH*GW)
+  float *out;               // (B, Nout, GH*GW); SRC_SELF: rows (B, GH*GW, Nout), Nout a multiple of 8
   int *status;
   int B, Nout, Npb, nblk, nchunks, tiles_x, tiles_y, stages;
 };
@@ -405,6 +405,15 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
                                  [&](int c, float (&v)[16]) {
         if (pix < 0) return;
         const int left = p.Nout - n0 - c;
+        if constexpr (SRC == SRC_SELF) {  // the column buffer of the multiply-first adjoint: this pixel's 16 columns are one 64-byte run
+          float *o = p.out + ((size_t)b * npix + pix) * p.Nout + n0 + c;
+#pragma unroll
+          for (int j = 0; j < 16; j += 8)
+            if (j < left)
+              asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + j), "f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]),
+                           "f"(v[j + 3]), "f"(v[j + 4]), "f"(v[j + 5]), "f"(v[j + 6]), "f"(v[j + 7]) : "memory");
+          return;
+        }
         if (p.bias) {
 #pragma unroll
           for (int j = 0; j < 16; j++)
@@ -640,22 +649,42 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_dw_kernel(const Dw3 p) {
 }
 
 // ---- layout pre-passes ---------------------------------------------------------------------------------------------------
-// (B, C, HW) -> (B, HW + 1, Cp) float32; padding channels and the extra pixel are zero.  32 pixels x 32 channels per block,
-// through shared memory.
-__global__ void __launch_bounds__(256) nchw_to_nhwc_kernel(const float *__restrict__ x, float *__restrict__ y, int C, int Cp, int HW) {
-  __shared__ float tile[32][33];
-  const int b = blockIdx.z, c0 = blockIdx.y * 32, p0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+// (B, C, HW) -> (B, HW + 1, Cp) float32; padding channels and the extra pixel are zero.  128 pixels x 32 channels per block,
+// through shared memory (blocks of 32 x 32 spent half their instructions on finding their place: 41 -> 27 us per 67 MB).  With
+// `sums` every block also leaves its channels' sums over its pixels, sums[(b * px_blocks + block) * Cp + c]: the bias gradient
+// where the gathered side is the output's gradient.
+constexpr int kNhwcPix = 128;
+struct Nhwc3 {
+  const float *x;
+  float *y, *sums;
+  int C, Cp, HW, px_blocks, ch_blocks, blocks;
+};
+using NhwcTile = float[32][kNhwcPix + 1];
+__device__ __forceinline__ void nhwc_block(const Nhwc3 &q, int block, NhwcTile &tile) {
+  const int bp = block % q.px_blocks, bc = block / q.px_blocks % q.ch_blocks, b = block / (q.px_blocks * q.ch_blocks);
+  const int c0 = bc * 32, p0 = bp * kNhwcPix, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    const int c = c0 + ty + 8 * i, p = p0 + tx;
-    tile[ty + 8 * i][tx] = c < C && p < HW ? __ldg(x + ((size_t)b * C + c) * HW + p) : 0.0f;
+    const int c = c0 + ty + 8 * i;
+    const float *x = q.x + ((size_t)b * q.C + c) * q.HW + p0 + tx;
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) v[j] = c < q.C && p0 + tx + 32 * j < q.HW ? __ldg(x + 32 * j) : 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; j++) tile[ty + 8 * i][tx + 32 * j] = v[j];
+    if (q.sums) {
+      float s = (v[0] + v[1]) + (v[2] + v[3]);
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+      if (tx == 0 && c < q.Cp) q.sums[((size_t)b * q.px_blocks + bp) * q.Cp + c] = s;
+    }
   }
   __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int p = p0 + ty + 8 * i, c = c0 + tx;
-    if (p <= HW && c < Cp) y[((size_t)b * (HW + 1) + p) * Cp + c] = tile[tx][ty + 8 * i];
-  }
+  const int c = c0 + tx, np = min(kNhwcPix, q.HW + 1 - p0);
+  if (c >= q.Cp) return;
+  float *y = q.y + ((size_t)b * (q.HW + 1) + p0) * q.Cp + c;
+#pragma unroll 4
+  for (int i = ty; i < np; i += 8) y[(size_t)i * q.Cp] = tile[tx][i];
 }
 
 __device__ __forceinline__ void split3(float x, uint16_t &h, uint16_t &m, uint16_t &l) {
@@ -665,37 +694,60 @@ __device__ __forceinline__ void split3(float x, uint16_t &h, uint16_t &m, uint16
   l = (uint16_t)(__float_as_uint(s) >> 16);
 }
 
-// Weights -> three-part tile images.  Rows n = nb * Npb + row; `premul`: rows are n = k * M + m of the multiply-first adjoint
+// Weights -> three-part tile images.  Rows n = nb * Npb + row; `premul`: rows are n = k * premul + m of the multiply-first adjoint
 // (columns: source channels), else rows are output channels and columns (slot, channel) items.  W[m * sm + ch * sc + k * sk].
-__global__ void weight_image3_kernel(const float *__restrict__ w, uint16_t *__restrict__ wp, int M, int CH, int Cp, int K, int Npb, int nblk,
-                                     int nchunks, int64_t sm, int64_t sc, int64_t sk, int premul) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (int64_t)nblk * nchunks * Npb * kCols) return;
-  const int col = (int)(i % kCols), r = (int)((i / kCols) % Npb), chunk = (int)((i / ((int64_t)kCols * Npb)) % nchunks);
-  const int nb = (int)(i / ((int64_t)kCols * Npb * nchunks)), n = nb * Npb + r;
-  int slot, c0;
+struct Weight3 {
+  const float *w;
+  uint16_t *wp;
+  int M, CH, Cp, K, Npb, nblk, nchunks, premul, blocks;  // premul: padded M, or 0
+  int64_t sm, sc, sk;
+};
+__device__ __forceinline__ void weight_block(const Weight3 &q, int block) {
+  const int i = block * 256 + threadIdx.x;
+  if (i >= q.nblk * q.nchunks * q.Npb * kCols) return;
+  const int col = i % kCols, r = i / kCols % q.Npb, chunk = i / (kCols * q.Npb) % q.nchunks, nb = i / (kCols * q.Npb * q.nchunks);
+  const int n = nb * q.Npb + r;
   float v = 0.0f;
-  if (premul) {
-    const int k = n / M, ch = chunk * kCols + col;
-    if (k < K && ch < CH) v = __ldg(w + (n - k * M) * sm + ch * sc + k * sk);
+  if (q.premul) {
+    const int k = n / q.premul, m = n - k * q.premul, ch = chunk * kCols + col;
+    if (k < q.K && m < q.M && ch < q.CH) v = __ldg(q.w + m * q.sm + ch * q.sc + k * q.sk);
   } else {
-    chunk_item3(Cp, K, chunk, col >> 3, slot, c0);
+    int slot, c0;
+    chunk_item3(q.Cp, q.K, chunk, col >> 3, slot, c0);
     const int ch = c0 + (col & 7);
-    if (n < M && slot < K && ch < CH) v = __ldg(w + n * sm + ch * sc + slot * sk);
+    if (n < q.M && slot < q.K && ch < q.CH) v = __ldg(q.w + n * q.sm + ch * q.sc + slot * q.sk);
   }
   uint16_t h, m, l;
   split3(v, h, m, l);
-  uint16_t *t = wp + ((int64_t)nb * nchunks + chunk) * 3 * Npb * kCols + r * kCols + ((((col >> 3) ^ ((r >> 1) & 3)) << 3) | (col & 7));
+  uint16_t *t = q.wp + ((int64_t)nb * q.nchunks + chunk) * 3 * q.Npb * kCols + r * kCols + ((((col >> 3) ^ ((r >> 1) & 3)) << 3) | (col & 7));
   t[0] = h;
-  t[(int64_t)Npb * kCols] = m;
-  t[(int64_t)2 * Npb * kCols] = l;
+  t[(int64_t)q.Npb * kCols] = m;
+  t[(int64_t)2 * q.Npb * kCols] = l;
+}
+
+// The pre-pass of x3_gemm in one launch: source, weights, the call's status word.
+__global__ void __launch_bounds__(256) gemm_prepare3_kernel(const Nhwc3 src, const Weight3 wgt, int *status) {
+  __shared__ NhwcTile tile;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+  if ((int)blockIdx.x < wgt.blocks) weight_block(wgt, blockIdx.x);
+  else nhwc_block(src, blockIdx.x - wgt.blocks, tile);
 }
 
 // Gradient (B, N, GH*GW) -> tile images [tile][row block][step][part][128 rows][32 pixels] and, with `sums`, the sum of every
 // row over the tile's pixels: sums[(tile * mbs + row block) * 128 + row].  One block = one tile and row block.
-__global__ void __launch_bounds__(256) grad_image3_kernel(const float *__restrict__ gsrc, uint8_t *__restrict__ gt, int N, int GH, int GW,
-                                                          int tiles_x, int tiles_y, int mbs, float *__restrict__ sums) {
-  const int t2 = blockIdx.x, mb = blockIdx.y, b = blockIdx.z, ty = t2 / tiles_x, tx = t2 % tiles_x;
+struct Grad3 {
+  const float *g;
+  uint8_t *gt;
+  float *sums;
+  int N, GH, GW, tiles_x, tiles_y, mbs, blocks;
+};
+__device__ __forceinline__ void grad_block(const Grad3 &q, int block) {
+  const int N = q.N, GH = q.GH, GW = q.GW, tiles_x = q.tiles_x, tiles_y = q.tiles_y, mbs = q.mbs;
+  const int mb = block % mbs, t2 = block / mbs % (tiles_x * tiles_y), b = block / (mbs * tiles_x * tiles_y);
+  const int ty = t2 / tiles_x, tx = t2 % tiles_x;
+  const float *gsrc = q.g;
+  uint8_t *gt = q.gt;
+  float *sums = q.sums;
   const size_t npix = (size_t)GH * GW, tile = (size_t)b * tiles_x * tiles_y + t2;
   uint8_t *dst = gt + (tile * mbs + mb) * 4 * kStepA;
   const bool vec = (GW & 3) == 0 && (((uintptr_t)gsrc) & 15) == 0;
@@ -731,31 +783,96 @@ __global__ void __launch_bounds__(256) grad_image3_kernel(const float *__restric
   }
 }
 
-// gw[m, ch, k] = sum over splits, in order, of the partial sums.
-__global__ void dw3_reduce_kernel(const float *__restrict__ partial, int splits, int rows, int cols, int M, int CH, int Cp, int K, int64_t sm,
-                                  int64_t sc, int64_t sk, float *__restrict__ gw) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M * CH * K) return;
-  const int ch = i % CH, k = (i / CH) % K, m = i / (CH * K);
-  const float *s = partial + (size_t)m * cols + k * Cp + ch;
-  float a = 0.0f;
-  for (int z = 0; z < splits; z++) a += __ldg(s + (size_t)z * rows * cols);
-  gw[m * sm + ch * sc + k * sk] = a;
+// The pre-pass of x3_dw in one launch: gathered side, gradient tile images, the call's status word.
+__global__ void __launch_bounds__(256) dw_prepare3_kernel(const Nhwc3 src, const Grad3 grad, int *status) {
+  __shared__ NhwcTile tile;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+  if ((int)blockIdx.x < grad.blocks) grad_block(grad, blockIdx.x);
+  else nhwc_block(src, blockIdx.x - grad.blocks, tile);
 }
 
-// gb[c] = sum over tiles of the row sums: one block per channel, fixed order.
-__global__ void __launch_bounds__(256) bias_sum3_kernel(const float *__restrict__ sums, int64_t tiles, int rows, float *__restrict__ gb) {
+// The post-pass of x3_dw in one launch: gw[m, ch, k] = sum over splits, in order, of the partial sums (256 values per block, columns
+// fastest), and gb[c] = sum over `parts` of sums[part * pitch + c], one block per channel, in a fixed order.
+struct Reduce3 {
+  const float *partial, *sums;
+  float *gw, *gb;
+  int splits, rows, cols, M, CH, Cp, K, blocks, parts, pitch;
+  int64_t sm, sc, sk;
+};
+__global__ void __launch_bounds__(256) dw_reduce3_kernel(const Reduce3 q) {
   __shared__ float red[256];
-  const int c = blockIdx.x;
+  if ((int)blockIdx.x < q.blocks) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= q.M * q.CH * q.K) return;
+    const int ch = i % q.CH, k = (i / q.CH) % q.K, m = i / (q.CH * q.K);
+    const float *s = q.partial + (size_t)m * q.cols + k * q.Cp + ch;
+    const size_t step = (size_t)q.rows * q.cols;
+    float a = 0.0f;
+    int z = 0;
+    for (; z + 4 <= q.splits; z += 4) {  // (four loads in flight, added in order)
+      const float v0 = __ldg(s + z * step), v1 = __ldg(s + (z + 1) * step), v2 = __ldg(s + (z + 2) * step), v3 = __ldg(s + (z + 3) * step);
+      a = (((a + v0) + v1) + v2) + v3;
+    }
+    for (; z < q.splits; z++) a += __ldg(s + z * step);
+    q.gw[m * q.sm + ch * q.sc + k * q.sk] = a;
+    return;
+  }
+  const int c = blockIdx.x - q.blocks;
   float s = 0.0f;
-  for (int64_t t = threadIdx.x; t < tiles; t += 256) s += __ldg(sums + t * rows + c);
+  for (int t = threadIdx.x; t < q.parts; t += 256) s += __ldg(q.sums + (size_t)t * q.pitch + c);
   red[threadIdx.x] = s;
   __syncthreads();
   for (int d = 128; d > 0; d >>= 1) {
     if (threadIdx.x < d) red[threadIdx.x] += red[threadIdx.x + d];
     __syncthreads();
   }
-  if (threadIdx.x == 0) gb[c] = red[0];
+  if (threadIdx.x == 0) q.gb[c] = red[0];
+}
+
+// Second half of the multiply-first adjoint: out[b][m][q] (+bias) = sum over the plan entries (p, k, w) of destination pixel q, in
+// plan order, of w * T[b][p][k * Mp + m].  Thread = one destination pixel and VP output channels; an entry is one contiguous
+// run of its row.
+template <int VP>
+__global__ void __launch_bounds__(128) plan_gather_rows3_kernel(const float *__restrict__ T, const void *__restrict__ plan_blob,
+                                                                const float *__restrict__ bias, float *__restrict__ out, int K, int M, int Mp,
+                                                                int n_src, int n_dst) {
+  const int q = blockIdx.x * 128 + threadIdx.x, m0 = blockIdx.y * VP, b = blockIdx.z;
+  if (q >= n_dst) return;
+  bool ok;
+  const PlanView<float> pv = plan_view<float>(plan_blob, n_dst * K, ok);
+  const uint32_t pitch = (uint32_t)(K * Mp) * 4u;
+  const char *rows = (const char *)(T + (size_t)b * n_src * (K * Mp) + m0);
+  V8 acc[VP / 8];
+#pragma unroll
+  for (int i = 0; i < VP / 8; i++)
+#pragma unroll
+    for (int j = 0; j < 8; j++) acc[i].f[j] = 0.0f;
+  if (ok) {
+    const int *off = pv.offsets + (size_t)q * K;
+    int e = __ldg(off);
+    const int end = __ldg(off + K);
+    for (int k = 0; k < K && e < end; k++, rows += Mp * 4) {
+      const int e1 = __ldg(off + k + 1);
+      for (; e < e1; e++) {
+        const int s = __ldg(pv.src + e);
+        if (!index_ok(s, n_src)) continue;
+        const float w = __ldg(pv.w + e);
+        const char *row = rows + (size_t)(unsigned)s * pitch;
+#pragma unroll
+        for (int i = 0; i < VP / 8; i++) {
+          const V8 v = load8(row + i * 32);
+#pragma unroll
+          for (int j = 0; j < 8; j++) acc[i].f[j] = fmaf(w, v.f[j], acc[i].f[j]);
+        }
+      }
+    }
+  }
+  float *o = out + ((size_t)b * M + m0) * n_dst + q;
+#pragma unroll
+  for (int i = 0; i < VP / 8; i++)
+#pragma unroll
+    for (int j = 0; j < 8; j++, o += n_dst)
+      if (m0 + i * 8 + j < M) *o = acc[i].f[j] + (bias ? __ldg(bias + m0 + i * 8 + j) : 0.0f);
 }
 
 // ---- host side -------------------------------------------------------------------------------------------------------------
@@ -821,13 +938,15 @@ GemmPlan3 gemm_plan3(int src, int64_t B, int64_t CH, int64_t SHW, int64_t K, int
 // Multiply first (conv_simt.cu says when and why): a dense product over the source grid with N = K * M rows.
 struct Premul3 {
   GemmPlan3 q;
+  int Mp;  // output channels padded to 8: a thread of the plan gather reads 8 (or 16) of a row at once
   size_t t_bytes;
   bool use;
 };
 Premul3 premul3(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t M, int64_t n_dst) {
   Premul3 r{};
-  r.q = gemm_plan3(SRC_SELF, B, CH, SHW, 1, K * M);
-  r.t_bytes = align_up((size_t)(B * K * M * SHW) * 4, 256);
+  r.Mp = (int)align_up((size_t)M, 8);
+  r.q = gemm_plan3(SRC_SELF, B, CH, SHW, 1, K * r.Mp);
+  r.t_bytes = align_up((size_t)(B * K * r.Mp * SHW) * 4, 256);
   r.use = r.q.ok && n_dst >= 3 * SHW && CH >= 16 && r.t_bytes <= ((size_t)8 << 30);
   return r;
 }
@@ -849,18 +968,22 @@ DwPlan3 dw_plan3(int src, int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t
   const int64_t tiles = B * d.tiles_x * d.tiles_y;
   int64_t s = sms3() / ((int64_t)d.groups * d.mbs);
   d.splits = (int)(s < 1 ? 1 : s > tiles ? tiles : s);
-  d.stages = 3;
-  d.smem = 1024 + (size_t)d.stages * (kStepA + kStepB) + 2 * align_up(table3(src, d.slots), 16) + bars_bytes(d.stages);
+  const auto dw_smem = [&](int s) { return 1024 + (size_t)s * (kStepA + kStepB) + 2 * align_up(table3(src, d.slots), 16) + bars_bytes(s); };
+  d.stages = dw_smem(3) <= kSmemMax ? 3 : 2;
+  d.smem = dw_smem(d.stages);
   d.xl_bytes = align_up((size_t)(B * (SHW + 1)) * d.Cp * 4, 256);
   d.gt_bytes = align_up((size_t)tiles * d.mbs * 4 * kStepA, 256);
   d.partial_bytes = align_up((size_t)d.splits * d.mbs * 128 * d.groups * kDwN * 4, 256);
-  d.sums_bytes = align_up((size_t)tiles * d.mbs * 128 * 4, 256);
+  // (row sums of the gradient's tiles, or channel sums of the gathered side's blocks)
+  d.sums_bytes = align_up((size_t)std::max<int64_t>(tiles * d.mbs * 128, B * cdiv(SHW + 1, kNhwcPix) * d.Cp) * 4, 256);
   d.ok = src >= 0 && src != SRC_PLAN && d.smem <= kSmemMax && (SHW + 1) * d.Cp * 4 < ((int64_t)1 << 32) && tiles < ((int64_t)1 << 28);
   return d;
 }
 
-void to_nhwc3(const void *x, float *y, int64_t B, int64_t C, int Cp, int64_t HW, cudaStream_t st) {
-  nchw_to_nhwc_kernel<<<dim3(cdiv(HW + 1, 32), cdiv(Cp, 32), (unsigned)B), 256, 0, st>>>((const float *)x, y, (int)C, Cp, (int)HW);
+Nhwc3 nhwc3(const void *x, float *y, int64_t B, int64_t C, int Cp, int64_t HW, float *sums = nullptr) {
+  Nhwc3 q{(const float *)x, y, sums, (int)C, Cp, (int)HW, cdiv(HW + 1, kNhwcPix), cdiv(Cp, 32), 0};
+  q.blocks = q.px_blocks * q.ch_blocks * (int)B;
+  return q;
 }
 
 template <int SRC> void launch_gemm3(const Gemm3 &p, int64_t tiles, size_t smem, cudaStream_t st) {
@@ -897,11 +1020,10 @@ int x3_gemm(bool use_plan, const void *src, const void *map, const void *iw, con
   float *xl = (float *)(w + 256);
   uint16_t *wp = (uint16_t *)(w + 256 + q.xl_bytes);
   float *T = (float *)(w + 256 + q.xl_bytes + q.wp_bytes);
-  if (cudaMemsetAsync(status, 0, 4, st) != cudaSuccess) return SPH_ERR_CUDA;
-  to_nhwc3(src, xl, B, CH, q.Cp, SH * SW, st);
-  const int64_t wtotal = (int64_t)q.nblk * q.nchunks * q.Npb * kCols;
-  weight_image3_kernel<<<cdiv(wtotal, 256), 256, 0, st>>>((const float *)wgt, wp, (int)Nout, (int)CH, q.Cp, (int)K, q.Npb, q.nblk, q.nchunks,
-                                                          sm, sc, sk, r.use ? 1 : 0);
+  const Nhwc3 pre = nhwc3(src, xl, B, CH, q.Cp, SH * SW);
+  const Weight3 wt{(const float *)wgt, wp, (int)Nout, (int)CH, q.Cp, (int)K, q.Npb, q.nblk, q.nchunks, r.use ? r.Mp : 0,
+                   cdiv((int64_t)q.nblk * q.nchunks * q.Npb * kCols, 256), sm, sc, sk};
+  gemm_prepare3_kernel<<<(unsigned)(wt.blocks + pre.blocks), 256, 0, st>>>(pre, wt, status);
   Gemm3 p{};
   p.g = Src3{(const char *)xl, (const float *)map, (const float *)iw, plan, q.Cp, (int)SH, (int)SW, r.use ? 1 : (int)K, (int)P,
              (int)(r.use ? SH : GH), (int)(r.use ? SW : GW), interp};
@@ -909,7 +1031,7 @@ int x3_gemm(bool use_plan, const void *src, const void *map, const void *iw, con
   p.bias = r.use ? nullptr : (const float *)bias;
   p.out = r.use ? T : (float *)out;
   p.status = status;
-  p.B = (int)B; p.Nout = (int)(r.use ? K * Nout : Nout); p.Npb = q.Npb; p.nblk = q.nblk; p.nchunks = q.nchunks;
+  p.B = (int)B; p.Nout = (int)(r.use ? K * r.Mp : Nout); p.Npb = q.Npb; p.nblk = q.nblk; p.nchunks = q.nchunks;
   p.tiles_x = cdiv(p.g.GW, kTileW); p.tiles_y = cdiv(p.g.GH, kTileH); p.stages = q.stages;
   const int64_t tiles = B * p.tiles_x * p.tiles_y * q.nblk;
   switch (kind) {
@@ -918,8 +1040,17 @@ int x3_gemm(bool use_plan, const void *src, const void *map, const void *iw, con
     case SRC_PLAN: launch_gemm3<SRC_PLAN>(p, tiles, q.smem, st); break;
     default: launch_gemm3<SRC_SELF>(p, tiles, q.smem, st); break;
   }
-  const int rc = launch_status(3);
-  return rc == SPH_OK && r.use ? simt_plan_gather_planes(T, plan, bias, out, K, Nout, SH * SW, GH * GW, B, st) : rc;
+  const int rc = launch_status(2);
+  if (rc != SPH_OK || !r.use) return rc;
+  const int vp = r.Mp % 16 == 0 ? 16 : 8;
+  const dim3 grid(cdiv(GH * GW, 128), r.Mp / vp, (unsigned)B);
+  if (vp == 16)
+    plan_gather_rows3_kernel<16><<<grid, 128, 0, st>>>(T, plan, (const float *)bias, (float *)out, (int)K, (int)Nout, r.Mp, (int)(SH * SW),
+                                                       (int)(GH * GW));
+  else
+    plan_gather_rows3_kernel<8><<<grid, 128, 0, st>>>(T, plan, (const float *)bias, (float *)out, (int)K, (int)Nout, r.Mp, (int)(SH * SW),
+                                                      (int)(GH * GW));
+  return launch_status();
 }
 
 size_t x3_dw_workspace(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int interp, int64_t M, int64_t GH, int64_t GW) {
@@ -927,10 +1058,11 @@ size_t x3_dw_workspace(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P,
   return d.ok ? 256 + d.xl_bytes + d.gt_bytes + d.partial_bytes + d.sums_bytes : 0;
 }
 
-// gw[m, ch, k] = sum A[b, m, pix] * Col[b, pix, (ch, k)];  with gb, also gb[m] = sum A[b, m, :].
+// gw[m, ch, k] = sum A[b, m, pix] * Col[b, pix, (ch, k)], and the bias gradient gb: the sums of A's rows or (bias_of_src: a
+// transposed convolution, whose gathered side is the output's gradient) of the source's channels.
 int x3_dw(const void *A, const void *src, const void *map, const void *iw, int64_t CH, int64_t SH, int64_t SW, int64_t K, int64_t P,
-          int64_t GH, int64_t GW, int interp, int64_t M, int64_t B, void *gw, int64_t sm, int64_t sc, int64_t sk, void *gb, void *ws,
-          cudaStream_t st) {
+          int64_t GH, int64_t GW, int interp, int64_t M, int64_t B, void *gw, int64_t sm, int64_t sc, int64_t sk, void *gb, bool bias_of_src,
+          void *ws, cudaStream_t st) {
   const int kind = source3(false, P, interp);
   const DwPlan3 d = dw_plan3(kind, B, CH, SH * SW, K, M, GH, GW);
   char *w = (char *)ws;
@@ -938,10 +1070,10 @@ int x3_dw(const void *A, const void *src, const void *map, const void *iw, int64
   float *xl = (float *)(w + 256);
   uint8_t *gt = (uint8_t *)(w + 256 + d.xl_bytes);
   float *partial = (float *)(w + 256 + d.xl_bytes + d.gt_bytes), *sums = (float *)((char *)partial + d.partial_bytes);
-  if (cudaMemsetAsync(status, 0, 4, st) != cudaSuccess) return SPH_ERR_CUDA;
-  to_nhwc3(src, xl, B, CH, d.Cp, SH * SW, st);
-  grad_image3_kernel<<<dim3(d.tiles_x * d.tiles_y, d.mbs, (unsigned)B), 256, 0, st>>>((const float *)A, gt, (int)M, (int)GH, (int)GW, d.tiles_x,
-                                                                                     d.tiles_y, d.mbs, gb ? sums : nullptr);
+  const Nhwc3 pre = nhwc3(src, xl, B, CH, d.Cp, SH * SW, bias_of_src ? sums : nullptr);
+  const int tiles = (int)(B * d.tiles_x * d.tiles_y);
+  const Grad3 grad{(const float *)A, gt, bias_of_src ? nullptr : sums, (int)M, (int)GH, (int)GW, d.tiles_x, d.tiles_y, d.mbs, tiles * d.mbs};
+  dw_prepare3_kernel<<<(unsigned)(grad.blocks + pre.blocks), 256, 0, st>>>(pre, grad, status);
   Dw3 p{};
   p.g = Src3{(const char *)xl, (const float *)map, (const float *)iw, nullptr, d.Cp, (int)SH, (int)SW, (int)K, (int)P, (int)GH, (int)GW, interp};
   p.gt = (const __nv_bfloat16 *)gt; p.partial = partial; p.status = status;
@@ -949,10 +1081,10 @@ int x3_dw(const void *A, const void *src, const void *map, const void *iw, int64
   p.splits = d.splits; p.stages = d.stages;
   if (kind == SRC_MAP1) launch_dw3<SRC_MAP1>(p, d.smem, st);
   else launch_dw3<SRC_MAP4>(p, d.smem, st);
-  dw3_reduce_kernel<<<cdiv(M * CH * K, 256), 256, 0, st>>>(partial, d.splits, d.mbs * 128, d.groups * kDwN, (int)M, (int)CH, d.Cp, (int)K, sm,
-                                                           sc, sk, (float *)gw);
-  if (gb) bias_sum3_kernel<<<(unsigned)M, 256, 0, st>>>(sums, B * d.tiles_x * d.tiles_y, d.mbs * 128, (float *)gb);
-  return launch_status(gb ? 5 : 4);
+  const Reduce3 red{partial, sums, (float *)gw, (float *)gb, d.splits, d.mbs * 128, d.groups * kDwN, (int)M, (int)CH, d.Cp, (int)K,
+                    cdiv(M * CH * K, 256), bias_of_src ? (int)B * pre.px_blocks : tiles, bias_of_src ? d.Cp : d.mbs * 128, sm, sc, sk};
+  dw_reduce3_kernel<<<(unsigned)(red.blocks + (bias_of_src ? CH : M)), 256, 0, st>>>(red);
+  return launch_status(3);
 }
 
 int x3_wait_status(int reset) {
