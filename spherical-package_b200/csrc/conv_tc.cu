@@ -294,6 +294,7 @@ struct TcParams {
   int out_pitch;            // multiply-first adjoint), no bias
   int *status;              // set to 1 if a bounded wait gave up
   int B, Nout, Npb, nblk, nchunks, tiles_x, tiles_y, stages;
+  int over;                 // plan mode, lean loop: entries five to eight of a key have a table of their own
   int use_out_map;          // outputs leave through the tensor map passed beside these parameters
   int relu;                 // clamp the outputs at zero (fused activation)
   __nv_bfloat16 *out_cl;    // if set: the outputs are also written as a channels-last bf16 copy (B, GH*GW + 1, cl_pitch)
@@ -303,7 +304,8 @@ struct TcParams {
 struct Smem {
   uint8_t *A, *Bw;
   Tap *taps;
-  int2 *rest;  // plan mode: [slot][pixel] range of plan entries beyond the table capacity
+  int2 *rest;  // plan mode: [slot][pixel] (first plan entry beyond the four of the tap table, number of such entries)
+  Tap *over;   // p.over: [slot][pixel][4], the first four of them
   uint64_t *full, *empty, *tfull, *tempty;
   uint32_t *tmem_ptr;
   volatile int *abort_flag;
@@ -314,11 +316,12 @@ constexpr int kOutStageCh = 16;
 constexpr int kClStageBytes = kEpilogueWarps * 32 * kOutStageCh * 2;  // channels-last copy: [warp][2 rows][16 px][16 ch] bf16
 constexpr int kOutStageBytes = kEpilogueWarps * kOutStageCh * 32 * 4 + kClStageBytes;
 
-inline size_t gemm_smem_bytes(int stages, int Npb, int K, int nt, bool direct) {
+inline size_t gemm_smem_bytes(int stages, int Npb, int K, int nt, bool direct, bool over = false) {
   size_t s = 1024;  // alignment slack
   s += (size_t)stages * (kAStageBytes + Npb * 128);
   s += (size_t)K * kTileM * nt * sizeof(Tap);
   if (!direct) s += (size_t)K * kTileM * sizeof(int2);
+  if (over) s += (size_t)K * kTileM * 4 * sizeof(Tap);
   s += 8 * (2 * stages + 4) + 16;
   s += kOutStageBytes + 128;
   return s;
@@ -334,6 +337,8 @@ __device__ inline Smem carve(uint8_t *raw, const TcParams &p, bool direct) {
   q += (size_t)p.g.K * kTileM * p.g.nt * sizeof(Tap);
   s.rest = (int2 *)q;
   q += direct ? 0 : (size_t)p.g.K * kTileM * sizeof(int2);
+  s.over = (Tap *)q;
+  q += p.over ? (size_t)p.g.K * kTileM * 4 * sizeof(Tap) : 0;
   s.full = (uint64_t *)q;
   s.empty = s.full + p.stages;
   s.tfull = s.empty + p.stages;
@@ -369,8 +374,8 @@ __device__ __forceinline__ void produce_chunk(const Gather &g, const Tap *taps, 
       gather_pair<NTI>(imgc, imgc, trow + (size_t)(r * kRowStep) * stride, trow + (size_t)((r + 1) * kRowStep) * stride, g.nt, a0, a1);
       if (PLAN) {
         const int2 r0 = rest[row0 + r * kRowStep], r1 = rest[row0 + (r + 1) * kRowStep];
-        if (r0.x < r0.y) gather_plan_rest(a0, imgc, pv, r0.x, r0.y, g.Cp * 2);
-        if (r1.x < r1.y) gather_plan_rest(a1, imgc, pv, r1.x, r1.y, g.Cp * 2);
+        if (r0.y > 0) gather_plan_rest(a0, imgc, pv, r0.x, r0.x + r0.y, g.Cp * 2);
+        if (r1.y > 0) gather_plan_rest(a1, imgc, pv, r1.x, r1.x + r1.y, g.Cp * 2);
       }
     }
     *(uint4 *)(dst + r * kRowStep * 128) = acc_pack(a0);
@@ -412,7 +417,7 @@ __device__ __forceinline__ void produce_chunk_pair(const Gather &g, const Tap *t
     }
     if (PLAN) {
       const int2 rr = rest[row];
-      for (int e = rr.x; e < rr.y; e++) {
+      for (int e = rr.x; e < rr.x + rr.y; e++) {
         uint4 xa, xb;
         const int sp = __ldg(pv.src + e);
         if (!index_ok(sp, pv.n_src)) continue;
@@ -442,7 +447,7 @@ __device__ __forceinline__ bool produce_tile_lean(const TcParams &p, const Smem 
   const uint32_t taps0 = smem_u32(sm.taps) + pl * (STRIDE * (uint32_t)sizeof(Tap));
   const uint32_t a0s = smem_u32(sm.A) + pl * 128 + (((2 * vp) ^ (pl & 7)) << 4);
   const uint32_t a1s = smem_u32(sm.A) + pl * 128 + (((2 * vp + 1) ^ (pl & 7)) << 4);
-  const uint32_t full0 = smem_u32(sm.full), empty0 = smem_u32(sm.empty);
+  const uint32_t full0 = smem_u32(sm.full), empty0 = smem_u32(sm.empty), over0 = PLAN ? smem_u32(sm.over) : 0u;
   const uint32_t bbytes = (uint32_t)p.Npb * 128;
   const __nv_bfloat16 *wsrc = p.wp + (size_t)nb * p.nchunks * p.Npb * kChunk;
   const char *imgc = img + vp * 32;  // advanced by 128 bytes per channel block
@@ -497,7 +502,23 @@ __device__ __forceinline__ bool produce_tile_lean(const TcParams &p, const Smem 
     }
     if (PLAN) {
       const int2 rr = sm.rest[slot * kTileM + pl];
-      for (int e = rr.x; e < rr.y; e++) {
+      int done = 0;
+      if (p.over) {  // two rows in flight, addresses from shared memory
+        const uint32_t over_s = over0 + (slot * kTileM + pl) * (4 * (uint32_t)sizeof(Tap));
+        for (; done < min(rr.y, 4); done += 2) {
+          const uint4 t2 = lds128(over_s + done * (uint32_t)sizeof(Tap));
+          uint4 xa, xb, ya = make_uint4(0u, 0u, 0u, 0u), yb = ya;
+          ldg32(imgc + (int)t2.x, xa, xb);
+          if (done + 1 < rr.y) ldg32(imgc + (int)t2.z, ya, yb);
+          acc_fma(a0, t2.y, xa);
+          acc_fma(a1, t2.y, xb);
+          if (done + 1 < rr.y) {
+            acc_fma(a0, t2.w, ya);
+            acc_fma(a1, t2.w, yb);
+          }
+        }
+      }
+      for (int e = rr.x + done; e < rr.x + rr.y; e++) {
         uint4 xa, xb;
         const int sp = __ldg(pv.src + e);
         if (!index_ok(sp, pv.n_src)) continue;
@@ -790,7 +811,17 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcParams p, 
           static_assert(kPlanTaps == 4, "two 16-byte stores per entry");
           ((uint4 *)dst)[0] = make_uint4((uint32_t)t[0].off, t[0].w, (uint32_t)t[1].off, t[1].w);
           ((uint4 *)dst)[1] = make_uint4((uint32_t)t[2].off, t[2].w, (uint32_t)t[3].off, t[3].w);
-          sm.rest[idx] = make_int2(min(e0 + kPlanTaps, e1), e1);
+          sm.rest[idx] = make_int2(e0 + kPlanTaps, max(e1 - e0 - kPlanTaps, 0));
+          if (LEAN && p.over && e1 - e0 > kPlanTaps) {
+            Tap *o = sm.over + (size_t)idx * 4;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+              const bool in = e0 + kPlanTaps + i < e1;
+              const int sp = in ? __ldg(pv.src + e0 + kPlanTaps + i) : 0;
+              o[i].off = (in && index_ok(sp, pv.n_src)) ? sp * pitch : zero_off;
+              o[i].w = in && index_ok(sp, pv.n_src) ? tap_weight(__ldg(pv.w + e0 + kPlanTaps + i)) : 0u;
+            }
+          }
         }
       }
       producer_bar();
@@ -895,10 +926,10 @@ inline size_t dw_smem_bytes(int stages, int grp, int mbs, int tap_rows, int nt) 
   return 1024 + stages * dw_stage_bytes(grp, mbs) + 2 * (size_t)tap_rows * kDwPix * nt * sizeof(Tap) + 8 * (2 * stages + 1) + 16;
 }
 
-// WT selects warp-private taps (unweighted maps, Cp >= 64, NT > 0): every producer warp decodes the taps of its own
+// WT selects warp-private taps (unweighted maps or, WQ, weighted nearest ones of at most four points; Cp >= 64, NT > 0): every producer warp decodes the taps of its own
 // four pixels, one step ahead, into its own slice of the table, so the producers share nothing but the stage
 // barriers; otherwise the whole producer group fills one table per step and meets at a named barrier.
-template <int NT, int GRP, bool WT>
+template <int NT, int GRP, bool WT, bool WQ = false>
 __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
   constexpr int MBS = 8 / GRP;
   constexpr int kDwColBytes = GRP * kDwPix * 128;  // gathered columns per stage
@@ -908,7 +939,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
   const int S = p.stages;
   const int grp = blockIdx.x, split = blockIdx.y, mb0 = blockIdx.z * MBS;
   const int mbs = min(MBS, p.mbs_total - mb0);
-  const int chunk0 = grp * GRP, ncg = min(GRP, p.nchunks - chunk0);
+  // column groups of equal width (at most GRP chunks): nine chunks make three groups of three, not four, four and one
+  const int chunk0 = grp * p.nchunks / (int)gridDim.x, ncg = (grp + 1) * p.nchunks / (int)gridDim.x - chunk0;
   const size_t stage_bytes = kDwColBytes + (size_t)mbs * kDwGtBytes;
 
   DwSmem sm;
@@ -1028,7 +1060,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
     // position (image, tile row, tile column) of the step whose map coordinate is fetched next
     int nb_ = step_lo / tiles_per_image, nty = (step_lo % tiles_per_image) / p.tiles_x, ntx = (step_lo % tiles_per_image) % p.tiles_x;
     int b_dec = 0, pix_dec = -1;
-    float mx = 0.0f, my = 0.0f;
+    constexpr int NP = WQ ? 4 : 1;
+    float mx[NP], my[NP], mw[NP];
+#pragma unroll
+    for (int i = 0; i < NP; i++) { mx[i] = my[i] = mw[i] = 0.0f; }
     auto fetch = [&]() {  // issue the map loads of the next step; they complete under the current step's gather
       b_dec = nb_;
       pix_dec = tile_pixel(e_pl, nty, ntx, kDwTH, g.GH, g.GW);
@@ -1037,15 +1072,29 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
         if (++nty == p.tiles_y) { nty = 0; nb_++; }
       }
       if (dec && pix_dec >= 0) {
-        const float *m = g.map + 2 * ((size_t)pix_dec * g.K + e_slot);
-        mx = __ldg(m);
-        my = __ldg(m + 1);
+        const size_t e = ((size_t)pix_dec * g.K + e_slot) * (WQ ? g.P : 1);
+#pragma unroll
+        for (int i = 0; i < NP; i++)
+          if (!WQ || i < g.P) {
+            mx[i] = __ldg(g.map + 2 * (e + i));
+            my[i] = __ldg(g.map + 2 * (e + i) + 1);
+            if (WQ) mw[i] = __ldg(g.iw + e + i);
+          }
       }
     };
     auto decode_to = [&](uint32_t dst_s) {
       if (lane < kEnt) {
         Tap t[NT];
-        if (dec && pix_dec >= 0) taps_from_xy<NT>(g, mx, my, t);
+        if (WQ && dec && pix_dec >= 0) {  // the points take the taps' places
+#pragma unroll
+          for (int i = 0; i < NT; i++) {
+            Tap q[1];
+            taps_from_xy<1>(g, mx[i < NP ? i : 0], my[i < NP ? i : 0], q);
+            const bool in = i < g.P && q[0].w != 0u;
+            t[i].off = in ? q[0].off : zero_off;
+            t[i].w = in ? tap_weight(mw[i < NP ? i : 0]) : 0u;
+          }
+        } else if (dec && pix_dec >= 0) taps_from_xy<NT>(g, mx[0], my[0], t);
         else {
 #pragma unroll
           for (int i = 0; i < NT; i++) { t[i].off = zero_off; t[i].w = 0u; }
@@ -1293,9 +1342,11 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_bf16_kernel(const float *__r
 
 // Weights -> bf16 tile images.  Row n of block nb, chunk `chunk`: 64 columns, 16-byte vector v stored at
 // position v ^ (n & 7) of the 128-byte row.  The source is addressed W[n*sn + ch*sc + slot*sk].
+// The kernel also clears the call's status word.
 __global__ void weight_image_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ wp, int Nout, int CH, int Cp,
-                                    int K, int Npb, int nblk, int nchunks, int64_t sn, int64_t sc, int64_t sk) {
+                                    int K, int Npb, int nblk, int nchunks, int64_t sn, int64_t sc, int64_t sk, int *status) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *status = 0;
   const int64_t total = (int64_t)nblk * nchunks * Npb * kChunk;
   if (i >= total) return;
   const int col = (int)(i % kChunk), n = (int)((i / kChunk) % Npb), chunk = (int)((i / ((int64_t)kChunk * Npb)) % nchunks);
@@ -1313,16 +1364,21 @@ __global__ void weight_image_kernel(const float *__restrict__ w, __nv_bfloat16 *
 // row_part[(b * tiles + tile) * mbs_total * 128 + row] (first stage of the bias gradient).
 // With `cl` the same (masked) values are also written as the channels-last bf16 copy (B, GH*GW + 1, cl_pitch) that the
 // input-gradient kernel gathers from, so the gradient is read from memory once for both of its consumers; the extra
-// zero pixel of every image is not written here.
+// zero pixel of every image is written too.  The kernel also clears a status word.
 constexpr int kClStride = 128 + 8;  // bf16 per staged pixel row: 16-byte aligned rows, shifted banks
 __global__ void __launch_bounds__(256) grad_image_kernel(const float *__restrict__ gsrc, __nv_bfloat16 *__restrict__ gt, int N,
                                                           int GH, int GW, int tiles_x, int tiles_y, int mbs_total,
                                                           float *__restrict__ row_part, const float *__restrict__ mask,
-                                                          __nv_bfloat16 *__restrict__ cl, int cl_pitch) {
+                                                          __nv_bfloat16 *__restrict__ cl, int cl_pitch, int *status) {
   __shared__ __align__(16) __nv_bfloat16 cls[64 * kClStride];  // [pixel of the 4x16 tile][channel of this 128-row block]
   const int t2 = blockIdx.x, mb = blockIdx.y, b = blockIdx.z;
   const int ty = t2 / tiles_x, tx = t2 % tiles_x;
   const size_t npix = (size_t)GH * GW;
+  if (t2 == 0) {
+    if (mb == 0 && b == 0 && threadIdx.x == 0) *status = 0;
+    const int c = mb * 128 + threadIdx.x;
+    if (cl != nullptr && threadIdx.x < 128 && c < cl_pitch) cl[((size_t)b * (npix + 1) + npix) * cl_pitch + c] = __float2bfloat16(0.0f);
+  }
   __nv_bfloat16 *dst = gt + (((size_t)b * tiles_x * tiles_y + t2) * mbs_total + mb) * (128 * 64);
   for (int i = threadIdx.x; i < 128 * 8; i += 256) {
     const int r = i >> 3, v = i & 7, n = mb * 128 + r;
@@ -1379,30 +1435,27 @@ __global__ void __launch_bounds__(256) grad_image_kernel(const float *__restrict
   }
 }
 
-// Second and third stage of the fused bias gradient: fixed-order sums over the (image, tile) blocks.
-constexpr int kRowSplits = 64;
-__global__ void row_sum_split_kernel(const float *__restrict__ row_part, int64_t nblocks, int rows_total, int C,
-                                     float *__restrict__ part2) {
+// Second stage of the fused bias gradient: sums of kRowSplits ranges of the (image, tile) blocks, in order; the third is part
+// of tc_dw_reduce_kernel.
+constexpr int kRowSplits = 256;
+__global__ void __launch_bounds__(128) row_sum_split_kernel(const float *__restrict__ row_part, int64_t nblocks, int rows_total, int C,
+                                                            float *__restrict__ part2) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x, sp = blockIdx.y;
   if (c >= C) return;
   const int64_t lo = nblocks * sp / kRowSplits, hi = nblocks * (sp + 1) / kRowSplits;
   float s = 0.0f;
+#pragma unroll 8
   for (int64_t i = lo; i < hi; i++) s += __ldg(row_part + i * rows_total + c);
   part2[(size_t)sp * C + c] = s;
-}
-__global__ void row_sum_final_kernel(const float *__restrict__ part2, int C, float *__restrict__ gb) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= C) return;
-  float s = 0.0f;
-  for (int sp = 0; sp < kRowSplits; sp++) s += part2[(size_t)sp * C + c];
-  gb[c] = s;
 }
 
 // Weight image of the multiply-first adjoint: rows n = k * Mp + m (slot-major, so that one map slot's M channels
 // are contiguous in the column buffer), columns = source channels; W addressed Wgt[m*sm + ch*sc + k*sk].
+// The kernel also clears the call's status word.
 __global__ void premul_weight_image_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ wp, int M, int Mp, int K,
-                                           int CH, int Npb, int nblk, int nchunks, int64_t sm, int64_t sc, int64_t sk) {
+                                           int CH, int Npb, int nblk, int nchunks, int64_t sm, int64_t sc, int64_t sk, int *status) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *status = 0;
   const int64_t total = (int64_t)nblk * nchunks * Npb * kChunk;
   if (i >= total) return;
   const int col = (int)(i % kChunk), n = (int)((i / kChunk) % Npb), chunk = (int)((i / ((int64_t)kChunk * Npb)) % nchunks);
@@ -1462,17 +1515,37 @@ plan_gather_rows_kernel(const __nv_bfloat16 *__restrict__ T, const void *__restr
   }
 }
 
-// gw[n*sn + ch*sc + slot*sk] = sum over splits (in order) of partial[split][n][column of (slot, ch)].
-__global__ void tc_dw_reduce_kernel(const float *__restrict__ partial, int splits, int rows_total, int ncols_total, int Nout,
-                                    int CH, int Cp, int K, int64_t sn, int64_t sc, int64_t sk, float *__restrict__ gw) {
+// gw[n*sn + ch*sc + slot*sk] = sum over splits (in order) of partial[split][n][column of (slot, ch)]: 256 values per block, channels
+// fastest (neighbouring threads read neighbouring columns), four splits in flight.  With part2, further blocks (eight channels
+// each, a warp per channel) add the bias gradient's kRowSplits partial sums in a fixed order.
+__global__ void __launch_bounds__(256) tc_dw_reduce_kernel(const float *__restrict__ partial, int splits, int rows_total, int ncols_total,
+                                                           int Nout, int CH, int Cp, int K, int64_t sn, int64_t sc, int64_t sk,
+                                                           float *__restrict__ gw, int gw_blocks, const float *__restrict__ part2, int C,
+                                                           float *__restrict__ gb) {
+  if ((int)blockIdx.x >= gw_blocks) {
+    const int c = (blockIdx.x - gw_blocks) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (c >= C) return;
+    float s = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kRowSplits / 32; i++) s += __ldg(part2 + (size_t)(lane + 32 * i) * C + c);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    if (lane == 0) gb[c] = s;
+    return;
+  }
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Nout * CH * K) return;
-  const int slot = i % K, ch = (i / K) % CH, n = i / (K * CH);
-  int col;
-  if (Cp >= 64) col = ((ch / 64) * K + slot) * 64 + (ch % 64);
-  else col = slot * Cp + ch;
+  const int ch = i % CH, slot = (i / CH) % K, n = i / (CH * K);
+  const int col = Cp >= 64 ? ((ch / 64) * K + slot) * 64 + (ch % 64) : slot * Cp + ch;
+  const float *src = partial + (size_t)n * ncols_total + col;
+  const size_t step = (size_t)rows_total * ncols_total;
   float s = 0.0f;
-  for (int z = 0; z < splits; z++) s += partial[((size_t)z * rows_total + n) * ncols_total + col];
+  int z = 0;
+  for (; z + 4 <= splits; z += 4) {
+    const float v0 = __ldg(src + z * step), v1 = __ldg(src + (z + 1) * step), v2 = __ldg(src + (z + 2) * step), v3 = __ldg(src + (z + 3) * step);
+    s = (((s + v0) + v1) + v2) + v3;
+  }
+  for (; z < splits; z++) s += __ldg(src + z * step);
   gw[n * sn + ch * sc + slot * sk] = s;
 }
 
@@ -1510,7 +1583,7 @@ void ensure_dynamic_smem(Kernel kernel, int *granted /* [kMaxDevices], zero-init
 }
 
 struct Geometry {
-  int Cp, nchunks, Npb, nblk, nt, stages;
+  int Cp, nchunks, Npb, nblk, nt, stages, over;
   size_t xh_bytes, wp_bytes, smem;
   bool ok;
 };
@@ -1534,16 +1607,22 @@ Geometry geometry(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int 
   // (layer-4 input gradient of the encoder: 3 stages at 207 KB 3.97 ms, 2 stages at 158 KB 3.77 ms).  So: as many stages
   // as fit 196 KB, and only if two do not fit, as many as fit the whole array.
   constexpr size_t kSoftLimit = 196 * 1024;
+  // Plan mode: a key has about four entries on a map that neither stretches nor folds the image, but their number varies - on a
+  // map without locality it is near a Poisson variable of mean four, and more than a third of the keys have five or more.
+  // Entries five to eight come from a second table where two stages still fit beside it; without it each is a dependent
+  // chain index -> address -> row (weighted random map, 64 -> 128 channels, 16 x 256 x 512: 3.90 ms without, 3.28 ms with;
+  // gnomonic maps, where few keys have a fifth entry: no difference).
+  g.over = !direct && g.Cp >= 64 && gemm_smem_bytes(2, g.Npb, (int)K, g.nt, direct, true) <= kSoftLimit;
   g.stages = 4;
-  while (g.stages > 2 && gemm_smem_bytes(g.stages, g.Npb, (int)K, g.nt, direct) > kSoftLimit) g.stages--;
-  if (gemm_smem_bytes(g.stages, g.Npb, (int)K, g.nt, direct) > kSoftLimit) {
+  while (g.stages > 2 && gemm_smem_bytes(g.stages, g.Npb, (int)K, g.nt, direct, g.over) > kSoftLimit) g.stages--;
+  if (gemm_smem_bytes(g.stages, g.Npb, (int)K, g.nt, direct, g.over) > kSoftLimit) {
     g.stages = 4;
     while (g.stages > 2 && gemm_smem_bytes(g.stages, g.Npb, (int)K, g.nt, direct) > (size_t)kSmemLimit) g.stages--;
   }
   // With at most 128 output columns the MMA of a chunk is short next to its gather, a deeper pipeline buys nothing, and
   // the shared memory two stages leave free goes to L1 (layer-2 forward of the encoder: 4 stages 1.14 ms, 2 stages 1.05 ms).
   if (direct && g.Npb <= 128 && map_mode_gather) g.stages = 2;
-  g.smem = gemm_smem_bytes(g.stages, g.Npb, (int)K, g.nt, direct);
+  g.smem = gemm_smem_bytes(g.stages, g.Npb, (int)K, g.nt, direct, g.over);
   if (g.smem > (size_t)kSmemLimit) g.ok = false;
   return g;
 }
@@ -1673,12 +1752,11 @@ int tc_adjoint_premul(const PremulGeometry &q, const void *src, const void *plan
   __nv_bfloat16 *xh = (__nv_bfloat16 *)((char *)ws + 256);
   __nv_bfloat16 *wp = (__nv_bfloat16 *)((char *)ws + 256 + g.xh_bytes);
   __nv_bfloat16 *T = (__nv_bfloat16 *)((char *)ws + 256 + g.xh_bytes + g.wp_bytes);
-  if (cudaMemsetAsync(status, 0, 4, st) != cudaSuccess) return SPH_ERR_CUDA;
   if (fz.src_cl != nullptr) xh = (__nv_bfloat16 *)fz.src_cl;  // already converted (and masked) by the caller
   else to_nhwc(src, xh, B, CH, g.Cp, SH * SW, st, fz.mask);   // adjoint: src is grad_output
   const int64_t wtotal = (int64_t)g.nblk * g.nchunks * g.Npb * kChunk;
   premul_weight_image_kernel<<<cdiv(wtotal, 256), 256, 0, st>>>((const float *)wgt, wp, (int)M, q.Mp, (int)K, (int)CH, g.Npb, g.nblk,
-                                                                g.nchunks, sm_, sc, sk);
+                                                                g.nchunks, sm_, sc, sk, status);
   TcParams p{};
   p.g = Gather{xh, nullptr, nullptr, nullptr, g.Cp, (int)SH, (int)SW, 1, 0, (int)SH, (int)SW, SPH_NEAREST, 1};
   p.out_cl = nullptr; p.cl_pitch = 0;
@@ -1711,12 +1789,11 @@ int tc_gemm(bool use_plan, const void *src, const void *map, const void *iw, con
   int *status = (int *)ws;
   __nv_bfloat16 *xh = (__nv_bfloat16 *)((char *)ws + 256);
   __nv_bfloat16 *wp = (__nv_bfloat16 *)((char *)ws + 256 + g.xh_bytes);
-  if (cudaMemsetAsync(status, 0, 4, st) != cudaSuccess) return SPH_ERR_CUDA;
   if (fz.src_cl != nullptr) xh = (__nv_bfloat16 *)fz.src_cl;  // the caller keeps a channels-last copy of src
   else to_nhwc(src, xh, B, CH, g.Cp, SH * SW, st, use_plan ? fz.mask : nullptr);
   const int64_t wtotal = (int64_t)g.nblk * g.nchunks * g.Npb * kChunk;
   weight_image_kernel<<<cdiv(wtotal, 256), 256, 0, st>>>((const float *)wgt, wp, (int)Nout, (int)CH, g.Cp, (int)K, g.Npb, g.nblk,
-                                                         g.nchunks, sn, sc, sk);
+                                                         g.nchunks, sn, sc, sk, status);
   TcParams p{};
   p.g = Gather{xh, (const float *)map, (const float *)iw, plan, g.Cp, (int)SH, (int)SW, (int)K, (int)P, (int)GH, (int)GW, interp, g.nt};
   p.wp = wp; p.bias = (const float *)bias; p.out = (float *)out; p.status = status;
@@ -1724,7 +1801,7 @@ int tc_gemm(bool use_plan, const void *src, const void *map, const void *iw, con
   p.out_cl = (__nv_bfloat16 *)fz.out_cl;
   p.cl_pitch = fz.out_cl ? padded_channels(Nout) : 0;
   p.B = (int)B; p.Nout = (int)Nout; p.Npb = g.Npb; p.nblk = g.nblk; p.nchunks = g.nchunks;
-  p.tiles_x = cdiv(GW, kTW); p.tiles_y = cdiv(GH, kTH); p.stages = g.stages;
+  p.tiles_x = cdiv(GW, kTW); p.tiles_y = cdiv(GH, kTH); p.stages = g.stages; p.over = g.over;
   const int64_t tiles = (int64_t)B * p.tiles_x * p.tiles_y * g.nblk;
   const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
   if (use_plan) launch_gemm<MODE_PLAN, kPlanTaps>(p, grid, g.smem, st);
@@ -1794,15 +1871,16 @@ DwGeometry dw_geometry(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P,
   return d;
 }
 
-template <int NT, int GRP, bool WT>
+template <int NT, int GRP, bool WT, bool WQ = false>
 void launch_dw_g(const DwParams &p, dim3 grid, size_t smem, cudaStream_t st) {
   static int granted[kMaxDevices];
-  ensure_dynamic_smem(tc_dw_kernel<NT, GRP, WT>, granted, smem);
-  tc_dw_kernel<NT, GRP, WT><<<grid, kThreads, smem, st>>>(p);
+  ensure_dynamic_smem(tc_dw_kernel<NT, GRP, WT, WQ>, granted, smem);
+  tc_dw_kernel<NT, GRP, WT, WQ><<<grid, kThreads, smem, st>>>(p);
 }
 template <int NT>
 void launch_dw(const DwParams &p, int grp, bool warp_taps, dim3 grid, size_t smem, cudaStream_t st) {
   if (grp == 8) launch_dw_g<NT, 8, false>(p, grid, smem, st);
+  else if (warp_taps && NT == 4 && p.g.P > 0) launch_dw_g<4, 4, true, true>(p, grid, smem, st);
   else if (warp_taps && NT > 0) launch_dw_g<NT, 4, (NT > 0)>(p, grid, smem, st);
   else launch_dw_g<NT, 4, false>(p, grid, smem, st);
 }
@@ -1826,7 +1904,6 @@ int tc_dw(const void *A, const void *src, const void *map, const void *iw, int64
   __nv_bfloat16 *gt = (__nv_bfloat16 *)(w8 + 256 + d.xh_bytes);
   float *partial = (float *)(w8 + 256 + d.xh_bytes + d.gt_bytes);
   void *bias_ws = w8 + 256 + d.xh_bytes + d.gt_bytes + d.partial_bytes;
-  if (cudaMemsetAsync(status, 0, 4, st) != cudaSuccess) return SPH_ERR_CUDA;
   if (fz.src_cl != nullptr) xh = (__nv_bfloat16 *)fz.src_cl;  // the caller keeps a channels-last copy of src
   else to_nhwc(src, xh, B, CH, d.Cp, SH * SW, st);
   // When the operand being imaged is also the tensor whose channel sums give the bias gradient (conv dW:
@@ -1835,28 +1912,29 @@ int tc_dw(const void *A, const void *src, const void *map, const void *iw, int64
   const int64_t nblocks = B * d.tiles_x * d.tiles_y;
   float *row_part = (float *)((char *)bias_ws + simt_bias_workspace(Cbias, 4));
   float *part2 = (float *)((char *)row_part + align_up((size_t)nblocks * d.mbs_total * 128 * 4, 256));
-  if (!fz.gt_ready)  // (else the caller's combined pre-pass has filled gt and row_part already)
+  if (!fz.gt_ready)  // (else the caller's combined pre-pass has filled gt and row_part and cleared the status already)
     grad_image_kernel<<<dim3(d.tiles_x * d.tiles_y, d.mbs_total, (unsigned)B), 256, 0, st>>>(
         (const float *)A, gt, (int)Nout, (int)GH, (int)GW, d.tiles_x, d.tiles_y, d.mbs_total, fuse_bias ? row_part : nullptr,
-        (const float *)fz.mask, nullptr, 0);
+        (const float *)fz.mask, nullptr, 0, status);
   DwParams p{};
   p.g = Gather{xh, (const float *)map, (const float *)iw, nullptr, d.Cp, (int)SH, (int)SW, (int)K, (int)P, (int)GH, (int)GW, interp, d.nt};
   p.gt = gt; p.partial = partial; p.status = status;
   p.B = (int)B; p.mbs_total = d.mbs_total; p.nchunks = d.nchunks; p.tiles_x = d.tiles_x; p.tiles_y = d.tiles_y;
   p.splits = d.splits; p.stages = d.stages; p.tap_rows = d.tap_rows;
   dim3 grid(d.ngroups, d.splits, (d.mbs_total + 8 / d.grp - 1) / (8 / d.grp));
-  const bool warp_taps = d.Cp >= 64 && P == 0;  // one slot per chunk and one coordinate per slot
+  // one slot per chunk and a slot's coordinates in a thread's registers: one, or up to four weighted nearest points
+  const bool warp_taps = d.Cp >= 64 && (P == 0 || (P == 4 && interp == SPH_NEAREST));
   if (d.nt == 4) launch_dw<4>(p, d.grp, warp_taps, grid, d.smem, st);
   else if (d.nt == 1) launch_dw<1>(p, d.grp, warp_taps, grid, d.smem, st);
   else launch_dw<0>(p, d.grp, false, grid, d.smem, st);
-  tc_dw_reduce_kernel<<<cdiv(Nout * CH * K, 256), 256, 0, st>>>(partial, d.splits, d.mbs_total * 128, d.nchunks * kChunk, (int)Nout,
-                                                               (int)CH, d.Cp, (int)K, sn, sc, sk, (float *)gw);
-  note_launches(2 + (fz.src_cl ? 0 : 1) + (fz.gt_ready ? 0 : 1));
-  if (fuse_bias) {
+  if (fuse_bias)
     row_sum_split_kernel<<<dim3(cdiv(Cbias, 128), kRowSplits), 128, 0, st>>>(row_part, nblocks, d.mbs_total * 128, (int)Cbias, part2);
-    row_sum_final_kernel<<<cdiv(Cbias, 128), 128, 0, st>>>(part2, (int)Cbias, (float *)gb);
-    return launch_status(2);
-  }
+  const int gw_blocks = cdiv(Nout * CH * K, 256);
+  tc_dw_reduce_kernel<<<gw_blocks + (fuse_bias ? cdiv(Cbias, 8) : 0), 256, 0, st>>>(
+      partial, d.splits, d.mbs_total * 128, d.nchunks * kChunk, (int)Nout, (int)CH, d.Cp, (int)K, sn, sc, sk, (float *)gw, gw_blocks,
+      fuse_bias ? part2 : nullptr, (int)Cbias, (float *)gb);
+  note_launches(2 + (fz.src_cl ? 0 : 1) + (fz.gt_ready ? 0 : 1));
+  if (fuse_bias) return launch_status(1);
   return simt_bias_grad<float>(gbias_src, B, Cbias, nbias, gb, bias_ws, st);
 }
 
@@ -1973,12 +2051,9 @@ int tc_conv_backward(const void *gout, const void *x, const void *plan, const vo
     ~PhaseScope() { g_phase_count = 0; }
   } phase_scope;
   mark_phase(0, st);
-  // the zero pixel behind every image of the channels-last copy (unused taps point there)
-  if (gx && cudaMemset2DAsync((char *)go_cl + npix * cp_go * 2, (npix + 1) * cp_go * 2, 0, (size_t)cp_go * 2, (size_t)B, st) != cudaSuccess)
-    return SPH_ERR_CUDA;
   grad_image_kernel<<<dim3(d.tiles_x * d.tiles_y, d.mbs_total, (unsigned)B), 256, 0, st>>>(
       (const float *)gout, gt, (int)Cout, (int)OH, (int)OW, d.tiles_x, d.tiles_y, d.mbs_total, row_part, (const float *)fz.mask,
-      gx ? go_cl : nullptr, cp_go);  // (the copy serves the input gradient only)
+      gx ? go_cl : nullptr, cp_go, (int *)ws_dw);  // (the copy serves the input gradient only)
   note_launches(1);
   mark_phase(1, st);
   // channels between mbs_total * 128 and cp_go do not exist (cp_go <= mbs_total * 128), so the copy is complete
