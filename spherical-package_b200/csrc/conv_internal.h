@@ -17,13 +17,13 @@ namespace sph {
 // caller that keeps such copies next to its float32 activations passes them here and the conversion pre-passes
 // disappear: src_cl is the copy of the gathered tensor, out_cl (forward only) is where the epilogue also writes the
 // output in that layout (real channels and pixels only: the buffer is zero-filled once by its owner).
-// gt_ready (weight gradient): the gradient tile images and bias partial sums already sit in the workspace.
+// a_cl (weight gradient): channels-last copy of the left operand, masked; its row sums already sit in the workspace.
 struct Fusion {
   bool relu_out = false;
   const void *mask = nullptr;
   const void *src_cl = nullptr;
   void *out_cl = nullptr;
-  bool gt_ready = false;
+  const void *a_cl = nullptr;
   bool active() const { return relu_out || mask != nullptr; }
 };
 

@@ -899,40 +899,46 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcParams p, 
 // weight-gradient kernel
 // =================================================================================================
 constexpr int kDwPix = 64, kDwTH = 4;      // pixels per reduction step (a 4x16 block)
-// A CTA accumulates GRP chunks (of 64 columns) for MBS = 8 / GRP row blocks (of 128 rows): 512 TMEM columns either
-// way.  GRP = 4 holds two row blocks and is what the host selects; GRP = 8 (one row block, more map slots per step)
-// is kept for experiments.
-constexpr int kDwGtBytes = 128 * 128;                  // one 128-row x 64-pixel gradient tile image
+// A CTA accumulates up to four chunks (of 64 columns) for up to two row blocks (of 128 rows): 512 TMEM columns.  (One row
+// block with twice the chunks leaves room for only two pipeline stages and measured 1.9x slower on the encoder's layers.)
+constexpr int kDwGrp = 4, kDwMbs = 2;
+constexpr int kDwColBytes = kDwGrp * kDwPix * 128;     // gathered columns per stage
+constexpr int kDwABytes = kDwPix * 128;                // 64 pixels x 64 channels of the left operand
 constexpr int kDwMaxTapBytes = 20 * 1024;
 
 struct DwParams {
   Gather g;
-  const __nv_bfloat16 *gt;  // gradient tile images [b][ptile][mb][128 rows][64 px], 128B-swizzled
   float *partial;           // [splits][mbs_total*128][nchunks*64]
   int *status;
   int B, mbs_total, nchunks, tiles_x, tiles_y, splits, stages, tap_rows;
+  int a_blocks;             // 64-channel blocks of the left operand
 };
 
 struct DwSmem {
-  uint8_t *stage;  // per stage: columns (32 KB) then gradient tiles (mbs * 16 KB)
+  uint8_t *stage;  // per stage: columns (32 KB) then left-operand blocks (two of 8 KB per row block)
   Tap *taps;
   uint64_t *full, *empty, *tfull;
   uint32_t *tmem_ptr;
   volatile int *abort_flag;
 };
 
-inline size_t dw_stage_bytes(int grp, int mbs) { return (size_t)grp * kDwPix * 128 + (size_t)mbs * kDwGtBytes; }
-inline size_t dw_smem_bytes(int stages, int grp, int mbs, int tap_rows, int nt) {
-  return 1024 + stages * dw_stage_bytes(grp, mbs) + 2 * (size_t)tap_rows * kDwPix * nt * sizeof(Tap) + 8 * (2 * stages + 1) + 16;
+inline size_t dw_stage_bytes(int mbs) { return kDwColBytes + (size_t)mbs * 2 * kDwABytes; }
+inline size_t dw_smem_bytes(int stages, int mbs, int tap_rows, int nt) {
+  return 1024 + stages * dw_stage_bytes(mbs) + 2 * (size_t)tap_rows * kDwPix * nt * sizeof(Tap) + 8 * (2 * stages + 1) + 16;
 }
 
-// WT selects warp-private taps (unweighted maps or, WQ, weighted nearest ones of at most four points; Cp >= 64, NT > 0): every producer warp decodes the taps of its own
-// four pixels, one step ahead, into its own slice of the table, so the producers share nothing but the stage
-// barriers; otherwise the whole producer group fills one table per step and meets at a named barrier.
-template <int NT, int GRP, bool WT, bool WQ = false>
-__global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
-  constexpr int MBS = 8 / GRP;
-  constexpr int kDwColBytes = GRP * kDwPix * 128;  // gathered columns per stage
+// Both operands are MN-major: the left one (the gradient) arrives from its channels-last copy - the one that the
+// input-gradient kernel gathers from - as 4 x 16 pixel x 64 channel boxes of a tensor map with the 128-byte swizzle, loaded by
+// one thread of the otherwise idle epilogue warps; pixels outside the image and channels beyond the copy read as zero.
+// (A transposed image of its own cost the pre-pass two bytes per element more: encoder, batch 64, the gradient pre-passes
+// took 2.90 ms with it and take 2.01 ms without.)
+// WT selects warp-private taps (unweighted maps or, WQ, weighted nearest ones of at most four points; Cp >= 64, NT > 0):
+// every producer warp decodes the taps of its own four pixels, one step ahead, into its own slice of the table, so the
+// producers share nothing but the stage barriers; otherwise the whole producer group fills one table per step and meets at a
+// named barrier.
+template <int NT, bool WT, bool WQ = false>
+__global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p, const __grid_constant__ CUtensorMap a_map) {
+  constexpr int GRP = kDwGrp, MBS = kDwMbs;
   extern __shared__ uint8_t smem_raw[];
   const Gather &g = p.g;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -941,7 +947,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
   const int mbs = min(MBS, p.mbs_total - mb0);
   // column groups of equal width (at most GRP chunks): nine chunks make three groups of three, not four, four and one
   const int chunk0 = grp * p.nchunks / (int)gridDim.x, ncg = (grp + 1) * p.nchunks / (int)gridDim.x - chunk0;
-  const size_t stage_bytes = kDwColBytes + (size_t)mbs * kDwGtBytes;
+  const size_t stage_bytes = kDwColBytes + (size_t)mbs * 2 * kDwABytes;
 
   DwSmem sm;
   {
@@ -981,6 +987,25 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
   const int ncols_total = p.nchunks * kChunk;
 
   if (warp < kEpilogueWarps) {
+    if (tid == 0 && step_hi > step_lo) {
+      // ---------------- left operand: one thread loads the gradient boxes of every step ----------------
+      const int blocks = min(2 * mbs, p.a_blocks - 2 * mb0);  // (a last row block of at most 64 rows has one)
+      int ab = step_lo / tiles_per_image, aty = (step_lo % tiles_per_image) / p.tiles_x, atx = (step_lo % tiles_per_image) % p.tiles_x;
+      Ring ring;
+      for (int step = step_lo; step < step_hi; step++, ring.next(S)) {
+        const int s = ring.s;
+        if (!mbar_wait(sm.empty + s, ring.ph ^ 1u, sm.abort_flag)) break;
+        const uint32_t dst = smem_u32(sm.stage + (size_t)s * stage_bytes + kDwColBytes), bar = smem_u32(sm.full + s);
+        mbar_arrive_expect_tx_s(bar, (uint32_t)(blocks * kDwABytes));
+        for (int i = 0; i < blocks; i++)
+          tensor_load_4d(dst + i * kDwABytes, &a_map, (2 * mb0 + i) * 64, atx * kTW, aty * kDwTH, ab, bar);
+        if (++atx == p.tiles_x) {
+          atx = 0;
+          if (++aty == p.tiles_y) { aty = 0; ab++; }
+        }
+      }
+    }
+    __syncwarp();
     // ---------------- epilogue: TMEM -> partial sums ----------------
     bool have = step_hi > step_lo;
     if (have) have = mbar_wait(sm.tfull, 0, sm.abort_flag);
@@ -988,7 +1013,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
     for (int mb = 0; mb < mbs; mb++) {
       const int row = (mb0 + mb) * 128 + warp * 32 + lane;
       float *prow = p.partial + ((size_t)split * p.mbs_total * 128 + row) * ncols_total + (size_t)chunk0 * kChunk;
-      const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + mb * (GRP / 4) * 256;
+      const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + mb * 256;
       for (int n0 = 0; n0 < ncg * kChunk; n0 += 32) {
         uint32_t r[32];
         if (have) {
@@ -1008,10 +1033,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
   } else if (warp == kEpilogueWarps) {
     // ---------------- MMA issuer ----------------
     if (lane == 0 && step_hi > step_lo) {
-      // A (gradient) K-major, B (columns) MN-major; the column group is issued in halves of at most 4 chunks (N <= 256)
-      const int nhalves = (ncg + 3) / 4;
-      const uint32_t idesc0 = idesc_bf16(128, min(4, ncg) * kChunk, 0, 1);
-      const uint32_t idesc1 = idesc_bf16(128, max(1, ncg - 4) * kChunk, 0, 1);
+      const uint32_t idesc = idesc_bf16(128, ncg * kChunk, 1, 1);
       bool alive = true;
       int it = 0;
       Ring ring;
@@ -1020,15 +1042,13 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
         if (!mbar_wait(sm.full + s, ring.ph, sm.abort_flag)) { alive = false; break; }
         tc_fence_after();
         uint8_t *st = sm.stage + (size_t)s * stage_bytes;
+        const uint64_t b0 = smem_desc_sw128(smem_u32(st), kDwPix * 128, 1024);
         for (int mb = 0; mb < mbs; mb++) {
-          const uint64_t a0 = smem_desc_sw128(smem_u32(st + kDwColBytes + (size_t)mb * kDwGtBytes), 16, 1024);
-          for (int h = 0; h < nhalves; h++) {
-            const uint64_t b0 = smem_desc_sw128(smem_u32(st + h * 4 * (kDwPix * 128)), kDwPix * 128, 1024);
-            const uint32_t d = tmem_base + (mb * (GRP / 4) + h) * 256;
+          const uint64_t a0 = smem_desc_sw128(smem_u32(st + kDwColBytes + (size_t)mb * 2 * kDwABytes), kDwABytes, 1024);
 #pragma unroll
-            for (int ks = 0; ks < kDwPix / 16; ks++)
-              umma_bf16(d, a0 + 2 * ks, b0 + (uint64_t)(ks * 16 * 128 >> 4), h ? idesc1 : idesc0, (it | ks) != 0);
-          }
+          for (int ks = 0; ks < kDwPix / 16; ks++)
+            umma_bf16(tmem_base + mb * 256, a0 + (uint64_t)(ks * 16 * 128 >> 4), b0 + (uint64_t)(ks * 16 * 128 >> 4), idesc,
+                      (it | ks) != 0);
         }
         umma_commit(sm.empty + s);
       }
@@ -1038,7 +1058,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
     // ---------------- producers, warp-private taps ----------------
     // Thread = (chunk pair h, pixel pl, vector pair vp): one pixel and 32 bytes of it for two chunks of the group;
     // a warp covers 8 pixels of one chunk pair and decodes exactly the 16 (chunk, pixel) tap entries it reads.
-    static_assert(GRP == 4 && kProducerThreads == 2 * kDwPix * 4, "two chunk pairs x 64 pixels x 4 vector pairs");
+    static_assert(kProducerThreads == 2 * kDwPix * 4, "two chunk pairs x 64 pixels x 4 vector pairs");
     const int pt = tid - kFirstProducerThread, pw = pt >> 5;
     const int h = pt >> 8, pl = (pt & 255) >> 2, vp = pt & 3, pxl = lane >> 2;
     constexpr int kEnt = 16;                                   // (chunk of the pair, pixel) entries per warp and step
@@ -1132,12 +1152,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
       const bool ok = mbar_wait_s(empty0 + 8 * s, ring.ph ^ 1u, sm.abort_flag);
       if (!__all_sync(0xffffffffu, ok)) break;  // the whole warp leaves together
       const uint32_t st_s = stage0_s + (uint32_t)(s * stage_bytes);
-      if (pt == 0) {
-        const uint32_t bytes = (uint32_t)mbs * kDwGtBytes;
-        mbar_arrive_expect_tx(sm.full + s, bytes);
-        bulk_copy_g2s(sm.stage + (size_t)s * stage_bytes + kDwColBytes, p.gt + ((size_t)step * p.mbs_total + mb0) * (kDwGtBytes / 2),
-                      bytes, sm.full + s);
-      }
       const bool more = step + 1 < step_hi;
       int b_next = b_cur;
       if (more) {
@@ -1240,11 +1254,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
       if (alive && !mbar_wait(sm.empty + s, ring.ph ^ 1u, sm.abort_flag)) alive = false;
       if (!alive) { producer_bar(); continue; }
       uint8_t *st = sm.stage + (size_t)s * stage_bytes;
-      if (pt == 0) {
-        const uint32_t bytes = (uint32_t)mbs * kDwGtBytes;
-        mbar_arrive_expect_tx(sm.full + s, bytes);
-        bulk_copy_g2s(st + kDwColBytes, p.gt + ((size_t)step * p.mbs_total + mb0) * (kDwGtBytes / 2), bytes, sm.full + s);
-      }
       if (step + 1 < step_hi) fill_step(sm.taps + ((it + 1) & 1) * tap_half);  // also moves cur_b on for the next step
       // thread pt: 16-byte vector v = pt & 7 of pixel pt >> 3, two chunks of the group at a time
       {
@@ -1290,11 +1299,15 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p) {
 // zero (unused taps point there).  64 pixels x 64 channels per block: 256-byte row segments in, 128-byte
 // pixel rows out.
 // With `mask` (same shape as x) elements whose mask value is not positive are taken as zero (gradient of a fused ReLU).
+// With `row_part` the kernel also writes the sums of the (masked) float32 values over the block's pixels to
+// row_part[(b * gridDim.x + block) * rows_total + channel] (first stage of the bias gradient); with `status` it clears that word.
 __global__ void __launch_bounds__(256) nchw_to_nhwc_bf16_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ y,
-                                                                 int C, int Cp, int HW, const float *__restrict__ mask) {
+                                                                 int C, int Cp, int HW, const float *__restrict__ mask,
+                                                                 float *__restrict__ row_part, int rows_total, int *status) {
   __shared__ float tile[64][65];
   const int b = blockIdx.z, c0 = blockIdx.y * 64, p0 = blockIdx.x * 64;
   const int tid = threadIdx.x;
+  if (status != nullptr && (blockIdx.x | blockIdx.y | blockIdx.z | tid) == 0) *status = 0;
   // rows of every channel start 16-byte aligned
   const bool vec_ok = (HW & 3) == 0 && (((uintptr_t)x | (uintptr_t)mask) & 15) == 0;
 #pragma unroll
@@ -1324,6 +1337,12 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_bf16_kernel(const float *__r
     tile[c][q + 1] = f.y;
     tile[c][q + 2] = f.z;
     tile[c][q + 3] = f.w;
+    if (row_part) {
+      float sum = (f.x + f.y) + (f.z + f.w);
+#pragma unroll
+      for (int d = 1; d < 16; d <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+      if (q == 0) row_part[((size_t)b * gridDim.x + blockIdx.x) * rows_total + c0 + c] = sum;
+    }
   }
   __syncthreads();
 #pragma unroll
@@ -1358,84 +1377,7 @@ __global__ void weight_image_kernel(const float *__restrict__ w, __nv_bfloat16 *
   wp[(((int64_t)nb * nchunks + chunk) * Npb + n) * kChunk + (((col >> 3) ^ (n & 7)) << 3) + (col & 7)] = __float2bfloat16(v);
 }
 
-// Gradient (B, N, GH*GW) float32 -> bf16 tile images [b][ptile][mb][128 rows][64 px]; the 64 pixels of a tile
-// are a 4x16 block of the (GH, GW) grid; 16-byte vector v (8 pixels) of row r sits at position v ^ (r & 7).
-// With `row_part` the kernel also writes the sum of every row over the tile's pixels to
-// row_part[(b * tiles + tile) * mbs_total * 128 + row] (first stage of the bias gradient).
-// With `cl` the same (masked) values are also written as the channels-last bf16 copy (B, GH*GW + 1, cl_pitch) that the
-// input-gradient kernel gathers from, so the gradient is read from memory once for both of its consumers; the extra
-// zero pixel of every image is written too.  The kernel also clears a status word.
-constexpr int kClStride = 128 + 8;  // bf16 per staged pixel row: 16-byte aligned rows, shifted banks
-__global__ void __launch_bounds__(256) grad_image_kernel(const float *__restrict__ gsrc, __nv_bfloat16 *__restrict__ gt, int N,
-                                                          int GH, int GW, int tiles_x, int tiles_y, int mbs_total,
-                                                          float *__restrict__ row_part, const float *__restrict__ mask,
-                                                          __nv_bfloat16 *__restrict__ cl, int cl_pitch, int *status) {
-  __shared__ __align__(16) __nv_bfloat16 cls[64 * kClStride];  // [pixel of the 4x16 tile][channel of this 128-row block]
-  const int t2 = blockIdx.x, mb = blockIdx.y, b = blockIdx.z;
-  const int ty = t2 / tiles_x, tx = t2 % tiles_x;
-  const size_t npix = (size_t)GH * GW;
-  if (t2 == 0) {
-    if (mb == 0 && b == 0 && threadIdx.x == 0) *status = 0;
-    const int c = mb * 128 + threadIdx.x;
-    if (cl != nullptr && threadIdx.x < 128 && c < cl_pitch) cl[((size_t)b * (npix + 1) + npix) * cl_pitch + c] = __float2bfloat16(0.0f);
-  }
-  __nv_bfloat16 *dst = gt + (((size_t)b * tiles_x * tiles_y + t2) * mbs_total + mb) * (128 * 64);
-  for (int i = threadIdx.x; i < 128 * 8; i += 256) {
-    const int r = i >> 3, v = i & 7, n = mb * 128 + r;
-    float f[8];
-    {
-      // the 8 pixels of vector v are consecutive in one image row: two 16-byte loads when the row segment is
-      // inside the image and 16-byte aligned
-      const int y = ty * kDwTH + (v >> 1), x0 = tx * kTW + (v & 1) * 8;
-      const float *src = gsrc + ((size_t)b * N + n) * npix + (size_t)y * GW + x0;
-      const float *msk = mask ? mask + (src - gsrc) : nullptr;  // same shape: a fused ReLU's output
-      if (n < N && y < GH && x0 + 8 <= GW && (GW & 3) == 0 && (((uintptr_t)gsrc | (uintptr_t)mask) & 15) == 0) {
-        const float4 a = __ldg((const float4 *)src), c = __ldg((const float4 *)src + 1);
-        f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
-        f[4] = c.x; f[5] = c.y; f[6] = c.z; f[7] = c.w;
-        if (msk) {
-          const float4 ma = __ldg((const float4 *)msk), mc = __ldg((const float4 *)msk + 1);
-          const float mv[8] = {ma.x, ma.y, ma.z, ma.w, mc.x, mc.y, mc.z, mc.w};
-#pragma unroll
-          for (int e = 0; e < 8; e++) f[e] = mv[e] > 0.0f ? f[e] : 0.0f;
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; e++)
-          f[e] = (n < N && y < GH && x0 + e < GW && (!msk || __ldg(msk + e) > 0.0f)) ? __ldg(src + e) : 0.0f;
-      }
-    }
-    uint4 o;
-    o.x = pack_bf16(f[0], f[1]);
-    o.y = pack_bf16(f[2], f[3]);
-    o.z = pack_bf16(f[4], f[5]);
-    o.w = pack_bf16(f[6], f[7]);
-    *(uint4 *)(dst + r * 64 + ((v ^ (r & 7)) << 3)) = o;
-    if (cl != nullptr) {
-#pragma unroll
-      for (int e = 0; e < 8; e++) cls[(v * 8 + e) * kClStride + r] = __float2bfloat16(f[e]);
-    }
-    if (row_part) {
-      float sum = ((f[0] + f[1]) + (f[2] + f[3])) + ((f[4] + f[5]) + (f[6] + f[7]));
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 4);
-      if (v == 0) row_part[(((size_t)b * tiles_x * tiles_y + t2) * mbs_total + mb) * 128 + r] = sum;
-    }
-  }
-  if (cl != nullptr) {
-    __syncthreads();
-    // pixel v * 8 + e of the tile is (row v >> 1, column (v & 1) * 8 + e); 16 threads write one pixel's 128 channels
-    for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-      const int pl = i >> 4, vec = i & 15, v = pl >> 3, e = pl & 7;
-      const int y = ty * kDwTH + (v >> 1), x = tx * kTW + (v & 1) * 8 + e, c = mb * 128 + vec * 8;
-      if (y < GH && x < GW && c + 8 <= cl_pitch)
-        *(uint4 *)(cl + ((size_t)b * (npix + 1) + (size_t)y * GW + x) * cl_pitch + c) = *(const uint4 *)(cls + pl * kClStride + vec * 8);
-    }
-  }
-}
-
-// Second stage of the fused bias gradient: sums of kRowSplits ranges of the (image, tile) blocks, in order; the third is part
+// Second stage of the fused bias gradient: sums of kRowSplits ranges of the (image, pixel block) rows, in order; the third is part
 // of tc_dw_reduce_kernel.
 constexpr int kRowSplits = 256;
 __global__ void __launch_bounds__(128) row_sum_split_kernel(const float *__restrict__ row_part, int64_t nblocks, int rows_total, int C,
@@ -1628,9 +1570,9 @@ Geometry geometry(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int 
 }
 
 void to_nhwc(const void *src, __nv_bfloat16 *xh, int64_t B, int64_t CH, int Cp, int64_t HW, cudaStream_t st,
-             const void *mask = nullptr) {
-  nchw_to_nhwc_bf16_kernel<<<dim3(cdiv(HW + 1, 64), cdiv(Cp, 64), (unsigned)B), 256, 0, st>>>((const float *)src, xh, (int)CH, Cp, (int)HW,
-                                                                                          (const float *)mask);
+             const void *mask = nullptr, float *row_part = nullptr, int *status = nullptr) {
+  nchw_to_nhwc_bf16_kernel<<<dim3(cdiv(HW + 1, 64), cdiv(Cp, 64), (unsigned)B), 256, 0, st>>>(
+      (const float *)src, xh, (int)CH, Cp, (int)HW, (const float *)mask, row_part, cdiv(Cp, 64) * 64, status);
 }
 
 // Tensor map of the float32 output (B, Nout, GH, GW) with the epilogue's box: 16 pixels x 2 rows x kOutStageCh channels.
@@ -1688,15 +1630,16 @@ bool make_out_map(CUtensorMap *m, float *out, int64_t B, int64_t Nout, int64_t G
 }
 
 // Tensor map of a channels-last bf16 copy (B, GH*GW + 1, pitch) seen as (B, GH, GW, pitch) with the image stride of
-// GH*GW + 1 pixels; box = 16 channels x 16 pixels x 2 rows.
-bool make_cl_map(CUtensorMap *m, __nv_bfloat16 *cl, int64_t B, int64_t pitch, int64_t GH, int64_t GW) {
+// GH*GW + 1 pixels; box = box_c channels x 16 pixels x box_h rows.
+bool make_cl_map(CUtensorMap *m, __nv_bfloat16 *cl, int64_t B, int64_t pitch, int64_t GH, int64_t GW, int box_c = kOutStageCh,
+                 int box_h = 2, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn || cl == nullptr || (pitch & 7) != 0 || ((uintptr_t)cl & 15) != 0) return false;
   const cuuint64_t dims[4] = {(cuuint64_t)pitch, (cuuint64_t)GW, (cuuint64_t)GH, (cuuint64_t)B};
   const cuuint64_t strides[3] = {(cuuint64_t)pitch * 2, (cuuint64_t)GW * pitch * 2, (cuuint64_t)(GH * GW + 1) * pitch * 2};
-  const cuuint32_t box[4] = {(cuuint32_t)kOutStageCh, (cuuint32_t)kTW, 2, 1}, estr[4] = {1, 1, 1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, cl, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  const cuuint32_t box[4] = {(cuuint32_t)box_c, (cuuint32_t)kTW, (cuuint32_t)box_h, 1}, estr[4] = {1, 1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, cl, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+            CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int MODE, int NT, bool ROWS, bool LEAN>
@@ -1823,66 +1766,63 @@ size_t gemm_ws(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int int
 }
 
 struct DwGeometry {
-  int Cp, nchunks, ngroups, mbs_total, nt, stages, splits, tap_rows, tiles_x, tiles_y, grp;
-  size_t xh_bytes, gt_bytes, partial_bytes, bias_bytes, smem;
+  int Cp, nchunks, ngroups, mbs_total, nt, stages, splits, tap_rows, tiles_x, tiles_y, a_pitch, rows_total;
+  int64_t row_blocks;
+  size_t xh_bytes, a_bytes, partial_bytes, row_bytes, bias_bytes, smem;
   bool ok;
+  size_t total() const { return 256 + xh_bytes + a_bytes + partial_bytes + bias_bytes; }
+  size_t bias_at() const { return 256 + xh_bytes + a_bytes + partial_bytes; }
 };
 
+// own_a: the workspace holds the left operand's channels-last copy (the combined backward keeps it with the input gradient's).
+// Cbias, nbias: channels and pixels of the tensor whose sums are the bias gradient.
 DwGeometry dw_geometry(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int interp, int64_t Nout, int64_t GH,
-                       int64_t GW, int64_t Cbias) {
+                       int64_t GW, int64_t Cbias, int64_t nbias, bool own_a = true) {
   DwGeometry d{};
   d.Cp = padded_channels(CH);
+  d.a_pitch = padded_channels(Nout);
   d.nchunks = num_chunks(d.Cp, (int)K);
-  // GRP = 8 (one row block, twice the slots per step) leaves room for only two pipeline stages and measured
-  // 1.9x slower on the encoder's layers than GRP = 4 with three stages, so it is not selected.
-  d.grp = 4;
-  d.ngroups = (d.nchunks + d.grp - 1) / d.grp;
+  d.ngroups = (d.nchunks + kDwGrp - 1) / kDwGrp;
   d.mbs_total = (int)((Nout + 127) / 128);
   d.nt = (int)((P > 0 ? P : 1) * (interp == SPH_NEAREST ? 1 : 4));
-  d.tap_rows = d.Cp >= 64 ? d.grp : (int)std::min<int64_t>(K, (int64_t)d.grp * (64 / d.Cp));
+  d.tap_rows = d.Cp >= 64 ? kDwGrp : (int)std::min<int64_t>(K, (int64_t)kDwGrp * (64 / d.Cp));
   d.tiles_x = cdiv(GW, kTW);
   d.tiles_y = cdiv(GH, kDwTH);
-  const int mbs_cta = 8 / d.grp;
-  const int mbs = d.mbs_total >= mbs_cta ? mbs_cta : 1;
+  const int mbs = d.mbs_total >= kDwMbs ? kDwMbs : 1;
   d.ok = (size_t)d.tap_rows * kDwPix * d.nt * sizeof(Tap) <= (size_t)kDwMaxTapBytes;
   // pipeline depth: as for the forward-type kernel, stay within 196 KB of shared memory if two stages fit there
   // (layer-4 dW of the encoder: 3 stages at 209 KB 3.62 ms, 2 stages at 145 KB 3.32 ms)
   constexpr size_t kSoftLimit = 196 * 1024;
   d.stages = 4;
-  while (d.stages > 2 && dw_smem_bytes(d.stages, d.grp, mbs, d.tap_rows, d.nt) > kSoftLimit) d.stages--;
-  if (dw_smem_bytes(d.stages, d.grp, mbs, d.tap_rows, d.nt) > kSoftLimit) {
+  while (d.stages > 2 && dw_smem_bytes(d.stages, mbs, d.tap_rows, d.nt) > kSoftLimit) d.stages--;
+  if (dw_smem_bytes(d.stages, mbs, d.tap_rows, d.nt) > kSoftLimit) {
     d.stages = 4;
-    while (d.stages > 2 && dw_smem_bytes(d.stages, d.grp, mbs, d.tap_rows, d.nt) > (size_t)kSmemLimit) d.stages--;
+    while (d.stages > 2 && dw_smem_bytes(d.stages, mbs, d.tap_rows, d.nt) > (size_t)kSmemLimit) d.stages--;
   }
-  d.smem = dw_smem_bytes(d.stages, d.grp, mbs, d.tap_rows, d.nt);
+  d.smem = dw_smem_bytes(d.stages, mbs, d.tap_rows, d.nt);
   if (d.smem > (size_t)kSmemLimit) d.ok = false;
   const int64_t steps = B * d.tiles_x * d.tiles_y;
-  const int zdim = (d.mbs_total + mbs_cta - 1) / mbs_cta;
+  const int zdim = (d.mbs_total + kDwMbs - 1) / kDwMbs;
   int64_t s = sm_count() / (d.ngroups * zdim);
   if (s < 1) s = 1;
   if (s > steps) s = steps;
   d.splits = (int)s;
   d.xh_bytes = align_up((size_t)(B * (SHW + 1)) * d.Cp * 2, 256);
   if ((SHW + 1) * d.Cp * 2 >= ((int64_t)1 << 31)) d.ok = false;
-  d.gt_bytes = align_up((size_t)steps * d.mbs_total * kDwGtBytes, 256);
+  d.a_bytes = own_a ? align_up((size_t)(B * (GH * GW + 1)) * d.a_pitch * 2, 256) : 0;
   d.partial_bytes = align_up((size_t)d.splits * d.mbs_total * 128 * d.nchunks * kChunk * 4, 256);
-  d.bias_bytes = simt_bias_workspace(Cbias, 4) + align_up((size_t)steps * d.mbs_total * 128 * 4, 256) +
-                 align_up((size_t)kRowSplits * Cbias * 4, 256);
+  d.row_blocks = B * cdiv(nbias + 1, 64);  // one row of sums per block of the conversion
+  d.rows_total = (int)align_up((size_t)Cbias, 64);
+  d.row_bytes = align_up((size_t)d.row_blocks * d.rows_total * 4, 256);
+  d.bias_bytes = std::max(simt_bias_workspace(Cbias, 4), d.row_bytes + align_up((size_t)kRowSplits * Cbias * 4, 256));
   return d;
 }
 
-template <int NT, int GRP, bool WT, bool WQ = false>
-void launch_dw_g(const DwParams &p, dim3 grid, size_t smem, cudaStream_t st) {
+template <int NT, bool WT, bool WQ = false>
+void launch_dw(const DwParams &p, const CUtensorMap &a_map, dim3 grid, size_t smem, cudaStream_t st) {
   static int granted[kMaxDevices];
-  ensure_dynamic_smem(tc_dw_kernel<NT, GRP, WT, WQ>, granted, smem);
-  tc_dw_kernel<NT, GRP, WT, WQ><<<grid, kThreads, smem, st>>>(p);
-}
-template <int NT>
-void launch_dw(const DwParams &p, int grp, bool warp_taps, dim3 grid, size_t smem, cudaStream_t st) {
-  if (grp == 8) launch_dw_g<NT, 8, false>(p, grid, smem, st);
-  else if (warp_taps && NT == 4 && p.g.P > 0) launch_dw_g<4, 4, true, true>(p, grid, smem, st);
-  else if (warp_taps && NT > 0) launch_dw_g<NT, 4, (NT > 0)>(p, grid, smem, st);
-  else launch_dw_g<NT, 4, false>(p, grid, smem, st);
+  ensure_dynamic_smem(tc_dw_kernel<NT, WT, WQ>, granted, smem);
+  tc_dw_kernel<NT, WT, WQ><<<grid, kThreads, smem, st>>>(p, a_map);
 }
 
 // gw[n,ch,slot] = sum_{b,pix} A[b,n,pix] * im2col(src)[b,pix,(slot,ch)]; gb = sum of gbias_src over batch and pixels.
@@ -1890,59 +1830,60 @@ int tc_dw(const void *A, const void *src, const void *map, const void *iw, int64
           int64_t P, int64_t GH, int64_t GW, int interp, int64_t Nout, int64_t B, void *gw, int64_t sn, int64_t sc, int64_t sk,
           const void *gbias_src, int64_t Cbias, int64_t nbias, void *gb, void *ws, size_t ws_bytes, cudaStream_t st,
           const Fusion &fz = Fusion{}) {
-  const DwGeometry d = dw_geometry(B, CH, SH * SW, K, P, interp, Nout, GH, GW, Cbias);
-  // a masked gradient needs its bias sums from the (masked) imaging pass
-  if (fz.active() && (!d.ok || !(gbias_src == A && Cbias == Nout && nbias == GH * GW))) return SPH_ERR_UNSUPPORTED;
+  const DwGeometry d = dw_geometry(B, CH, SH * SW, K, P, interp, Nout, GH, GW, Cbias, nbias, fz.a_cl == nullptr);
+  // The bias gradient's sums ride along with the conversion of the tensor they are taken over, the left operand of a
+  // convolution and the gathered tensor of a transposed one.  A masked gradient needs its sums from the (masked) conversion.
+  const bool bias_of_a = gbias_src == A && Cbias == Nout && nbias == GH * GW;
+  const bool bias_of_src = !bias_of_a && gbias_src == src && Cbias == CH && nbias == SH * SW && fz.src_cl == nullptr;
+  if (fz.active() && (!d.ok || !bias_of_a)) return SPH_ERR_UNSUPPORTED;
   if (!d.ok)
     return simt_dw<float>(A, src, map, iw, CH, SH, SW, K, P, GH * GW, interp, Nout, B, gw, sn, sc, sk, gbias_src, Cbias, nbias, gb,
                           ws, ws_bytes, st);
-  if (!ws || ws_bytes < 256 + d.xh_bytes + d.gt_bytes + d.partial_bytes + d.bias_bytes) return SPH_ERR_WORKSPACE_TOO_SMALL;
+  if (!ws || ws_bytes < d.total()) return SPH_ERR_WORKSPACE_TOO_SMALL;
   if ((uintptr_t)ws & 255) return SPH_ERR_INVALID_ARGUMENT;  // vector loads and bulk copies assume the alignment
   char *w8 = (char *)ws;
   int *status = (int *)w8;
-  __nv_bfloat16 *xh = (__nv_bfloat16 *)(w8 + 256);
-  __nv_bfloat16 *gt = (__nv_bfloat16 *)(w8 + 256 + d.xh_bytes);
-  float *partial = (float *)(w8 + 256 + d.xh_bytes + d.gt_bytes);
-  void *bias_ws = w8 + 256 + d.xh_bytes + d.gt_bytes + d.partial_bytes;
+  __nv_bfloat16 *xh = (__nv_bfloat16 *)(w8 + 256), *a_cl = (__nv_bfloat16 *)(w8 + 256 + d.xh_bytes);
+  float *partial = (float *)(w8 + 256 + d.xh_bytes + d.a_bytes);
+  void *bias_ws = w8 + d.bias_at();
+  float *row_part = (float *)bias_ws, *part2 = (float *)((char *)bias_ws + d.row_bytes);
+  if (fz.a_cl != nullptr) a_cl = (__nv_bfloat16 *)fz.a_cl;  // converted (and masked) by the caller, status cleared, sums written
+  CUtensorMap a_map;
+  if (!make_cl_map(&a_map, a_cl, B, d.a_pitch, GH, GW, 64, kDwTH, CU_TENSOR_MAP_SWIZZLE_128B)) return SPH_ERR_CUDA;
+  if (fz.a_cl == nullptr) to_nhwc(A, a_cl, B, Nout, d.a_pitch, GH * GW, st, fz.mask, bias_of_a ? row_part : nullptr, status);
   if (fz.src_cl != nullptr) xh = (__nv_bfloat16 *)fz.src_cl;  // the caller keeps a channels-last copy of src
-  else to_nhwc(src, xh, B, CH, d.Cp, SH * SW, st);
-  // When the operand being imaged is also the tensor whose channel sums give the bias gradient (conv dW:
-  // both are grad_output), the sums ride along with the imaging pass instead of re-reading the tensor.
-  const bool fuse_bias = gbias_src == A && Cbias == Nout && nbias == GH * GW;
-  const int64_t nblocks = B * d.tiles_x * d.tiles_y;
-  float *row_part = (float *)((char *)bias_ws + simt_bias_workspace(Cbias, 4));
-  float *part2 = (float *)((char *)row_part + align_up((size_t)nblocks * d.mbs_total * 128 * 4, 256));
-  if (!fz.gt_ready)  // (else the caller's combined pre-pass has filled gt and row_part and cleared the status already)
-    grad_image_kernel<<<dim3(d.tiles_x * d.tiles_y, d.mbs_total, (unsigned)B), 256, 0, st>>>(
-        (const float *)A, gt, (int)Nout, (int)GH, (int)GW, d.tiles_x, d.tiles_y, d.mbs_total, fuse_bias ? row_part : nullptr,
-        (const float *)fz.mask, nullptr, 0, status);
+  else to_nhwc(src, xh, B, CH, d.Cp, SH * SW, st, nullptr, bias_of_src ? row_part : nullptr);
   DwParams p{};
   p.g = Gather{xh, (const float *)map, (const float *)iw, nullptr, d.Cp, (int)SH, (int)SW, (int)K, (int)P, (int)GH, (int)GW, interp, d.nt};
-  p.gt = gt; p.partial = partial; p.status = status;
+  p.partial = partial; p.status = status;
   p.B = (int)B; p.mbs_total = d.mbs_total; p.nchunks = d.nchunks; p.tiles_x = d.tiles_x; p.tiles_y = d.tiles_y;
-  p.splits = d.splits; p.stages = d.stages; p.tap_rows = d.tap_rows;
-  dim3 grid(d.ngroups, d.splits, (d.mbs_total + 8 / d.grp - 1) / (8 / d.grp));
-  // one slot per chunk and a slot's coordinates in a thread's registers: one, or up to four weighted nearest points
-  const bool warp_taps = d.Cp >= 64 && (P == 0 || (P == 4 && interp == SPH_NEAREST));
-  if (d.nt == 4) launch_dw<4>(p, d.grp, warp_taps, grid, d.smem, st);
-  else if (d.nt == 1) launch_dw<1>(p, d.grp, warp_taps, grid, d.smem, st);
-  else launch_dw<0>(p, d.grp, false, grid, d.smem, st);
+  p.splits = d.splits; p.stages = d.stages; p.tap_rows = d.tap_rows; p.a_blocks = cdiv(d.a_pitch, 64);
+  const dim3 grid(d.ngroups, d.splits, (d.mbs_total + kDwMbs - 1) / kDwMbs);
+  // warp-private taps: one slot per chunk, and a slot's coordinates in a thread's registers (one, or up to four weighted
+  // nearest points)
+  const bool one_slot = d.Cp >= 64;
+  if (d.nt == 4 && one_slot && P == 0) launch_dw<4, true>(p, a_map, grid, d.smem, st);
+  else if (d.nt == 4 && one_slot && interp == SPH_NEAREST) launch_dw<4, true, true>(p, a_map, grid, d.smem, st);
+  else if (d.nt == 4) launch_dw<4, false>(p, a_map, grid, d.smem, st);
+  else if (d.nt == 1 && one_slot && P == 0) launch_dw<1, true>(p, a_map, grid, d.smem, st);
+  else if (d.nt == 1) launch_dw<1, false>(p, a_map, grid, d.smem, st);
+  else launch_dw<0, false>(p, a_map, grid, d.smem, st);
+  const bool fuse_bias = bias_of_a || bias_of_src;
   if (fuse_bias)
-    row_sum_split_kernel<<<dim3(cdiv(Cbias, 128), kRowSplits), 128, 0, st>>>(row_part, nblocks, d.mbs_total * 128, (int)Cbias, part2);
+    row_sum_split_kernel<<<dim3(cdiv(Cbias, 128), kRowSplits), 128, 0, st>>>(row_part, d.row_blocks, d.rows_total, (int)Cbias, part2);
   const int gw_blocks = cdiv(Nout * CH * K, 256);
   tc_dw_reduce_kernel<<<gw_blocks + (fuse_bias ? cdiv(Cbias, 8) : 0), 256, 0, st>>>(
       partial, d.splits, d.mbs_total * 128, d.nchunks * kChunk, (int)Nout, (int)CH, d.Cp, (int)K, sn, sc, sk, (float *)gw, gw_blocks,
       fuse_bias ? part2 : nullptr, (int)Cbias, (float *)gb);
-  note_launches(2 + (fz.src_cl ? 0 : 1) + (fz.gt_ready ? 0 : 1));
+  note_launches(2 + (fz.src_cl ? 0 : 1) + (fz.a_cl ? 0 : 1));
   if (fuse_bias) return launch_status(1);
   return simt_bias_grad<float>(gbias_src, B, Cbias, nbias, gb, bias_ws, st);
 }
 
 size_t dw_ws(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int interp, int64_t Nout, int64_t GH, int64_t GW,
-             int64_t Cbias) {
-  const DwGeometry d = dw_geometry(B, CH, SHW, K, P, interp, Nout, GH, GW, Cbias);
-  if (!d.ok) return simt_dw_workspace(B, GH * GW, Nout, CH, K, Cbias, 4);
-  return 256 + d.xh_bytes + d.gt_bytes + d.partial_bytes + d.bias_bytes;
+             int64_t Cbias, int64_t nbias) {
+  const DwGeometry d = dw_geometry(B, CH, SHW, K, P, interp, Nout, GH, GW, Cbias, nbias);
+  return d.ok ? d.total() : simt_dw_workspace(B, GH * GW, Nout, CH, K, Cbias, 4);
 }
 
 }  // namespace
@@ -1987,10 +1928,10 @@ size_t tc_workspace_bytes(int op, int64_t B, int64_t Cin, int64_t Cout, int64_t 
   switch (op) {
     case SPH_CONV_FORWARD: return gemm_ws(B, Cin, IH * IW, K, P, interp, Cout, true);
     case SPH_CONV_BACKWARD_INPUT: return gemm_ws(B, Cout, OH * OW, K, 0, 0, Cin, false, IH * IW);
-    case SPH_CONV_BACKWARD_WEIGHT: return dw_ws(B, Cin, IH * IW, K, P, interp, Cout, OH, OW, Cout);
+    case SPH_CONV_BACKWARD_WEIGHT: return dw_ws(B, Cin, IH * IW, K, P, interp, Cout, OH, OW, Cout, OH * OW);
     case SPH_TCONV_FORWARD: return gemm_ws(B, Cin, IH * IW, K, 0, 0, Cout, false, OH * OW);
     case SPH_TCONV_BACKWARD_INPUT: return gemm_ws(B, Cout, OH * OW, K, P, interp, Cin, true);
-    case SPH_TCONV_BACKWARD_WEIGHT: return dw_ws(B, Cout, OH * OW, K, P, interp, Cin, IH, IW, Cout);
+    case SPH_TCONV_BACKWARD_WEIGHT: return dw_ws(B, Cout, OH * OW, K, P, interp, Cin, IH, IW, Cout, OH * OW);
     default: return 0;
   }
 }
@@ -2016,47 +1957,36 @@ int tc_conv_backward_weight(const void *gout, const void *x, const void *map, co
                ws_bytes, st, fz);
 }
 
-// Combined backward of one convolution.  grad_output feeds two kernels in two layouts - channels-last bf16 for the
-// input-gradient gather, 128-row tile images for the weight-gradient MMA - and, with a fused ReLU, has to be masked
-// for both.  One pre-pass reads it (and the mask) once and writes both, where the separate entry points read it
-// twice; the reference likewise computes all three gradients in one call
+// Combined backward of one convolution.  grad_output feeds two kernels, the input-gradient gather and the weight-gradient
+// MMA, from one channels-last bf16 copy and, with a fused ReLU, has to be masked for both.  One pre-pass reads it (and the
+// mask) once; the reference likewise computes all three gradients in one call
 // (ext_modules/include/layers/mapped_convolution_layer.h:89-134).  Workspace: the input-gradient part first, then
 // the weight-gradient part, each laid out as its own operator expects.
 size_t tc_conv_backward_workspace(int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH, int64_t OW,
                                   int64_t K, int64_t P, int interp) {
   const size_t a = gemm_ws(B, Cout, OH * OW, K, 0, 0, Cin, false, IH * IW);
-  const DwGeometry d = dw_geometry(B, Cin, IH * IW, K, P, interp, Cout, OH, OW, Cout);
+  const DwGeometry d = dw_geometry(B, Cin, IH * IW, K, P, interp, Cout, OH, OW, Cout, OH * OW, false);
   if (a == 0 || !d.ok) return 0;
-  return align_up(a, 256) + dw_ws(B, Cin, IH * IW, K, P, interp, Cout, OH, OW, Cout);
+  return align_up(a, 256) + d.total();
 }
 
 int tc_conv_backward(const void *gout, const void *x, const void *plan, const void *map, const void *iw, const void *weight,
                      void *gx, void *gw, void *gb, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH,
                      int64_t OW, int64_t K, int64_t P, int interp, void *ws, size_t ws_bytes, cudaStream_t st, const Fusion &fz) {
   const size_t dx_bytes = gemm_ws(B, Cout, OH * OW, K, 0, 0, Cin, false, IH * IW);
-  const DwGeometry d = dw_geometry(B, Cin, IH * IW, K, P, interp, Cout, OH, OW, Cout);
+  const DwGeometry d = dw_geometry(B, Cin, IH * IW, K, P, interp, Cout, OH, OW, Cout, OH * OW, false);
   if (dx_bytes == 0 || !d.ok) return SPH_ERR_UNSUPPORTED;  // one of the two runs on other kernels: use the separate entry points
-  const size_t dw_bytes = dw_ws(B, Cin, IH * IW, K, P, interp, Cout, OH, OW, Cout);
-  if (!ws || ws_bytes < align_up(dx_bytes, 256) + dw_bytes) return SPH_ERR_WORKSPACE_TOO_SMALL;
+  if (!ws || ws_bytes < align_up(dx_bytes, 256) + d.total()) return SPH_ERR_WORKSPACE_TOO_SMALL;
   if ((uintptr_t)ws & 255) return SPH_ERR_INVALID_ARGUMENT;
   char *ws_dx = (char *)ws, *ws_dw = (char *)ws + align_up(dx_bytes, 256);
-  // where the two operators expect their operands (see tc_gemm / tc_adjoint_premul and tc_dw)
-  const int cp_go = padded_channels(Cout);
-  __nv_bfloat16 *go_cl = (__nv_bfloat16 *)(ws_dx + 256);
-  __nv_bfloat16 *gt = (__nv_bfloat16 *)(ws_dw + 256 + d.xh_bytes);
-  char *bias_ws = ws_dw + 256 + d.xh_bytes + d.gt_bytes + d.partial_bytes;
-  float *row_part = (float *)(bias_ws + simt_bias_workspace(Cout, 4));
-  const size_t npix = (size_t)(OH * OW);
+  __nv_bfloat16 *go_cl = (__nv_bfloat16 *)(ws_dx + 256);  // where tc_gemm / tc_adjoint_premul keep their source
   struct PhaseScope {  // the event list is consumed by this call, whatever its outcome
     ~PhaseScope() { g_phase_count = 0; }
   } phase_scope;
   mark_phase(0, st);
-  grad_image_kernel<<<dim3(d.tiles_x * d.tiles_y, d.mbs_total, (unsigned)B), 256, 0, st>>>(
-      (const float *)gout, gt, (int)Cout, (int)OH, (int)OW, d.tiles_x, d.tiles_y, d.mbs_total, row_part, (const float *)fz.mask,
-      gx ? go_cl : nullptr, cp_go, (int *)ws_dw);  // (the copy serves the input gradient only)
+  to_nhwc(gout, go_cl, B, Cout, d.a_pitch, OH * OW, st, fz.mask, (float *)(ws_dw + d.bias_at()), (int *)ws_dw);
   note_launches(1);
   mark_phase(1, st);
-  // channels between mbs_total * 128 and cp_go do not exist (cp_go <= mbs_total * 128), so the copy is complete
   Fusion fx;
   fx.src_cl = go_cl;  // already masked
   int rc = SPH_OK;
@@ -2067,9 +1997,9 @@ int tc_conv_backward(const void *gout, const void *x, const void *plan, const vo
   mark_phase(2, st);
   Fusion fw;
   fw.src_cl = fz.src_cl;  // channels-last copy of x, if the caller keeps one
-  fw.gt_ready = true;
+  fw.a_cl = go_cl;
   rc = tc_dw(gout, x, map, iw, Cin, IH, IW, K, P, OH, OW, interp, Cout, B, gw, Cin * K, K, 1, gout, Cout, OH * OW, gb, ws_dw,
-             dw_bytes, st, fw);
+             d.total(), st, fw);
   mark_phase(3, st);
   return rc;
 }

@@ -132,6 +132,17 @@ __device__ __forceinline__ void tensor_store_4d(const void *tmap, uint32_t src_s
                "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                : "memory");
 }
+// Tiled tensor load global -> shared through a tensor map, completion on an mbarrier.  The innermost coordinate times the
+// element size must be a multiple of 16 bytes; what lies outside the tensor reads as the map's fill value.  No multicast.
+__device__ __forceinline__ void tensor_load_4d(uint32_t dst_s, const void *tmap, int c0, int c1, int c2, int c3, uint32_t bar_s) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst_s),
+      "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar_s)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx_s(uint32_t bar_s, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_s), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // until the copies issued by this thread have read their shared-memory source (it may be overwritten then)
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
