@@ -378,7 +378,8 @@ int sph_mapped_conv_relu_backward_weight(const void *gout, const void *act_out, 
  * layers can keep the copies ("companions") next to its float32 activations:
  *   sph_conv_companion_bytes  size of the companion of a (B,C,H,W) tensor.
  *       The owner zero-fills it once (cudaMemsetAsync); the kernels only ever
- *       write real channels of real pixels.
+ *       write real channels of real pixels and zeros into the extra pixels, so
+ *       a companion whose Cp is C may start uninitialised.
  *   sph_mapped_conv_forward_cl  the forward operator (with the fused ReLU if
  *       relu != 0).  x_cl: companion of x, or NULL (then converted as usual).
  *       out_cl: if not NULL the kernel epilogue also writes the output as a

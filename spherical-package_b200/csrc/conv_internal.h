@@ -16,7 +16,7 @@ namespace sph {
 // (Cp = channels padded as padded_channels() says; pixel H*W of every image and the padding channels are zero).  A
 // caller that keeps such copies next to its float32 activations passes them here and the conversion pre-passes
 // disappear: src_cl is the copy of the gathered tensor, out_cl (forward only) is where the epilogue also writes the
-// output in that layout (real channels and pixels only: the buffer is zero-filled once by its owner).
+// output in that layout (real channels, and zeros into the extra pixels; padding channels are zero-filled once by the owner).
 // a_cl (weight gradient): channels-last copy of the left operand, masked; its row sums already sit in the workspace.
 struct Fusion {
   bool relu_out = false;
@@ -26,6 +26,26 @@ struct Fusion {
   const void *a_cl = nullptr;
   bool active() const { return relu_out || mask != nullptr; }
 };
+
+// ---- dependent launches ---------------------------------------------------
+// Launches `kernel` so that its blocks may start while the last blocks of the kernel launched before it on `st`, its pre-pass,
+// are still running; it waits for that kernel on the device (wait_for_launcher in tc_common.cuh).  Hides the launch gap and the
+// start of the kernel: one image through the encoder 197 -> 174 us together with the memsets that went into the
+// pre-passes.
+template <typename... KP, typename... A>
+inline void launch_after(void (*kernel)(KP...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &attr;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, KP(args)...);
+}
 
 // ---- exact SIMT kernels (conv_simt.cu) -----------------------------------
 template <typename T>

@@ -583,6 +583,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcParams p, 
   const int npix = g.GH * g.GW;
   const size_t shw = (size_t)g.SH * g.SW;
 
+  if (warp <= kEpilogueWarps) wait_for_launcher();  // (the producers: after their first tile's taps)
   if (warp < kEpilogueWarps) {
     // ---------------- epilogue: TMEM -> registers -> (+bias) -> global ----------------
     int tl = 0;
@@ -824,6 +825,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcParams p, 
           }
         }
       }
+      if (tile == (int)blockIdx.x) wait_for_launcher();
       producer_bar();
       if (pt == 0) { TC_TOC(t_fill, 0); TC_COUNT(7); }
       TC_TIC(t_loop);
@@ -1359,13 +1361,79 @@ __global__ void __launch_bounds__(256) nchw_to_nhwc_bf16_kernel(const float *__r
   }
 }
 
+// What a call's pre-pass clears besides: the status word and, if the call writes a channels-last copy of its output, the zero
+// pixel behind every image of it (`vecs` 16-byte vectors at p + b * step).
+struct Clears {
+  int *status;
+  uint4 *p;
+  int64_t step;
+  int vecs, B;
+};
+__device__ __forceinline__ void clear_all(const Clears &c) {
+  if (blockIdx.x != 0) return;
+  if (threadIdx.x == 0) *c.status = 0;
+  for (int i = threadIdx.x; i < c.B * c.vecs; i += blockDim.x) c.p[i / c.vecs * c.step + i % c.vecs] = make_uint4(0u, 0u, 0u, 0u);
+}
+Clears clears(int *status, const Fusion &fz, int64_t B, int64_t Nout, int64_t npix) {
+  Clears c{status, nullptr, 0, 0, 0};
+  if (fz.out_cl != nullptr) {
+    c.vecs = padded_channels(Nout) / 8;
+    c.step = (npix + 1) * c.vecs;
+    c.p = (uint4 *)fz.out_cl + npix * c.vecs;
+    c.B = (int)B;
+  }
+  return c;
+}
+
 // Weights -> bf16 tile images.  Row n of block nb, chunk `chunk`: 64 columns, 16-byte vector v stored at
-// position v ^ (n & 7) of the 128-byte row.  The source is addressed W[n*sn + ch*sc + slot*sk].
-// The kernel also clears the call's status word.
-__global__ void weight_image_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ wp, int Nout, int CH, int Cp,
-                                    int K, int Npb, int nblk, int nchunks, int64_t sn, int64_t sc, int64_t sk, int *status) {
+// position v ^ (n & 7) of the 128-byte row.  The source is addressed W[n*sn + ch*sc + slot*sk], sk = 1 or not.
+// Cp >= 64 (one slot per chunk): a block takes 8 rows x 64 channels x up to nine slots through shared memory, read in the order
+// in which they lie in the source and written as 16-byte vectors (one value per thread read with the stride of a slot group took
+// 5.3 us for 256 x 256 x 9, this takes 4.3).
+constexpr int kWiRows = 8, kWiSlots = 9, kWiPitch = kWiRows * 66 + 1;
+__global__ void __launch_bounds__(256) weight_image_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ wp, int Nout, int CH,
+                                                           int Cp, int K, int Npb, int nblk, int nchunks, int64_t sn, int64_t sc,
+                                                           int64_t sk, const Clears clr) {
+  __shared__ float tile[kWiSlots * kWiPitch];
+  launch_dependents();
+  clear_all(clr);
+  const int cblocks = Cp / 64, groups = (K + kWiSlots - 1) / kWiSlots;
+  const int grp = blockIdx.x % groups, cb = blockIdx.x / groups % cblocks, n0 = blockIdx.x / (groups * cblocks) * kWiRows;
+  const int k0 = grp * kWiSlots, nk = min(kWiSlots, K - k0);
+  const bool ch_inner = sc < sn;
+  const float *src = w + n0 * sn + cb * 64 * sc + k0 * sk;
+  constexpr int kLoads = kWiRows * 64 * kWiSlots / 256;
+  float f[kLoads];
+#pragma unroll
+  for (int it = 0; it < kLoads; it++) {  // all loads in flight
+    const int i = threadIdx.x + it * 256, k = i % kWiSlots, q = i / kWiSlots;
+    const int n = ch_inner ? q >> 6 : q & (kWiRows - 1), ch = ch_inner ? q & 63 : q / kWiRows;
+    f[it] = n0 + n < Nout && cb * 64 + ch < CH && k < nk ? __ldg(src + n * sn + ch * sc + k * sk) : 0.0f;
+  }
+#pragma unroll
+  for (int it = 0; it < kLoads; it++) {
+    const int i = threadIdx.x + it * 256, k = i % kWiSlots, q = i / kWiSlots;
+    const int n = ch_inner ? q >> 6 : q & (kWiRows - 1), ch = ch_inner ? q & 63 : q / kWiRows;
+    tile[k * kWiPitch + n * 66 + ch] = f[it];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kWiRows * 8 * nk; i += 256) {
+    const int v = i & 7, n = i >> 3 & (kWiRows - 1), k = i >> 6, ng = n0 + n, nb = ng / Npb, r = ng - nb * Npb;
+    const float *t = tile + k * kWiPitch + n * 66 + v * 8;
+    uint4 o;
+    o.x = pack_bf16(t[0], t[1]);
+    o.y = pack_bf16(t[2], t[3]);
+    o.z = pack_bf16(t[4], t[5]);
+    o.w = pack_bf16(t[6], t[7]);
+    *(uint4 *)(wp + (((int64_t)nb * nchunks + cb * K + k0 + k) * Npb + r) * kChunk + ((v ^ (r & 7)) << 3)) = o;
+  }
+}
+// Cp < 64: several slots per chunk, small images; one value per thread.
+__global__ void weight_image_narrow_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ wp, int Nout, int CH, int Cp, int K,
+                                           int Npb, int nblk, int nchunks, int64_t sn, int64_t sc, int64_t sk, const Clears clr) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) *status = 0;
+  launch_dependents();
+  clear_all(clr);
   const int64_t total = (int64_t)nblk * nchunks * Npb * kChunk;
   if (i >= total) return;
   const int col = (int)(i % kChunk), n = (int)((i / kChunk) % Npb), chunk = (int)((i / ((int64_t)kChunk * Npb)) % nchunks);
@@ -1397,6 +1465,7 @@ __global__ void __launch_bounds__(128) row_sum_split_kernel(const float *__restr
 __global__ void premul_weight_image_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ wp, int M, int Mp, int K,
                                            int CH, int Npb, int nblk, int nchunks, int64_t sm, int64_t sc, int64_t sk, int *status) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  launch_dependents();
   if (i == 0) *status = 0;
   const int64_t total = (int64_t)nblk * nchunks * Npb * kChunk;
   if (i >= total) return;
@@ -1652,7 +1721,7 @@ void launch_gemm_l(TcParams p, int grid, size_t smem, cudaStream_t st) {
   if (p.use_out_map && p.out_cl != nullptr && !make_cl_map(&cl_map, p.out_cl, p.B, p.cl_pitch, p.g.GH, p.g.GW)) p.use_out_map = 0;
   static int granted[kMaxDevices];
   ensure_dynamic_smem(tc_gemm_kernel<MODE, NT, ROWS, LEAN>, granted, smem);
-  tc_gemm_kernel<MODE, NT, ROWS, LEAN><<<grid, kThreads, smem, st>>>(p, out_map, cl_map);
+  launch_after(tc_gemm_kernel<MODE, NT, ROWS, LEAN>, dim3(grid), kThreads, smem, st, p, out_map, cl_map);
 }
 template <int MODE, int NT, bool ROWS = false>
 void launch_gemm(const TcParams &p, int grid, size_t smem, cudaStream_t st) {
@@ -1734,9 +1803,13 @@ int tc_gemm(bool use_plan, const void *src, const void *map, const void *iw, con
   __nv_bfloat16 *wp = (__nv_bfloat16 *)((char *)ws + 256 + g.xh_bytes);
   if (fz.src_cl != nullptr) xh = (__nv_bfloat16 *)fz.src_cl;  // the caller keeps a channels-last copy of src
   else to_nhwc(src, xh, B, CH, g.Cp, SH * SW, st, use_plan ? fz.mask : nullptr);
-  const int64_t wtotal = (int64_t)g.nblk * g.nchunks * g.Npb * kChunk;
-  weight_image_kernel<<<cdiv(wtotal, 256), 256, 0, st>>>((const float *)wgt, wp, (int)Nout, (int)CH, g.Cp, (int)K, g.Npb, g.nblk,
-                                                         g.nchunks, sn, sc, sk, status);
+  const Clears clr = clears(status, fz, B, Nout, GH * GW);
+  if (g.Cp >= 64)  // (Npb is a multiple of 16: a block's rows lie in one row block)
+    weight_image_kernel<<<g.nblk * g.Npb / kWiRows * (g.Cp / 64) * cdiv(K, kWiSlots), 256, 0, st>>>(
+        (const float *)wgt, wp, (int)Nout, (int)CH, g.Cp, (int)K, g.Npb, g.nblk, g.nchunks, sn, sc, sk, clr);
+  else
+    weight_image_narrow_kernel<<<cdiv((int64_t)g.nblk * g.nchunks * g.Npb * kChunk, 256), 256, 0, st>>>(
+        (const float *)wgt, wp, (int)Nout, (int)CH, g.Cp, (int)K, g.Npb, g.nblk, g.nchunks, sn, sc, sk, clr);
   TcParams p{};
   p.g = Gather{xh, (const float *)map, (const float *)iw, plan, g.Cp, (int)SH, (int)SW, (int)K, (int)P, (int)GH, (int)GW, interp, g.nt};
   p.wp = wp; p.bias = (const float *)bias; p.out = (float *)out; p.status = status;

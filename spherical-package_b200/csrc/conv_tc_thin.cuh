@@ -160,7 +160,8 @@ __global__ void __launch_bounds__(kThinThreads, 2) tc_thin_fwd_kernel(const Thin
   }
   // operand stages start as zeros (the padding columns are never written again); the weight block is copied once
   for (int i = tid; i < 2 * kAStageBytes / 16; i += kThinThreads) ((uint4 *)A)[i] = make_uint4(0, 0, 0, 0);
-  for (int i = tid; i < p.Npb * 8; i += kThinThreads) ((uint4 *)Bw)[i] = __ldg((const uint4 *)p.wp + i);
+  wait_for_launcher();
+  for (int i = tid; i < p.Npb * 8; i += kThinThreads) ((uint4 *)Bw)[i] = *((const uint4 *)p.wp + i);
   for (int i = tid; i < p.Npb; i += kThinThreads) bias_s[i] = (p.bias && i < p.Nout) ? __ldg(p.bias + i) : 0.0f;
   fence_proxy_async();
   if (warp == kEpilogueWarps) {
@@ -273,8 +274,10 @@ __global__ void __launch_bounds__(kThinThreads, 2) tc_thin_fwd_kernel(const Thin
 
 // Weight block of the thin forward: wp[n][j] = w[n*sn + c*sc + k*sk] for column j = k * CH + c, zero elsewhere.
 __global__ void thin_weight_image_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ wp, int Nout, int CH, int K, int Npb,
-                                         int64_t sn, int64_t sc, int64_t sk) {
+                                         int64_t sn, int64_t sc, int64_t sk, const Clears clr) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  launch_dependents();
+  clear_all(clr);
   if (i >= Npb * kChunk) return;
   const int col = i % kChunk, n = i / kChunk;
   float v = 0.0f;
@@ -295,7 +298,7 @@ template <int INTERP>
 void launch_thin_fwd(const ThinFwdParams &p, const CUtensorMap &out_map, const CUtensorMap &cl_map, int grid, size_t smem, cudaStream_t st) {
   static int granted[kMaxDevices];
   ensure_dynamic_smem(tc_thin_fwd_kernel<INTERP>, granted, smem);
-  tc_thin_fwd_kernel<INTERP><<<grid, kThinThreads, smem, st>>>(p, out_map, cl_map);
+  launch_after(tc_thin_fwd_kernel<INTERP>, dim3(grid), kThinThreads, smem, st, p, out_map, cl_map);
 }
 
 // Out[b, n, pix] = bias[n] + sum_j Col[b, pix, j] * W[n, j] (+ ReLU, + channels-last bf16 copy) for a thin gathered side.
@@ -313,7 +316,6 @@ int tc_thin_forward(const void *src, const void *map, const void *iw, int64_t CH
   if (fz.out_cl != nullptr && !make_cl_map(&cl_map, (__nv_bfloat16 *)fz.out_cl, B, padded_channels(Nout), GH, GW)) return SPH_ERR_UNSUPPORTED;
   int *status = (int *)ws;
   __nv_bfloat16 *wp = (__nv_bfloat16 *)((char *)ws + 256);
-  if (cudaMemsetAsync(status, 0, 4, st) != cudaSuccess) return SPH_ERR_CUDA;
   ThinFwdParams p{};
   p.src = (const float *)src; p.map = (const float *)map; p.iw = (const float *)iw; p.wp = wp; p.bias = (const float *)bias;
   p.status = status;
@@ -322,7 +324,8 @@ int tc_thin_forward(const void *src, const void *map, const void *iw, int64_t CH
   p.relu = fz.relu_out ? 1 : 0; p.has_cl = fz.out_cl != nullptr ? 1 : 0;
   p.tmem_cols = 32;
   while (p.tmem_cols < 2 * p.Npb) p.tmem_cols *= 2;
-  thin_weight_image_kernel<<<cdiv(p.Npb * kChunk, 256), 256, 0, st>>>((const float *)wgt, wp, (int)Nout, (int)CH, (int)K, p.Npb, sn, sc, sk);
+  thin_weight_image_kernel<<<cdiv(p.Npb * kChunk, 256), 256, 0, st>>>((const float *)wgt, wp, (int)Nout, (int)CH, (int)K, p.Npb, sn, sc, sk,
+                                                                   clears(status, fz, B, Nout, GH * GW));
   const int64_t tiles = (int64_t)B * p.tiles_x * p.tiles_y;
   const int grid = (int)std::min<int64_t>(tiles, 2 * (int64_t)sm_count());
   const size_t smem = thin_fwd_smem(p.Npb);
@@ -600,8 +603,9 @@ __global__ void __launch_bounds__(kThinThreads, 2) tc_thin_bwd_kernel(const Thin
 
 // Wt[j][o] = w[o*so + c*sc + k*sk] for row j = k * CH + c (zero elsewhere), 128 rows x 64 columns, 128B-swizzled.
 __global__ void thin_wt_image_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ wt, int N, int CH, int K, int64_t so,
-                                     int64_t sc, int64_t sk) {
+                                     int64_t sc, int64_t sk, int *status) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *status = 0;
   if (i >= 128 * kChunk) return;
   const int o = i % kChunk, j = i / kChunk;
   float v = 0.0f;
@@ -719,7 +723,7 @@ int tc_thin_backward(const void *gout, const void *act, const void *x, const voi
   if ((uintptr_t)ws & 255) return SPH_ERR_INVALID_ARGUMENT;
   char *w8 = (char *)ws;
   int *status = (int *)w8;
-  if (cudaMemsetAsync(status, 0, 4, st) != cudaSuccess) return SPH_ERR_CUDA;
+  if (!do_dx && cudaMemsetAsync(status, 0, 4, st) != cudaSuccess) return SPH_ERR_CUDA;
   ThinBwdParams p{};
   p.gout = (const float *)gout; p.act = (const float *)act; p.src = (const float *)x; p.map = (const float *)map; p.iw = (const float *)iw;
   p.wt = (const __nv_bfloat16 *)(w8 + L.off_wt); p.t2 = (__nv_bfloat16 *)(w8 + L.off_t2); p.partial = (float *)(w8 + L.off_partial);
@@ -735,7 +739,7 @@ int tc_thin_backward(const void *gout, const void *act, const void *x, const voi
   mark_phase(0, st);
   if (do_dx)
     thin_wt_image_kernel<<<cdiv(128 * kChunk, 256), 256, 0, st>>>((const float *)weight, (__nv_bfloat16 *)(w8 + L.off_wt), (int)N, (int)CH,
-                                                                (int)K, CH * K, K, 1);
+                                                                (int)K, CH * K, K, 1, status);
   mark_phase(1, st);
   SPH_DISPATCH_INTERP(interp, launch_thin_bwd<INTERP>(p, L.grid, st));
   if (do_dw)

@@ -394,6 +394,8 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
   const int seg = p.nchunks <= kOneSeg ? kOneSeg : kSeg, nseg = (p.nchunks + seg - 1) / seg;
   const int nc = nseg == 1 ? 2 : 1;  // buffers of the small products
 
+  // (The producers of map modes wait after their first tile's taps; in plan mode, a wait inside the tile loop cost its gather 6 %.)
+  if (SRC == SRC_PLAN || warp <= kEpi) wait_for_launcher();
   if (warp < kEpi) {
     int sg = 0, tl = 0;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x, tl++) {
@@ -474,6 +476,7 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
       const char *img = g.xl + (size_t)b * image;
       producer_bar3();  // the previous tile's taps have been read
       fill_taps3<SRC>(g, taps, pv, plan_ok, 0, g.K, ty, tx, pt);
+      if (SRC != SRC_PLAN && tile == (int)blockIdx.x) wait_for_launcher();
       producer_bar3();
       if (!alive) continue;
       uint32_t self = 0u;
@@ -562,6 +565,7 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_dw_kernel(const Dw3 p) {
   const int lo = (int)(total * split / p.splits), hi = (int)(total * (split + 1) / p.splits);
   const int nseg = (hi - lo) * 4 / kSeg;
 
+  if (warp <= kEpi) wait_for_launcher();  // (the producers: after their first tile's taps)
   if (warp < kEpi) {
     int sg = 0;
     float *o = p.partial + ((size_t)split * p.mbs * 128 + mb * 128 + warp * 32 + lane) * (p.groups * kDwN) + grp * kDwN;
@@ -604,6 +608,7 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_dw_kernel(const Dw3 p) {
     };
     int image_of = lo / tiles_per_image, t2 = lo - image_of * tiles_per_image;  // image and tile of `tile`
     if (lo < hi) fill(t2, 0);
+    wait_for_launcher();
     Ring3 ring;
     bool alive = true;
     for (int tile = lo; tile < hi; tile++) {
@@ -728,6 +733,7 @@ __device__ __forceinline__ void weight_block(const Weight3 &q, int block) {
 // The pre-pass of x3_gemm in one launch: source, weights, the call's status word.
 __global__ void __launch_bounds__(256) gemm_prepare3_kernel(const Nhwc3 src, const Weight3 wgt, int *status) {
   __shared__ NhwcTile tile;
+  launch_dependents();
   if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
   if ((int)blockIdx.x < wgt.blocks) weight_block(wgt, blockIdx.x);
   else nhwc_block(src, blockIdx.x - wgt.blocks, tile);
@@ -786,6 +792,7 @@ __device__ __forceinline__ void grad_block(const Grad3 &q, int block) {
 // The pre-pass of x3_dw in one launch: gathered side, gradient tile images, the call's status word.
 __global__ void __launch_bounds__(256) dw_prepare3_kernel(const Nhwc3 src, const Grad3 grad, int *status) {
   __shared__ NhwcTile tile;
+  launch_dependents();
   if (blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
   if ((int)blockIdx.x < grad.blocks) grad_block(grad, blockIdx.x);
   else nhwc_block(src, blockIdx.x - grad.blocks, tile);
@@ -989,12 +996,12 @@ Nhwc3 nhwc3(const void *x, float *y, int64_t B, int64_t C, int Cp, int64_t HW, f
 template <int SRC> void launch_gemm3(const Gemm3 &p, int64_t tiles, size_t smem, cudaStream_t st) {
   static int granted[kMaxDev3];
   allow_smem3(x3_gemm_kernel<SRC>, granted, smem);
-  x3_gemm_kernel<SRC><<<(unsigned)std::min<int64_t>(tiles, sms3()), kThreads3, smem, st>>>(p);
+  launch_after(x3_gemm_kernel<SRC>, dim3((unsigned)std::min<int64_t>(tiles, sms3())), kThreads3, smem, st, p);
 }
 template <int SRC> void launch_dw3(const Dw3 &p, size_t smem, cudaStream_t st) {
   static int granted[kMaxDev3];
   allow_smem3(x3_dw_kernel<SRC>, granted, smem);
-  x3_dw_kernel<SRC><<<dim3(p.groups, p.splits, p.mbs), kThreads3, smem, st>>>(p);
+  launch_after(x3_dw_kernel<SRC>, dim3(p.groups, p.splits, p.mbs), kThreads3, smem, st, p);
 }
 
 }  // namespace

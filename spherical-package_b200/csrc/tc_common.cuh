@@ -152,6 +152,14 @@ __device__ __forceinline__ void sts32(uint32_t addr_s, uint32_t v) {
   asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr_s), "r"(v) : "memory");
 }
 
+// ---- dependent launches -----------------------------------------------------
+// A tensor-core kernel that follows its pre-pass is launched with programmatic stream serialization (launch_after in
+// conv_internal.h): its blocks may start once every block of the pre-pass has called launch_dependents() or ended, set up
+// their barriers and tensor memory and decode their first tile's taps, and call wait_for_launcher() before they touch
+// anything that the pre-pass writes.  The pre-pass itself is an ordinary launch, so everything before it is complete.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_launcher() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- tensor memory ----------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst_smem, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols)

@@ -229,19 +229,14 @@ const void *find_companion(const torch::Tensor &t) {
   return nullptr;
 }
 
-// Fresh companion buffer for a (B, C, H, W) activation: only the zero pixel behind every image (and, if the channel
-// count is padded, the padding) has to be cleared; the kernel writes the rest.
+// Fresh companion buffer for a (B, C, H, W) activation: only the padding, if the channel count is padded, has to be cleared; the
+// call writes the rest.
 torch::Tensor new_companion(const torch::Tensor &like, int64_t B, int64_t C, int64_t H, int64_t W) {
   const size_t bytes = sph_conv_companion_bytes(B, C, H, W);
   TORCH_CHECK(bytes > 0, "activation too large for a channels-last companion");
   const int64_t cp = sph_conv_companion_channels(C);
   if (cp != C) return torch::zeros({(int64_t)bytes}, like.options().dtype(torch::kUInt8));
-  torch::Tensor c = torch::empty({(int64_t)bytes}, like.options().dtype(torch::kUInt8));
-  const size_t px = (size_t)cp * 2, img = (size_t)(H * W + 1) * px;
-  TORCH_CHECK(cudaMemset2DAsync((char *)c.data_ptr() + (size_t)(H * W) * px, img, 0, px, (size_t)B,
-                                at::cuda::getCurrentCUDAStream().stream()) == cudaSuccess,
-              "clearing the companion's zero pixels failed");
-  return c;
+  return torch::empty({(int64_t)bytes}, like.options().dtype(torch::kUInt8));
 }
 
 void register_companion(const torch::Tensor &t, torch::Tensor companion) {
