@@ -906,6 +906,9 @@ constexpr int kDwPix = 64, kDwTH = 4;      // pixels per reduction step (a 4x16 
 constexpr int kDwGrp = 4, kDwMbs = 2;
 constexpr int kDwColBytes = kDwGrp * kDwPix * 128;     // gathered columns per stage
 constexpr int kDwABytes = kDwPix * 128;                // 64 pixels x 64 channels of the left operand
+// Four epilogue warps - idle until the end, so one thread of the first loads the left operand and one of the second issues the
+// MMAs - and the producers: 20 warps leave 96 registers per thread, a 21st would leave 80.
+constexpr int kDwFirstProducer = 32 * kEpilogueWarps, kDwThreads = kDwFirstProducer + kProducerThreads;
 constexpr int kDwMaxTapBytes = 20 * 1024;
 
 struct DwParams {
@@ -939,7 +942,7 @@ inline size_t dw_smem_bytes(int stages, int mbs, int tap_rows, int nt) {
 // producers share nothing but the stage barriers; otherwise the whole producer group fills one table per step and meets at a
 // named barrier.
 template <int NT, bool WT, bool WQ = false>
-__global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p, const __grid_constant__ CUtensorMap a_map) {
+__global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, const __grid_constant__ CUtensorMap a_map) {
   constexpr int GRP = kDwGrp, MBS = kDwMbs;
   extern __shared__ uint8_t smem_raw[];
   const Gather &g = p.g;
@@ -973,7 +976,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p, co
     *sm.abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == kEpilogueWarps) {
+  if (warp == 0) {
     tmem_alloc(sm.tmem_ptr, kTmemCols);
     tmem_relinquish();
   }
@@ -1007,6 +1010,29 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p, co
         }
       }
     }
+    // ---------------- MMA issuer: one thread of another ----------------
+    if (tid == 32 && step_hi > step_lo) {
+      const uint32_t idesc = idesc_bf16(128, ncg * kChunk, 1, 1);
+      bool alive = true;
+      int it = 0;
+      Ring ring;
+      for (int step = step_lo; alive && step < step_hi; step++, it++, ring.next(S)) {
+        const int s = ring.s;
+        if (!mbar_wait(sm.full + s, ring.ph, sm.abort_flag)) { alive = false; break; }
+        tc_fence_after();
+        uint8_t *st = sm.stage + (size_t)s * stage_bytes;
+        const uint64_t b0 = smem_desc_sw128(smem_u32(st), kDwPix * 128, 1024);
+        for (int mb = 0; mb < mbs; mb++) {
+          const uint64_t a0 = smem_desc_sw128(smem_u32(st + kDwColBytes + (size_t)mb * 2 * kDwABytes), kDwABytes, 1024);
+#pragma unroll
+          for (int ks = 0; ks < kDwPix / 16; ks++)
+            umma_bf16(tmem_base + mb * 256, a0 + (uint64_t)(ks * 16 * 128 >> 4), b0 + (uint64_t)(ks * 16 * 128 >> 4), idesc,
+                      (it | ks) != 0);
+        }
+        umma_commit(sm.empty + s);
+      }
+      if (alive) umma_commit(sm.tfull);
+    }
     __syncwarp();
     // ---------------- epilogue: TMEM -> partial sums ----------------
     bool have = step_hi > step_lo;
@@ -1032,69 +1058,54 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p, co
       }
     }
     tc_fence_before();
-  } else if (warp == kEpilogueWarps) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0 && step_hi > step_lo) {
-      const uint32_t idesc = idesc_bf16(128, ncg * kChunk, 1, 1);
-      bool alive = true;
-      int it = 0;
-      Ring ring;
-      for (int step = step_lo; alive && step < step_hi; step++, it++, ring.next(S)) {
-        const int s = ring.s;
-        if (!mbar_wait(sm.full + s, ring.ph, sm.abort_flag)) { alive = false; break; }
-        tc_fence_after();
-        uint8_t *st = sm.stage + (size_t)s * stage_bytes;
-        const uint64_t b0 = smem_desc_sw128(smem_u32(st), kDwPix * 128, 1024);
-        for (int mb = 0; mb < mbs; mb++) {
-          const uint64_t a0 = smem_desc_sw128(smem_u32(st + kDwColBytes + (size_t)mb * 2 * kDwABytes), kDwABytes, 1024);
-#pragma unroll
-          for (int ks = 0; ks < kDwPix / 16; ks++)
-            umma_bf16(tmem_base + mb * 256, a0 + (uint64_t)(ks * 16 * 128 >> 4), b0 + (uint64_t)(ks * 16 * 128 >> 4), idesc,
-                      (it | ks) != 0);
-        }
-        umma_commit(sm.empty + s);
-      }
-      if (alive) umma_commit(sm.tfull);
-    }
   } else if constexpr (WT && NT > 0) {
     // ---------------- producers, warp-private taps ----------------
-    // Thread = (chunk pair h, pixel pl, vector pair vp): one pixel and 32 bytes of it for two chunks of the group;
-    // a warp covers 8 pixels of one chunk pair and decodes exactly the 16 (chunk, pixel) tap entries it reads.
+    // Thread = (half h, pixel pl, vector pair vp): one pixel and 32 bytes of it.  The group's chunks fall into two sets, the
+    // larger first; the halves take one each and change places every step, so that three chunks load them equally over two
+    // steps.  A warp covers 8 pixels of one set and decodes exactly the up to 16 (chunk, pixel) tap entries it reads.  The
+    // loads roll: those of the next chunk (or step) go out as soon as a chunk's values are folded into the accumulators.
     static_assert(kProducerThreads == 2 * kDwPix * 4, "two chunk pairs x 64 pixels x 4 vector pairs");
-    const int pt = tid - kFirstProducerThread, pw = pt >> 5;
+    const int pt = tid - kDwFirstProducer, pw = pt >> 5;
     const int h = pt >> 8, pl = (pt & 255) >> 2, vp = pt & 3, pxl = lane >> 2;
     constexpr int kEnt = 16;                                   // (chunk of the pair, pixel) entries per warp and step
     constexpr uint32_t kEntBytes = NT * sizeof(Tap);
     const uint32_t wt_s = smem_u32(sm.taps) + pw * (2 * kEnt * kEntBytes);  // this warp's two table halves
-    // decoding role: lane e < 16 owns chunk 2h + (e >> 3) of the group and pixel e & 7 of the warp
-    const bool dec = lane < kEnt && (2 * h + (lane >> 3)) < ncg;
+    const int n0 = (ncg + 1) / 2;  // chunks 0 .. n0 - 1 of the group are set 0, the others set 1
+    // decoding role: lane e < 16 owns chunk e >> 3 of the set and pixel e & 7 of the warp
     const int e_pl = (pw & 7) * 8 + (lane & 7);
-    int e_slot = 0;
-    if (dec) { int c0; chunk_vec(g.Cp, g.K, chunk0 + 2 * h + (lane >> 3), 0, e_slot, c0); }
-    int coff[2];
+    int e_slot[2], coff[2][2];  // by set: the decoded slot (-1: none); byte offset of this thread's channels in a pixel
 #pragma unroll
-    for (int c = 0; c < 2; c++) {
-      int slot = 0, c0 = 0;
-      if (2 * h + c < ncg) chunk_vec(g.Cp, g.K, chunk0 + 2 * h + c, 2 * vp, slot, c0);
-      coff[c] = c0 * 2;
+    for (int t = 0; t < 2; t++) {
+      const int first = t ? n0 : 0, n = t ? ncg - n0 : n0;
+      int c0;
+      e_slot[t] = -1;
+      if (lane < kEnt && (lane >> 3) < n) chunk_vec(g.Cp, g.K, chunk0 + first + (lane >> 3), 0, e_slot[t], c0);
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        int slot;
+        c0 = 0;
+        if (c < n) chunk_vec(g.Cp, g.K, chunk0 + first + c, 2 * vp, slot, c0);
+        coff[t][c] = c0 * 2;
+      }
     }
     const int zero_off = g.SH * g.SW * g.Cp * 2;
     // position (image, tile row, tile column) of the step whose map coordinate is fetched next
     int nb_ = step_lo / tiles_per_image, nty = (step_lo % tiles_per_image) / p.tiles_x, ntx = (step_lo % tiles_per_image) % p.tiles_x;
-    int b_dec = 0, pix_dec = -1;
+    int b_dec = 0, pix_dec = -1, slot_dec = -1;
     constexpr int NP = WQ ? 4 : 1;
     float mx[NP], my[NP], mw[NP];
 #pragma unroll
     for (int i = 0; i < NP; i++) { mx[i] = my[i] = mw[i] = 0.0f; }
-    auto fetch = [&]() {  // issue the map loads of the next step; they complete under the current step's gather
+    auto fetch = [&](int set) {  // issue the map loads of the next step; they complete under the current step's gather
+      slot_dec = set ? e_slot[1] : e_slot[0];
       b_dec = nb_;
       pix_dec = tile_pixel(e_pl, nty, ntx, kDwTH, g.GH, g.GW);
       if (++ntx == p.tiles_x) {
         ntx = 0;
         if (++nty == p.tiles_y) { nty = 0; nb_++; }
       }
-      if (dec && pix_dec >= 0) {
-        const size_t e = ((size_t)pix_dec * g.K + e_slot) * (WQ ? g.P : 1);
+      if (slot_dec >= 0 && pix_dec >= 0) {
+        const size_t e = ((size_t)pix_dec * g.K + slot_dec) * (WQ ? g.P : 1);
 #pragma unroll
         for (int i = 0; i < NP; i++)
           if (!WQ || i < g.P) {
@@ -1107,7 +1118,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p, co
     auto decode_to = [&](uint32_t dst_s) {
       if (lane < kEnt) {
         Tap t[NT];
-        if (WQ && dec && pix_dec >= 0) {  // the points take the taps' places
+        if (WQ && slot_dec >= 0 && pix_dec >= 0) {  // the points take the taps' places
 #pragma unroll
           for (int i = 0; i < NT; i++) {
             Tap q[1];
@@ -1116,7 +1127,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p, co
             t[i].off = in ? q[0].off : zero_off;
             t[i].w = in ? tap_weight(mw[i < NP ? i : 0]) : 0u;
           }
-        } else if (dec && pix_dec >= 0) taps_from_xy<NT>(g, mx[0], my[0], t);
+        } else if (slot_dec >= 0 && pix_dec >= 0) taps_from_xy<NT>(g, mx[0], my[0], t);
         else {
 #pragma unroll
           for (int i = 0; i < NT; i++) { t[i].off = zero_off; t[i].w = 0u; }
@@ -1134,56 +1145,50 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p, co
         }
       }
     };
-    int b_cur = 0;
+    uint4 qa[NT], qb[NT];
+    uint32_t w[NT];
+    const auto issue = [&](uint32_t trow, const char *ic) {
+      if constexpr (NT == 4) {
+        const uint4 ta = lds128(trow), tb = lds128(trow + 16);
+        w[0] = ta.y; w[1] = ta.w; w[2] = tb.y; w[3] = tb.w;
+        ldg32(ic + (int)ta.x, qa[0], qb[0]);
+        ldg32(ic + (int)ta.z, qa[1], qb[1]);
+        ldg32(ic + (int)tb.x, qa[2], qb[2]);
+        ldg32(ic + (int)tb.z, qa[3], qb[3]);
+      } else {
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+          const uint2 tt = lds64(trow + 8 * t);
+          w[t] = tt.y;
+          ldg32(ic + (int)tt.x, qa[t], qb[t]);
+        }
+      }
+    };
+    const size_t image = (shw + 1) * g.Cp * 2;
+    const uint32_t my_taps = wt_s + pxl * kEntBytes;
+    const char *img = nullptr;
     if (step_lo < step_hi) {
-      fetch();
-      b_cur = b_dec;
+      fetch(h);
+      img = (const char *)g.xh + (size_t)b_dec * image;
       decode_to(wt_s);
     }
     __syncwarp();
+    if (step_lo < step_hi && (h == 0 || ncg > n0)) issue(my_taps, img + coff[h][0]);
     const uint32_t stage0_s = smem_u32(sm.stage);
     const uint32_t full0 = smem_u32(sm.full), empty0 = smem_u32(sm.empty);
     // this thread's two 16-byte slots of a chunk's row pl (128-byte swizzle)
     const uint32_t d0 = pl * 128 + (((2 * vp) ^ (pl & 7)) << 4), d1 = pl * 128 + (((2 * vp + 1) ^ (pl & 7)) << 4);
-    int it = 0;
+    int set = h, half = 0;
     Ring ring;
-    for (int step = step_lo; step < step_hi; step++, it++, ring.next(S)) {
-      const char *img = (const char *)g.xh + (size_t)b_cur * (shw + 1) * g.Cp * 2;
-      const uint32_t taps_s = wt_s + (it & 1) * (kEnt * kEntBytes) + pxl * kEntBytes;
-      const int s = ring.s;
+    for (int step = step_lo; step < step_hi; step++, ring.next(S)) {
+      const int n = set ? ncg - n0 : n0, n_next = ncg - n, s = ring.s;
+      const bool more = step + 1 < step_hi;
+      if (more) fetch(set ^ 1);
       const bool ok = mbar_wait_s(empty0 + 8 * s, ring.ph ^ 1u, sm.abort_flag);
       if (!__all_sync(0xffffffffu, ok)) break;  // the whole warp leaves together
-      const uint32_t st_s = stage0_s + (uint32_t)(s * stage_bytes);
-      const bool more = step + 1 < step_hi;
-      int b_next = b_cur;
-      if (more) {
-        fetch();
-        b_next = b_dec;
-      }
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        const int gi = 2 * h + c;
-        if (gi >= ncg) break;
-        uint4 qa[NT], qb[NT];
-        uint32_t w[NT];
-        const uint32_t trow = taps_s + c * (8 * kEntBytes);
-        if constexpr (NT == 4) {
-          const uint4 ta = lds128(trow), tb = lds128(trow + 16);
-          w[0] = ta.y; w[1] = ta.w; w[2] = tb.y; w[3] = tb.w;
-          const char *ic = img + coff[c];
-          ldg32(ic + (int)ta.x, qa[0], qb[0]);
-          ldg32(ic + (int)ta.z, qa[1], qb[1]);
-          ldg32(ic + (int)tb.x, qa[2], qb[2]);
-          ldg32(ic + (int)tb.z, qa[3], qb[3]);
-        } else {
-#pragma unroll
-          for (int t = 0; t < NT; t++) {
-            const uint2 tt = lds64(trow + 8 * t);
-            w[t] = tt.y;
-            ldg32(img + coff[c] + (int)tt.x, qa[t], qb[t]);
-          }
-        }
-        Acc8 a0, a1;
+      const uint32_t st_s = stage0_s + (uint32_t)(s * stage_bytes) + (set ? n0 : 0) * (kDwPix * 128);
+      Acc8 a0, a1;
+      if (n > 0) {
         acc_zero(a0);
         acc_zero(a1);
 #pragma unroll
@@ -1191,18 +1196,38 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p, co
           acc_fma(a0, w[t], qa[t]);
           acc_fma(a1, w[t], qb[t]);
         }
-        sts128(st_s + gi * (kDwPix * 128) + d0, acc_pack(a0));
-        sts128(st_s + gi * (kDwPix * 128) + d1, acc_pack(a1));
+        if (n > 1) issue(my_taps + half * (kEnt * kEntBytes) + 8 * kEntBytes, img + (set ? coff[1][1] : coff[0][1]));
+        sts128(st_s + d0, acc_pack(a0));
+        sts128(st_s + d1, acc_pack(a1));
       }
-      if (more) decode_to(wt_s + ((it + 1) & 1) * (kEnt * kEntBytes));
+      if (more) decode_to(wt_s + (half ^ 1) * (kEnt * kEntBytes));
+      __syncwarp();
+      if (n > 1) {
+        acc_zero(a0);
+        acc_zero(a1);
+#pragma unroll
+        for (int t = 0; t < NT; t++) {
+          acc_fma(a0, w[t], qa[t]);
+          acc_fma(a1, w[t], qb[t]);
+        }
+      }
+      set ^= 1;
+      half ^= 1;
+      if (more) {
+        img = (const char *)g.xh + (size_t)b_dec * image;
+        if (n_next > 0) issue(my_taps + half * (kEnt * kEntBytes), img + (set ? coff[1][0] : coff[0][0]));
+      }
+      if (n > 1) {
+        sts128(st_s + (kDwPix * 128) + d0, acc_pack(a0));
+        sts128(st_s + (kDwPix * 128) + d1, acc_pack(a1));
+      }
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive_s(full0 + 8 * s);
-      b_cur = b_next;
     }
   } else {
     // ---------------- producers, shared tap table ----------------
-    const int pt = tid - kFirstProducerThread;
+    const int pt = tid - kDwFirstProducer;
     bool alive = true;
     int it = 0;
     // table row r holds the taps of slot `slot_base + r`
@@ -1286,7 +1311,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_dw_kernel(const DwParams p, co
 
   tc_fence_before();
   __syncthreads();
-  if (warp == kEpilogueWarps) tmem_dealloc(tmem_base, kTmemCols);
+  if (warp == 0) tmem_dealloc(tmem_base, kTmemCols);
   if (tid == 0 && *sm.abort_flag) {
     *p.status = 1;
     g_wait_status = 1;
@@ -1895,7 +1920,7 @@ template <int NT, bool WT, bool WQ = false>
 void launch_dw(const DwParams &p, const CUtensorMap &a_map, dim3 grid, size_t smem, cudaStream_t st) {
   static int granted[kMaxDevices];
   ensure_dynamic_smem(tc_dw_kernel<NT, WT, WQ>, granted, smem);
-  tc_dw_kernel<NT, WT, WQ><<<grid, kThreads, smem, st>>>(p, a_map);
+  tc_dw_kernel<NT, WT, WQ><<<grid, kDwThreads, smem, st>>>(p, a_map);
 }
 
 // gw[n,ch,slot] = sum_{b,pix} A[b,n,pix] * im2col(src)[b,pix,(slot,ch)]; gb = sum of gbias_src over batch and pixels.
