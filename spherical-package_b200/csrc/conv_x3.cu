@@ -222,13 +222,25 @@ __device__ __forceinline__ V8 item_value(const Item<SRC> &it, const TapTable<SRC
       for (int i = 1; i < 4; i++) v.f[j] = fmaf(it.w[i], it.q[i].f[j], v.f[j]);
     }
     const uint2 r = lds64(t.rest + entry * 8);
-    for (int e = (int)r.x; e < (int)r.y; e++) {  // segments longer than the table
-      const int s = __ldg(pv.src + e);
-      if (!index_ok(s, pv.n_src)) continue;
-      const float w = __ldg(pv.w + e);
-      const V8 x = load8(img + (size_t)s * pitch);
+    if (r.x < r.y) {
+      // Segments longer than the table: the next entry's index and weight are on their way with this one's row.  (Each entry's
+      // loads in turn: 691 us for the input gradient of 64 -> 128 channels, 8 x 128 x 256; so 565 us; four rows in flight
+      // spill, 975 us.)
+      int s = __ldg(pv.src + r.x);
+      float w = __ldg(pv.w + r.x);
+      for (int e = (int)r.x + 1;; e++) {
+        const bool ok = index_ok(s, pv.n_src);
+        const V8 x = load8(img + (size_t)(ok ? s : 0) * pitch);
+        const float we = ok ? w : 0.0f;
+        const bool more = e < (int)r.y;
+        if (more) {
+          s = __ldg(pv.src + e);
+          w = __ldg(pv.w + e);
+        }
 #pragma unroll
-      for (int j = 0; j < 8; j++) v.f[j] = fmaf(w, x.f[j], v.f[j]);
+        for (int j = 0; j < 8; j++) v.f[j] = fmaf(we, x.f[j], v.f[j]);
+        if (!more) break;
+      }
     }
   }
   return v;
@@ -837,49 +849,65 @@ __global__ void __launch_bounds__(256) dw_reduce3_kernel(const Reduce3 q) {
 }
 
 // Second half of the multiply-first adjoint: out[b][m][q] (+bias) = sum over the plan entries (p, k, w) of destination pixel q, in
-// plan order, of w * T[b][p][k * Mp + m].  Thread = one destination pixel and VP output channels; an entry is one contiguous
-// run of its row.
-template <int VP>
-__global__ void __launch_bounds__(128) plan_gather_rows3_kernel(const float *__restrict__ T, const void *__restrict__ plan_blob,
+// plan order, of w * T[b][p][k * Mp + m].  L neighbouring threads share a destination pixel; each adds NV vectors of eight channels,
+// L apart, so that an instruction reads whole lines of a row.  The next entry's index and weight are on their way with this
+// one's row.  (Transposed 128 -> 64 channels, 8 x 128 x 256: one thread per pixel and 16 channels 92 us; so 69 us.)
+template <int NV, int L>
+__global__ void __launch_bounds__(256) plan_gather_rows3_kernel(const float *__restrict__ T, const void *__restrict__ plan_blob,
                                                                 const float *__restrict__ bias, float *__restrict__ out, int K, int M, int Mp,
                                                                 int n_src, int n_dst) {
-  const int q = blockIdx.x * 128 + threadIdx.x, m0 = blockIdx.y * VP, b = blockIdx.z;
-  if (q >= n_dst) return;
+  const int q = blockIdx.x * (256 / L) + threadIdx.x / L, m0 = (blockIdx.y * NV * L + threadIdx.x % L) * 8, b = blockIdx.z;
+  if (q >= n_dst || m0 >= Mp) return;
   bool ok;
   const PlanView<float> pv = plan_view<float>(plan_blob, n_dst * K, ok);
   const uint32_t pitch = (uint32_t)(K * Mp) * 4u;
   const char *rows = (const char *)(T + (size_t)b * n_src * (K * Mp) + m0);
-  V8 acc[VP / 8];
+  V8 acc[NV];
 #pragma unroll
-  for (int i = 0; i < VP / 8; i++)
+  for (int i = 0; i < NV; i++)
 #pragma unroll
     for (int j = 0; j < 8; j++) acc[i].f[j] = 0.0f;
   if (ok) {
     const int *off = pv.offsets + (size_t)q * K;
-    int e = __ldg(off);
+    int e = __ldg(off), e1 = __ldg(off + 1);
     const int end = __ldg(off + K);
-    for (int k = 0; k < K && e < end; k++, rows += Mp * 4) {
-      const int e1 = __ldg(off + k + 1);
-      for (; e < e1; e++) {
-        const int s = __ldg(pv.src + e);
-        if (!index_ok(s, n_src)) continue;
-        const float w = __ldg(pv.w + e);
-        const char *row = rows + (size_t)(unsigned)s * pitch;
-#pragma unroll
-        for (int i = 0; i < VP / 8; i++) {
-          const V8 v = load8(row + i * 32);
-#pragma unroll
-          for (int j = 0; j < 8; j++) acc[i].f[j] = fmaf(w, v.f[j], acc[i].f[j]);
-        }
+    int s = 0;
+    float w = 0.0f;
+    if (e < end) {
+      s = __ldg(pv.src + e);
+      w = __ldg(pv.w + e);
+    }
+    while (e < end) {
+      while (e >= e1) {
+        off++;
+        e1 = __ldg(off + 1);
+        rows += Mp * 4;
       }
+      const bool in = index_ok(s, n_src);
+      const float we = in ? w : 0.0f;
+      const char *row = rows + (size_t)(unsigned)(in ? s : 0) * pitch;
+      V8 v[NV];
+#pragma unroll
+      for (int i = 0; i < NV; i++)
+        if (i == 0 || m0 + i * L * 8 < Mp) v[i] = load8(row + i * L * 32);
+      if (++e < end) {
+        s = __ldg(pv.src + e);
+        w = __ldg(pv.w + e);
+      }
+#pragma unroll
+      for (int i = 0; i < NV; i++)
+        if (i == 0 || m0 + i * L * 8 < Mp)
+#pragma unroll
+          for (int j = 0; j < 8; j++) acc[i].f[j] = fmaf(we, v[i].f[j], acc[i].f[j]);
     }
   }
-  float *o = out + ((size_t)b * M + m0) * n_dst + q;
 #pragma unroll
-  for (int i = 0; i < VP / 8; i++)
+  for (int i = 0; i < NV; i++)
 #pragma unroll
-    for (int j = 0; j < 8; j++, o += n_dst)
-      if (m0 + i * 8 + j < M) *o = acc[i].f[j] + (bias ? __ldg(bias + m0 + i * 8 + j) : 0.0f);
+    for (int j = 0; j < 8; j++) {
+      const int m = m0 + i * L * 8 + j;
+      if (m < M) out[((size_t)b * M + m) * n_dst + q] = acc[i].f[j] + (bias ? __ldg(bias + m) : 0.0f);
+    }
 }
 
 // ---- host side -------------------------------------------------------------------------------------------------------------
@@ -1049,14 +1077,11 @@ int x3_gemm(bool use_plan, const void *src, const void *map, const void *iw, con
   }
   const int rc = launch_status(2);
   if (rc != SPH_OK || !r.use) return rc;
-  const int vp = r.Mp % 16 == 0 ? 16 : 8;
-  const dim3 grid(cdiv(GH * GW, 128), r.Mp / vp, (unsigned)B);
-  if (vp == 16)
-    plan_gather_rows3_kernel<16><<<grid, 128, 0, st>>>(T, plan, (const float *)bias, (float *)out, (int)K, (int)Nout, r.Mp, (int)(SH * SW),
-                                                       (int)(GH * GW));
-  else
-    plan_gather_rows3_kernel<8><<<grid, 128, 0, st>>>(T, plan, (const float *)bias, (float *)out, (int)K, (int)Nout, r.Mp, (int)(SH * SW),
-                                                      (int)(GH * GW));
+  const int vecs = r.Mp / 8, lanes = vecs >= 4 ? 4 : vecs >= 2 ? 2 : 1, nv = vecs > 4 ? 2 : 1;
+  const dim3 grid(cdiv(GH * GW, 256 / lanes), cdiv(vecs, nv * lanes), (unsigned)B);
+  const auto rows = nv == 2 ? plan_gather_rows3_kernel<2, 4>
+                            : (lanes == 4 ? plan_gather_rows3_kernel<1, 4> : lanes == 2 ? plan_gather_rows3_kernel<1, 2> : plan_gather_rows3_kernel<1, 1>);
+  rows<<<grid, 256, 0, st>>>(T, plan, (const float *)bias, (float *)out, (int)K, (int)Nout, r.Mp, (int)(SH * SW), (int)(GH * GW));
   return launch_status();
 }
 
