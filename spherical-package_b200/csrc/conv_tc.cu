@@ -1071,7 +1071,10 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
     constexpr uint32_t kEntBytes = NT * sizeof(Tap);
     const uint32_t wt_s = smem_u32(sm.taps) + pw * (2 * kEnt * kEntBytes);  // this warp's two table halves
     const int n0 = (ncg + 1) / 2;  // chunks 0 .. n0 - 1 of the group are set 0, the others set 1
-    // decoding role: lane e < 16 owns chunk e >> 3 of the set and pixel e & 7 of the warp
+    // decoding role: lane e < 16 owns chunk e >> 3 of the set and pixel e & 7 of the warp; with weighted points lanes e and
+    // e + 16 share the entry, two points each
+    const int ent = lane & (kEnt - 1), half_of = WQ ? lane >> 4 : 0;
+    const bool decodes = WQ || lane < kEnt;
     const int e_pl = (pw & 7) * 8 + (lane & 7);
     int e_slot[2], coff[2][2];  // by set: the decoded slot (-1: none); byte offset of this thread's channels in a pixel
 #pragma unroll
@@ -1079,7 +1082,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
       const int first = t ? n0 : 0, n = t ? ncg - n0 : n0;
       int c0;
       e_slot[t] = -1;
-      if (lane < kEnt && (lane >> 3) < n) chunk_vec(g.Cp, g.K, chunk0 + first + (lane >> 3), 0, e_slot[t], c0);
+      if (decodes && (ent >> 3) < n) chunk_vec(g.Cp, g.K, chunk0 + first + (ent >> 3), 0, e_slot[t], c0);
 #pragma unroll
       for (int c = 0; c < 2; c++) {
         int slot;
@@ -1092,7 +1095,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
     // position (image, tile row, tile column) of the step whose map coordinate is fetched next
     int nb_ = step_lo / tiles_per_image, nty = (step_lo % tiles_per_image) / p.tiles_x, ntx = (step_lo % tiles_per_image) % p.tiles_x;
     int b_dec = 0, pix_dec = -1, slot_dec = -1;
-    constexpr int NP = WQ ? 4 : 1;
+    constexpr int NP = WQ ? 2 : 1;
     float mx[NP], my[NP], mw[NP];
 #pragma unroll
     for (int i = 0; i < NP; i++) { mx[i] = my[i] = mw[i] = 0.0f; }
@@ -1105,10 +1108,10 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
         if (++nty == p.tiles_y) { nty = 0; nb_++; }
       }
       if (slot_dec >= 0 && pix_dec >= 0) {
-        const size_t e = ((size_t)pix_dec * g.K + slot_dec) * (WQ ? g.P : 1);
+        const size_t e = ((size_t)pix_dec * g.K + slot_dec) * (WQ ? g.P : 1) + 2 * half_of;
 #pragma unroll
         for (int i = 0; i < NP; i++)
-          if (!WQ || i < g.P) {
+          if (!WQ || 2 * half_of + i < g.P) {
             mx[i] = __ldg(g.map + 2 * (e + i));
             my[i] = __ldg(g.map + 2 * (e + i) + 1);
             if (WQ) mw[i] = __ldg(g.iw + e + i);
@@ -1116,32 +1119,33 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
       }
     };
     auto decode_to = [&](uint32_t dst_s) {
-      if (lane < kEnt) {
-        Tap t[NT];
-        if (WQ && slot_dec >= 0 && pix_dec >= 0) {  // the points take the taps' places
+      if (decodes) {
+        const bool any = slot_dec >= 0 && pix_dec >= 0;
+        constexpr int ND = WQ ? 2 : NT;  // taps this lane writes
+        Tap t[ND];
+        if constexpr (WQ) {  // the points take the taps' places
 #pragma unroll
-          for (int i = 0; i < NT; i++) {
+          for (int i = 0; i < ND; i++) {
             Tap q[1];
-            taps_from_xy<1>(g, mx[i < NP ? i : 0], my[i < NP ? i : 0], q);
-            const bool in = i < g.P && q[0].w != 0u;
+            taps_from_xy<1>(g, mx[i], my[i], q);
+            const bool in = any && 2 * half_of + i < g.P && q[0].w != 0u;
             t[i].off = in ? q[0].off : zero_off;
-            t[i].w = in ? tap_weight(mw[i < NP ? i : 0]) : 0u;
+            t[i].w = in ? tap_weight(mw[i]) : 0u;
           }
-        } else if (slot_dec >= 0 && pix_dec >= 0) taps_from_xy<NT>(g, mx[0], my[0], t);
-        else {
-#pragma unroll
-          for (int i = 0; i < NT; i++) { t[i].off = zero_off; t[i].w = 0u; }
-        }
-        const uint32_t d = dst_s + lane * kEntBytes;
-        if constexpr (NT == 4) {
-          sts128(d, make_uint4((uint32_t)t[0].off, t[0].w, (uint32_t)t[1].off, t[1].w));
-          sts128(d + 16, make_uint4((uint32_t)t[2].off, t[2].w, (uint32_t)t[3].off, t[3].w));
+        } else if (any) {
+          taps_from_xy<NT>(g, mx[0], my[0], t);
         } else {
 #pragma unroll
-          for (int i = 0; i < NT; i++) {
-            sts32(d + 8 * i, (uint32_t)t[i].off);
-            sts32(d + 8 * i + 4, t[i].w);
-          }
+          for (int i = 0; i < ND; i++) { t[i].off = zero_off; t[i].w = 0u; }
+        }
+        const uint32_t d = dst_s + ent * kEntBytes + half_of * 16;
+        if constexpr (ND > 1) {
+#pragma unroll
+          for (int i = 0; i < ND; i += 2)
+            sts128(d + 8 * i, make_uint4((uint32_t)t[i].off, t[i].w, (uint32_t)t[i + 1].off, t[i + 1].w));
+        } else {
+          sts32(d, (uint32_t)t[0].off);
+          sts32(d + 4, t[0].w);
         }
       }
     };
