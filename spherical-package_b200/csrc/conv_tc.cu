@@ -1071,10 +1071,11 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
     constexpr uint32_t kEntBytes = NT * sizeof(Tap);
     const uint32_t wt_s = smem_u32(sm.taps) + pw * (2 * kEnt * kEntBytes);  // this warp's two table halves
     const int n0 = (ncg + 1) / 2;  // chunks 0 .. n0 - 1 of the group are set 0, the others set 1
-    // decoding role: lane e < 16 owns chunk e >> 3 of the set and pixel e & 7 of the warp; with weighted points lanes e and
-    // e + 16 share the entry, two points each
-    const int ent = lane & (kEnt - 1), half_of = WQ ? lane >> 4 : 0;
-    const bool decodes = WQ || lane < kEnt;
+    // Decoding roles: lane e and lane e + 16 own chunk e >> 3 of the set and pixel e & 7 of the warp.  With weighted points they
+    // share the entry, two points each, and decode one step at a time; without, lane e decodes for one step and lane e + 16 for
+    // the step after it, every other step (its set is the other one: the same one every time).
+    constexpr int kAhead = WQ ? 1 : 2;  // steps decoded at a time
+    const int ent = lane & (kEnt - 1), hi = lane >> 4;
     const int e_pl = (pw & 7) * 8 + (lane & 7);
     int e_slot[2], coff[2][2];  // by set: the decoded slot (-1: none); byte offset of this thread's channels in a pixel
 #pragma unroll
@@ -1082,7 +1083,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
       const int first = t ? n0 : 0, n = t ? ncg - n0 : n0;
       int c0;
       e_slot[t] = -1;
-      if (decodes && (ent >> 3) < n) chunk_vec(g.Cp, g.K, chunk0 + first + (ent >> 3), 0, e_slot[t], c0);
+      if ((ent >> 3) < n) chunk_vec(g.Cp, g.K, chunk0 + first + (ent >> 3), 0, e_slot[t], c0);
 #pragma unroll
       for (int c = 0; c < 2; c++) {
         int slot;
@@ -1091,27 +1092,33 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
         coff[t][c] = c0 * 2;
       }
     }
+    if (!WQ) e_slot[0] = e_slot[h ^ hi];
     const int zero_off = g.SH * g.SW * g.Cp * 2;
-    // position (image, tile row, tile column) of the step whose map coordinate is fetched next
-    int nb_ = step_lo / tiles_per_image, nty = (step_lo % tiles_per_image) / p.tiles_x, ntx = (step_lo % tiles_per_image) % p.tiles_x;
-    int b_dec = 0, pix_dec = -1, slot_dec = -1;
+    // tile position of the step whose coordinates this lane fetches next, and that step
+    int nty = (step_lo % tiles_per_image) / p.tiles_x, ntx = (step_lo % tiles_per_image) % p.tiles_x, next = step_lo;
+    int pix_dec = -1, slot_dec = -1;
+    const auto advance = [&]() {
+      next++;
+      if (++ntx == p.tiles_x) {
+        ntx = 0;
+        if (++nty == p.tiles_y) nty = 0;
+      }
+    };
+    if (!WQ && hi) advance();
     constexpr int NP = WQ ? 2 : 1;
     float mx[NP], my[NP], mw[NP];
 #pragma unroll
     for (int i = 0; i < NP; i++) { mx[i] = my[i] = mw[i] = 0.0f; }
-    auto fetch = [&](int set) {  // issue the map loads of the next step; they complete under the current step's gather
-      slot_dec = set ? e_slot[1] : e_slot[0];
-      b_dec = nb_;
-      pix_dec = tile_pixel(e_pl, nty, ntx, kDwTH, g.GH, g.GW);
-      if (++ntx == p.tiles_x) {
-        ntx = 0;
-        if (++nty == p.tiles_y) { nty = 0; nb_++; }
-      }
+    auto fetch = [&](int set) {  // issue the map loads of the next step (or two); they complete under the current step's gather
+      slot_dec = (WQ && set) ? e_slot[1] : e_slot[0];
+      pix_dec = next < step_hi ? tile_pixel(e_pl, nty, ntx, kDwTH, g.GH, g.GW) : -1;
+#pragma unroll
+      for (int i = 0; i < kAhead; i++) advance();
       if (slot_dec >= 0 && pix_dec >= 0) {
-        const size_t e = ((size_t)pix_dec * g.K + slot_dec) * (WQ ? g.P : 1) + 2 * half_of;
+        const size_t e = ((size_t)pix_dec * g.K + slot_dec) * (WQ ? g.P : 1) + (WQ ? 2 * hi : 0);
 #pragma unroll
         for (int i = 0; i < NP; i++)
-          if (!WQ || 2 * half_of + i < g.P) {
+          if (!WQ || 2 * hi + i < g.P) {
             mx[i] = __ldg(g.map + 2 * (e + i));
             my[i] = __ldg(g.map + 2 * (e + i) + 1);
             if (WQ) mw[i] = __ldg(g.iw + e + i);
@@ -1119,34 +1126,32 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
       }
     };
     auto decode_to = [&](uint32_t dst_s) {
-      if (decodes) {
-        const bool any = slot_dec >= 0 && pix_dec >= 0;
-        constexpr int ND = WQ ? 2 : NT;  // taps this lane writes
-        Tap t[ND];
-        if constexpr (WQ) {  // the points take the taps' places
+      const bool any = slot_dec >= 0 && pix_dec >= 0;
+      constexpr int ND = WQ ? 2 : NT;  // taps this lane writes
+      Tap t[ND];
+      if constexpr (WQ) {  // the points take the taps' places
 #pragma unroll
-          for (int i = 0; i < ND; i++) {
-            Tap q[1];
-            taps_from_xy<1>(g, mx[i], my[i], q);
-            const bool in = any && 2 * half_of + i < g.P && q[0].w != 0u;
-            t[i].off = in ? q[0].off : zero_off;
-            t[i].w = in ? tap_weight(mw[i]) : 0u;
-          }
-        } else if (any) {
-          taps_from_xy<NT>(g, mx[0], my[0], t);
-        } else {
-#pragma unroll
-          for (int i = 0; i < ND; i++) { t[i].off = zero_off; t[i].w = 0u; }
+        for (int i = 0; i < ND; i++) {
+          Tap q[1];
+          taps_from_xy<1>(g, mx[i], my[i], q);
+          const bool in = any && 2 * hi + i < g.P && q[0].w != 0u;
+          t[i].off = in ? q[0].off : zero_off;
+          t[i].w = in ? tap_weight(mw[i]) : 0u;
         }
-        const uint32_t d = dst_s + ent * kEntBytes + half_of * 16;
-        if constexpr (ND > 1) {
+      } else if (any) {
+        taps_from_xy<NT>(g, mx[0], my[0], t);
+      } else {
 #pragma unroll
-          for (int i = 0; i < ND; i += 2)
-            sts128(d + 8 * i, make_uint4((uint32_t)t[i].off, t[i].w, (uint32_t)t[i + 1].off, t[i + 1].w));
-        } else {
-          sts32(d, (uint32_t)t[0].off);
-          sts32(d + 4, t[0].w);
-        }
+        for (int i = 0; i < ND; i++) { t[i].off = zero_off; t[i].w = 0u; }
+      }
+      const uint32_t d = dst_s + ent * kEntBytes + (WQ ? hi * 16 : 0);
+      if constexpr (ND > 1) {
+#pragma unroll
+        for (int i = 0; i < ND; i += 2)
+          sts128(d + 8 * i, make_uint4((uint32_t)t[i].off, t[i].w, (uint32_t)t[i + 1].off, t[i + 1].w));
+      } else {
+        sts32(d, (uint32_t)t[0].off);
+        sts32(d + 4, t[0].w);
       }
     };
     uint4 qa[NT], qb[NT];
@@ -1170,11 +1175,11 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
     };
     const size_t image = (shw + 1) * g.Cp * 2;
     const uint32_t my_taps = wt_s + pxl * kEntBytes;
-    const char *img = nullptr;
+    const char *img = (const char *)g.xh + (size_t)(step_lo / tiles_per_image) * image;
+    int left = tiles_per_image - step_lo % tiles_per_image;  // steps of this image from the current one on
     if (step_lo < step_hi) {
       fetch(h);
-      img = (const char *)g.xh + (size_t)b_dec * image;
-      decode_to(wt_s);
+      decode_to(wt_s + (WQ ? 0 : hi * (kEnt * kEntBytes)));
     }
     __syncwarp();
     if (step_lo < step_hi && (h == 0 || ncg > n0)) issue(my_taps, img + coff[h][0]);
@@ -1187,7 +1192,8 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
     for (int step = step_lo; step < step_hi; step++, ring.next(S)) {
       const int n = set ? ncg - n0 : n0, n_next = ncg - n, s = ring.s;
       const bool more = step + 1 < step_hi;
-      if (more) fetch(set ^ 1);
+      const bool decode = more && (WQ || half == 1);  // (two steps at a time: when the table holds this step only)
+      if (decode) fetch(set ^ 1);
       const bool ok = mbar_wait_s(empty0 + 8 * s, ring.ph ^ 1u, sm.abort_flag);
       if (!__all_sync(0xffffffffu, ok)) break;  // the whole warp leaves together
       const uint32_t st_s = stage0_s + (uint32_t)(s * stage_bytes) + (set ? n0 : 0) * (kDwPix * 128);
@@ -1204,8 +1210,11 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
         sts128(st_s + d0, acc_pack(a0));
         sts128(st_s + d1, acc_pack(a1));
       }
-      if (more) decode_to(wt_s + (half ^ 1) * (kEnt * kEntBytes));
-      __syncwarp();
+      if (decode) {
+        if (!WQ) __syncwarp();  // every lane has read this step's half of the table
+        decode_to(wt_s + (WQ ? half ^ 1 : hi) * (kEnt * kEntBytes));
+        __syncwarp();
+      }
       if (n > 1) {
         acc_zero(a0);
         acc_zero(a1);
@@ -1218,7 +1227,10 @@ __global__ void __launch_bounds__(kDwThreads, 1) tc_dw_kernel(const DwParams p, 
       set ^= 1;
       half ^= 1;
       if (more) {
-        img = (const char *)g.xh + (size_t)b_dec * image;
+        if (--left == 0) {
+          left = tiles_per_image;
+          img += image;
+        }
         if (n_next > 0) issue(my_taps + half * (kEnt * kEntBytes), img + (set ? coff[1][0] : coff[0][0]));
       }
       if (n > 1) {
