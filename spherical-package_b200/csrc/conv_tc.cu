@@ -47,6 +47,7 @@ constexpr int kEpilogueWarps = 4, kProducerWarps = 16;
 constexpr int kProducerThreads = 32 * kProducerWarps;
 constexpr int kThreads = 32 * (kEpilogueWarps + 1 + kProducerWarps);
 constexpr int kFirstProducerThread = 32 * (kEpilogueWarps + 1);
+constexpr int kRowThreads = 32 * (kEpilogueWarps + 2);  // the dense GEMM of the multiply-first adjoint: one loading warp
 constexpr int kSmemLimit = 227 * 1024;
 constexpr int kTmemCols = 512;
 
@@ -315,6 +316,8 @@ struct Smem {
 constexpr int kOutStageCh = 16;
 constexpr int kClStageBytes = kEpilogueWarps * 32 * kOutStageCh * 2;  // channels-last copy: [warp][2 rows][16 px][16 ch] bf16
 constexpr int kOutStageBytes = kEpilogueWarps * kOutStageCh * 32 * 4 + kClStageBytes;
+constexpr int kRowStage = 32 * 128;  // bf16 rows: [warp][2 buffers][32 pixels][64 columns], 128-byte swizzle
+constexpr int kRowStageBytes = kEpilogueWarps * 2 * kRowStage + 1024;
 
 inline size_t gemm_smem_bytes(int stages, int Npb, int K, int nt, bool direct, bool over = false) {
   size_t s = 1024;  // alignment slack
@@ -550,7 +553,7 @@ __device__ __forceinline__ bool produce_tile_lean(const TcParams &p, const Smem 
 // LEAN: channel copies of at least 64 padded channels with a static tap count - the producers run the lean per-chunk
 // loop and the instantiation carries no code for the general one (and the other way round).
 template <int MODE, int NT, bool ROWS = false, bool LEAN = false>
-__global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcParams p, const __grid_constant__ CUtensorMap out_map,
+__global__ void __launch_bounds__(ROWS ? kRowThreads : kThreads, 1) tc_gemm_kernel(const TcParams p, const __grid_constant__ CUtensorMap out_map,
                                                                const __grid_constant__ CUtensorMap cl_map) {
   extern __shared__ uint8_t smem_raw[];
   const Smem sm = carve(smem_raw, p, MODE == MODE_DIRECT);
@@ -560,7 +563,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcParams p, 
 
   if (tid == 0) {
     for (int s = 0; s < S; s++) {
-      mbar_init(sm.full + s, kProducerWarps + 1);
+      mbar_init(sm.full + s, ROWS ? 1 : kProducerWarps + 1);
       mbar_init(sm.empty + s, 1);
     }
     for (int i = 0; i < 2; i++) {
@@ -586,7 +589,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcParams p, 
   if (warp <= kEpilogueWarps) wait_for_launcher();  // (the producers: after their first tile's taps)
   if (warp < kEpilogueWarps) {
     // ---------------- epilogue: TMEM -> registers -> (+bias) -> global ----------------
-    int tl = 0;
+    int tl = 0, row_pass = 0;
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, tl++) {
       const int nb = tile % p.nblk, rest = tile / p.nblk;
       const int b = rest / tiles_per_image, t2 = rest % tiles_per_image;
@@ -651,6 +654,42 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcParams p, 
         if (tid == 0) { TC_TOC(t_drain, 6); }
         continue;
       }
+      if constexpr (ROWS) {
+        // bf16 rows, 64 columns of the warp's 32 pixels at a time: each pixel's 128 bytes go to one of two staging buffers
+        // (16-byte chunks XOR-swizzled, conflict-free) and leave as a tiled tensor store, which clips columns beyond the row
+        // and pixels outside the image.  The epilogue's own stores, 64 bytes per pixel through shared memory and back, bound
+        // this kernel (encoder layer 2, batch 64: 950 -> 895 us).
+        const uint32_t rows_s = ((smem_u32(sm.ostage) + 1023) & ~1023u) + warp * (2 * kRowStage);
+        for (int n0 = 0; n0 < p.Npb; n0 += 64, row_pass ^= 1) {
+          const uint32_t buf_s = rows_s + row_pass * kRowStage + lane * 128;
+          if (lane == 0) bulk_wait_read_but_last();  // this buffer's previous store has read it
+          __syncwarp();
+#pragma unroll
+          for (int half = 0; half < 2; half++) {
+            uint32_t r[32];
+            tmem_ld_32x32(taddr + n0 + half * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+              sts128(buf_s + (((half * 4 + j) ^ (lane & 7)) << 4),
+                     make_uint4(pack_bf16(__uint_as_float(r[8 * j]), __uint_as_float(r[8 * j + 1])),
+                                pack_bf16(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3])),
+                                pack_bf16(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5])),
+                                pack_bf16(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]))));
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            tensor_store_4d(&cl_map, buf_s, nb * p.Npb + n0, tx * kTW, ty * kTH + 2 * warp, b);
+            bulk_commit();
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(sm.tempty + buf);
+        if (tid == 0) { TC_TOC(t_drain, 6); }
+        continue;
+      }
       float *orow = p.out + ((size_t)b * p.Nout) * npix + (pix >= 0 ? pix : 0);
       for (int n0 = 0; n0 < p.Npb; n0 += 32) {
         uint32_t r[32];
@@ -663,31 +702,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcParams p, 
           for (int j = 0; j < 16; j++) { r[j] = h[j]; r[j + 16] = 0; }
         }
         tmem_ld_wait();
-        if constexpr (ROWS) {
-          // 32 consecutive columns of every pixel's row, as bf16 (out_pitch and Npb are multiples of 8).  A thread holds
-          // its own pixel's 64 bytes; stored directly, one instruction would touch 32 rows with 16 bytes each.  The warp's
-          // 32 x 64 bytes go through shared memory (16-byte chunks XOR-swizzled, conflict-free both ways) and leave with
-          // eight pixels of 64 contiguous bytes per instruction.
-          const uint32_t hs = smem_u32(sm.ostage) + warp * (kOutStageCh * 32 * 4);
-          __syncwarp();  // the previous pass has been read
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            sts128(hs + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4),
-                   make_uint4(pack_bf16(__uint_as_float(r[8 * j]), __uint_as_float(r[8 * j + 1])),
-                              pack_bf16(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3])),
-                              pack_bf16(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5])),
-                              pack_bf16(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]))));
-          __syncwarp();
-          const int c = lane & 3, col = nb * p.Npb + n0 + c * 8;
-#pragma unroll
-          for (int it = 0; it < 4; it++) {
-            const int pl = it * 8 + (lane >> 2);
-            const int ppix = tile_pixel(warp * 32 + pl, ty, tx, kTH, g.GH, g.GW);
-            const uint4 v = lds128(hs + pl * 64 + ((c ^ ((pl >> 1) & 3)) << 4));
-            if (ppix >= 0 && n0 + c * 8 < p.Npb && col < p.out_pitch)
-              *(uint4 *)(p.out_h + ((size_t)b * npix + ppix) * p.out_pitch + col) = v;
-          }
-        } else if (pix >= 0) {
+        if (pix >= 0) {
           float ov[32];
 #pragma unroll
           for (int j = 0; j < 32; j++) {
@@ -744,6 +759,28 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const TcParams p, 
           umma_commit(sm.empty + s);
         }
         if (alive) umma_commit(sm.tfull + buf);
+      }
+    }
+  } else if constexpr (ROWS) {
+    // ---------------- one thread loads both operands: boxes of 8 x 16 pixels x 64 channels of the dense source ----------------
+    // (out_map is the map of the source's channels-last copy here.)  Gathered by the producers like any other source, every
+    // tile of two or four chunks started with its loads' latency; with loads that run ahead over tiles 895 -> 600 us (encoder
+    // layer 2, batch 64), 121 -> 76 us (batch 8).
+    wait_for_launcher();
+    if (lane == 0) {
+      const uint32_t bbytes = (uint32_t)p.Npb * 128;
+      bool alive = true;
+      Ring ring;
+      for (int tile = blockIdx.x; alive && tile < total_tiles; tile += gridDim.x) {
+        const int nb = tile % p.nblk, rest = tile / p.nblk, b = rest / tiles_per_image, t2 = rest % tiles_per_image;
+        for (int chunk = 0; chunk < p.nchunks; chunk++, ring.next(S)) {
+          const int s = ring.s;
+          if (!mbar_wait(sm.empty + s, ring.ph ^ 1u, sm.abort_flag)) { alive = false; break; }
+          mbar_arrive_expect_tx(sm.full + s, bbytes + kAStageBytes);
+          bulk_copy_g2s(sm.Bw + (size_t)s * bbytes, p.wp + ((size_t)nb * p.nchunks + chunk) * p.Npb * kChunk, bbytes, sm.full + s);
+          tensor_load_4d(smem_u32(sm.A + (size_t)s * kAStageBytes), &out_map, chunk * kChunk, t2 % p.tiles_x * kTW, t2 / p.tiles_x * kTH, b,
+                         smem_u32(sm.full + s));
+        }
       }
     }
   } else {
@@ -1752,37 +1789,44 @@ bool make_out_map(CUtensorMap *m, float *out, int64_t B, int64_t Nout, int64_t G
 }
 
 // Tensor map of a channels-last bf16 copy (B, GH*GW + 1, pitch) seen as (B, GH, GW, pitch) with the image stride of
-// GH*GW + 1 pixels; box = box_c channels x 16 pixels x box_h rows.
+// GH*GW + 1 pixels (extra_pixels = 0: rows without the zero pixel); box = box_c channels x 16 pixels x box_h rows.
 bool make_cl_map(CUtensorMap *m, __nv_bfloat16 *cl, int64_t B, int64_t pitch, int64_t GH, int64_t GW, int box_c = kOutStageCh,
-                 int box_h = 2, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE) {
+                 int box_h = 2, CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE, int64_t extra_pixels = 1) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn || cl == nullptr || (pitch & 7) != 0 || ((uintptr_t)cl & 15) != 0) return false;
   const cuuint64_t dims[4] = {(cuuint64_t)pitch, (cuuint64_t)GW, (cuuint64_t)GH, (cuuint64_t)B};
-  const cuuint64_t strides[3] = {(cuuint64_t)pitch * 2, (cuuint64_t)GW * pitch * 2, (cuuint64_t)(GH * GW + 1) * pitch * 2};
+  const cuuint64_t strides[3] = {(cuuint64_t)pitch * 2, (cuuint64_t)GW * pitch * 2, (cuuint64_t)(GH * GW + extra_pixels) * pitch * 2};
   const cuuint32_t box[4] = {(cuuint32_t)box_c, (cuuint32_t)kTW, (cuuint32_t)box_h, 1}, estr[4] = {1, 1, 1, 1};
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, cl, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
             CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int MODE, int NT, bool ROWS, bool LEAN>
-void launch_gemm_l(TcParams p, int grid, size_t smem, cudaStream_t st) {
+bool launch_gemm_l(TcParams p, int grid, size_t smem, cudaStream_t st) {
   CUtensorMap out_map, cl_map;
   memset(&out_map, 0, sizeof(out_map));
   memset(&cl_map, 0, sizeof(cl_map));
-  p.use_out_map = (p.out_h == nullptr && cached_out_map(&out_map, p.out, p.B, p.Nout, p.g.GH, p.g.GW)) ? 1 : 0;
+  if (ROWS) {
+    if (!make_cl_map(&cl_map, p.out_h, p.B, p.out_pitch, p.g.GH, p.g.GW, 64, 2, CU_TENSOR_MAP_SWIZZLE_128B, 0) ||
+        !make_cl_map(&out_map, (__nv_bfloat16 *)p.g.xh, p.B, p.g.Cp, p.g.GH, p.g.GW, kChunk, kTH, CU_TENSOR_MAP_SWIZZLE_128B))
+      return false;
+    smem += kRowStageBytes - kOutStageBytes;
+  }
+  if (!ROWS) p.use_out_map = (p.out_h == nullptr && cached_out_map(&out_map, p.out, p.B, p.Nout, p.g.GH, p.g.GW)) ? 1 : 0;
   // the copy leaves through its own tensor map when the float32 output does; otherwise with plain stores
   if (p.use_out_map && p.out_cl != nullptr && !make_cl_map(&cl_map, p.out_cl, p.B, p.cl_pitch, p.g.GH, p.g.GW)) p.use_out_map = 0;
   static int granted[kMaxDevices];
   ensure_dynamic_smem(tc_gemm_kernel<MODE, NT, ROWS, LEAN>, granted, smem);
-  launch_after(tc_gemm_kernel<MODE, NT, ROWS, LEAN>, dim3(grid), kThreads, smem, st, p, out_map, cl_map);
+  launch_after(tc_gemm_kernel<MODE, NT, ROWS, LEAN>, dim3(grid), ROWS ? kRowThreads : kThreads, smem, st, p, out_map, cl_map);
+  return true;
 }
+// False if the operands of the multiply-first adjoint (ROWS) do not fit a tensor map.
 template <int MODE, int NT, bool ROWS = false>
-void launch_gemm(const TcParams &p, int grid, size_t smem, cudaStream_t st) {
-  if (p.g.Cp >= 64 && (MODE == MODE_PLAN || NT > 0)) {
-    if constexpr (MODE == MODE_PLAN || NT > 0) launch_gemm_l<MODE, NT, ROWS, true>(p, grid, smem, st);
-  } else {
-    launch_gemm_l<MODE, NT, ROWS, false>(p, grid, smem, st);
-  }
+bool launch_gemm(const TcParams &p, int grid, size_t smem, cudaStream_t st) {
+  if constexpr (MODE == MODE_PLAN || NT > 0)
+    if (ROWS || p.g.Cp >= 64) return launch_gemm_l<MODE, NT, ROWS, true>(p, grid, smem, st);
+  if constexpr (!ROWS) return launch_gemm_l<MODE, NT, ROWS, false>(p, grid, smem, st);
+  return false;
 }
 
 // ---- multiply-first adjoint -------------------------------------------------------------------------
@@ -1829,7 +1873,7 @@ int tc_adjoint_premul(const PremulGeometry &q, const void *src, const void *plan
   p.B = (int)B; p.Nout = (int)(K * q.Mp); p.Npb = g.Npb; p.nblk = g.nblk; p.nchunks = g.nchunks;
   p.tiles_x = cdiv(SW, kTW); p.tiles_y = cdiv(SH, kTH); p.stages = g.stages;
   const int64_t tiles = (int64_t)B * p.tiles_x * p.tiles_y * g.nblk;
-  launch_gemm<MODE_DIRECT, 1, true>(p, (int)(tiles < sm_count() ? tiles : sm_count()), g.smem, st);
+  if (!launch_gemm<MODE_DIRECT, 1, true>(p, (int)(tiles < sm_count() ? tiles : sm_count()), g.smem, st)) return SPH_ERR_CUDA;
   // 32-byte reads need rows that start at multiples of 32 bytes
   const int vc = q.Mp % 16 == 0 ? 16 : 8, vecs = q.Mp / vc, lanes = vecs >= 4 ? 4 : vecs >= 2 ? 2 : 1;
   const dim3 rgrid(cdiv(GH * GW, 256 / lanes), cdiv(vecs, lanes), (unsigned)B);

@@ -486,11 +486,16 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
       const int nb = tile % p.nblk, rest = tile / p.nblk, b = rest / tiles_per_image, t2 = rest % tiles_per_image;
       const int ty = t2 / p.tiles_x, tx = t2 % p.tiles_x;
       const char *img = g.xl + (size_t)b * image;
-      producer_bar3();  // the previous tile's taps have been read
-      fill_taps3<SRC>(g, taps, pv, plan_ok, 0, g.K, ty, tx, pt);
-      if (SRC != SRC_PLAN && tile == (int)blockIdx.x) wait_for_launcher();
-      producer_bar3();
-      if (!alive) continue;
+      if constexpr (SRC != SRC_SELF) {
+        producer_bar3();  // the previous tile's taps have been read
+        fill_taps3<SRC>(g, taps, pv, plan_ok, 0, g.K, ty, tx, pt);
+        if (SRC != SRC_PLAN && tile == (int)blockIdx.x) wait_for_launcher();
+        producer_bar3();
+        if (!alive) continue;
+      } else {
+        if (!alive) break;
+        if (tile == (int)blockIdx.x) wait_for_launcher();
+      }
       uint32_t self = 0u;
       if (SRC == SRC_SELF) {
         const int q = tile_pixel3(px, ty, tx, g.GH, g.GW);

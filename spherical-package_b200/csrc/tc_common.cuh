@@ -146,6 +146,8 @@ __device__ __forceinline__ void mbar_arrive_expect_tx_s(uint32_t bar_s, uint32_t
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // until the copies issued by this thread have read their shared-memory source (it may be overwritten then)
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// the same but for the copies of the last commit
+__device__ __forceinline__ void bulk_wait_read_but_last() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 // until the copies issued by this thread are complete
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void sts32(uint32_t addr_s, uint32_t v) {
