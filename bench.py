@@ -327,7 +327,7 @@ def run_encoder(args, rank, local, world):
                     "bwd": "tc_thin_bwd_kernel + thin_plan_gather_kernel (combined backward call)"}.get(
                         ph, "small_%s (SIMT, thin contraction)" % ph)
         return {"dw": "tc_dw_kernel", "bwd": "tc_gemm_kernel + tc_dw_kernel (combined backward call)",
-                "bwd.prepass": "grad_image_kernel (layout pre-pass of the backward call)"}.get(ph, "tc_gemm_kernel")
+                "bwd.prepass": "nchw_to_nhwc_bf16_kernel (layout pre-pass of the backward call)"}.get(ph, "tc_gemm_kernel")
 
     def launch_flops(li, ph):
         ci, co, _, (oh, ow), _ = cfg["layers"][li]

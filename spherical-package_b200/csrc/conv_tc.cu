@@ -1559,7 +1559,8 @@ __global__ void premul_weight_image_kernel(const float *__restrict__ w, __nv_bfl
 // T is the bf16 column buffer (B, n_src, pitch = K*Mp) written by the GEMM on the source grid.  L neighbouring threads share a
 // destination pixel and read VC channels each, so that a row segment of 64 channels is one 128-byte line of one instruction; the
 // next entry's index and weight are on their way with this one's row. (Encoder layer 2, batch 64: one thread per pixel, 64
-// channels of it, 1.93 ms; so 1.77 ms; pixel blocks of 16 x 4 1.81, two rows in flight 1.94.)
+// channels of it, 1.93 ms; so 1.77 ms; pixel blocks of 16 x 4 1.81, two rows in flight 1.94, an inner loop per
+// slot 2.09: a warp meets at every slot then.)
 template <int VC, int L>
 __global__ void __launch_bounds__(256)
 plan_gather_rows_kernel(const __nv_bfloat16 *__restrict__ T, const void *__restrict__ plan_blob, const float *__restrict__ bias,
