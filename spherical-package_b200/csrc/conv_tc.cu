@@ -1465,10 +1465,10 @@ Clears clears(int *status, const Fusion &fz, int64_t B, int64_t Nout, int64_t np
 
 // Weights -> bf16 tile images.  Row n of block nb, chunk `chunk`: 64 columns, 16-byte vector v stored at
 // position v ^ (n & 7) of the 128-byte row.  The source is addressed W[n*sn + ch*sc + slot*sk], sk = 1 or not.
-// Cp >= 64 (one slot per chunk): a block takes 8 rows x 64 channels x up to nine slots through shared memory, read in the order
+// Cp >= 64 (one slot per chunk): a block takes 4 rows x 64 channels x up to nine slots through shared memory, read in the order
 // in which they lie in the source and written as 16-byte vectors (one value per thread read with the stride of a slot group took
-// 5.3 us for 256 x 256 x 9, this takes 4.3).
-constexpr int kWiRows = 8, kWiSlots = 9, kWiPitch = kWiRows * 66 + 1;
+// 5.3 us for 256 x 256 x 9, this takes 3.6; with 8 rows, 128 blocks, 4.3).
+constexpr int kWiRows = 4, kWiSlots = 9, kWiPitch = kWiRows * 66 + 1;
 __global__ void __launch_bounds__(256) weight_image_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ wp, int Nout, int CH,
                                                            int Cp, int K, int Npb, int nblk, int nchunks, int64_t sn, int64_t sc,
                                                            int64_t sk, const Clears clr) {
@@ -1496,7 +1496,7 @@ __global__ void __launch_bounds__(256) weight_image_kernel(const float *__restri
   }
   __syncthreads();
   for (int i = threadIdx.x; i < kWiRows * 8 * nk; i += 256) {
-    const int v = i & 7, n = i >> 3 & (kWiRows - 1), k = i >> 6, ng = n0 + n, nb = ng / Npb, r = ng - nb * Npb;
+    const int v = i & 7, n = i >> 3 & (kWiRows - 1), k = i / (8 * kWiRows), ng = n0 + n, nb = ng / Npb, r = ng - nb * Npb;
     const float *t = tile + k * kWiPitch + n * 66 + v * 8;
     uint4 o;
     o.x = pack_bf16(t[0], t[1]);

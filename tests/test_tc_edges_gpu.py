@@ -1,4 +1,4 @@
-"""bf16 tensor-core convolutions at the edges of their weight images (8 rows x 64 channels x 9 slots per block), of the
+"""bf16 tensor-core convolutions at the edges of their weight images (4 rows x 64 channels x 9 slots per block), of the
 weight gradient's 128-row blocks and column groups, and of the plan tables (four and eight entries of a key), against the
 CPU oracle; and the extra pixels of a channels-last copy that starts uninitialised."""
 import pytest
