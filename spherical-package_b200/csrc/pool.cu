@@ -66,6 +66,16 @@ max_pool_kernel(const T *__restrict__ x, const T *__restrict__ map, const T *__r
     }
 }
 
+// Whether neighbouring positions of a map read neighbouring pixels: 256 pairs spread over it, slot 0; *flag = 1 if three quarters
+// of the pairs are at most 8 pixels apart in both directions, else 2.
+__global__ void __launch_bounds__(256) map_locality_kernel(const float *__restrict__ map, long long n, int K, int *flag) {
+  const long long o = (n - 1) * (long long)threadIdx.x / 256;
+  const float *a = map + 2 * (size_t)(o * K), *b = a + 2 * (o + 1 < n ? K : 0);
+  const bool near = fabsf(__ldg(b) - __ldg(a)) <= 8.0f && fabsf(__ldg(b + 1) - __ldg(a + 1)) <= 8.0f;
+  const int c = __syncthreads_count(near);
+  if (threadIdx.x == 0) *(volatile int *)flag = c >= 192 ? 1 : 2;
+}
+
 // Nearest-neighbour, unweighted pooling with at most kPoolMaxK slots: the K tap offsets of the output position are
 // decoded first and kept in registers, then every plane issues its K loads back to back (no load depends on
 // another), which is what lets the kernel run at memory speed instead of at K round-trip latencies per plane.
@@ -216,6 +226,7 @@ struct PoolOp {
     return b <= 48 * 1024 ? b : 0;
   }
 
+  size_t stage_smem() const { return stage_aligned(x, c.n_src) ? 0 : kStageBlock<PG>; }
   __device__ __forceinline__ void stage(int p0, char *rows, int tile) const { stage_quad<PG>(x, c.planes, c.n_src, p0, tile, rows); }
   __device__ __forceinline__ void use(int p0, const char *rows, int tile) const {
     extern __shared__ __align__(16) unsigned char pool_table[];
@@ -309,6 +320,7 @@ struct UnpoolOp {
   FastDiv divK, div2P, stage_tiles, use_tiles;
 
   __device__ __forceinline__ size_t winners_at() const { return (size_t)(c.n_src + 1) * PG * 4; }
+  size_t stage_smem() const { return stage_aligned(g, c.n_src) ? 0 : kStageBlock<PG>; }
   __device__ __forceinline__ void stage(int p0, char *rows, int tile) const {
     constexpr int LP = PG / 4;
     stage_quad<PG>(g, c.planes, c.n_src, p0, tile, rows);
@@ -540,6 +552,12 @@ extern "C" int sph_mapped_pool_ws(const void *x, const void *map, const void *iw
   }
   return dtype == SPH_F32 ? pool<float>(x, map, iw, out, idx, B * C, IH, IW, OH * OW, K, P, interp, st, average != 0)
                           : pool<double>(x, map, iw, out, idx, B * C, IH, IW, OH * OW, K, P, interp, st, average != 0);
+}
+
+extern "C" int sph_map_locality(const void *map, int64_t n, int64_t K, int *flag, void *stream) {
+  if (!map || !flag || n <= 0 || K <= 0 || K >= ((int64_t)1 << 31)) return SPH_ERR_INVALID_ARGUMENT;
+  map_locality_kernel<<<1, 256, 0, (cudaStream_t)stream>>>((const float *)map, (long long)n, (int)K, flag);
+  return launch_status();
 }
 
 extern "C" int sph_mapped_max_pool(const void *x, const void *map, const void *iw, void *out, int64_t *idx, int64_t B,

@@ -174,6 +174,7 @@ struct ScatterOp {
   int n_dst;
   FastDiv stage_tiles, use_tiles;
 
+  size_t stage_smem() const { return stage_aligned(x, c.n_src) ? 0 : kStageBlock<PG>; }
   __device__ __forceinline__ void stage(int p0, char *rows, int tile) const { stage_quad<PG>(x, c.planes, c.n_src, p0, tile, rows); }
   __device__ __forceinline__ void use(int p0, const char *rows, int tile) const {
     constexpr int VP = PG < 8 ? PG : 8, NV = PG / VP;
@@ -243,6 +244,7 @@ struct GatherOp {
   TileGrid grid;
   FastDiv stage_tiles, use_tiles;
 
+  size_t stage_smem() const { return stage_aligned(x, c.n_src) ? 0 : kStageBlock<PG>; }
   __device__ __forceinline__ void stage(int p0, char *rows, int tile) const { stage_quad<PG>(x, c.planes, c.n_src, p0, tile, rows); }
   __device__ __forceinline__ void use(int p0, const char *rows, int tile) const {
     constexpr int VP = Split<PG>::VP, LP = Split<PG>::LP;

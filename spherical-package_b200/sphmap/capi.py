@@ -30,7 +30,7 @@ SYMBOLS = [
     "sph_mapped_conv_relu_forward", "sph_mapped_conv_relu_backward_input", "sph_mapped_conv_relu_backward_weight",
     "sph_device_status", "sph_debug_bounded_wait", "sph_mapped_max_unpool_planned", "sph_mapped_avg_pool",
     "sph_mapped_avg_unpool", "sph_resample_to_map_normalized", "sph_resample_from_uv_maps", "sph_plan_build_uv",
-    "sph_voting_resample_to_map", "sph_build_kernel_map", "sph_build_is_checked", "sph_conv_companion_bytes",
+    "sph_voting_resample_to_map", "sph_map_locality", "sph_build_kernel_map", "sph_build_is_checked", "sph_conv_companion_bytes",
     "sph_staging_bytes", "sph_conv_workspace_preferred_bytes", "sph_resample_from_map_ws", "sph_resample_to_map_ws", "sph_mapped_pool_ws", "sph_mapped_max_unpool_ws",
     "sph_conv_companion_channels", "sph_conv_companion_fill", "sph_trace_phases", "sph_mapped_conv_forward_cl", "sph_mapped_conv_backward_cl",
 ]

@@ -55,3 +55,31 @@ def test_resampling_matches_direct_kernels(planes, interp, P):
         assert torch.equal(back, capi.resample_to_map(go, plan, ih, iw))
         norm = C.resample_to_map_normalized(go, m, w, ih, iw, it)
         assert torch.equal(norm, capi.resample_to_map_normalized(go, plan, ih, iw))
+
+
+@pytest.mark.parametrize("local", [True, False])
+def test_nearest_pooling_by_locality(local):
+    """The host extension reads the planes in place over a local map, once it knows that the map is one: same bits."""
+    import ctypes
+    from spherical_distortion.nn import InterpolationType, MappedMaxPool
+    from spherical_distortion.util import inverse_gnomonic_projection_map
+    from sphmap import capi
+    H, W = 66, 131
+    if local:
+        m = inverse_gnomonic_projection_map((H, W), (3, 3), stride=2, device="cuda")
+    else:
+        m = torch.rand(33, 66, 9, 2, generator=torch.Generator().manual_seed(3)).mul(torch.tensor([W - 1.0, H - 1.0])).cuda()
+    x = torch.randn(2, 35, H, W, generator=torch.Generator().manual_seed(4)).cuda()
+    n = m.shape[0] * m.shape[1]
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    capi._ok(capi.lib.sph_map_locality(capi._ptr(m), ctypes.c_int64(n), ctypes.c_int64(9), capi._ptr(flag), capi._stream()), "locality")
+    assert flag.item() == (1 if local else 2)
+    pool = MappedMaxPool(9, InterpolationType.NEAREST, return_indices=True)
+    runs = []
+    for _ in range(3):
+        runs.append(pool(x, m))
+        torch.cuda.synchronize()
+    for out, idx in runs[1:]:
+        assert torch.equal(out, runs[0][0]) and torch.equal(idx, runs[0][1])
+    want, at = capi.mapped_max_pool(x, m, 9, 0)
+    assert torch.equal(runs[0][0], want) and torch.equal(runs[0][1], at)
