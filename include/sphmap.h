@@ -113,8 +113,9 @@ int sph_resample_from_map(const void *x, const void *map, const void *iw, void *
  *   slots x points x 1 or 4), else ignored.
  * No counterpart in the reference.
  * ---------------------------------------------------------------------- */
-/* Max pooling by nearest neighbours, unweighted, K <= 16, is the exception to "pays": over a map whose neighbouring positions
- * read neighbouring pixels the kernel without scratch is 8 to 75 % faster.  sph_map_locality() looks at 256 pairs of a float32
+/* Gathers that read a pixel less than eight times, and max pooling by nearest neighbours (unweighted, K <= 16), are the
+ * exceptions to "pays": over a map whose neighbouring positions read neighbouring pixels the kernels without scratch are faster,
+ * pooling by 8 to 75 %.  sph_map_locality() looks at 256 pairs of a float32
  * map (n positions, K slots) and writes 1 (they do) or 2 to *flag, device-accessible memory, on the stream. */
 int sph_map_locality(const void *map, int64_t n, int64_t K, int *flag, void *stream);
 enum sph_stage_op { SPH_STAGE_GATHER = 0, SPH_STAGE_POOL = 1, SPH_STAGE_ARGMAX = 2, SPH_STAGE_SCATTER = 3 };

@@ -193,10 +193,11 @@ int64_t plan_cache_size() {
 }
 
 // ---- locality of sample maps ------------------------------------------------------
-// Max pooling by nearest neighbours reads the planes where they lie if neighbouring outputs read neighbouring pixels, and
-// transposed groups of planes if not.  Which it is depends only on the map: a small kernel looks, the first time a map is seen, and
-// writes the answer into pinned memory; until it is there, and while a stream is captured, the groups are used.  (Both ways give
-// the same bits, so an answer that comes late or belongs to a map whose place was given away costs time only.)
+// Gathers and max pooling by nearest neighbours read the planes where they lie if neighbouring outputs read neighbouring pixels,
+// and transposed groups of planes if not.  Which it is depends only on the map: a small kernel looks, the first time a map is seen,
+// and writes the answer into pinned memory; until it is there, and while a stream is captured, it is unknown.  (Both ways give the
+// same bits, so an answer that comes late or belongs to a map whose place was given away costs time only.)
+enum class Locality { Unknown = 0, Local = 1, Scattered = 2 };
 struct LocalityEntry {
   c10::weak_intrusive_ptr<c10::StorageImpl> map_s;
   const void *map_p;
@@ -207,7 +208,7 @@ struct LocalityEntry {
 std::mutex g_locality_mu;
 constexpr int kMaxLocalities = 64;
 
-bool map_is_local(const torch::Tensor &map, int64_t n, int64_t K) {
+Locality locality_of(const torch::Tensor &map, int64_t n, int64_t K) {
   static auto *entries = new std::list<LocalityEntry>();
   static volatile int *flags = nullptr;
   static int next = 0;
@@ -215,15 +216,16 @@ bool map_is_local(const torch::Tensor &map, int64_t n, int64_t K) {
   for (const LocalityEntry &e : *entries)
     if (e.map_p == map.data_ptr() && e.map_v == version_of(map) && e.n == n && e.K == K &&
         e.map_s.lock().get() == map.storage().unsafeGetStorageImpl())
-      return flags[e.slot] == 1;
+      return (Locality)flags[e.slot];
   const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
+    return Locality::Unknown;
   if (flags == nullptr) {
     void *p = nullptr;
     if (cudaHostAlloc(&p, kMaxLocalities * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
       cudaGetLastError();
-      return false;
+      return Locality::Unknown;
     }
     flags = (volatile int *)p;
   }
@@ -234,7 +236,7 @@ bool map_is_local(const torch::Tensor &map, int64_t n, int64_t K) {
   ok(sph_map_locality(map.data_ptr(), n, K, (int *)flags + slot, st), "sph_map_locality");
   entries->push_front(LocalityEntry{c10::weak_intrusive_ptr<c10::StorageImpl>(map.storage().getWeakStorageImpl()), map.data_ptr(),
                                     version_of(map), n, K, slot});
-  return false;
+  return Locality::Unknown;
 }
 
 // ---- channels-last companions of activations (bf16 precision) -------------------
@@ -323,7 +325,14 @@ torch::Tensor resample_from_map_impl(torch::Tensor x, torch::Tensor map, const t
   const MapInfo m = map_info(map, iw, false, 1);
   c10::cuda::CUDAGuard guard(x.device());
   torch::Tensor y = torch::empty({x.size(0), x.size(1), m.H, m.W}, x.options());
-  const Staging sg(SPH_STAGE_GATHER, x.size(0) * x.size(1), x.size(2) * x.size(3), m.H * m.W * std::max<int64_t>(m.P, 1) * taps_of(it), x);
+  // Over a map that is not known to be scattered, groups of planes pay where a pixel is read eight times or more (bilinear tangent
+  // images of 300 x 600, direct and in groups: 24 planes, 2.5 reads 13 and 15 us, 5 reads 20 and 20, 12 reads 34 and 29; 6 planes
+  // 12 reads 12.5 and 11.8).
+  const int64_t planes = x.size(0) * x.size(1), reads = m.H * m.W * std::max<int64_t>(m.P, 1) * taps_of(it);
+  const bool grouped = planes >= 3 && x.scalar_type() == torch::kFloat && reads > 0 && x.numel() > 0 &&
+                       ((planes >= 8 && reads >= 8 * x.size(2) * x.size(3)) ||
+                        (reads >= x.size(2) * x.size(3) && locality_of(map, m.H * m.W, std::max<int64_t>(m.P, 1)) == Locality::Scattered));
+  const Staging sg(SPH_STAGE_GATHER, grouped ? planes : 0, x.size(2) * x.size(3), reads, x);
   ok(sph_resample_from_map_ws(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, y.data_ptr(), x.size(0), x.size(1),
                               x.size(2), x.size(3), m.H, m.W, m.P, dtype_of(x), (int)it, sg.ptr(), sg.bytes, stream()),
      "sph_resample_from_map");
@@ -511,8 +520,8 @@ std::vector<torch::Tensor> max_pool_impl(torch::Tensor x, torch::Tensor map, con
   const int64_t pixels = x.size(2) * x.size(3), wave = 4 * at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
   const int64_t blocks = (planes + 31) / 32 * ((m.H + 7) / 8) * ((m.W + 7) / 8);
   const bool few = nearest && (values <= ((int64_t)1 << 19) || (pixels <= ((int64_t)1 << 14) && values <= ((int64_t)5 << 18)));
-  const bool thin_wave = !nearest && float_taps && planes >= 64 && blocks > wave && 4 * blocks <= 5 * wave;
-  const bool direct = few || ((nearest || thin_wave) && map_is_local(map, m.H * m.W, m.K));
+  const bool thin_wave = !nearest && float_taps && planes >= 64 && blocks > wave && 5 * blocks <= 7 * wave;
+  const bool direct = few || ((nearest || thin_wave) && locality_of(map, m.H * m.W, m.K) == Locality::Local);
   const Staging sg(SPH_STAGE_POOL, direct ? 0 : planes, x.size(2) * x.size(3), m.H * m.W * m.K * std::max<int64_t>(m.P, 1) * taps_of(it), x);
   ok(sph_mapped_pool_ws(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, out.data_ptr(), idx.data_ptr<int64_t>(),
                         x.size(0), x.size(1), x.size(2), x.size(3), m.H, m.W, m.K, m.P, 0, dtype_of(x), (int)it, sg.ptr(), sg.bytes,
