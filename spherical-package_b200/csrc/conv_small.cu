@@ -234,6 +234,8 @@ small_fwd_tile_kernel(const float *__restrict__ src, const float *__restrict__ m
         o.w = pack_bf16x2(c[6], c[7]);
         *(uint4 *)(out_cl + ((size_t)b * (npix + 1) + px) * cl_pitch + mw) = o;
       }
+      if (p0 == 0 && lane == 0)  // the extra pixel, which taps outside the image read
+        *(uint4 *)(out_cl + ((size_t)b * (npix + 1) + npix) * cl_pitch + mw) = make_uint4(0u, 0u, 0u, 0u);
     }
   }
 }
