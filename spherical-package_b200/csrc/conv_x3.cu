@@ -1001,7 +1001,8 @@ DwPlan3 dw_plan3(int src, int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t
   d.Cp = padded3(CH);
   d.groups = (int)((K * d.Cp + kDwN - 1) / kDwN);
   d.mbs = (int)((M + 127) / 128);
-  for (int g = 0; g < d.groups && g < 64; g++)
+  // (the position of a group's first column within its slot repeats after at most Cp / 32 groups)
+  for (int g = 0; g < d.groups && g < std::max(d.Cp / 32, 1); g++)
     d.slots = std::max(d.slots, (g * kDwN + kDwN - 1) / d.Cp - g * kDwN / d.Cp + 1);
   d.tiles_x = cdiv(GW, kTileW);
   d.tiles_y = cdiv(GH, kTileH);

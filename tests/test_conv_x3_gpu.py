@@ -15,7 +15,8 @@ CASES = [(2, 16, 32, (16, 32), (16, 32), 9, 1, 0),
          (2, 40, 200, (20, 30), (7, 11), 9, 1, 0),
          (1, 100, 50, (20, 33), (20, 33), 5, 0, 3),
          (1, 96, 16, (24, 40), (24, 40), 25, 1, 0),
-         (1, 260, 256, (16, 32), (16, 32), 9, 1, 0)]
+         (1, 260, 256, (16, 32), (16, 32), 9, 1, 0),
+         (1, 8200, 16, (4, 8), (4, 8), 9, 1, 0)]     # dW: the first column group of two slots is the 65th
 
 
 def _rel(a, ref):
