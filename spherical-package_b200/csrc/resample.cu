@@ -182,12 +182,12 @@ struct ScatterOp {
     if (q >= n_dst) return;
     bool ok;
     const PlanView<float> pv = plan_view<float>(plan, n_dst, ok, c.n_src);
-    const int e0 = __ldg(pv.offsets + q), e1 = __ldg(pv.offsets + q + 1);
+    const int e0 = ok ? __ldg(pv.offsets + q) : 0, e1 = ok ? __ldg(pv.offsets + q + 1) : 0;
     Vec<VP> acc[NV];
 #pragma unroll
     for (int i = 0; i < NV; i++) acc[i] = vec_fill<VP>(0.0f);
     float wsum = 0.0f;
-    if (ok && e0 < e1) {
+    if (e0 < e1) {
       const int *sp = pv.src + e0, *end = pv.src + e1;
       const float *wp = pv.w + e0;
       int s = __ldg(sp);

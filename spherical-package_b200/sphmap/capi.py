@@ -139,11 +139,24 @@ def plan_build(smap, iw, n_src, K, interp, dstH, dstW):
     return plan
 
 
-def resample_to_map(x, plan, oh, ow):
+STAGE_GATHER, STAGE_POOL, STAGE_ARGMAX, STAGE_SCATTER = 0, 1, 2, 3
+
+
+def staging(op, planes, n_src, reads, like):
+    """Scratch of the plane-group kernels for an operator's `ws` argument, or None where sph_staging_bytes() reports none."""
+    n = lib.sph_staging_bytes(_int(op), *_ints(planes, n_src, reads), _int(_dt(like)))
+    return _bytes(n, like) if n else None
+
+
+def resample_to_map(x, plan, oh, ow, ws=None):
     B, C, MH, MW = x.shape
     out = torch.empty(B, C, int(oh), int(ow), dtype=x.dtype, device=x.device)
-    _ok(lib.sph_resample_to_map(_ptr(x), _ptr(plan), _ptr(out), *_ints(B, C, MH, MW, oh, ow), _int(_dt(x)), _stream()),
-        "sph_resample_to_map")
+    if ws is None:
+        rc = lib.sph_resample_to_map(_ptr(x), _ptr(plan), _ptr(out), *_ints(B, C, MH, MW, oh, ow), _int(_dt(x)), _stream())
+    else:
+        rc = lib.sph_resample_to_map_ws(_ptr(x), _ptr(plan), _ptr(out), *_ints(B, C, MH, MW, oh, ow), _int(0), _int(_dt(x)), _ptr(ws),
+                                        _sz(ws.numel()), _stream())
+    _ok(rc, "sph_resample_to_map")
     return out
 
 

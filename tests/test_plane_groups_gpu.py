@@ -83,3 +83,16 @@ def test_nearest_pooling_by_locality(local):
         assert torch.equal(out, runs[0][0]) and torch.equal(idx, runs[0][1])
     want, at = capi.mapped_max_pool(x, m, 9, 0)
     assert torch.equal(runs[0][0], want) and torch.equal(runs[0][1], at)
+
+
+@pytest.mark.parametrize("planes", [3, 8, 16])
+def test_scatter_with_a_plan_of_another_size_yields_zeros(planes):
+    """A plan that was built for another destination, or is none, is not followed: zeros, as from the direct kernel."""
+    from sphmap import capi
+    _, m, _, go = _case(planes, 6, 7, 13, 11, 1, 0)
+    m = m[:, :, 0].contiguous()
+    ws = capi.staging(capi.STAGE_SCATTER, planes, 13 * 11, 0, go)
+    smaller = capi.plan_build(m, None, 13 * 11, 1, 1, 6, 7)
+    for plan in (smaller, torch.zeros_like(smaller)):
+        for scratch in (None, ws):
+            assert not capi.resample_to_map(go, plan, 60, 70, ws=scratch).any()
