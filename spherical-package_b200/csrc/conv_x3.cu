@@ -8,7 +8,9 @@
 //   - the large products h*h go to an accumulator of their own, which takes at most kSeg chunks (64 columns, four additions)
 //     before the epilogue warps add it, round to nearest, to float32 sums (kept in tensor memory); two such accumulators
 //     alternate;
-//   - the five small ones share a second accumulator for the whole tile: its losses are 2^-8 of the large one's.
+//   - the five small ones go to a second accumulator, whose losses are 2^-7 of the large one's: it takes kRun segments (800
+//     additions, ten per chunk: 4e-7) before it is added to the sums too.  (One accumulator for a whole weight gradient of 768 tiles
+//     was off by 1.6e-5, so 7e-7, the CUDA cores' sums 1.4e-6; it cost a weight gradient of 70 tiles per block 1.6 %.)
 // (Tiles of one segment need no sums: their columns are the small products' second buffer, and the next tile's products run
 // while this one's results are stored.)
 // The result is at least as close to the exact sum as the SIMT kernels' (conv_simt.cu; tests/test_conv_x3_gpu.py compares
@@ -44,6 +46,7 @@ constexpr int kThreads3 = 32 * (kEpi + 1 + kProd);
 constexpr int kProd0 = 32 * (kEpi + 1);                 // first producer thread
 constexpr int kSeg = 2;                                 // chunks per segment of large products; tiles of at most kOneSeg chunks
 constexpr int kOneSeg = 4;                              // (the multiply-first product) are one segment
+constexpr int kRun = 40;                                // segments that share an accumulator of small products
 constexpr int kPartA = kPix * 64;                       // bytes of one part of a 128-row x 32-column operand tile
 constexpr int kNMax = 128;
 constexpr size_t kSmemMax = 227 * 1024;
@@ -324,9 +327,11 @@ __device__ __forceinline__ void issue_step(uint32_t hh, uint32_t corr, uint64_t 
 
 // One tile's sums in an epilogue warp (lanes 32 * warp ..): every finished segment of large products is added to the running
 // sums in tensor memory; with the last one the small products join and the 16-column blocks go to `put(first column, values)`.
-// `sg` counts segments over all tiles; `cb`: the small products' buffer.  False if a wait gave up.
+// `sg` and `rn` count segments and runs over all tiles; `nc`: buffers of the small products.  False if a wait gave up.
 template <class Put>
-__device__ __forceinline__ bool drain_tile(const Bars &b, uint32_t lane_addr, int ncols, int nseg, int &sg, int lane, int cb, Put put) {
+__device__ __forceinline__ bool drain_tile(const Bars &b, uint32_t lane_addr, int ncols, int nseg, int &sg, int &rn, int nc, int lane,
+                                           Put put) {
+  const int cb = nc == 2 ? rn & 1 : 0;
   for (int s = 0; s < nseg; s++, sg++) {
     const int buf = sg & 1;
     if (!mbar_wait(b.seg_full + buf, (sg >> 1) & 1, b.abort_flag)) return false;
@@ -359,7 +364,58 @@ __device__ __forceinline__ bool drain_tile(const Bars &b, uint32_t lane_addr, in
       if (last) mbar_arrive(b.corr_empty + cb);
     }
   }
+  rn++;
   return true;
+}
+
+// The same for tiles of more than one run: a finished run of small products is added like a segment of large ones, and the sums go
+// to `put` after the last buffers were given back.  (A kernel of its own, because the forward product of tiles of one run lost 5 %
+// to the registers of this form.)
+template <class Put>
+__device__ __forceinline__ bool drain_long_tile(const Bars &b, uint32_t lane_addr, int ncols, int nseg, int &sg, int &rn, int lane, Put put) {
+  for (int s = 0; s < nseg; s++, sg++) {
+    const int buf = sg & 1;
+    if (!mbar_wait(b.seg_full + buf, (sg >> 1) & 1, b.abort_flag)) return false;
+    tc_fence_after();
+    const bool flush = s + 1 == nseg || s % kRun == kRun - 1;  // (the run's last small product was committed with this segment)
+    for (int pass = 0; pass < (flush ? 2 : 1); pass++) {
+      for (int c = 0; c < ncols; c += 16) {
+        uint32_t r[16], t[16];
+        tmem_ld_32x16(lane_addr + (pass ? kCorr : kHh + buf * 128) + c, r);
+        if (s + pass > 0) tmem_ld_32x16(lane_addr + kSum + c, t);
+        tmem_ld_wait();
+        if (s + pass > 0) {
+#pragma unroll
+          for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(t[j]), __uint_as_float(r[j])));
+        }
+        tmem_st_32x16(lane_addr + kSum + c, r);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(pass ? b.corr_empty : b.seg_empty + buf);
+    }
+    if (flush) rn++;
+  }
+#pragma unroll 1
+  for (int c = 0; c < ncols; c += 16) {
+    uint32_t r[16];
+    tmem_ld_32x16(lane_addr + kSum + c, r);
+    tmem_ld_wait();
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
+    put(c, v);
+  }
+  return true;
+}
+
+// The MMA thread's wait for the buffer of a new run of small products; its index in `cb`.
+__device__ __forceinline__ bool start_run(const Bars &b, int &rn, int nc, int &cb) {
+  cb = nc == 2 ? rn & 1 : 0;
+  const int use = nc == 2 ? rn >> 1 : rn;  // this buffer's use count
+  rn++;
+  return mbar_wait(b.corr_empty + cb, (use & 1) ^ 1, b.abort_flag);
 }
 
 struct Gemm3 {
@@ -390,7 +446,8 @@ template <int SRC> inline size_t gemm3_smem(int stages, int Npb, int K) {
   return 1024 + (size_t)stages * (3 * kPartA + 3 * Npb * 64) + align_up(TapTable<SRC>::bytes(K), 16) + bars_bytes(stages);
 }
 
-template <int SRC>
+// LONG: the small products of a tile take more than one run
+template <int SRC, bool LONG>
 __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -409,14 +466,13 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
   // (The producers of map modes wait after their first tile's taps; in plan mode, a wait inside the tile loop cost its gather 6 %.)
   if (SRC == SRC_PLAN || warp <= kEpi) wait_for_launcher();
   if (warp < kEpi) {
-    int sg = 0, tl = 0;
-    for (int tile = blockIdx.x; tile < total; tile += gridDim.x, tl++) {
+    int sg = 0, rn = 0;
+    for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
       const int nb = tile % p.nblk, rest = tile / p.nblk, b = rest / tiles_per_image, t2 = rest % tiles_per_image;
       const int pix = tile_pixel3(warp * 32 + lane, t2 / p.tiles_x, t2 % p.tiles_x, g.GH, g.GW);
       const int n0 = nb * p.Npb;
       float *out = p.out + ((size_t)b * p.Nout + n0) * npix + pix;
-      const bool ok = drain_tile(bars, tmem + ((uint32_t)(warp * 32) << 16), p.Npb, nseg, sg, lane, nc == 2 ? tl & 1 : 0,
-                                 [&](int c, float (&v)[16]) {
+      const auto put = [&](int c, float (&v)[16]) {
         if (pix < 0) return;
         const int left = p.Nout - n0 - c;
         if constexpr (SRC == SRC_SELF) {  // the column buffer of the multiply-first adjoint: this pixel's 16 columns are one 64-byte run
@@ -442,27 +498,31 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_gemm_kernel(const Gemm3 p) {
           for (int j = 0; j < 16; j++, o += npix)
             if (j < left) *o = v[j];
         }
-      });
+      };
+      const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+      bool ok;
+      if constexpr (LONG) ok = drain_long_tile(bars, lane_addr, p.Npb, nseg, sg, rn, lane, put);
+      else ok = drain_tile(bars, lane_addr, p.Npb, nseg, sg, rn, nc, lane, put);
       if (!ok) break;
     }
   } else if (warp == kEpi) {
     if (lane == 0) {
       const uint32_t idesc = idesc_bf16(kPix, p.Npb, 0, 0);
-      int tl = 0, sg = 0;
+      int sg = 0, rn = 0, cb = 0;
       Ring3 ring;
       bool alive = true;
-      for (int tile = blockIdx.x; alive && tile < total; tile += gridDim.x, tl++) {
-        const int cb = nc == 2 ? tl & 1 : 0, use = nc == 2 ? tl >> 1 : tl;  // this buffer's use count
-        if (!mbar_wait(bars.corr_empty + cb, (use & 1) ^ 1, bars.abort_flag)) break;
+      for (int tile = blockIdx.x; alive && tile < total; tile += gridDim.x) {
+        if (!start_run(bars, rn, nc, cb)) break;
         for (int chunk = 0; chunk < p.nchunks; chunk++, ring.next(S)) {
-          const bool first = chunk % seg == 0;
+          const bool first = chunk % seg == 0, first_corr = LONG ? chunk % (kSeg * kRun) == 0 : chunk == 0;
           const int buf = sg & 1;
+          if (LONG && first_corr && chunk > 0 && !start_run(bars, rn, nc, cb)) { alive = false; break; }
           if (first && !mbar_wait(bars.seg_empty + buf, ((sg >> 1) & 1) ^ 1, bars.abort_flag)) { alive = false; break; }
           if (!mbar_wait(bars.full + ring.s, ring.ph, bars.abort_flag)) { alive = false; break; }
           tc_fence_after();
           const uint32_t a = stage0 + ring.s * stage_bytes, bw = a + 3 * kPartA;
           issue_step(tmem + kHh + buf * 128, tmem + kCorr + cb * 128, smem_desc_sw64(a), smem_desc_sw64(bw), kPartA >> 4,
-                     (uint32_t)p.Npb * 4u, 2, 2, idesc, first, chunk == 0);
+                     (uint32_t)p.Npb * 4u, 2, 2, idesc, first, first_corr);
           umma_commit(bars.empty + ring.s);
           if (chunk % seg == seg - 1 || chunk + 1 == p.nchunks) {
             umma_commit(bars.seg_full + buf);
@@ -584,27 +644,29 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_dw_kernel(const Dw3 p) {
 
   if (warp <= kEpi) wait_for_launcher();  // (the producers: after their first tile's taps)
   if (warp < kEpi) {
-    int sg = 0;
+    int sg = 0, rn = 0;
     float *o = p.partial + ((size_t)split * p.mbs * 128 + mb * 128 + warp * 32 + lane) * (p.groups * kDwN) + grp * kDwN;
     const auto put = [&](int c, const float (&v)[16]) {
 #pragma unroll
       for (int j = 0; j < 16; j += 4) *(float4 *)(o + c + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     };
-    drain_tile(bars, tmem + ((uint32_t)(warp * 32) << 16), kDwN, nseg, sg, lane, 0, put);
+    drain_long_tile(bars, tmem + ((uint32_t)(warp * 32) << 16), kDwN, nseg, sg, rn, lane, put);
   } else if (warp == kEpi) {
     if (lane == 0) {
       const uint32_t idesc = idesc_bf16(128, kDwN, 0, 1);
       Ring3 ring;
       const int steps = (hi - lo) * 4;
+      int rn = 0, cb = 0;
       for (int st = 0; st < steps; st++, ring.next(S)) {
         const int sg = st / kSeg, buf = sg & 1;
-        const bool first = st % kSeg == 0;
+        const bool first = st % kSeg == 0, first_corr = st % (kSeg * kRun) == 0;
+        if (first_corr && !start_run(bars, rn, 1, cb)) break;
         if (first && !mbar_wait(bars.seg_empty + buf, ((sg >> 1) & 1) ^ 1, bars.abort_flag)) break;
         if (!mbar_wait(bars.full + ring.s, ring.ph, bars.abort_flag)) break;
         tc_fence_after();
         const uint32_t a = stage0 + ring.s * stage_bytes;
         issue_step(tmem + kHh + buf * 128, tmem + kCorr, smem_desc_sw64(a), smem_desc_sw128(a + kStepA, kDwPix3 * 128, 1024), kPartA >> 4,
-                   kPartB3 >> 4, 2, 16 * 128 >> 4, idesc, first, st == 0);
+                   kPartB3 >> 4, 2, 16 * 128 >> 4, idesc, first, first_corr);
         umma_commit(bars.empty + ring.s);
         if (st % kSeg == kSeg - 1) umma_commit(bars.seg_full + buf);
       }
@@ -1027,10 +1089,14 @@ Nhwc3 nhwc3(const void *x, float *y, int64_t B, int64_t C, int Cp, int64_t HW, f
   return q;
 }
 
-template <int SRC> void launch_gemm3(const Gemm3 &p, int64_t tiles, size_t smem, cudaStream_t st) {
+template <int SRC, bool LONG> void launch_gemm3_as(const Gemm3 &p, int64_t tiles, size_t smem, cudaStream_t st) {
   static int granted[kMaxDev3];
-  allow_smem3(x3_gemm_kernel<SRC>, granted, smem);
-  launch_after(x3_gemm_kernel<SRC>, dim3((unsigned)std::min<int64_t>(tiles, sms3())), kThreads3, smem, st, p);
+  allow_smem3(x3_gemm_kernel<SRC, LONG>, granted, smem);
+  launch_after(x3_gemm_kernel<SRC, LONG>, dim3((unsigned)std::min<int64_t>(tiles, sms3())), kThreads3, smem, st, p);
+}
+template <int SRC> void launch_gemm3(const Gemm3 &p, int64_t tiles, size_t smem, cudaStream_t st) {
+  if (p.nchunks > kSeg * kRun) launch_gemm3_as<SRC, true>(p, tiles, smem, st);
+  else launch_gemm3_as<SRC, false>(p, tiles, smem, st);
 }
 template <int SRC> void launch_dw3(const Dw3 &p, size_t smem, cudaStream_t st) {
   static int granted[kMaxDev3];

@@ -16,6 +16,7 @@ CASES = [(2, 16, 32, (16, 32), (16, 32), 9, 1, 0),
          (1, 100, 50, (20, 33), (20, 33), 5, 0, 3),
          (1, 96, 16, (24, 40), (24, 40), 25, 1, 0),
          (1, 260, 256, (16, 32), (16, 32), 9, 1, 0),
+         (1, 300, 320, (9, 17), (9, 17), 9, 2, 0),    # products of 90 chunks: more than one run of small products
          (1, 8200, 16, (4, 8), (4, 8), 9, 1, 0)]     # dW: the first column group of two slots is the 65th
 
 
@@ -77,3 +78,20 @@ def test_cancellation_and_one_sided_sums():
         old, ref = simt(x, m, w, b, go), simt(*(t.double() for t in (x, m, w, b, go)))
         for what, n, o, f in zip(("forward", "dInput", "dW"), new, old, ref):
             assert _rel(n, f) <= 1.25 * _rel(o, f) + 5e-8, (sign, what, _rel(n, f), _rel(o, f))
+
+
+def test_long_one_sided_reduction():
+    """Weight gradient whose blocks reduce 768 tiles each (147 column groups, so one split): 3072 steps of products of one sign.
+    Each step cuts ten small products (2^-7 of the sum at most) and, per two steps, four large ones off toward zero, about
+    5e-8 of an accumulator each.  With at most 800 small ones to an accumulator that is 4e-7 + 2e-7; rounding 1536 float32
+    additions adds 2^-25 sqrt(1536 / 3) = 7e-7.  An accumulator of all 30720 would be off by 1.6e-5 on its own."""
+    import _spherical_distortion_ext._C as C
+    from sphmap import capi
+    g = torch.Generator().manual_seed(11)
+    B, ci, co, H, W, K = 768, 384, 16, 8, 16, 49
+    m = (torch.rand(H, W, K, 2, generator=g) * torch.tensor([W - 1.0, H - 1.0])).cuda()
+    x, w, go = (torch.rand(*s, generator=g).cuda() + 0.5 for s in ((B, ci, H, W), (co, ci, K), (B, co, H, W)))
+    new = C.mapped_conv_backward(go, m, x, w, torch.zeros(co, device="cuda"), K, C.InterpolationType(1))[1]
+    old = capi.conv_backward_weight(go, x, m, K, 1)[0]
+    ref = capi.conv_backward_weight(go.double(), x.double(), m.double(), K, 1)[0]
+    assert _rel(new, ref) <= 1.5e-6, (_rel(new, ref), _rel(old, ref))
