@@ -14,7 +14,7 @@
 // (Tiles of one segment need no sums: their columns are the small products' second buffer, and the next tile's products run
 // while this one's results are stored.)
 // The result is at least as close to the exact sum as the SIMT kernels' (conv_simt.cu; tests/test_conv_x3_gpu.py compares
-// both with float64).  An infinite operand gives NaN where float32 arithmetic could have kept an infinity.
+// both with float64).  Infinities and NaNs come out as from float32 arithmetic: see add_small().
 //
 // The two kernels mirror conv_tc.cu (tiles of 128 pixels, producer warps that gather, weights or gradient tile images by
 // bulk copies, one MMA thread, epilogue warps), but gather float32 values from a channels-last float32 copy of the source
@@ -26,6 +26,7 @@
 // the SM's 128-byte data path carries 512 wavefronts of gathered taps, 192 + 192 of operand stores and 768 of operand
 // reads; 32-column chunks (64-byte swizzled rows, 48 KB a stage for both operands in three parts) leave the L1 room for
 // the tile's neighbourhood, which 64-column chunks (96 KB a stage) do not.
+#include <float.h>
 #include <string.h>
 
 #include <algorithm>
@@ -325,6 +326,14 @@ __device__ __forceinline__ void issue_step(uint32_t hh, uint32_t corr, uint64_t 
   }
 }
 
+// The small products join.  An operand that is infinite has parts (inf, NaN, NaN): the large products then carry the sum, infinite
+// or NaN as in float32 arithmetic, and the small ones are NaN.  fmaxf() makes a number of a NaN, which changes neither an infinity
+// nor a NaN, and leaves numbers as they are.  (One instruction per value: a comparison and a selection cost the forward product
+// 1.4 %, one test for 16 values its registers.)
+__device__ __forceinline__ uint32_t add_small(uint32_t large, uint32_t small) {
+  return __float_as_uint(__fadd_rn(__uint_as_float(large), fmaxf(__uint_as_float(small), -FLT_MAX)));
+}
+
 // One tile's sums in an epilogue warp (lanes 32 * warp ..): every finished segment of large products is added to the running
 // sums in tensor memory; with the last one the small products join and the 16-column blocks go to `put(first column, values)`.
 // `sg` and `rn` count segments and runs over all tiles; `nc`: buffers of the small products.  False if a wait gave up.
@@ -350,7 +359,7 @@ __device__ __forceinline__ bool drain_tile(const Bars &b, uint32_t lane_addr, in
       if (last) {  // (the small products' last one was committed with this segment)
         float v[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = __fadd_rn(__uint_as_float(r[j]), __uint_as_float(u[j]));
+        for (int j = 0; j < 16; j++) v[j] = __uint_as_float(add_small(r[j], u[j]));
         put(c, v);
       } else {
         tmem_st_32x16(lane_addr + kSum + c, r);
@@ -384,7 +393,10 @@ __device__ __forceinline__ bool drain_long_tile(const Bars &b, uint32_t lane_add
         tmem_ld_32x16(lane_addr + (pass ? kCorr : kHh + buf * 128) + c, r);
         if (s + pass > 0) tmem_ld_32x16(lane_addr + kSum + c, t);
         tmem_ld_wait();
-        if (s + pass > 0) {
+        if (pass) {
+#pragma unroll
+          for (int j = 0; j < 16; j++) r[j] = add_small(t[j], r[j]);
+        } else if (s > 0) {
 #pragma unroll
           for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(t[j]), __uint_as_float(r[j])));
         }
@@ -732,6 +744,9 @@ __global__ void __launch_bounds__(kThreads3, 1) x3_dw_kernel(const Dw3 p) {
   }
 }
 
+// A NaN whose payload lies in the lower half alone would have an infinity for its upper part: NaNs become the canonical one.
+__device__ __forceinline__ float quiet(float x) { return x != x ? __int_as_float(0x7fffffff) : x; }
+
 // ---- layout pre-passes ---------------------------------------------------------------------------------------------------
 // (B, C, HW) -> (B, HW + 1, Cp) float32; padding channels and the extra pixel are zero.  128 pixels x 32 channels per block,
 // through shared memory (blocks of 32 x 32 spent half their instructions on finding their place: 41 -> 27 us per 67 MB).  With
@@ -768,10 +783,11 @@ __device__ __forceinline__ void nhwc_block(const Nhwc3 &q, int block, NhwcTile &
   if (c >= q.Cp) return;
   float *y = q.y + ((size_t)b * (q.HW + 1) + p0) * q.Cp + c;
 #pragma unroll 4
-  for (int i = ty; i < np; i += 8) y[(size_t)i * q.Cp] = tile[tx][i];
+  for (int i = ty; i < np; i += 8) y[(size_t)i * q.Cp] = quiet(tile[tx][i]);
 }
 
 __device__ __forceinline__ void split3(float x, uint16_t &h, uint16_t &m, uint16_t &l) {
+  x = quiet(x);
   const float r = x - __uint_as_float(__float_as_uint(x) & 0xffff0000u), s = r - __uint_as_float(__float_as_uint(r) & 0xffff0000u);
   h = (uint16_t)(__float_as_uint(x) >> 16);
   m = (uint16_t)(__float_as_uint(r) >> 16);

@@ -95,3 +95,47 @@ def test_long_one_sided_reduction():
     old = capi.conv_backward_weight(go, x, m, K, 1)[0]
     ref = capi.conv_backward_weight(go.double(), x.double(), m.double(), K, 1)[0]
     assert _rel(new, ref) <= 1.5e-6, (_rel(new, ref), _rel(old, ref))
+
+
+@pytest.mark.parametrize("case", [(2, 16, 32, (16, 32), (16, 32), 9, 1, 0), (1, 40, 48, (24, 40), (11, 19), 9, 0, 0),
+                                  (1, 20, 32, (9, 17), (9, 17), 4, 0, 3), (1, 300, 32, (9, 17), (9, 17), 9, 1, 0)])
+@pytest.mark.parametrize("kind", ["inf", "mixed", "overflow"])
+def test_infinities_and_nans_are_those_of_float32(case, kind):
+    """Infinite and NaN operands (one NaN with its payload in the lower half alone) and products beyond the float32 range: the same
+    elements of every result are NaN, plus and minus infinity as from the CUDA cores."""
+    import _spherical_distortion_ext._C as C
+    from sphmap import capi
+    B, ci, co, (H, W), (OH, OW), K, interp, P = case
+    g = torch.Generator().manual_seed(co)
+    r = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    x, w, b, go = r(B, ci, H, W), r(co, ci, K), r(co), r(B, co, OH, OW)
+    wt, bt, xt, got = r(ci, co, K), r(co), r(B, ci, OH, OW), r(B, co, H, W)
+    m = torch.rand(*((OH, OW, K, P, 2) if P else (OH, OW, K, 2)), generator=g) * torch.tensor([W + 1.0, H + 1.0]) - 1.0
+    iw = torch.rand(OH, OW, K, P, generator=g) if P else None
+    odd_nan = torch.tensor([0x7f800001], dtype=torch.int32).view(torch.float32)
+    if kind == "overflow":  # (of one sign: with two, whether a sum overflows depends on its order)
+        x, w, b, go, wt, bt, xt, got = (t.abs() + 0.5 for t in (x, w, b, go, wt, bt, xt, got))
+    for t in (x, go, xt, got):
+        if kind == "overflow":
+            t[0, 0, 3, 4] = 3e38
+            continue
+        t[0, 0, 3, 4] = float("inf")
+        t[0, 1, 2, 7] = float("-inf")
+        if kind == "mixed":
+            t[-1, 2, 6, 1] = odd_nan[0]
+            t[-1, 3, 5, 5] = float("nan")
+    if kind == "mixed":
+        w[1, 2, 3], w[2, 0, 1], wt[1, 2, 3], wt[2, 1, 0] = float("inf"), odd_nan[0], float("-inf"), float("nan")
+    x, w, b, go, m, iw, wt, bt, xt, got = (None if t is None else t.cuda() for t in (x, w, b, go, m, iw, wt, bt, xt, got))
+    plan = capi.plan_build(m, iw, OH * OW, K, interp, H, W)
+    old = [capi.conv_forward(x, m, w, b, K, interp, iw), capi.conv_backward_input(go, plan, w, H, W, K),
+           *capi.conv_backward_weight(go, x, m, K, interp, iw), capi.tconv_forward(xt, plan, wt, bt, H, W, K),
+           capi.tconv_backward_input(got, m, wt, K, interp, iw), *capi.tconv_backward_weight(got, xt, m, K, interp, iw)]
+    it, ws = C.InterpolationType(interp), (m, iw) if P else (m,)
+    name = "weighted_" if P else ""
+    new = [getattr(C, name + "mapped_conv_forward")(x, *ws, w, b, K, it), *getattr(C, name + "mapped_conv_backward")(go, *ws, x, w, b, K, it),
+           getattr(C, name + "mapped_transposed_conv_forward")(xt, *ws, wt, bt, H, W, K, it),
+           *getattr(C, name + "mapped_transposed_conv_backward")(got, *ws, xt, wt, bt, K, it)]
+    for what, n, o in zip(("forward", "dInput", "dW", "dBias", "t forward", "t dInput", "t dW", "t dBias"), new, old):
+        for which, f in (("NaN", torch.isnan), ("+inf", torch.isposinf), ("-inf", torch.isneginf)):
+            assert torch.equal(f(n), f(o)), (what, which, int(f(n).sum()), int(f(o).sum()))
