@@ -7,6 +7,7 @@
 // module names.  There is no CPU path: CPU tensors raise.
 #include <torch/extension.h>
 
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -930,6 +931,16 @@ bool args_ok(const torch::Tensor &x, const torch::Tensor &map, const OptTensor &
   if (iw && (iw->dim() != want - 1 || x.scalar_type() != iw->scalar_type() || map.size(-2) != iw->size(-1))) return false;
   return (in_channels < 0 || x.size(1) == in_channels) && (!k || map.size(2) == kernel_size);
 }
+// What the native nodes are invisible to: a torch.jit trace, torch.func transforms, forward-mode tangents.  Such a call returns
+// nothing either, and the Python layer takes it through an autograd Function; `inside`: the call that comes from there.
+bool transformed(std::initializer_list<const torch::Tensor *> ts) {
+  if (at::tracer::impl::is_dispatch_enabled() || c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode))
+    return true;
+  for (const torch::Tensor *t : ts)
+    if (t != nullptr && t->defined() && t->_fw_grad(0).defined()) return true;
+  return false;
+}
+const torch::Tensor *opt(const OptTensor &t) { return t ? &*t : nullptr; }
 bool map_covers(const torch::Tensor &x, const torch::Tensor &map) { return x.size(2) == map.size(0) && x.size(3) == map.size(1); }
 
 // A node's saved tensors (an absent one stays undefined) and the operator's plain arguments.
@@ -984,7 +995,8 @@ struct MappedConvNode : public MapNode {
   }
 };
 OptTensor mapped_convolution(const torch::Tensor &x, const torch::Tensor &weight, const torch::Tensor &bias, const torch::Tensor &map,
-                             int64_t K, InterpolationType it, const OptTensor &iw, bool relu) {
+                             int64_t K, InterpolationType it, const OptTensor &iw, bool relu, bool inside) {
+  if (!inside && transformed({&x, &weight, &bias, &map, opt(iw)})) return c10::nullopt;
   if (weight.dim() != 3 || !args_ok(x, map, iw, weight.size(1), weight.size(2))) return c10::nullopt;
   torch::Tensor out;
   {
@@ -1015,7 +1027,8 @@ struct MappedTransposedConvNode : public MapNode {
 };
 OptTensor mapped_transposed_convolution(const torch::Tensor &x, const torch::Tensor &weight, const torch::Tensor &bias,
                                         const torch::Tensor &map, int64_t oh, int64_t ow, int64_t K, InterpolationType it,
-                                        const OptTensor &iw) {
+                                        const OptTensor &iw, bool inside) {
+  if (!inside && transformed({&x, &weight, &bias, &map, opt(iw)})) return c10::nullopt;
   if (weight.dim() != 3 || !args_ok(x, map, iw, weight.size(0), weight.size(2)) || !map_covers(x, map)) return c10::nullopt;
   torch::Tensor out;
   {
@@ -1042,7 +1055,8 @@ struct MappedMaxPoolNode : public MapNode {
   }
 };
 c10::optional<std::tuple<torch::Tensor, torch::Tensor>> max_pool_op(const torch::Tensor &x, const torch::Tensor &map, int64_t K,
-                                                                   InterpolationType it, const OptTensor &iw) {
+                                                                   InterpolationType it, const OptTensor &iw, bool inside) {
+  if (!inside && transformed({&x, &map, opt(iw)})) return c10::nullopt;
   if (!args_ok(x, map, iw, -1, K)) return c10::nullopt;
   std::vector<torch::Tensor> r;
   {
@@ -1072,7 +1086,8 @@ struct ResampleNode : public MapNode {
   }
 };
 OptTensor resample_op(const torch::Tensor &x, const torch::Tensor &map, InterpolationType it, const OptTensor &iw, bool scatter, int64_t oh,
-                      int64_t ow) {
+                      int64_t ow, bool inside) {
+  if (!inside && transformed({&x, &map, opt(iw)})) return c10::nullopt;
   if (!args_ok(x, map, iw, -1, -1) || (scatter && !map_covers(x, map))) return c10::nullopt;
   torch::Tensor out;
   {
@@ -1104,10 +1119,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .value("BROWN", DistortionType::BROWN)
       .value("FISHEYE", DistortionType::FISHEYE);
 
-  m.def("mapped_convolution_op", &mapped_convolution);
-  m.def("mapped_transposed_convolution_op", &mapped_transposed_convolution);
-  m.def("mapped_max_pool_op", &max_pool_op);
-  m.def("resample_op", &resample_op);
+  m.def("mapped_convolution_op", &mapped_convolution, py::arg("x"), py::arg("weight"), py::arg("bias"), py::arg("map"), py::arg("K"),
+        py::arg("interp"), py::arg("interp_weights"), py::arg("relu"), py::arg("inside") = false);
+  m.def("mapped_transposed_convolution_op", &mapped_transposed_convolution, py::arg("x"), py::arg("weight"), py::arg("bias"), py::arg("map"),
+        py::arg("oh"), py::arg("ow"), py::arg("K"), py::arg("interp"), py::arg("interp_weights"), py::arg("inside") = false);
+  m.def("mapped_max_pool_op", &max_pool_op, py::arg("x"), py::arg("map"), py::arg("K"), py::arg("interp"), py::arg("interp_weights"),
+        py::arg("inside") = false);
+  m.def("resample_op", &resample_op, py::arg("x"), py::arg("map"), py::arg("interp"), py::arg("interp_weights"), py::arg("scatter"),
+        py::arg("oh"), py::arg("ow"), py::arg("inside") = false);
   m.def("resample_to_map", &resample_to_map);
   m.def("resample_from_map", &resample_from_map);
   m.def("weighted_resample_to_map", &weighted_resample_to_map);

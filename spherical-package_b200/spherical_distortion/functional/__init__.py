@@ -23,11 +23,37 @@ def _scalars(kernel_size, interp):
     return torch.tensor(kernel_size), torch.tensor(int(interp))
 
 
-def _failed(*check):
-    """The native operator returned nothing: its arguments fail the checks, whose assertions are raised here."""
-    for fn, *args in check:
-        fn(*args)
-    raise AssertionError("arguments do not fit the operator")
+class _AsFunction(torch.autograd.Function):
+    """A native operator inside a Python autograd Function, for what its own node is invisible to: torch.jit traces record the
+    Function as one opaque node; forward-mode differentiation and torch.func transforms refuse it, as they do any without rules
+    of their own."""
+
+    @staticmethod
+    def forward(ctx, op, *args):
+        wanted = [i for i in range(len(args)) if ctx.needs_input_grad[i + 1]]
+        inner = [a.detach().requires_grad_(i in wanted) if isinstance(a, torch.Tensor) else a for i, a in enumerate(args)]
+        with torch.set_grad_enabled(bool(wanted)):
+            out = op(*inner, True)
+        if out is None:
+            raise AssertionError("arguments do not fit the operator")
+        many = isinstance(out, tuple)
+        ctx.wanted, ctx.inputs, ctx.output = wanted, [inner[i] for i in wanted], out[0] if many else out
+        result = [o.detach() for o in (out if many else (out,))]
+        ctx.mark_non_differentiable(*[o for o in result if not o.is_floating_point()])
+        return tuple(result) if many else result[0]
+
+    @staticmethod
+    def backward(ctx, grad_output, *_):
+        grads = iter(torch.autograd.grad(ctx.output, ctx.inputs, grad_output, retain_graph=True, allow_unused=True))
+        return (None,) + tuple(next(grads) if i in ctx.wanted else None for i in range(len(ctx.needs_input_grad) - 1))
+
+
+def _by_function(op, args, *checks):
+    """The native operator returned nothing: its arguments fail the checks, whose assertions are raised here, or something
+    that its autograd node is invisible to looks at the call."""
+    for fn, *a in checks:
+        fn(*a)
+    return _AsFunction.apply(op, *args)
 
 
 # The operators' autograd nodes are part of the native extension: one call per operator.
@@ -35,26 +61,30 @@ def mapped_convolution(input, weight, bias, sample_map, kernel_size, interp, int
     """`activation` (None or "relu") is an extension of this library: the ReLU runs inside the convolution kernels
     instead of as separate passes over the output and its gradient."""
     assert activation in (None, "relu"), "activation must be None or 'relu'"
-    out = _C.mapped_convolution_op(input, weight, bias, sample_map, kernel_size, interp, interp_weights, activation is not None)
+    args = (input, weight, bias, sample_map, kernel_size, interp, interp_weights, activation is not None)
+    out = _C.mapped_convolution_op(*args)
     if out is None:
-        _failed((check_args, input, sample_map, interp_weights, weight.shape[1], weight.shape[2]))
+        out = _by_function(_C.mapped_convolution_op, args,
+                           (check_args, input, sample_map, interp_weights, weight.shape[1], weight.shape[2]))
     return out
 
 
 def mapped_transposed_convolution(input, weight, bias, sample_map, output_height, output_width, kernel_size, interp,
                                   interp_weights=None):
-    out = _C.mapped_transposed_convolution_op(input, weight, bias, sample_map, output_height, output_width, kernel_size,
-                                              interp, interp_weights)
+    args = (input, weight, bias, sample_map, output_height, output_width, kernel_size, interp, interp_weights)
+    out = _C.mapped_transposed_convolution_op(*args)
     if out is None:
-        _failed((check_args, input, sample_map, interp_weights, weight.shape[0], weight.shape[2]),
-                (check_input_map_shape, input, sample_map))
+        out = _by_function(_C.mapped_transposed_convolution_op, args,
+                           (check_args, input, sample_map, interp_weights, weight.shape[0], weight.shape[2]),
+                           (check_input_map_shape, input, sample_map))
     return out
 
 
 def mapped_max_pool(input, sample_map, kernel_size, interp, interp_weights=None):
-    out = _C.mapped_max_pool_op(input, sample_map, kernel_size, interp, interp_weights)
+    args = (input, sample_map, kernel_size, interp, interp_weights)
+    out = _C.mapped_max_pool_op(*args)
     if out is None:
-        _failed((check_args, input, sample_map, interp_weights, None, kernel_size))
+        out = _by_function(_C.mapped_max_pool_op, args, (check_args, input, sample_map, interp_weights, None, kernel_size))
     return out
 
 
@@ -68,9 +98,11 @@ def _with_batch(fn, input, *args):
 def resample(input, sample_map, output_shape, interp, interp_weights=None):
     """Scatter forward, gather backward (layers/functional/resample.py:11-48)."""
     def run(x):
-        out = _C.resample_op(x, sample_map, interp, interp_weights, True, output_shape[0], output_shape[1])
+        args = (x, sample_map, interp, interp_weights, True, output_shape[0], output_shape[1])
+        out = _C.resample_op(*args)
         if out is None:
-            _failed((check_args, x, sample_map, interp_weights, None, None), (check_input_map_shape, x, sample_map))
+            out = _by_function(_C.resample_op, args, (check_args, x, sample_map, interp_weights, None, None),
+                               (check_input_map_shape, x, sample_map))
         return out
     return _with_batch(run, input)
 
@@ -78,9 +110,10 @@ def resample(input, sample_map, output_shape, interp, interp_weights=None):
 def unresample(input, sample_map, interp, interp_weights=None):
     """Gather forward, scatter backward (layers/functional/resample.py:51-83)."""
     def run(x):
-        out = _C.resample_op(x, sample_map, interp, interp_weights, False, 0, 0)
+        args = (x, sample_map, interp, interp_weights, False, 0, 0)
+        out = _C.resample_op(*args)
         if out is None:
-            _failed((check_args, x, sample_map, interp_weights, None, None))
+            out = _by_function(_C.resample_op, args, (check_args, x, sample_map, interp_weights, None, None))
         return out
     return _with_batch(run, input)
 
