@@ -963,7 +963,7 @@ struct MapNode : public Node {
   variable_list apply(variable_list &&g) override {
     std::lock_guard<std::mutex> lock(mu);
     variable_list r(num_outputs());
-    if (!g[0].defined()) return r;
+    if (!g[0].defined()) g[0] = input_metadata(0).zeros_like();  // an output nobody depended on: zero gradients, as autograd Functions give
     at::NoGradGuard no_grad;
     const torch::Tensor m = map.unpack(), q = weighted ? iw.unpack() : torch::Tensor();
     gradients(r, g[0], m, weighted ? &q : nullptr);

@@ -70,3 +70,15 @@ def test_saved_tensor_hooks(name):
     with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t) or t.cpu(), lambda t: t.cuda()):
         got = _gradient(f, x)
     assert packed and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_undefined_output_gradient_gives_zeros(name):
+    class Blocks(torch.autograd.Function):
+        forward = staticmethod(lambda ctx, x: x.clone())
+        backward = staticmethod(lambda ctx, g: None)
+
+    f, x = _operators()[name]
+    x.requires_grad_(True)
+    Blocks.apply(f(x)).sum().backward()
+    assert x.grad is not None and not x.grad.any()
