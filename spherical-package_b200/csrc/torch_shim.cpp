@@ -972,10 +972,11 @@ struct MapNode : public Node {
   virtual void gradients(variable_list &r, torch::Tensor go, const torch::Tensor &m, const torch::Tensor *q) = 0;
 };
 
+// (A map or its weights that require a gradient make the result require one and get none, as from an autograd Function.)
 bool wants_grad(std::initializer_list<const torch::Tensor *> ts) {
   if (!at::GradMode::is_enabled()) return false;
   for (const torch::Tensor *t : ts)
-    if (t->requires_grad()) return true;
+    if (t != nullptr && t->requires_grad()) return true;
   return false;
 }
 template <class N> std::shared_ptr<N> new_node(const torch::autograd::edge_list &edges) {
@@ -1003,8 +1004,8 @@ OptTensor mapped_convolution(const torch::Tensor &x, const torch::Tensor &weight
     at::NoGradGuard no_grad;
     out = conv_forward_impl(x, map, iw ? &*iw : nullptr, weight, bias, K, it, relu);
   }
-  if (wants_grad({&x, &weight, &bias})) {
-    auto n = new_node<MappedConvNode>(torch::autograd::collect_next_edges(x, weight, bias));
+  if (wants_grad({&x, &weight, &bias, &map, opt(iw)})) {
+    auto n = new_node<MappedConvNode>(torch::autograd::collect_next_edges(x, weight, bias, map, iw.value_or(torch::Tensor())));
     n->x = SavedVariable(x, false);
     n->weight = SavedVariable(weight, false);
     n->bias = SavedVariable(bias, false);
@@ -1035,8 +1036,8 @@ OptTensor mapped_transposed_convolution(const torch::Tensor &x, const torch::Ten
     at::NoGradGuard no_grad;
     out = tconv_forward_impl(x, map, iw ? &*iw : nullptr, weight, bias, oh, ow, K, it);
   }
-  if (wants_grad({&x, &weight, &bias})) {
-    auto n = new_node<MappedTransposedConvNode>(torch::autograd::collect_next_edges(x, weight, bias));
+  if (wants_grad({&x, &weight, &bias, &map, opt(iw)})) {
+    auto n = new_node<MappedTransposedConvNode>(torch::autograd::collect_next_edges(x, weight, bias, map, iw.value_or(torch::Tensor())));
     n->x = SavedVariable(x, false);
     n->weight = SavedVariable(weight, false);
     n->bias = SavedVariable(bias, false);
@@ -1063,8 +1064,8 @@ c10::optional<std::tuple<torch::Tensor, torch::Tensor>> max_pool_op(const torch:
     at::NoGradGuard no_grad;
     r = max_pool_impl(x, map, iw ? &*iw : nullptr, K, it);
   }
-  if (wants_grad({&x})) {
-    auto n = new_node<MappedMaxPoolNode>(torch::autograd::collect_next_edges(x));
+  if (wants_grad({&x, &map, opt(iw)})) {
+    auto n = new_node<MappedMaxPoolNode>(torch::autograd::collect_next_edges(x, map, iw.value_or(torch::Tensor())));
     n->x = SavedVariable(r[1], false);
     n->save_map(map, iw);
     n->K = K;
@@ -1094,8 +1095,8 @@ OptTensor resample_op(const torch::Tensor &x, const torch::Tensor &map, Interpol
     at::NoGradGuard no_grad;
     out = scatter ? resample_to_map_impl(x, map, iw ? &*iw : nullptr, oh, ow, it) : resample_from_map_impl(x, map, iw ? &*iw : nullptr, it);
   }
-  if (wants_grad({&x})) {
-    auto n = new_node<ResampleNode>(torch::autograd::collect_next_edges(x));
+  if (wants_grad({&x, &map, opt(iw)})) {
+    auto n = new_node<ResampleNode>(torch::autograd::collect_next_edges(x, map, iw.value_or(torch::Tensor())));
     n->save_map(map, iw);
     n->it = it;
     n->scatter = scatter;

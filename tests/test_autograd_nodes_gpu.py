@@ -82,3 +82,30 @@ def test_undefined_output_gradient_gives_zeros(name):
     x.requires_grad_(True)
     Blocks.apply(f(x)).sum().backward()
     assert x.grad is not None and not x.grad.any()
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_maps_that_require_gradients(weighted):
+    """They get none, but the result requires one and backward runs, whatever else takes part."""
+    from spherical_distortion import functional as F
+    from spherical_distortion.nn import InterpolationType
+    it = InterpolationType.NEAREST
+    g = torch.Generator().manual_seed(3)
+    r = lambda *s: torch.rand(*s, generator=g).cuda()  # noqa: E731
+    x, m = r(1, 3, 8, 9), r(8, 9, 4, 2, 2) * 7 if weighted else r(8, 9, 4, 2) * 7
+    iw = r(8, 9, 4, 2) if weighted else None
+    w, b = r(2, 3, 4), r(2)
+    wanting = iw if weighted else m
+    m1, iw1 = m[:, :, 0].contiguous(), iw[:, :, 0].contiguous() if weighted else None
+    for t in (wanting, iw1 if weighted else m1):
+        t.requires_grad_(True)
+    for out, t in ((F.mapped_convolution(x, w, b, m, 4, it, iw), wanting),
+                   (F.mapped_transposed_convolution(x, w.transpose(0, 1).contiguous(), b, m, 8, 9, 4, it, iw), wanting),
+                   (F.mapped_max_pool(x, m, 4, it, iw)[0], wanting),
+                   (F.resample(x, m1, (8, 9), it, iw1), iw1 if weighted else m1), (F.unresample(x, m1, it, iw1), iw1 if weighted else m1)):
+        assert out.requires_grad
+        out.sum().backward()
+        assert t.grad is None
+    x.requires_grad_(True)
+    F.mapped_convolution(x, w, b, m, 4, it, iw).sum().backward()
+    assert x.grad.any() and wanting.grad is None
