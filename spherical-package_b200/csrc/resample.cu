@@ -322,18 +322,23 @@ SPH_TU_STATUS(resample)
 
 extern "C" size_t sph_staging_bytes(int op, int64_t planes, int64_t n_src, int64_t reads, int dtype) {
   if (dtype != SPH_F32 || planes < 3 || n_src <= 0 || n_src >= ((int64_t)1 << 31)) return 0;
+  PlaneChunks c;
   switch (op) {
     // A gather that reads a pixel less than once on average leaves whole sectors of the source untouched, which the
     // transposition would fetch; and the few taps per position of a resampling map do not pay for rows that go through HBM.
-    case SPH_STAGE_GATHER: {
-      const PlaneChunks c = stage_chunks(planes, n_src, 4);
-      return reads < n_src || c.group_bytes > kStageGroup ? 0 : stage_bytes(c);
-    }
-    case SPH_STAGE_SCATTER: return stage_bytes(stage_chunks(planes, n_src, 4, kScatterGroup));
-    case SPH_STAGE_POOL: return reads < n_src ? 0 : stage_bytes(stage_chunks(planes, n_src, 4));
-    case SPH_STAGE_ARGMAX: return stage_bytes(stage_chunks(planes, n_src, 5));
+    case SPH_STAGE_GATHER:
+      c = stage_chunks(planes, n_src, 4);
+      if (reads < n_src || c.group_bytes > kStageGroup) return 0;
+      break;
+    case SPH_STAGE_SCATTER: c = stage_chunks(planes, n_src, 4, kScatterGroup); break;
+    case SPH_STAGE_POOL:
+      c = stage_chunks(planes, n_src, 4);
+      if (reads < n_src) return 0;
+      break;
+    case SPH_STAGE_ARGMAX: c = stage_chunks(planes, n_src, 5); break;
     default: return 0;
   }
+  return stage_fits(c) ? stage_bytes(c) : 0;
 }
 
 extern "C" int sph_resample_from_map(const void *x, const void *map, const void *iw, void *y, int64_t B, int64_t C,
