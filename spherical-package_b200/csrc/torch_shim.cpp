@@ -303,13 +303,18 @@ torch::Tensor workspace(size_t bytes, const torch::Tensor &like) {
   return torch::empty({(int64_t)(bytes ? bytes : 1)}, like.options().dtype(torch::kUInt8));
 }
 
-// Scratch of the plane-group kernels of resampling and pooling; undefined where they would not pay.
+// Scratch of the plane-group kernels of resampling and pooling; none where they would not pay or memory is short.
 struct Staging {
   torch::Tensor buf;
   size_t bytes = 0;
   Staging(int op, int64_t planes, int64_t n_src, int64_t reads, const torch::Tensor &like) {
-    bytes = sph_staging_bytes(op, planes, n_src, reads, dtype_of(like));
-    if (bytes) buf = workspace(bytes, like);
+    const size_t n = sph_staging_bytes(op, planes, n_src, reads, dtype_of(like));
+    if (n == 0) return;
+    try {
+      buf = workspace(n, like);
+      bytes = n;
+    } catch (const c10::OutOfMemoryError &) {
+    }
   }
   void *ptr() const { return bytes ? buf.data_ptr() : nullptr; }
 };
@@ -633,6 +638,25 @@ struct ConvArgs {
   int dtype, interp, prec;
 };
 
+// Scratch of a convolution: what its fastest kernels want, or, where that is not to be had, what it cannot do without.
+struct ConvScratch {
+  torch::Tensor buf;
+  size_t bytes = 0;
+  void get(int op, const ConvArgs &a, const torch::Tensor &like) {
+    if (buf.defined()) return;
+    bytes = sph_conv_workspace_preferred_bytes(op, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec);
+    try {
+      buf = workspace(bytes, like);
+    } catch (const c10::OutOfMemoryError &) {
+      const size_t least = sph_conv_workspace_bytes(op, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec);
+      if (least >= bytes) throw;
+      bytes = least;
+      buf = workspace(bytes, like);
+    }
+  }
+  void *ptr() const { return buf.data_ptr(); }
+};
+
 // relu: the fused variant (sph_mapped_conv_relu_*, an extension without a reference counterpart); shapes the
 // library does not fuse fall back to the plain operator plus a separate activation.
 torch::Tensor conv_forward_impl(torch::Tensor x, torch::Tensor map, const torch::Tensor *iw, torch::Tensor weight,
@@ -650,9 +674,8 @@ torch::Tensor conv_forward_impl(torch::Tensor x, torch::Tensor map, const torch:
   const ConvArgs a{x.size(0), x.size(1), weight.size(0), x.size(2), x.size(3), m.H, m.W, K, m.P, dtype_of(x), (int)it,
                    dtype_of(x) == SPH_F32 ? precision() : SPH_PRECISION_EXACT};
   torch::Tensor out = torch::empty({a.B, a.Cout, a.OH, a.OW}, x.options());
-  const size_t wb = sph_conv_workspace_preferred_bytes(SPH_CONV_FORWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
-                                             a.interp, a.prec);
-  torch::Tensor ws = workspace(wb, x);
+  ConvScratch ws;
+  ws.get(SPH_CONV_FORWARD, a, x);
   if (a.prec == SPH_PRECISION_BF16 && g_use_companions) {
     // channels-last companions: gather from the input's copy if a previous layer left one; with the fused ReLU also
     // write the copy of the output for the next layer
@@ -671,14 +694,14 @@ torch::Tensor conv_forward_impl(torch::Tensor x, torch::Tensor map, const torch:
       int rc = sph_mapped_conv_forward_cl(x.data_ptr(), x_cl, map.data_ptr(), iw ? iw->data_ptr() : nullptr, weight.data_ptr(),
                                           bias.data_ptr(), out.data_ptr(), out_cl.defined() ? out_cl.data_ptr() : nullptr, a.B,
                                           a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec, relu ? 1 : 0,
-                                          ws.data_ptr(), wb, stream());
+                                          ws.ptr(), ws.bytes, stream());
       if (rc == SPH_ERR_UNSUPPORTED && out_cl.defined()) {   // this shape cannot write the copy (or cannot fuse): without it
         out_cl = torch::Tensor();
         rc = x_cl == nullptr ? SPH_ERR_UNSUPPORTED
                              : sph_mapped_conv_forward_cl(x.data_ptr(), x_cl, map.data_ptr(), iw ? iw->data_ptr() : nullptr,
                                                           weight.data_ptr(), bias.data_ptr(), out.data_ptr(), nullptr, a.B, a.Cin,
                                                           a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec,
-                                                          relu ? 1 : 0, ws.data_ptr(), wb, stream());
+                                                          relu ? 1 : 0, ws.ptr(), ws.bytes, stream());
       }
       if (rc != SPH_ERR_UNSUPPORTED) {
         ok(rc, "sph_mapped_conv_forward_cl");
@@ -691,7 +714,7 @@ torch::Tensor conv_forward_impl(torch::Tensor x, torch::Tensor map, const torch:
   if (relu) {
     const int rc = sph_mapped_conv_relu_forward(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, weight.data_ptr(),
                                                 bias.data_ptr(), out.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K,
-                                                a.P, a.dtype, a.interp, a.prec, ws.data_ptr(), wb, stream());
+                                                a.P, a.dtype, a.interp, a.prec, ws.ptr(), ws.bytes, stream());
     if (rc != SPH_ERR_UNSUPPORTED) {
       ok(rc, "sph_mapped_conv_relu_forward");
       maybe_check_device("mapped convolution");
@@ -700,7 +723,7 @@ torch::Tensor conv_forward_impl(torch::Tensor x, torch::Tensor map, const torch:
   }
   ok(sph_mapped_conv_forward(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, weight.data_ptr(), bias.data_ptr(),
                              out.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec,
-                             ws.data_ptr(), wb, stream()),
+                             ws.ptr(), ws.bytes, stream()),
      "sph_mapped_conv_forward");
   if (relu) out.clamp_min_(0);
   maybe_check_device("mapped convolution");
@@ -737,7 +760,7 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
   if (a.prec == SPH_PRECISION_BF16) {
     // all three gradients in one call: grad_output is converted (and masked) once for both of its consumers, and the
     // input's channels-last copy is used if a previous layer left one
-    const size_t wbc = sph_conv_workspace_preferred_bytes(SPH_CONV_BACKWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
+    const size_t wbc = sph_conv_workspace_bytes(SPH_CONV_BACKWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
                                                 a.interp, a.prec);
     if (wbc > 0) {
       torch::Tensor wsc = workspace(wbc, x);
@@ -753,26 +776,37 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
       }
     }
   }
-  size_t wb = !need_gx ? 0 : sph_conv_workspace_preferred_bytes(SPH_CONV_BACKWARD_INPUT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
-                                       a.dtype, a.interp, a.prec);
-  torch::Tensor ws = workspace(wb, x);
-  size_t wb2 = sph_conv_workspace_preferred_bytes(SPH_CONV_BACKWARD_WEIGHT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
-                                        a.interp, a.prec);
-  torch::Tensor ws2 = workspace(wb2, x);
+  // The scratch of the input gradient is given back before the weight gradient's is taken.
+  const void *q = iw ? iw->data_ptr() : nullptr;
+  ConvScratch wsx, wsw;
+  const auto input_gradient = [&](const torch::Tensor *mask) -> int {
+    if (!need_gx) return SPH_OK;
+    wsx.get(SPH_CONV_BACKWARD_INPUT, a, x);
+    if (mask)
+      return sph_mapped_conv_relu_backward_input(go.data_ptr(), mask->data_ptr(), plan.data_ptr(), weight.data_ptr(), gx.data_ptr(), a.B,
+                                                 a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.dtype, a.prec, wsx.ptr(), wsx.bytes, stream());
+    return sph_mapped_conv_backward_input(go.data_ptr(), plan.data_ptr(), weight.data_ptr(), gx.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW,
+                                          a.OH, a.OW, a.K, a.dtype, a.prec, wsx.ptr(), wsx.bytes, stream());
+  };
+  const auto weight_gradient = [&](const torch::Tensor *mask) -> int {
+    wsx = ConvScratch();
+    wsw.get(SPH_CONV_BACKWARD_WEIGHT, a, x);
+    if (mask)
+      return sph_mapped_conv_relu_backward_weight(go.data_ptr(), mask->data_ptr(), x.data_ptr(), map.data_ptr(), q, gw.data_ptr(),
+                                                  gb.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp,
+                                                  a.prec, wsw.ptr(), wsw.bytes, stream());
+    return sph_mapped_conv_backward_weight(go.data_ptr(), x.data_ptr(), map.data_ptr(), q, gw.data_ptr(), gb.data_ptr(), a.B, a.Cin, a.Cout,
+                                           a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec, wsw.ptr(), wsw.bytes, stream());
+  };
+  bool have_gx = false;
   if (act_out) {  // gradient of the fused ReLU: the kernels read grad_output * (act_out > 0)
-    const int rc = !need_gx ? SPH_OK : sph_mapped_conv_relu_backward_input(go.data_ptr(), act_out->data_ptr(), plan.data_ptr(), weight.data_ptr(),
-                                                       gx.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.dtype,
-                                                       a.prec, ws.data_ptr(), wb, stream());
     // The two fused operators are eligible independently (the weight-gradient kernel's tap table is smaller than the
     // gather-GEMM's), so each one that declines falls back on its own to a masked copy and the plain operator.
-    bool have_gx = false;
+    const int rc = input_gradient(act_out);
     if (rc != SPH_ERR_UNSUPPORTED) {
       ok(rc, "sph_mapped_conv_relu_backward_input");
       have_gx = true;
-      const int rc2 = sph_mapped_conv_relu_backward_weight(go.data_ptr(), act_out->data_ptr(), x.data_ptr(), map.data_ptr(),
-                                                           iw ? iw->data_ptr() : nullptr, gw.data_ptr(), gb.data_ptr(), a.B,
-                                                           a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp,
-                                                           a.prec, ws2.data_ptr(), wb2, stream());
+      const int rc2 = weight_gradient(act_out);
       if (rc2 != SPH_ERR_UNSUPPORTED) {
         ok(rc2, "sph_mapped_conv_relu_backward_weight");
         maybe_check_device("mapped convolution");
@@ -780,24 +814,9 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
       }
     }
     go = at::threshold_backward(go, *act_out, 0);
-    if (have_gx) {
-      ok(sph_mapped_conv_backward_weight(go.data_ptr(), x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr,
-                                         gw.data_ptr(), gb.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
-                                         a.dtype, a.interp, a.prec, ws2.data_ptr(), wb2, stream()),
-         "sph_mapped_conv_backward_weight");
-      maybe_check_device("mapped convolution");
-      return {gx, gw, gb};
-    }
   }
-  if (need_gx)
-    ok(sph_mapped_conv_backward_input(go.data_ptr(), plan.data_ptr(), weight.data_ptr(), gx.data_ptr(), a.B, a.Cin, a.Cout,
-                                      a.IH, a.IW, a.OH, a.OW, a.K, a.dtype, a.prec, ws.data_ptr(), wb, stream()),
-       "sph_mapped_conv_backward_input");
-  wb = wb2;
-  ok(sph_mapped_conv_backward_weight(go.data_ptr(), x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr,
-                                     gw.data_ptr(), gb.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
-                                     a.dtype, a.interp, a.prec, ws2.data_ptr(), wb, stream()),
-     "sph_mapped_conv_backward_weight");
+  if (!have_gx) ok(input_gradient(nullptr), "sph_mapped_conv_backward_input");
+  ok(weight_gradient(nullptr), "sph_mapped_conv_backward_weight");
   maybe_check_device("mapped convolution");
   return {gx, gw, gb};
 }
@@ -849,11 +868,10 @@ torch::Tensor tconv_forward_impl(torch::Tensor x, torch::Tensor map, const torch
                    dtype_of(x) == SPH_F32 ? precision() : SPH_PRECISION_EXACT};
   torch::Tensor plan = get_plan(map, iw, a.IH * a.IW, a.K, a.P, a.interp, a.OH, a.OW);
   torch::Tensor out = torch::empty({a.B, a.Cout, a.OH, a.OW}, x.options());
-  const size_t wb = sph_conv_workspace_preferred_bytes(SPH_TCONV_FORWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
-                                             a.interp, a.prec);
-  torch::Tensor ws = workspace(wb, x);
+  ConvScratch ws;
+  ws.get(SPH_TCONV_FORWARD, a, x);
   ok(sph_mapped_tconv_forward(x.data_ptr(), plan.data_ptr(), weight.data_ptr(), bias.data_ptr(), out.data_ptr(), a.B, a.Cin,
-                              a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.dtype, a.prec, ws.data_ptr(), wb, stream()),
+                              a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.dtype, a.prec, ws.ptr(), ws.bytes, stream()),
      "sph_mapped_tconv_forward");
   maybe_check_device("mapped convolution");
   return out;
@@ -877,19 +895,17 @@ std::vector<torch::Tensor> tconv_backward_impl(torch::Tensor go, torch::Tensor m
   const ConvArgs a{x.size(0), x.size(1), weight.size(1), x.size(2), x.size(3), go.size(2), go.size(3), K, m.P, dtype_of(x),
                    (int)it, dtype_of(x) == SPH_F32 ? precision() : SPH_PRECISION_EXACT};
   torch::Tensor gx = torch::empty_like(x), gw = torch::empty_like(weight), gb = torch::empty({a.Cout}, x.options());
-  size_t wb = sph_conv_workspace_preferred_bytes(SPH_TCONV_BACKWARD_INPUT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
-                                       a.dtype, a.interp, a.prec);
-  torch::Tensor ws = workspace(wb, x);
+  ConvScratch ws;
+  ws.get(SPH_TCONV_BACKWARD_INPUT, a, x);
   ok(sph_mapped_tconv_backward_input(go.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, weight.data_ptr(),
                                      gx.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp,
-                                     a.prec, ws.data_ptr(), wb, stream()),
+                                     a.prec, ws.ptr(), ws.bytes, stream()),
      "sph_mapped_tconv_backward_input");
-  wb = sph_conv_workspace_preferred_bytes(SPH_TCONV_BACKWARD_WEIGHT, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
-                                a.interp, a.prec);
-  torch::Tensor ws2 = workspace(wb, x);
+  ws = ConvScratch();
+  ws.get(SPH_TCONV_BACKWARD_WEIGHT, a, x);
   ok(sph_mapped_tconv_backward_weight(go.data_ptr(), x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr,
                                       gw.data_ptr(), gb.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
-                                      a.dtype, a.interp, a.prec, ws2.data_ptr(), wb, stream()),
+                                      a.dtype, a.interp, a.prec, ws.ptr(), ws.bytes, stream()),
      "sph_mapped_tconv_backward_weight");
   maybe_check_device("mapped convolution");
   return {gx, gw, gb};
