@@ -118,12 +118,28 @@ def debug_bounded_wait(limit_ns=1000000):
     return int(st.item())
 
 
-def resample_from_map(x, smap, interp, iw=None):
+STAGE_GATHER, STAGE_POOL, STAGE_ARGMAX, STAGE_SCATTER = 0, 1, 2, 3
+
+
+def staging(op, planes, n_src, reads, like):
+    """Scratch of the plane-group kernels for an operator's `ws` argument, or None where sph_staging_bytes() reports none."""
+    n = lib.sph_staging_bytes(_int(op), *_ints(planes, n_src, reads), _int(_dt(like)))
+    return _bytes(n, like) if n else None
+
+
+def _staged(name, args, ws, ws_name=None, ws_args=None):
+    """Entry point `name`, or, with scratch, its *_ws form (of another name and other arguments if given)."""
+    if ws is None:
+        return getattr(lib, name)(*args, _stream())
+    return getattr(lib, ws_name or name + "_ws")(*(ws_args or args), _ptr(ws), _sz(ws.numel()), _stream())
+
+
+def resample_from_map(x, smap, interp, iw=None, ws=None):
     B, C, H, W = x.shape
     MH, MW = smap.shape[:2]
     y = torch.empty(B, C, MH, MW, dtype=x.dtype, device=x.device)
-    _ok(lib.sph_resample_from_map(_ptr(x), _ptr(smap), _ptr(iw), _ptr(y), *_ints(B, C, H, W, MH, MW, _P(iw)),
-                                  _int(_dt(x)), _int(int(interp)), _stream()), "sph_resample_from_map")
+    args = (_ptr(x), _ptr(smap), _ptr(iw), _ptr(y), *_ints(B, C, H, W, MH, MW, _P(iw)), _int(_dt(x)), _int(int(interp)))
+    _ok(_staged("sph_resample_from_map", args, ws), "sph_resample_from_map")
     return y
 
 
@@ -139,24 +155,11 @@ def plan_build(smap, iw, n_src, K, interp, dstH, dstW):
     return plan
 
 
-STAGE_GATHER, STAGE_POOL, STAGE_ARGMAX, STAGE_SCATTER = 0, 1, 2, 3
-
-
-def staging(op, planes, n_src, reads, like):
-    """Scratch of the plane-group kernels for an operator's `ws` argument, or None where sph_staging_bytes() reports none."""
-    n = lib.sph_staging_bytes(_int(op), *_ints(planes, n_src, reads), _int(_dt(like)))
-    return _bytes(n, like) if n else None
-
-
 def resample_to_map(x, plan, oh, ow, ws=None):
     B, C, MH, MW = x.shape
     out = torch.empty(B, C, int(oh), int(ow), dtype=x.dtype, device=x.device)
-    if ws is None:
-        rc = lib.sph_resample_to_map(_ptr(x), _ptr(plan), _ptr(out), *_ints(B, C, MH, MW, oh, ow), _int(_dt(x)), _stream())
-    else:
-        rc = lib.sph_resample_to_map_ws(_ptr(x), _ptr(plan), _ptr(out), *_ints(B, C, MH, MW, oh, ow), _int(0), _int(_dt(x)), _ptr(ws),
-                                        _sz(ws.numel()), _stream())
-    _ok(rc, "sph_resample_to_map")
+    args = (_ptr(x), _ptr(plan), _ptr(out), *_ints(B, C, MH, MW, oh, ow))
+    _ok(_staged("sph_resample_to_map", (*args, _int(_dt(x))), ws, None, (*args, _int(0), _int(_dt(x)))), "sph_resample_to_map")
     return out
 
 
@@ -174,15 +177,15 @@ def resample_to_map_static(x, smap, oh, ow, interp, iw=None, out=None):
     return out
 
 
-def mapped_max_pool(x, smap, K, interp, iw=None, out=None, idx=None):
+def mapped_max_pool(x, smap, K, interp, iw=None, out=None, idx=None, ws=None):
     B, C, IH, IW = x.shape
     OH, OW = smap.shape[:2]
     if out is None:
         out = torch.empty(B, C, OH, OW, dtype=x.dtype, device=x.device)
         idx = torch.empty(B, C, OH, OW, dtype=torch.int64, device=x.device)
-    _ok(lib.sph_mapped_max_pool(_ptr(x), _ptr(smap), _ptr(iw), _ptr(out), _ptr(idx),
-                                *_ints(B, C, IH, IW, OH, OW, K, _P(iw)), _int(_dt(x)), _int(int(interp)), _stream()),
-        "sph_mapped_max_pool")
+    args = (_ptr(x), _ptr(smap), _ptr(iw), _ptr(out), _ptr(idx), *_ints(B, C, IH, IW, OH, OW, K, _P(iw)))
+    kinds = (_int(_dt(x)), _int(int(interp)))
+    _ok(_staged("sph_mapped_max_pool", args + kinds, ws, "sph_mapped_pool_ws", (*args, _int(0), *kinds)), "sph_mapped_max_pool")
     return out, idx
 
 
@@ -203,21 +206,22 @@ def slot_plan_build(smap, iw, K, interp, dstH, dstW):
     return plan_build(smap, iw, OH * OW * K, 1, interp, dstH, dstW)
 
 
-def mapped_max_unpool_planned(g, idx, plan, ih, iw_, K, P=0, out=None):
+def mapped_max_unpool_planned(g, idx, plan, ih, iw_, K, P=0, out=None, ws=None):
     B, C, OH, OW = g.shape
     if out is None:
         out = torch.empty(B, C, int(ih), int(iw_), dtype=g.dtype, device=g.device)
-    _ok(lib.sph_mapped_max_unpool_planned(_ptr(g), _ptr(idx), _ptr(plan), _ptr(out), *_ints(B, C, ih, iw_, OH, OW, K, P),
-                                          _int(_dt(g)), _stream()), "sph_mapped_max_unpool_planned")
+    args = (_ptr(g), _ptr(idx), _ptr(plan), _ptr(out), *_ints(B, C, ih, iw_, OH, OW, K, P), _int(_dt(g)))
+    _ok(_staged("sph_mapped_max_unpool_planned", args, ws, "sph_mapped_max_unpool_ws"), "sph_mapped_max_unpool_planned")
     return out
 
 
-def mapped_avg_pool(x, smap, K, interp, iw=None):
+def mapped_avg_pool(x, smap, K, interp, iw=None, ws=None):
     B, C, IH, IW = x.shape
     OH, OW = smap.shape[:2]
     out = torch.empty(B, C, OH, OW, dtype=x.dtype, device=x.device)
-    _ok(lib.sph_mapped_avg_pool(_ptr(x), _ptr(smap), _ptr(iw), _ptr(out), *_ints(B, C, IH, IW, OH, OW, K, _P(iw)),
-                                _int(_dt(x)), _int(int(interp)), _stream()), "sph_mapped_avg_pool")
+    sizes, kinds = _ints(B, C, IH, IW, OH, OW, K, _P(iw)), (_int(_dt(x)), _int(int(interp)))
+    _ok(_staged("sph_mapped_avg_pool", (_ptr(x), _ptr(smap), _ptr(iw), _ptr(out), *sizes, *kinds), ws, "sph_mapped_pool_ws",
+                (_ptr(x), _ptr(smap), _ptr(iw), _ptr(out), _ptr(None), *sizes, _int(1), *kinds)), "sph_mapped_avg_pool")
     return out
 
 
@@ -229,13 +233,21 @@ def mapped_avg_unpool(g, plan, ih, iw_, K):
     return out
 
 
-def resample_to_map_normalized(x, plan, oh, ow, out=None):
+def resample_to_map_normalized(x, plan, oh, ow, out=None, ws=None):
     B, C, MH, MW = x.shape
     if out is None:
         out = torch.empty(B, C, int(oh), int(ow), dtype=x.dtype, device=x.device)
-    _ok(lib.sph_resample_to_map_normalized(_ptr(x), _ptr(plan), _ptr(out), *_ints(B, C, MH, MW, oh, ow), _int(_dt(x)),
-                                           _stream()), "sph_resample_to_map_normalized")
+    args = (_ptr(x), _ptr(plan), _ptr(out), *_ints(B, C, MH, MW, oh, ow))
+    _ok(_staged("sph_resample_to_map_normalized", (*args, _int(_dt(x))), ws, "sph_resample_to_map_ws", (*args, _int(1), _int(_dt(x)))),
+        "sph_resample_to_map_normalized")
     return out
+
+
+def map_locality(smap, K):
+    """1 if neighbouring positions of a float32 map read neighbouring pixels, else 2; synchronises."""
+    flag = torch.zeros(1, dtype=torch.int32, device=smap.device)
+    _ok(lib.sph_map_locality(_ptr(smap), *_ints(smap.numel() // (2 * K), K), _ptr(flag), _stream()), "sph_map_locality")
+    return int(flag.item())
 
 
 def resample_from_uv_maps(tex, quad, uv, interp):
@@ -286,9 +298,11 @@ def build_kernel_map(H, W, kh, kw, stride=1, dilation=1, kind=MAP_INVERSE_GNOMON
     return m
 
 
-def conv_workspace(op, B, Cin, Cout, IH, IW, OH, OW, K, P, dtype, interp, precision, like):
-    n = lib.sph_conv_workspace_bytes(_int(op), *_ints(B, Cin, Cout, IH, IW, OH, OW, K, P), _int(dtype),
-                                     _int(int(interp)), _int(precision))
+def conv_workspace(op, B, Cin, Cout, IH, IW, OH, OW, K, P, dtype, interp, precision, like, preferred=False):
+    """Scratch of a convolution operator; preferred: as much as its fastest kernels want (float32 in the exact precision: the
+    split products on the tensor cores, which the host extension runs; with less, the CUDA-core kernels)."""
+    query = lib.sph_conv_workspace_preferred_bytes if preferred else lib.sph_conv_workspace_bytes
+    n = query(_int(op), *_ints(B, Cin, Cout, IH, IW, OH, OW, K, P), _int(dtype), _int(int(interp)), _int(precision))
     return _bytes(n, like), n
 
 

@@ -1,11 +1,27 @@
 """Adapters that expose the CUDA library with the call signatures of oracle.port /
 oracle.ref, (a) through the C ABI via ctypes and (b) through the plugin modules
 of `_spherical_distortion_ext`, so parity tests can run one case on any of them."""
+import contextlib
+import functools
+
 import torch
 
 
 def _d(*ts):
     return [None if t is None else t.detach().cuda().contiguous() for t in ts]
+
+
+@contextlib.contextmanager
+def preferred_scratch():
+    """sphmap.capi with the scratch that the host extension brings: float32 convolutions in the exact precision run as split
+    products on the tensor cores, else on the CUDA cores."""
+    from sphmap import capi
+    least = capi.conv_workspace
+    capi.conv_workspace = functools.partial(least, preferred=True)
+    try:
+        yield
+    finally:
+        capi.conv_workspace = least
 
 
 class CApi:

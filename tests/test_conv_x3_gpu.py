@@ -16,6 +16,9 @@ CASES = [(2, 16, 32, (16, 32), (16, 32), 9, 1, 0),
          (1, 100, 50, (20, 33), (20, 33), 5, 0, 3),
          (1, 96, 16, (24, 40), (24, 40), 25, 1, 0),
          (1, 260, 256, (16, 32), (16, 32), 9, 1, 0),
+         (3, 16, 40, (64, 128), (64, 128), 9, 1, 0),  # more tiles than SMs, several images: every block takes a second tile
+         (2, 40, 24, (72, 136), (72, 136), 4, 0, 0),
+         (4, 40, 48, (128, 256), (64, 128), 9, 1, 0), # the same where the adjoints multiply first (tiles of one segment)
          (1, 300, 320, (9, 17), (9, 17), 9, 2, 0),    # products of 90 chunks: more than one run of small products
          (1, 8200, 16, (4, 8), (4, 8), 9, 1, 0)]     # dW: the first column group of two slots is the 65th
 

@@ -1,7 +1,9 @@
 """The large-tile kernels of the exact float32 path (128 / 64 x 128 gather-GEMM, 128 x 128 weight gradient, the
 multiply-first adjoint) on shapes that do not fill their tiles and fast paths: odd channel counts, ragged images, every
 interpolation type, weighted maps, down-sampling maps.  Against the CPU oracle at the exact path's tolerance
-|err| <= 1e-5 |ref| + 1e-5 max|ref|."""
+|err| <= 1e-5 |ref| + 1e-5 max|ref|.  With the preferred scratch the same cases run as split products on the tensor cores."""
+import contextlib
+
 import pytest
 import torch
 
@@ -26,7 +28,14 @@ def _close(got, ref, what):
 
 
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "s%d" % c[0])
-def test_exact_conv_and_transposed_conv(case):
+@pytest.mark.parametrize("scratch", ["least", "preferred"])
+def test_exact_conv_and_transposed_conv(case, scratch):
+    from _gpu_impl import preferred_scratch
+    with preferred_scratch() if scratch == "preferred" else contextlib.nullcontext():
+        _check(case)
+
+
+def _check(case):
     from _gpu_impl import CApi
     seed, B, Cin, Cout, IH, IW, OH, OW, K, interp, P = case
     g = torch.Generator().manual_seed(1000 + seed)

@@ -1,7 +1,8 @@
-"""Resampling and pooling over plane groups (the kernels the host extension selects by giving them scratch) against the
-direct kernels of the same library, which the other tests compare with the oracle: bit-identical, at plane counts around
-the group sizes, images whose pixel count is no multiple of a tile or of four, and maps whose tap table does and does not
-fit shared memory."""
+"""Resampling and pooling over plane groups (the entry points with scratch) against the direct kernels of the same library, which
+the other tests compare with the oracle: bit-identical, at plane counts around the group sizes, images whose pixel count is no
+multiple of a tile or of four, and maps whose tap table does and does not fit shared memory.  Which kernels ran is read off
+the library's launch counter: a direct kernel is one launch, a chunk of plane groups two.  Then the host extension, which
+chooses between the two."""
 import pytest
 import torch
 
@@ -18,6 +19,26 @@ def _case(planes, ih, iw, oh, ow, K, P, seed=0):
     return [t.cuda() if t is not None else None for t in (x, m, w, go)]
 
 
+def _launches(fn):
+    from sphmap import capi
+    before = capi.lib.sph_launch_count()
+    r = fn()
+    return r, capi.lib.sph_launch_count() - before
+
+
+def _grouped(op, ws):
+    """op(ws) over plane groups: two launches, and the bits of op(None), one launch."""
+    assert ws is not None
+    (got, n), (want, n1) = _launches(lambda: op(ws)), _launches(lambda: op(None))
+    assert n == 2 and n1 == 1
+    for a, b in zip(*((t if isinstance(t, tuple) else (t,)) for t in (got, want))):
+        assert torch.equal(a, b)
+    return got
+
+
+ANY = 1 << 40    # reads enough for the scratch to be reported
+
+
 @pytest.mark.parametrize("planes", [3, 5, 8, 16, 17, 33, 70])
 @pytest.mark.parametrize("interp,P", [(0, 0), (1, 0), (2, 0), (0, 3), (1, 2)])
 def test_pooling_matches_direct_kernels(planes, interp, P):
@@ -26,16 +47,19 @@ def test_pooling_matches_direct_kernels(planes, interp, P):
     it = C.InterpolationType(interp)
     for ih, iw, oh, ow, K in ((7, 9, 6, 11, 9), (16, 20, 9, 17, 20)):
         x, m, w, go = _case(planes, ih, iw, oh, ow, K, P)
-        assert capi.lib.sph_staging_bytes(1, *capi._ints(planes, ih * iw, oh * ow * K), 0) > 0
-        out, idx = C.weighted_mapped_max_pool(x, m, w, K, it) if P else C.mapped_max_pool(x, m, K, it)
-        ref, ridx = capi.mapped_max_pool(x, m, K, interp, w)
-        assert torch.equal(out, ref) and torch.equal(idx, ridx)
-        avg = C.weighted_mapped_avg_pool(x, m, w, K, it) if P else C.mapped_avg_pool(x, m, K, it)
-        assert torch.equal(avg, capi.mapped_avg_pool(x, m, K, interp, w))
+        ws = capi.staging(capi.STAGE_POOL, planes, ih * iw, ANY, x)
+        ref, ridx = _grouped(lambda s: capi.mapped_max_pool(x, m, K, interp, w, ws=s), ws)
+        avg = _grouped(lambda s: capi.mapped_avg_pool(x, m, K, interp, w, ws=s), ws)
+        idx = ridx.clone()
         idx[0, 0].view(-1)[:5] = torch.tensor([-1, -2, 1 << 40, 3, 1])          # not this output's slots: no contribution
-        gin = C.weighted_mapped_max_unpool(go, idx, m, w, ih, iw, K, it) if P else C.mapped_max_unpool(go, idx, m, ih, iw, K, it)
         plan = capi.slot_plan_build(m, w, K, interp, ih, iw)
-        assert torch.equal(gin, capi.mapped_max_unpool_planned(go, idx, plan, ih, iw, K, P))
+        gin = _grouped(lambda s: capi.mapped_max_unpool_planned(go, idx, plan, ih, iw, K, P, ws=s),
+                       capi.staging(capi.STAGE_ARGMAX, planes, oh * ow, 0, go))
+        out, i = C.weighted_mapped_max_pool(x, m, w, K, it) if P else C.mapped_max_pool(x, m, K, it)
+        assert torch.equal(out, ref) and torch.equal(i, ridx)
+        assert torch.equal(avg, C.weighted_mapped_avg_pool(x, m, w, K, it) if P else C.mapped_avg_pool(x, m, K, it))
+        assert torch.equal(gin, C.weighted_mapped_max_unpool(go, idx, m, w, ih, iw, K, it) if P else
+                           C.mapped_max_unpool(go, idx, m, ih, iw, K, it))
 
 
 @pytest.mark.parametrize("planes", [3, 5, 8, 16, 17, 33, 70])
@@ -47,42 +71,79 @@ def test_resampling_matches_direct_kernels(planes, interp, P):
     for ih, iw, oh, ow in ((7, 9, 13, 11), (12, 20, 40, 33)):
         x, m, w, go = _case(planes, ih, iw, oh, ow, 1, P, seed=1)
         m, w = m[:, :, 0].contiguous(), w[:, :, 0].contiguous() if P else None
-        assert capi.lib.sph_staging_bytes(0, *capi._ints(planes, ih * iw, oh * ow), 0) > 0
-        y = C.weighted_resample_from_map(x, m, w, it) if P else C.resample_from_map(x, m, it)
-        assert torch.equal(y, capi.resample_from_map(x, m, interp, w))
+        y = _grouped(lambda s: capi.resample_from_map(x, m, interp, w, ws=s), capi.staging(capi.STAGE_GATHER, planes, ih * iw, ANY, x))
+        assert torch.equal(y, C.weighted_resample_from_map(x, m, w, it) if P else C.resample_from_map(x, m, it))
         plan = capi.plan_build(m, w, oh * ow, 1, interp, ih, iw)
-        back = C.weighted_resample_to_map(go, m, w, ih, iw, it) if P else C.resample_to_map(go, m, ih, iw, it)
-        assert torch.equal(back, capi.resample_to_map(go, plan, ih, iw))
-        norm = C.resample_to_map_normalized(go, m, w, ih, iw, it)
-        assert torch.equal(norm, capi.resample_to_map_normalized(go, plan, ih, iw))
+        ws = capi.staging(capi.STAGE_SCATTER, planes, oh * ow, 0, go)
+        back = _grouped(lambda s: capi.resample_to_map(go, plan, ih, iw, ws=s), ws)
+        assert torch.equal(back, C.weighted_resample_to_map(go, m, w, ih, iw, it) if P else C.resample_to_map(go, m, ih, iw, it))
+        norm = _grouped(lambda s: capi.resample_to_map_normalized(go, plan, ih, iw, ws=s), ws)
+        assert torch.equal(norm, C.resample_to_map_normalized(go, m, w, ih, iw, it))
+
+
+def _chosen(run, first, then):
+    """The host extension's launches of the first call on a map, while nothing is known of it, and of later ones; equal bits."""
+    want, n = _launches(run)
+    torch.cuda.synchronize()
+    assert n == first
+    for _ in range(2):
+        got, n = _launches(run)
+        assert n == then
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+    return want
+
+
+def _map(local, h, w, oh, ow, K):
+    from spherical_distortion.util import inverse_gnomonic_projection_map
+    if local:
+        return inverse_gnomonic_projection_map((h, w), (3, 3), stride=2, device="cuda")
+    return torch.rand(oh, ow, K, 2, generator=torch.Generator().manual_seed(3)).mul(torch.tensor([w - 1.0, h - 1.0])).cuda()
 
 
 @pytest.mark.parametrize("local", [True, False])
 def test_nearest_pooling_by_locality(local):
-    """The host extension reads the planes in place over a local map, once it knows that the map is one: same bits."""
-    import ctypes
+    """Planes are read in place over a local map, in groups over a scattered one or one not looked at yet (one launch more)."""
     from spherical_distortion.nn import InterpolationType, MappedMaxPool
-    from spherical_distortion.util import inverse_gnomonic_projection_map
     from sphmap import capi
-    H, W = 66, 131
-    if local:
-        m = inverse_gnomonic_projection_map((H, W), (3, 3), stride=2, device="cuda")
-    else:
-        m = torch.rand(33, 66, 9, 2, generator=torch.Generator().manual_seed(3)).mul(torch.tensor([W - 1.0, H - 1.0])).cuda()
-    x = torch.randn(2, 35, H, W, generator=torch.Generator().manual_seed(4)).cuda()
-    n = m.shape[0] * m.shape[1]
-    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
-    capi._ok(capi.lib.sph_map_locality(capi._ptr(m), ctypes.c_int64(n), ctypes.c_int64(9), capi._ptr(flag), capi._stream()), "locality")
-    assert flag.item() == (1 if local else 2)
+    m = _map(local, 144, 288, 72, 144, 9)
+    assert capi.map_locality(m, 9) == (1 if local else 2)
+    x = torch.randn(2, 8, 144, 288, generator=torch.Generator().manual_seed(4)).cuda()
     pool = MappedMaxPool(9, InterpolationType.NEAREST, return_indices=True)
-    runs = []
-    for _ in range(3):
-        runs.append(pool(x, m))
-        torch.cuda.synchronize()
-    for out, idx in runs[1:]:
-        assert torch.equal(out, runs[0][0]) and torch.equal(idx, runs[0][1])
+    out, idx = _chosen(lambda: pool(x, m), 3, 1 if local else 2)
     want, at = capi.mapped_max_pool(x, m, 9, 0)
-    assert torch.equal(runs[0][0], want) and torch.equal(runs[0][1], at)
+    assert torch.equal(out, want) and torch.equal(idx, at)
+
+
+@pytest.mark.parametrize("planes,h,w", [(70, 65, 131), (4, 144, 288)])
+def test_few_values_are_pooled_in_place(planes, h, w):
+    """Nearest neighbours of few values: in place whatever the map, which is not looked at."""
+    from spherical_distortion.nn import InterpolationType, MappedMaxPool
+    m = _map(False, h, w, 33, 66, 9)
+    x = torch.randn(1, planes, h, w, generator=torch.Generator().manual_seed(4)).cuda()
+    _chosen(lambda: MappedMaxPool(9, InterpolationType.NEAREST, return_indices=True)(x, m), 1, 1)
+
+
+@pytest.mark.parametrize("local", [True, False])
+def test_second_wave_of_pooling_blocks(local):
+    """Four taps, and blocks of plane groups that fill the GPU once and a little: in place over a local map."""
+    from spherical_distortion.nn import InterpolationType, MappedMaxPool
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the size is one of 148 SMs")
+    m = _map(local, 144, 288, 72, 144, 9)
+    x = torch.randn(2, 64, 144, 288, generator=torch.Generator().manual_seed(4)).cuda()
+    _chosen(lambda: MappedMaxPool(9, InterpolationType.BILINEAR, return_indices=True)(x, m), 3, 1 if local else 2)
+
+
+@pytest.mark.parametrize("local", [True, False])
+def test_gather_by_locality(local):
+    """Between one and eight reads a pixel: in place over a local map or one not looked at yet, in groups over a scattered one."""
+    import _spherical_distortion_ext._C as C
+    from sphmap import capi
+    m = (_map(True, 80, 160, 0, 0, 9)[:, :, 4] if local else _map(False, 80, 160, 40, 80, 1)[:, :, 0]).contiguous()
+    x = torch.randn(2, 8, 40, 80, generator=torch.Generator().manual_seed(4)).cuda()
+    y, = _chosen(lambda: [C.resample_from_map(x, m, C.InterpolationType.BILINEAR)], 2, 1 if local else 2)
+    assert torch.equal(y, capi.resample_from_map(x, m, 1))
 
 
 @pytest.mark.parametrize("planes", [3, 8, 16])
