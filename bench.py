@@ -317,10 +317,10 @@ def run_encoder(args, rank, local, world):
 
     def kernel_of(li, ph):
         ci = cfg["layers"][li][0]
-        if exact:   # the exact float32 path: thin register-tiled kernels for layer 1, large-tile SIMT kernels for the rest
+        if exact:   # the exact float32 path: thin register-tiled kernels for layer 1, split products for the rest
             if ci * 9 <= 32:
                 return "small_%s (SIMT, thin contraction)" % ph
-            return "conv_dw128_kernel" if ph == "dw" else "conv_gemm128_kernel"
+            return "x3_dw_kernel" if ph == "dw" else "x3_gemm_kernel"
         if ci * 9 <= 32:
             return {"fwd": "tc_thin_fwd_kernel", "bwd.main": "tc_thin_bwd_kernel (dW, dBias, column buffer of dInput)",
                     "bwd.gather": "thin_plan_gather_kernel (dInput)", "bwd.prepass": "thin_wt_image_kernel",
@@ -343,9 +343,9 @@ def run_encoder(args, rank, local, world):
     dom_ms, dom_flops_total, dom_n = groups[dom_kernel]
     tensor_peak = peaks["bf16_tflops_sustained"]
     peak_source = peaks["source"] + " bf16 sustained (kernel timed inside a long step)"
-    if exact:   # no measured float32 figure exists: nominal FMA rate of the CUDA cores at the maximum SM clock
-        tensor_peak = round(148 * 128 * 2 * 1.965e9 / 1e12, 1)
-        peak_source = "nominal float32 FMA rate, 148 SMs x 128 lanes x 2 x 1.965 GHz (no measured figure)"
+    if exact:   # a float32 product is six bf16 products on the tensor cores
+        tensor_peak = round(tensor_peak / 6, 1)
+        peak_source += ", over the six products of a split float32 one"
     achieved = dom_flops_total / (dom_ms * 1e-3) / 1e12
     out = {
         "metric": "mapped-conv fwd+bwd TFLOP/s", "value": round(value, 3), "unit": "TFLOP/s", "n_gpus": world,
@@ -368,7 +368,7 @@ def run_encoder(args, rank, local, world):
                         "d2h_bytes_per_step": 4 * world, "ms_per_step": round(e2e["e2e_unfused"][0] / args.steps, 3),
                         "api": "spherical_distortion.nn.MappedConvolution + torch.relu + autograd (the reference's API, no fused activation)"},
         "gpu_launches": int(launches_per_step * args.steps),
-        "roofline": {"bound": "fp32" if exact else "tensor", "kernel": dom_kernel, "launches_per_step": dom_n,
+        "roofline": {"bound": "tensor", "kernel": dom_kernel, "launches_per_step": dom_n,
                      "avg_launch_ms": round(dom_ms / dom_n, 3),
                      "algorithmic_gflop_per_launch": round(dom_flops_total / dom_n / 1e9, 1),
                      "share_of_conv_time": round(dom_ms / sum(per_launch.values()), 3),
@@ -463,6 +463,10 @@ def run_pool(args, rank, local, world):
     x, go, m = cfg["x"][lo:hi].to(dev), cfg["grad_output"][lo:hi].to(dev), cfg["map"].to(dev)
     out, idx = capi.mapped_max_pool(x, m, 9, 0)
     gin = torch.empty_like(x)
+    # the scratch that the host extension brings: forward over plane groups unless the map is local, the deterministic backward always
+    planes, npix, nout = x.shape[0] * x.shape[1], x.shape[2] * x.shape[3], out.shape[2] * out.shape[3]
+    ws_fwd, ws_bwd = capi.staging(capi.STAGE_POOL, planes, npix, 9 * nout, x), capi.staging(capi.STAGE_ARGMAX, planes, nout, 0, x)
+    local = {id(m): capi.map_locality(m, 9) == 1}
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     ef = [torch.cuda.Event(enable_timing=True) for _ in range(6)]
     tf, tb, td = [], [], []
@@ -471,7 +475,7 @@ def run_pool(args, rank, local, world):
     def step():
         flush.zero_()
         ef[0].record()
-        capi.mapped_max_pool(x, m, 9, 0, None, out, idx)
+        capi.mapped_max_pool(x, m, 9, 0, None, out, idx, ws=None if local[id(m)] else ws_fwd)
         ef[1].record()
         flush.zero_()
         ef[2].record()
@@ -481,7 +485,7 @@ def run_pool(args, rank, local, world):
             plans[id(m)] = capi.slot_plan_build(m, None, 9, 0, x.shape[2], x.shape[3])
         flush.zero_()
         ef[4].record()
-        capi.mapped_max_unpool_planned(go, idx, plans[id(m)], x.shape[2], x.shape[3], 9, 0, gin)   # deterministic (plan walk)
+        capi.mapped_max_unpool_planned(go, idx, plans[id(m)], x.shape[2], x.shape[3], 9, 0, gin, ws=ws_bwd)   # deterministic
         ef[5].record()
         torch.cuda.synchronize()
         tf.append(ef[0].elapsed_time(ef[1]))
@@ -495,12 +499,15 @@ def run_pool(args, rank, local, world):
     barrier_sync(world)
     if sampler:
         sampler.start()
+    l0 = capi.lib.sph_launch_count()
     for _ in range(args.steps):
         step()
+    launches = capi.lib.sph_launch_count() - l0
     clocks = sampler.stop() if sampler else None
     # the same kernels on a map with locality (3x3 gnomonic, stride 2: what a pooling layer of a spherical network
     # uses), same tensor sizes: shows the kernels' bandwidth when the taps are not uniformly random
     ml = wl.gnomonic_map(x.shape[2], x.shape[3], 2).to(dev)
+    local[id(ml)] = capi.map_locality(ml, 9) == 1
     tf_r, tb_r, det_ms = list(tf), list(tb), sum(td) / len(td)
     tf.clear(), tb.clear(), td.clear()
     m_random, m = m, ml
@@ -531,14 +538,13 @@ def run_pool(args, rank, local, world):
             "scaling": "strong", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": "mapped max pool: B=%d C=64 256x512 -> 128x256, K=9, nearest, "
                                    "uniform-random map" % B, "l2": "256 MB flush before every launch", "local_batch": n},
-            "gpu_launches": 2 * args.steps,
-            "roofline": {"bound": "hbm", "kernel": "max_pool_kernel (forward)", "achieved": round(fwd_bytes / (f_ms * 1e-3) / 1e9, 1),
+            "gpu_launches": int(launches),
+            "roofline": {"bound": "hbm", "kernel": "plane_group_kernel<PoolOp> (forward: transposition and pooling)", "achieved": round(fwd_bytes / (f_ms * 1e-3) / 1e9, 1),
                          "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": round(fwd_bytes / (f_ms * 1e-3) / 1e9 / peaks["hbm_gbs"], 4),
-                         # DRAM read+write of the forward launch from an ncu capture at B=8, scaled by the local batch
-                         "traffic": int(450.7e6 * n / 8), "traffic_of": "constant from an ncu capture, not measured in this run", "fwd_ms": round(f_ms, 4), "bwd_ms": round(b_ms, 4),
+                         "traffic": None, "fwd_ms": round(f_ms, 4), "bwd_ms": round(b_ms, 4),
                          "bwd_achieved": round(fwd_bytes / (b_ms * 1e-3) / 1e9, 1),
                          "bwd_note": "value and bwd_ms use the atomic argmax backward (the reference's scheme); the "
-                                     "deterministic plan-walk backward the layers use by default takes bwd_deterministic_ms",
+                                     "deterministic backward the layers use by default (plane groups) takes bwd_deterministic_ms",
                          "bwd_deterministic_ms": round(det_ms, 4),
                          "local_map": {"map": "3x3 gnomonic, stride 2", "fwd_ms": round(lf_ms, 4), "bwd_ms": round(lb_ms, 4),
                                        "fwd_gbs": round(fwd_bytes / (lf_ms * 1e-3) / 1e9, 1),
@@ -548,25 +554,30 @@ def run_pool(args, rank, local, world):
 
 
 def _time_resample(capi, x, m, plan, H, W, steps, warmup, flush):
+    """(gather ms, scatter ms, launches): the gather reads the planes in place (less than one read a pixel), the scatter goes over
+    plane groups, as in the host extension."""
     y = capi.resample_from_map(x, m, 1)
     out = torch.empty_like(x)
+    ws = capi.staging(capi.STAGE_SCATTER, x.shape[0] * x.shape[1], m.shape[0] * m.shape[1], 0, x)
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
     tg, ts = [], []
     for i in range(warmup + steps):
+        if i == warmup:
+            l0 = capi.lib.sph_launch_count()
         flush.zero_()
         ev[0].record()
         capi.resample_from_map(x, m, 1)
         ev[1].record()
         flush.zero_()
         ev[2].record()
-        capi.resample_to_map(y, plan, H, W)
+        capi.resample_to_map(y, plan, H, W, ws=ws)
         ev[3].record()
         torch.cuda.synchronize()
         if i >= warmup:
             tg.append(ev[0].elapsed_time(ev[1]))
             ts.append(ev[2].elapsed_time(ev[3]))
     del out
-    return sum(tg) / len(tg), sum(ts) / len(ts)
+    return sum(tg) / len(tg), sum(ts) / len(ts), capi.lib.sph_launch_count() - l0
 
 
 def _resample_bytes(n, C, ns, H, W, map_numel):
@@ -588,13 +599,13 @@ def run_resample(args, rank, local, world):
     H, W = cfg["out_hw"]
     plan = capi.plan_build(m, None, m.shape[0] * m.shape[1], 1, 1, H, W)
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
-    g_ms, s_ms = _time_resample(capi, x, m, plan, H, W, args.steps, args.warmup, flush)
+    g_ms, s_ms, launches = _time_resample(capi, x, m, plan, H, W, args.steps, args.warmup, flush)
     n, C, ns = hi - lo, x.shape[1], m.shape[0] * m.shape[1]
     g_bytes, s_bytes = _resample_bytes(n, C, ns, H, W, m.numel())
     # scaled variant: 256 images, seeded the same way
     gbig = torch.Generator().manual_seed(1)
     xb = torch.rand(256 // world, C, H, W, generator=gbig).to(dev)
-    gb_ms, sb_ms = _time_resample(capi, xb, m, plan, H, W, max(3, args.steps // 2), 2, flush)
+    gb_ms, sb_ms, _ = _time_resample(capi, xb, m, plan, H, W, max(3, args.steps // 2), 2, flush)
     gb_bytes, sb_bytes = _resample_bytes(xb.shape[0], C, ns, H, W, m.numel())
     g_ms, s_ms = max_over_ranks(g_ms, world, dev), max_over_ranks(s_ms, world, dev)
     gb_ms, sb_ms = max_over_ranks(gb_ms, world, dev), max_over_ranks(sb_ms, world, dev)
@@ -615,7 +626,7 @@ def run_resample(args, rank, local, world):
             "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": "tangent-image resampling: B=%d C=3 512x1024 <-> 20x64x64, bilinear" % B,
                        "l2": "256 MB flush before every launch"},
-            "gpu_launches": 2 * args.steps,
+            "gpu_launches": int(launches),
             "roofline": {"bound": "hbm", "kernel": "resample_from_map_kernel", "achieved": round(g_bytes / (g_ms * 1e-3) / 1e9, 1),
                          "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": round(g_bytes / (g_ms * 1e-3) / 1e9 / peaks["hbm_gbs"], 4),
                          # DRAM read+write of the gather launch from an ncu capture at B=8, scaled by the local batch

@@ -137,7 +137,7 @@ class EncoderStack:
                 self.out_cl[li] = capi.companion(local_batch, co, oh, ow, device)
             for op in (capi.CONV_FORWARD, capi.CONV_BACKWARD_INPUT, capi.CONV_BACKWARD_WEIGHT, capi.CONV_BACKWARD):
                 self.ws[(li, op)] = capi.conv_workspace(op, local_batch, ci, co, ih, iw, oh, ow, self.K, 0, capi.F32,
-                                                        self.interp, precision, self.w[li])
+                                                        self.interp, precision, self.w[li], preferred=True)
         self.gx = [torch.empty(local_batch, ci, ih, iw, **f32) for ci, co, (ih, iw), _, _ in self.layers]
         # weight and bias gradients live in fixed buffers (one flat allocation per layer when a reducer owns them)
         if reducer is not None:
