@@ -240,16 +240,32 @@ Locality locality_of(const torch::Tensor &map, int64_t n, int64_t K) {
   return Locality::Unknown;
 }
 
+// Id of the capture that a stream takes part in; 0 outside one.
+unsigned long long capture_of(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 // ---- channels-last companions of activations (bf16 precision) -------------------
 // The tensor-core kernels gather from a channels-last bf16 copy of their input.  A layer with the fused ReLU writes
 // that copy of its output from its own epilogue; it is remembered here under the identity of the output tensor, so
 // that the next layer (whose input that tensor is) finds it in forward and in backward and skips its conversion
-// pass.  An entry dies with the tensor's storage, on an in-place modification (version counter) or by eviction.
+// pass.  An entry dies with the tensor's storage, on an in-place modification (version counter) or by eviction.  It
+// serves calls on the stream that wrote it alone (no other one waits for it), and a CUDA graph's capture alone if it was
+// written in one, or outside any: a replay finds new contents in the same tensor.  Inference tensors, whose modifications
+// nothing counts, have none.
 struct CompanionEntry {
   c10::weak_intrusive_ptr<c10::StorageImpl> storage;
   const void *ptr;
   uint32_t version;
   std::vector<int64_t> sizes;
+  cudaStream_t stream;
+  unsigned long long capture;
   torch::Tensor companion;
 };
 std::list<CompanionEntry> &companion_cache() {  // never destroyed, like the plan cache
@@ -261,20 +277,23 @@ std::mutex g_companion_mu;
 constexpr size_t kMaxCompanions = 8;
 bool g_use_companions = true;
 
-const void *find_companion(const torch::Tensor &t) {
-  if (!g_use_companions) return nullptr;
+// (Undefined: none.  The caller holds the tensor until its kernels are launched.)
+torch::Tensor find_companion(const torch::Tensor &t) {
+  if (!g_use_companions || t.is_inference()) return torch::Tensor();
+  const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
+  const unsigned long long capture = capture_of(st);
   std::lock_guard<std::mutex> lock(g_companion_mu);
   for (auto it = g_companions.begin(); it != g_companions.end();) {
     if (it->storage.expired()) {
       it = g_companions.erase(it);
       continue;
     }
-    if (it->ptr == t.data_ptr() && it->version == version_of(t) && it->sizes == t.sizes().vec() &&
-        it->storage.lock().get() == t.storage().unsafeGetStorageImpl())
-      return it->companion.data_ptr();
+    if (it->ptr == t.data_ptr() && it->version == version_of(t) && it->stream == st && it->capture == capture &&
+        it->sizes == t.sizes().vec() && it->storage.lock().get() == t.storage().unsafeGetStorageImpl())
+      return it->companion;
     ++it;
   }
-  return nullptr;
+  return torch::Tensor();
 }
 
 // Fresh companion buffer for a (B, C, H, W) activation: only the padding, if the channel count is padded, has to be cleared; the
@@ -288,9 +307,12 @@ torch::Tensor new_companion(const torch::Tensor &like, int64_t B, int64_t C, int
 }
 
 void register_companion(const torch::Tensor &t, torch::Tensor companion) {
+  if (t.is_inference()) return;
+  const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
+  const unsigned long long capture = capture_of(st);
   std::lock_guard<std::mutex> lock(g_companion_mu);
   g_companions.push_front(CompanionEntry{c10::weak_intrusive_ptr<c10::StorageImpl>(t.storage().getWeakStorageImpl()), t.data_ptr(),
-                                         version_of(t), t.sizes().vec(), std::move(companion)});
+                                         version_of(t), t.sizes().vec(), st, capture, std::move(companion)});
   while (g_companions.size() > kMaxCompanions) g_companions.pop_back();
 }
 
@@ -679,15 +701,15 @@ torch::Tensor conv_forward_impl(torch::Tensor x, torch::Tensor map, const torch:
   if (a.prec == SPH_PRECISION_BF16 && g_use_companions) {
     // channels-last companions: gather from the input's copy if a previous layer left one; with the fused ReLU also
     // write the copy of the output for the next layer
-    const void *x_cl = find_companion(x);
-    if (x_cl == nullptr && a.Cin * a.K > 63 && x.numel() > 0) {
+    torch::Tensor cl = find_companion(x);
+    if (!cl.defined() && a.Cin * a.K > 63 && x.numel() > 0) {
       // no previous layer left a copy of this input (the reference's own composition: convolution, then a separate
       // activation): convert it once here, for this call and for the weight gradient in backward
-      torch::Tensor cl = torch::empty({(int64_t)sph_conv_companion_bytes(a.B, a.Cin, a.IH, a.IW)}, x.options().dtype(torch::kUInt8));
+      cl = torch::empty({(int64_t)sph_conv_companion_bytes(a.B, a.Cin, a.IH, a.IW)}, x.options().dtype(torch::kUInt8));
       ok(sph_conv_companion_fill(x.data_ptr(), cl.data_ptr(), a.B, a.Cin, a.IH, a.IW, stream()), "sph_conv_companion_fill");
       register_companion(x, cl);
-      x_cl = cl.data_ptr();
     }
+    const void *x_cl = cl.defined() ? cl.data_ptr() : nullptr;
     torch::Tensor out_cl;
     if (relu && a.Cout % 8 == 0) out_cl = new_companion(x, a.B, a.Cout, a.OH, a.OW);
     if (x_cl != nullptr || out_cl.defined()) {
@@ -763,9 +785,10 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
     const size_t wbc = sph_conv_workspace_bytes(SPH_CONV_BACKWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
                                                 a.interp, a.prec);
     if (wbc > 0) {
+      const torch::Tensor cl = find_companion(x);
       torch::Tensor wsc = workspace(wbc, x);
       const int rc = sph_mapped_conv_backward_cl(go.data_ptr(), act_out ? act_out->data_ptr() : nullptr, x.data_ptr(),
-                                                 find_companion(x), need_gx ? plan.data_ptr() : nullptr, map.data_ptr(), iw ? iw->data_ptr() : nullptr,
+                                                 cl.defined() ? cl.data_ptr() : nullptr, need_gx ? plan.data_ptr() : nullptr, map.data_ptr(), iw ? iw->data_ptr() : nullptr,
                                                  weight.data_ptr(), need_gx ? gx.data_ptr() : nullptr, gw.data_ptr(), gb.data_ptr(), a.B,
                                                  a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec, wsc.data_ptr(), wbc,
                                                  stream());
