@@ -41,8 +41,8 @@ def test_convolutions(op):
 
     forward, backward = run()
     want = [t.cpu() for t in forward + list(backward())]
-    forward, backward = _short_of_memory(run, 42 << 20)
-    more = 42 << 20 if op != "relu" else 110 << 20       # (the masked gradient is a tensor more)
+    forward, backward = _short_of_memory(run, 60 << 20)   # (34 MB, and 22 in the allocator's steps for small ones)
+    more = 60 << 20 if op != "relu" else 110 << 20       # (the masked gradient is a tensor more)
     got = [t.cpu() for t in forward + list(_short_of_memory(backward, more))]
     for a, b_ in zip(got, want):
         assert ((a - b_).norm() / b_.norm()).item() < 5e-6
@@ -65,7 +65,7 @@ def test_plane_groups(op):
         r, m = _case(1, 1, 256, 512, 128, 256, 9)
         x, g = r(1, 64, 256, 512), r(1, 64, 128, 256)
         idx = C.mapped_max_pool(x, m, 9, it)[1]
-        run, spare = {"max_pool": (lambda: C.mapped_max_pool(x, m, 9, it), 30 << 20),
+        run, spare = {"max_pool": (lambda: C.mapped_max_pool(x, m, 9, it), 46 << 20),
                       "avg_pool": (lambda: [C.mapped_avg_pool(x, m, 9, it)], 24 << 20),
                       "unpool": (lambda: [C.mapped_max_unpool(g, idx, m, 256, 512, 9, it)], 38 << 20)}[op]
     want = run()
