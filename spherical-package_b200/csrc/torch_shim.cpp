@@ -10,6 +10,7 @@
 #include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/functions/utils.h>
 
@@ -104,10 +105,23 @@ MapInfo map_info(const torch::Tensor &map, const torch::Tensor *iw, bool has_k, 
   return m;
 }
 
+// Id of the capture that a stream takes part in; 0 outside one.
+unsigned long long capture_of(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 // ---- scatter-plan cache ---------------------------------------------------
 // A plan depends only on the map (and weights); training loops call the same
 // layer with the same map every step, so plans are kept, keyed by the
-// identity and version of the tensors' storage.
+// identity and version of the tensors' storage.  A plan that was built inside a CUDA graph's capture exists when the
+// graph is replayed, so it serves that capture alone; one that a capture reads stays for as long as its map lives.  (Nothing
+// counts the modifications of inference tensors: who changes such a map in place clears the cache.)
 struct PlanKey {
   c10::weak_intrusive_ptr<c10::StorageImpl> map_s, iw_s;
   const void *map_p, *iw_p;
@@ -118,9 +132,11 @@ struct PlanKey {
   torch::Tensor blob;
   std::shared_ptr<at::cuda::CUDAEvent> built;  // recorded after the build kernels, on the stream that ran them
   cudaStream_t build_stream;
+  unsigned long long capture;  // the capture that the build was part of, or 0
+  bool captured;               // a graph reads this plan
 };
 
-// Version counter of a tensor; inference tensors have none (and cannot be modified in place): 0.
+// Version counter of a tensor; inference tensors have none: 0.
 uint32_t version_of(const torch::Tensor &t) { return t.is_inference() ? 0u : (uint32_t)t._version(); }
 // (The caches are never destroyed: at interpreter shutdown the CUDA runtime may already be gone when static destructors
 // run, and releasing an event or a tensor then throws.  The process exit reclaims them.)
@@ -138,6 +154,8 @@ torch::Tensor get_plan(const torch::Tensor &map, const torch::Tensor *iw, int64_
                        int64_t dstH, int64_t dstW, int64_t uv_textures = 0) {
   const int dtype = dtype_of(map), device = map.get_device();
   if (uv_textures > 0) K = -uv_textures;  // keeps UV plans apart from ordinary ones in the cache
+  const cudaStream_t cur = at::cuda::getCurrentCUDAStream().stream();
+  const unsigned long long capture = capture_of(cur);
   std::lock_guard<std::mutex> lock(g_plan_mu);
   for (auto it = g_plans.begin(); it != g_plans.end();) {
     if (it->map_s.expired() || (it->iw_p && it->iw_s.expired())) {
@@ -150,13 +168,19 @@ torch::Tensor get_plan(const torch::Tensor &map, const torch::Tensor *iw, int64_
                             it->iw_s.lock().get() == iw->storage().unsafeGetStorageImpl())
                          : it->iw_p == nullptr) &&
                      it->n_src == n_src && it->K == K && it->P == P && it->dstH == dstH && it->dstW == dstW &&
-                     it->interp == interp && it->dtype == dtype && it->device == device;
+                     it->interp == interp && it->dtype == dtype && it->device == device &&
+                     (it->capture == 0 || it->capture == capture);
     if (hit) {
       g_plans.splice(g_plans.begin(), g_plans, it);
-      // a caller on another stream than the one that built the plan waits for the build first
-      const cudaStream_t cur = at::cuda::getCurrentCUDAStream().stream();
-      if (cur != g_plans.front().build_stream) g_plans.front().built->block(at::cuda::getCurrentCUDAStream());
-      return g_plans.front().blob;
+      PlanKey &k = g_plans.front();
+      k.captured |= capture != 0;
+      // a caller on another stream than the one that built the plan waits for the build first (a capture cannot wait for what
+      // ran before it, and need not once that is complete)
+      if (cur != k.build_stream) {
+        c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+        if (capture == 0 || k.capture != 0 || !k.built->query()) k.built->block(at::cuda::getCurrentCUDAStream());
+      }
+      return k.blob;
     }
     ++it;
   }
@@ -176,10 +200,15 @@ torch::Tensor get_plan(const torch::Tensor &map, const torch::Tensor *iw, int64_
                : c10::weak_intrusive_ptr<c10::StorageImpl>(map.storage().getWeakStorageImpl()),
             map.data_ptr(), iw ? iw->data_ptr() : nullptr, map.storage_offset(), iw ? iw->storage_offset() : 0,
             version_of(map), iw ? version_of(*iw) : 0u, n_src, K, P, dstH, dstW, interp, dtype, device, blob,
-            std::make_shared<at::cuda::CUDAEvent>(), at::cuda::getCurrentCUDAStream().stream()};
+            std::make_shared<at::cuda::CUDAEvent>(), cur, capture, capture != 0};
   k.built->record(at::cuda::getCurrentCUDAStream());
   g_plans.push_front(std::move(k));
-  if (g_plans.size() > kMaxPlans) g_plans.pop_back();
+  if (g_plans.size() > kMaxPlans)
+    for (auto it = g_plans.end(); it != g_plans.begin();)
+      if (!(--it)->captured) {
+        g_plans.erase(it);
+        break;
+      }
   return blob;
 }
 
@@ -238,17 +267,6 @@ Locality locality_of(const torch::Tensor &map, int64_t n, int64_t K) {
   entries->push_front(LocalityEntry{c10::weak_intrusive_ptr<c10::StorageImpl>(map.storage().getWeakStorageImpl()), map.data_ptr(),
                                     version_of(map), n, K, slot});
   return Locality::Unknown;
-}
-
-// Id of the capture that a stream takes part in; 0 outside one.
-unsigned long long capture_of(cudaStream_t st) {
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  unsigned long long id = 0;
-  if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return status == cudaStreamCaptureStatusActive ? id : 0;
 }
 
 // ---- channels-last companions of activations (bf16 precision) -------------------
