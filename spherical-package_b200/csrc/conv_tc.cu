@@ -10,12 +10,14 @@
 //                    weight gradients; split over pixel ranges, partial sums reduced in a fixed order.
 //
 // j runs over (slot, channel) pairs of the sample map.  Col is never written
-// to HBM: eight producer warps gather it (through the sample map's taps, or
+// to HBM: sixteen producer warps gather it (through the sample map's taps, or
 // through a scatter plan for the adjoint direction) from a channels-last bf16
 // copy of the source image straight into the 128-byte-swizzled shared-memory
-// layout tcgen05.mma reads; the other operand (weights, or the gradient tile
-// image) arrives by bulk async copies from a pre-swizzled bf16 image; one
-// thread issues the MMAs into TMEM; four epilogue warps drain TMEM.  The
+// layout tcgen05.mma reads; the other operand arrives by asynchronous copies
+// (weights from a pre-swizzled bf16 image, the gradient by tensor-map loads of
+// its channels-last copy); one thread issues the MMAs into TMEM; four epilogue
+// warps drain TMEM.  The dense product of the multiply-first adjoint has no
+// producers: one thread loads both operands.  The
 // reference does the same work per image as im2col kernel + cuBLAS SGEMM + bias
 // kernel with a (Cin*K, OH*OW) column buffer in HBM
 // (src/cuda/mapped_convolution_layer.cu:16-193).
@@ -145,11 +147,6 @@ __device__ __forceinline__ void fill_taps(const Gather &g, int pix, int slot, Ta
 }
 
 __device__ __forceinline__ void fill_taps_any(const Gather &g, int pix, int slot, Tap *dst) {
-  if (g.map == nullptr) {  // identity gather (dense GEMM over the source grid): one tap, the pixel itself
-    dst[0].off = pix * g.Cp * 2;
-    dst[0].w = tap_weight(1.0f);
-    return;
-  }
   SPH_DISPATCH_INTERP(g.interp, fill_taps<INTERP>(g, pix, slot, dst));
 }
 
@@ -814,7 +811,7 @@ __global__ void __launch_bounds__(ROWS ? kRowThreads : kThreads, 1) tc_gemm_kern
         Tap *dst = sm.taps + (size_t)idx * g.nt;
         if (MODE == MODE_DIRECT) {
           if constexpr (NT == 4) {
-            if (g.P == 0 && g.map != nullptr) {
+            if (g.P == 0) {
               // entry built in registers and stored as two 16-byte vectors (field-by-field stores at this
               // 32-byte stride collide eight ways)
               Tap t[4];
@@ -1813,7 +1810,7 @@ bool launch_gemm_l(TcParams p, int grid, size_t smem, cudaStream_t st) {
       return false;
     smem += kRowStageBytes - kOutStageBytes;
   }
-  if (!ROWS) p.use_out_map = (p.out_h == nullptr && cached_out_map(&out_map, p.out, p.B, p.Nout, p.g.GH, p.g.GW)) ? 1 : 0;
+  if (!ROWS) p.use_out_map = cached_out_map(&out_map, p.out, p.B, p.Nout, p.g.GH, p.g.GW) ? 1 : 0;
   // the copy leaves through its own tensor map when the float32 output does; otherwise with plain stores
   if (p.use_out_map && p.out_cl != nullptr && !make_cl_map(&cl_map, p.out_cl, p.B, p.cl_pitch, p.g.GH, p.g.GW)) p.use_out_map = 0;
   static int granted[kMaxDevices];

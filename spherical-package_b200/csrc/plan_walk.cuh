@@ -1,4 +1,5 @@
-// Warp-cooperative walk of a scatter plan: the engine of every adjoint ("scatter") operator.
+// Warp-cooperative walk of a scatter plan: the argmax backward of max pooling where it does not go over plane groups
+// (plane_groups.cuh): float64, fewer than three planes, 127 slots or more, no scratch.
 //
 // A plan lists, for every destination pixel q, the entries (source id, weight) that contribute to it, segments laid
 // out one after the other in q order.  A warp owns 32 consecutive destination pixels, whose segments are therefore
@@ -20,19 +21,18 @@ namespace sph {
 constexpr int kWalkUnroll = 2;                      // entries per lane and window
 constexpr int kWalkWindow = 32 * kWalkUnroll;       // entries per window
 
-// Shared memory one warp needs: PL planes (+ 1 row of weights when the sum is normalised) x window entries.
-template <typename T, int PL, bool NORM>
-__host__ __device__ constexpr int walk_smem_per_warp() { return (PL + (NORM ? 1 : 0)) * kWalkWindow * (int)sizeof(T); }
+// Shared memory one warp needs: PL planes x window entries.
+template <typename T, int PL>
+__host__ __device__ constexpr int walk_smem_per_warp() { return PL * kWalkWindow * (int)sizeof(T); }
 
 // prepare(s) -> per-entry value shared by all planes (source offset, decoded slot ...); contrib(pre, w, j) ->
 // contribution of that entry to plane j of this CTA's plane group.  Pixels [q_begin, q_end) are walked by the calling
 // CTA's warps; out_plane0 points at plane 0 of the group and planes are n_dst apart; np <= PL planes are written.
-template <typename T, int PL, bool NORM, typename FP, typename FC>
+template <typename T, int PL, typename FP, typename FC>
 __device__ __forceinline__ void plan_walk(const PlanView<T> &plan, bool ok, int n_dst, int q_begin, int q_end, T *cbuf_all,
                                           FP prepare, FC contrib, T *__restrict__ out_plane0, int np) {
-  constexpr int ROWS = PL + (NORM ? 1 : 0);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  T *cbuf = cbuf_all + (size_t)warp * ROWS * kWalkWindow;
+  T *cbuf = cbuf_all + (size_t)warp * PL * kWalkWindow;
   const bool full = np == PL;
   int q0 = q_begin + warp * 32;
   // segment bounds of the block this warp handles next, fetched one block ahead
@@ -49,7 +49,7 @@ __device__ __forceinline__ void plan_walk(const PlanView<T> &plan, bool ok, int 
       n1 = __ldg(plan.offsets + min(qn + lane + 1, n_dst));
     }
     const int a = __shfl_sync(0xffffffffu, e0, 0), b = __shfl_sync(0xffffffffu, e1, 31);
-    T acc[PL], wsum = T(0);
+    T acc[PL];
 #pragma unroll
     for (int j = 0; j < PL; j++) acc[j] = T(0);
     for (int t = a; t < b; t += kWalkWindow) {
@@ -66,7 +66,6 @@ __device__ __forceinline__ void plan_walk(const PlanView<T> &plan, bool ok, int 
           const auto pre = prepare(s);
 #pragma unroll
           for (int j = 0; j < PL; j++) cbuf[j * kWalkWindow + u * 32 + lane] = (valid && (full || j < np)) ? contrib(pre, w, j) : T(0);
-          if (NORM) cbuf[PL * kWalkWindow + u * 32 + lane] = w;
         }
       }
       __syncwarp();
@@ -75,22 +74,14 @@ __device__ __forceinline__ void plan_walk(const PlanView<T> &plan, bool ok, int 
       for (int e = lo; e < hi; e++) {
 #pragma unroll
         for (int j = 0; j < PL; j++) acc[j] += cbuf[j * kWalkWindow + e];
-        if (NORM) wsum += cbuf[PL * kWalkWindow + e];
       }
       __syncwarp();
     }
     if (q < q_end) {
       T *o = out_plane0 + q;
-      if (NORM) {
-        const T inv_den = wsum + T(1e-12);
 #pragma unroll
-        for (int j = 0; j < PL; j++)
-          if (full || j < np) o[(size_t)j * n_dst] = acc[j] / inv_den;
-      } else {
-#pragma unroll
-        for (int j = 0; j < PL; j++)
-          if (full || j < np) o[(size_t)j * n_dst] = acc[j];
-      }
+      for (int j = 0; j < PL; j++)
+        if (full || j < np) o[(size_t)j * n_dst] = acc[j];
     }
   }
 }

@@ -167,7 +167,7 @@ max_unpool_plan_kernel(const T *__restrict__ g, const int64_t *__restrict__ idx,
                        T *__restrict__ gin, int n, int n_dst, int planes, int K, int PP, int chunk, FastDiv divK) {
   extern __shared__ unsigned char unpool_smem[];
   T *cbuf = (T *)unpool_smem;
-  uint8_t *ksm = unpool_smem + (size_t)(blockDim.x >> 5) * walk_smem_per_warp<T, PL, false>();  // [PL][n]
+  uint8_t *ksm = unpool_smem + (size_t)(blockDim.x >> 5) * walk_smem_per_warp<T, PL>();  // [PL][n]
   const int p0 = blockIdx.y * PL;
   const int np = min(PL, planes - p0);
   if (STAGED) {
@@ -191,7 +191,7 @@ max_unpool_plan_kernel(const T *__restrict__ g, const int64_t *__restrict__ idx,
   const T *gp = g + (size_t)p0 * n;
   const int64_t *ip = idx + (size_t)p0 * n;
   struct Slot { int o, k, s; };
-  plan_walk<T, PL, false>(plan, ok, n_dst, q_begin, q_end, cbuf,
+  plan_walk<T, PL>(plan, ok, n_dst, q_begin, q_end, cbuf,
                           [&](int s) {
                             const int o = (int)divK.div((unsigned)s);
                             return Slot{o, s - o * K, s};
@@ -442,12 +442,12 @@ static int unpool_planned(const void *g, const int64_t *idx, const void *plan, v
   constexpr int PL = 4;
   const int groups = cdiv(planes, PL);
   const size_t stage = (size_t)PL * n;
-  if (K <= 254 && stage + 32 * (size_t)walk_smem_per_warp<T, PL, false>() <= 200 * 1024) {
+  if (K <= 254 && stage + 32 * (size_t)walk_smem_per_warp<T, PL>() <= 200 * 1024) {
     // one CTA of 32 warps per SM (the staged slots fill its shared memory); CTAs = plane groups x pixel chunks
     int chunks = cdiv((int64_t)148 * 2, groups);
     if (chunks > cdiv(n_dst, 1024)) chunks = cdiv(n_dst, 1024);
     const int chunk = cdiv(cdiv(n_dst, chunks), 1024) * 1024;
-    const size_t smem = stage + 32 * (size_t)walk_smem_per_warp<T, PL, false>();
+    const size_t smem = stage + 32 * (size_t)walk_smem_per_warp<T, PL>();
     cudaFuncSetAttribute(max_unpool_plan_kernel<T, PL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     max_unpool_plan_kernel<T, PL, true><<<dim3(cdiv(n_dst, chunk), groups), 1024, smem, st>>>(
         (const T *)g, idx, plan, (T *)gin, (int)n, (int)n_dst, (int)planes, (int)K, PP, chunk, FastDiv::make((unsigned)K));
@@ -455,7 +455,7 @@ static int unpool_planned(const void *g, const int64_t *idx, const void *plan, v
     int64_t chunks = ((int64_t)148 * 16 + groups - 1) / groups;
     if (chunks > (n_dst + 255) / 256) chunks = (n_dst + 255) / 256;
     const int chunk = (int)(((n_dst + chunks - 1) / chunks + 255) / 256 * 256);
-    const size_t smem = 8 * (size_t)walk_smem_per_warp<T, PL, false>();
+    const size_t smem = 8 * (size_t)walk_smem_per_warp<T, PL>();
     max_unpool_plan_kernel<T, PL, false><<<dim3(cdiv(n_dst, chunk), groups), 256, smem, st>>>(
         (const T *)g, idx, plan, (T *)gin, (int)n, (int)n_dst, (int)planes, (int)K, PP, chunk, FastDiv::make((unsigned)K));
   }
