@@ -18,8 +18,13 @@
  *   iw      interpolation weights (OH,OW,K,P), or NULL with P = 0.
  *   interp  0 nearest, 1 bilinear (zero outside), 2 bispherical (x wraps).
  *   dtype   0 float32, 1 float64.
- *   precision  0: arithmetic in the tensor's own type (SIMT path, the one
- *           compared bit-for-bit / to 1e-5 with the reference CPU code);
+ *   precision  0: the tensor's own precision, compared bit-for-bit / to 1e-5
+ *           with the reference CPU code.  float32 convolutions run on the
+ *           tensor cores as products of operands split into three bf16 parts
+ *           (no less accurate than float32 arithmetic; infinities and NaNs
+ *           as from it) where the caller brings
+ *           sph_conv_workspace_preferred_bytes() of scratch, else on the CUDA
+ *           cores, as float64 always does;
  *           1: bf16 operands with fp32 accumulation on the tcgen05 tensor
  *           cores (float32 tensors only).
  *
@@ -103,20 +108,27 @@ int sph_resample_from_map(const void *x, const void *map, const void *iw, void *
  * Scratch for resampling and pooling (optional).  The *_ws entry points are
  * the operators of this header with caller scratch: with at least
  * sph_staging_bytes() bytes (32-byte aligned, contents irrelevant) float32
- * tensors are processed in groups of 8 or 4 planes, transposed chunk by chunk
- * into the scratch, so that one load per tap serves a whole group; without
- * (NULL, or too small) they run the kernels of the entry points that take no
- * scratch.  Results are bit-identical either way.  sph_staging_bytes()
- * returns 0 where the transposition does not pay.
+ * tensors are processed in groups of up to 32 planes (16 in scatters),
+ * transposed chunk by chunk into the scratch, so that one load per tap serves
+ * eight planes; without (NULL, or too small) they run the kernels of the entry
+ * points that take no scratch.  Results are bit-identical either way.
+ * sph_staging_bytes() returns 0 where the transposition does not pay and where
+ * one group takes 4 GiB or more.
  *   planes  B*C;  n_src  pixels of a plane that is read (GATHER, POOL: H*W;
  *   SCATTER: MH*MW, ARGMAX: OH*OW);  reads  taps GATHER and POOL read per plane (positions x
  *   slots x points x 1 or 4), else ignored.
+ * "Pays" does not know the map.  Where neighbouring positions of the map read
+ * neighbouring pixels, a caller does better without scratch for gathers that
+ * read a pixel less than eight times, for max pooling by nearest neighbours
+ * (unweighted, K <= 16; by 8 to 75 %), and for max pooling of four taps whose
+ * blocks (64 outputs x 32 planes, four per SM) fill the GPU 1 to 1.4 times (by
+ * 6 to 23 %); and, whatever the map, for nearest-neighbour pooling of half a
+ * million values or fewer.  The host extension follows these rules.
+ * sph_map_locality() looks at 256 pairs of a float32 map (n positions, K slots)
+ * and writes 1 (they do) or 2 to *flag, device-accessible memory, on the
+ * stream.
  * No counterpart in the reference.
  * ---------------------------------------------------------------------- */
-/* Gathers that read a pixel less than eight times, and max pooling by nearest neighbours (unweighted, K <= 16), are the
- * exceptions to "pays": over a map whose neighbouring positions read neighbouring pixels the kernels without scratch are faster,
- * pooling by 8 to 75 %.  sph_map_locality() looks at 256 pairs of a float32
- * map (n positions, K slots) and writes 1 (they do) or 2 to *flag, device-accessible memory, on the stream. */
 int sph_map_locality(const void *map, int64_t n, int64_t K, int *flag, void *stream);
 enum sph_stage_op { SPH_STAGE_GATHER = 0, SPH_STAGE_POOL = 1, SPH_STAGE_ARGMAX = 2, SPH_STAGE_SCATTER = 3 };
 size_t sph_staging_bytes(int op, int64_t planes, int64_t n_src, int64_t reads, int dtype);
@@ -327,7 +339,7 @@ size_t sph_conv_workspace_bytes(int op, int64_t B, int64_t Cin, int64_t Cout, in
                                 int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp,
                                 int precision);
 /* Scratch with which the float32 operators of precision 0 run on the tensor cores (operands split into three bf16 parts
- * each, float32-accurate: csrc/conv_x3.cu); with less, down to sph_conv_workspace_bytes(), they run on the CUDA cores.
+ * each: csrc/conv_x3.cu); with less, down to sph_conv_workspace_bytes(), they run on the CUDA cores.
  * For everything else the two are equal. */
 size_t sph_conv_workspace_preferred_bytes(int op, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW,
                                           int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp,

@@ -558,8 +558,10 @@ std::vector<torch::Tensor> max_pool_impl(torch::Tensor x, torch::Tensor map, con
   // and where random reads hit L1 or L2 and cost less than the second launch: up to half a million values, and some more if a
   // plane fits L1 (random map, direct and in groups: 64 planes of 65 x 131 5.9 and 8.7 us, 128 planes 8.5 and 9.7 us, 512 planes 28
   // and 17 us; 16 planes of 144 x 288 12.6 and 9.0 us).
-  // Four taps: the groups are faster or level, but for a second wave of blocks that is nearly empty (four blocks of 64 outputs x
-  // 32 planes per SM; 128 planes of 144 x 288: 30 us direct, 34 us in groups), where a local map is read directly, too.
+  // Four taps: the groups are faster, but for a second wave of blocks that is nearly empty (four blocks of 64 outputs x 32 planes
+  // per SM), where a local map is read directly, too (3 x 3 gnomonic maps of stride 2, direct and in groups, by waves: 0.55 23 and
+  // 20 us, 0.82 28 and 25, 1.09 32 and 36, 1.28 32 and 38, 1.37 37.5 and 39.8, 1.52 37.5 and 37.9, 1.64 46 and 42, 1.92 49 and 44,
+  // 2.19 54 and 55, 2.74 69 and 60).
   const int64_t planes = x.size(0) * x.size(1), values = planes * x.size(2) * x.size(3);
   const bool float_taps = m.P == 0 && x.scalar_type() == torch::kFloat && x.numel() > 0 && m.H * m.W > 0;
   const bool nearest = it == InterpolationType::NEAREST && float_taps && m.K <= 16;
@@ -1227,7 +1229,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("weighted_mapped_transposed_conv_forward", &weighted_mapped_transposed_conv_forward);
   m.def("weighted_mapped_transposed_conv_backward", &weighted_mapped_transposed_conv_backward);
 
-  m.def("set_precision", &set_precision, "'fp32' (exact SIMT path) or 'bf16' (tcgen05 tensor cores) for float32 convolutions");
+  m.def("set_precision", &set_precision, "'fp32' (float32's own precision) or 'bf16' (bf16 operands) for float32 convolutions");
   m.def("get_precision", &get_precision);
   m.def("clear_plan_cache", &clear_plan_cache);
   m.def("plan_cache_size", &plan_cache_size);
