@@ -50,3 +50,32 @@ def test_extra_pixels_of_an_uninitialised_copy(cin, cout, width):
     copy = cl.view(torch.bfloat16)[:3 * (16 * width + 1) * cout].view(3, 16 * width + 1, cout)
     assert not copy[:, -1].any()
     assert torch.equal(copy[:, :-1].transpose(1, 2).reshape(3, cout, 16, width), out.bfloat16())
+
+
+@pytest.mark.parametrize("cin,cout,h,w,P,first", [
+    (20, 40, 140, 141, 4, True),     # a copy of 64 channels, ragged tiles
+    (64, 96, 149, 128, 3, True),     # the fewest points, and tiles, that multiply first; a copy of 128 channels
+    (64, 96, 148, 128, 3, False),    # as many pixels as one wave of tiles holds
+    (64, 64, 149, 128, 4, False),    # rows as wide as the gather's
+    (20, 40, 140, 141, 2, False),    # two points
+])
+def test_weighted_input_gradient_multiplies_first(cin, cout, h, w, P, first):
+    """With the preferred scratch, over weighted maps of three points a slot or more; in either form against the oracle."""
+    from sphmap import capi
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the sizes are those of 148 SMs")
+    K = 2
+    x, wgt, b, m, iw, go = _case(41, 1, cin, cout, h, w, h, w, K, 0, P)
+    want = port.mapped_conv_backward(go, m, x, wgt, b, K, 0, iw)
+    x, wgt, m, iw, go = [t.cuda() for t in (x, wgt, m, iw, go)]
+    plan = capi.plan_build(m, iw, h * w, K, 0, h, w)
+    launches = []
+    for preferred in (False, True):
+        ws = capi.conv_workspace(capi.CONV_BACKWARD, 1, cin, cout, h, w, h, w, K, P, capi.F32, 0, capi.BF16, x, preferred=preferred)
+        before = capi.lib.sph_launch_count()
+        got = capi.conv_backward_cl(go, None, x, None, plan, m, wgt, K, 0, iw, capi.BF16, ws=ws)
+        launches.append(capi.lib.sph_launch_count() - before)
+        for name, a, ref in zip(("grad_input", "grad_weight", "grad_bias"), got, want):
+            _close(a.cpu(), ref, name)
+    assert launches[1] - launches[0] == (1 if first else 0)
+    assert capi.device_status() == 0
