@@ -120,9 +120,8 @@ int sph_resample_from_map(const void *x, const void *map, const void *iw, void *
  * "Pays" does not know the map.  Where neighbouring positions of the map read
  * neighbouring pixels, a caller does better without scratch for gathers that
  * read a pixel less than eight times, for max pooling by nearest neighbours
- * (unweighted, K <= 16; by 8 to 75 %), and for max pooling of four taps whose
- * blocks (64 outputs x 32 planes, four per SM) fill the GPU 1 to 1.4 times (by
- * 6 to 23 %); and, whatever the map, for nearest-neighbour pooling of half a
+ * (unweighted, K <= 16; by 8 to 75 %) and of four taps (unweighted; by 8 to
+ * 48 %); and, whatever the map, for nearest-neighbour pooling of half a
  * million values or fewer.  The host extension follows these rules.
  * sph_map_locality() looks at 256 pairs of a float32 map (n positions, K slots)
  * and writes 1 (they do) or 2 to *flag, device-accessible memory, on the

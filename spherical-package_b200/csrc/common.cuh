@@ -143,6 +143,19 @@ __device__ __forceinline__ T gather(const T *__restrict__ plane, const Taps<T> &
   return gather_combine<T, INTERP>(t, v);
 }
 
+// Four taps that are a square of 2 x 2 pixels inside the image (all but those at its edges and, for bispherical ones, across the
+// seam), and their value from the address of the first.  An address costs more instructions than a load: this form has two per value
+// where four independent taps have four, and no test.
+__device__ __forceinline__ bool square_taps(const Taps<float> &t, int W) {
+  return t.off[0] >= 0 && t.off[3] >= 0 && t.off[1] == t.off[0] + 1 && t.off[2] == t.off[0] + W && t.off[3] == t.off[2] + 1 &&
+         index_ok(t.off[3], t.limit);
+}
+__device__ __forceinline__ float gather_square(const float *at, int W, const Taps<float> &t) {
+  const float *below = at + W;
+  const float v[4] = {__ldg(at), __ldg(at + 1), __ldg(below), __ldg(below + 1)};
+  return gather_combine<float, SPH_BILINEAR>(t, v);
+}
+
 // Value of one map slot: plain, or the weighted sum over its P points
 // (core/resample.h:143-161: acc += w_i * interp_i, in order).
 template <typename T, int INTERP, bool WEIGHTED>
@@ -260,6 +273,24 @@ struct FastDiv {
 };
 
 inline int cdiv(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
+
+// Outputs (height x width) cut into tiles of 256, one per block, 2^log_tx wide or narrower where the outputs are: neighbours in both
+// directions read the same lines.
+struct BlockTile {
+  int width, height, log_tx;
+  FastDiv across;
+  static BlockTile make(int64_t height, int64_t width, int log_tx) {
+    while (log_tx > 2 && (1 << log_tx) >= 2 * width) log_tx--;
+    return BlockTile{(int)width, (int)height, log_tx, FastDiv::make((unsigned)cdiv(width, 1 << log_tx))};
+  }
+  unsigned blocks() const { return across.d * (unsigned)cdiv(height, 256 >> log_tx); }
+  // This thread's output, or -1.
+  __device__ __forceinline__ int output() const {
+    const int ty = (int)across.div(blockIdx.x), tx = blockIdx.x - ty * (int)across.d;
+    const int x = (tx << log_tx) + (threadIdx.x & ((1 << log_tx) - 1)), y = ty * (256 >> log_tx) + (threadIdx.x >> log_tx);
+    return x < width && y < height ? y * width + x : -1;
+  }
+};
 
 // Dispatch a runtime interpolation code to a template parameter.
 #define SPH_DISPATCH_INTERP(interp, ...)                                              \

@@ -20,9 +20,9 @@ namespace sph {
 template <typename T, int INTERP, bool WEIGHTED, bool AVG>
 __global__ void __launch_bounds__(256)
 max_pool_kernel(const T *__restrict__ x, const T *__restrict__ map, const T *__restrict__ iw, T *__restrict__ out,
-                int64_t *__restrict__ idx, int n, int planes, int H, int W, int K, int P) {
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= n) return;
+                int64_t *__restrict__ idx, BlockTile bt, int planes, int H, int W, int K, int P) {
+  const int o = bt.output(), n = bt.width * bt.height;
+  if (o < 0) return;
   const int p0 = blockIdx.y * kPlanesPerThread;
   const int np = min(kPlanesPerThread, planes - p0);
   const size_t hw = (size_t)H * W;
@@ -63,6 +63,61 @@ max_pool_kernel(const T *__restrict__ x, const T *__restrict__ map, const T *__r
         out[(size_t)(p0 + j) * n + o] = best[j];
         idx[(size_t)(p0 + j) * n + o] = bk[j] < 0 ? (int64_t)-1 : ((int64_t)o * K + bk[j]) * PP * 2;
       }
+    }
+}
+
+// Max pooling of unweighted float32 maps of four taps, the planes read where they lie: the kernel above with fewer instructions per
+// value where the taps of a warp are squares of pixels, which they are but at the image's edges, and the next slot's coordinates
+// fetched with this one's pixels.  Bound: the SM's path to L1 (two to three wavefronts per load of 32 taps two pixels apart, and what
+// it fetches from L2, 80 %) and issue (65 %).  3 x 3 gnomonic map of stride 2, 1024 planes of 256 x 512: the kernel above on blocks of
+// 256 outputs of a row 547 us, over plane groups 568; on blocks of 32 x 8 447; so 407, on blocks of 64 x 4 385.  (Five blocks per SM
+// 421, six 433; sixteen planes per thread 466, four 453; three slots at a time, so that their lines are fetched once, 434: it fetches
+// a third and holds 80 registers; pairs as eight-byte loads where a warp's are aligned: 405, odd widths 463.)
+template <int INTERP>
+__global__ void __launch_bounds__(256, 4)
+max_pool_square_kernel(const float *__restrict__ x, const float *__restrict__ map, float *__restrict__ out, int64_t *__restrict__ idx,
+                       BlockTile bt, int planes, int H, int W, int K) {
+  constexpr int PPT = kPlanesPerThread;
+  const int o = bt.output(), n = bt.width * bt.height;
+  if (o < 0) return;
+  const int p0 = blockIdx.y * PPT, np = min(PPT, planes - p0);
+  const size_t hw = (size_t)H * W;
+  const float *xp = x + (size_t)p0 * hw, *m = map + 2 * (size_t)o * K;
+  const bool pairs = ((uintptr_t)map & 7) == 0;
+  const unsigned active = __activemask();
+  float best[PPT];
+  int bk[PPT];
+#pragma unroll
+  for (int j = 0; j < PPT; j++) { best[j] = -FLT_MAX; bk[j] = -1; }
+  float2 next = pairs ? __ldg((const float2 *)m) : make_float2(__ldg(m), __ldg(m + 1));
+#pragma unroll 1
+  for (int k = 0; k < K; k++) {
+    const float2 xy = next;
+    m += 2;
+    if (k + 1 < K) next = pairs ? __ldg((const float2 *)m) : make_float2(__ldg(m), __ldg(m + 1));
+    Taps<float> t;
+    decode<float, INTERP>(xy.x, xy.y, H, W, t);
+    if (__all_sync(active, np == PPT && square_taps(t, W))) {
+      const float *at = xp + t.off[0];
+#pragma unroll
+      for (int j = 0; j < PPT; j++, at += hw) {
+        const float v = gather_square(at, W, t);
+        if (v > best[j]) { best[j] = v; bk[j] = k; }
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < PPT; j++)
+        if (j < np) {
+          const float v = gather<float, INTERP>(xp + j * hw, t);
+          if (v > best[j]) { best[j] = v; bk[j] = k; }
+        }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < PPT; j++)
+    if (j < np) {
+      __stcs(out + (size_t)(p0 + j) * n + o, best[j]);
+      __stcs((long long *)idx + (size_t)(p0 + j) * n + o, bk[j] < 0 ? -1ll : ((long long)o * K + bk[j]) * 2);
     }
 }
 
@@ -464,37 +519,41 @@ static int unpool_planned(const void *g, const int64_t *idx, const void *plan, v
 
 template <typename T>
 static int pool(const void *x, const void *map, const void *iw, void *out, int64_t *idx, int64_t planes, int64_t H,
-                int64_t W, int64_t n, int64_t K, int64_t P, int interp, cudaStream_t st, bool avg = false) {
+                int64_t W, int64_t OH, int64_t OW, int64_t K, int64_t P, int interp, cudaStream_t st, bool avg = false) {
+  const BlockTile bt = BlockTile::make(OH, OW, 6);
   if (avg) {
-    dim3 grid(cdiv(n, 256), cdiv(planes, kPlanesPerThread));
+    dim3 grid(bt.blocks(), cdiv(planes, kPlanesPerThread));
     SPH_DISPATCH_INTERP(interp, {
       if (P > 0)
         max_pool_kernel<T, INTERP, true, true><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, (const T *)iw, (T *)out,
-                                                                     nullptr, (int)n, (int)planes, (int)H, (int)W, (int)K, (int)P);
+                                                                     nullptr, bt, (int)planes, (int)H, (int)W, (int)K, (int)P);
       else
         max_pool_kernel<T, INTERP, false, true><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, nullptr, (T *)out, nullptr,
-                                                                      (int)n, (int)planes, (int)H, (int)W, (int)K, 0);
+                                                                      bt, (int)planes, (int)H, (int)W, (int)K, 0);
     });
     return launch_status();
   }
   if (interp == SPH_NEAREST && P == 0 && K <= kPoolMaxK) {
     constexpr int PPT = 4;
-    dim3 grid(cdiv(n, 256), cdiv(planes, PPT));
+    dim3 grid(cdiv(OH * OW, 256), cdiv(planes, PPT));
 #define SPH_POOL_NEAREST(KMAX) \
-    max_pool_nearest_kernel<T, PPT, KMAX><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, (T *)out, idx, (int)n, (int)planes, (int)H, (int)W, (int)K)
+    max_pool_nearest_kernel<T, PPT, KMAX><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, (T *)out, idx, (int)(OH * OW), (int)planes, (int)H, (int)W, (int)K)
     if (K <= 4) SPH_POOL_NEAREST(4);
     else if (K <= 9) SPH_POOL_NEAREST(9);
     else SPH_POOL_NEAREST(16);
 #undef SPH_POOL_NEAREST
     return launch_status();
   }
-  dim3 grid(cdiv(n, 256), cdiv(planes, kPlanesPerThread));
+  dim3 grid(bt.blocks(), cdiv(planes, kPlanesPerThread));
   SPH_DISPATCH_INTERP(interp, {
     if (P > 0)
       max_pool_kernel<T, INTERP, true, false><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, (const T *)iw, (T *)out, idx,
-                                                             (int)n, (int)planes, (int)H, (int)W, (int)K, (int)P);
+                                                             bt, (int)planes, (int)H, (int)W, (int)K, (int)P);
+    else if constexpr (sizeof(T) == 4 && INTERP != SPH_NEAREST)
+      max_pool_square_kernel<INTERP><<<grid, 256, 0, st>>>((const float *)x, (const float *)map, (float *)out, idx, bt, (int)planes, (int)H, (int)W,
+                                                        (int)K);
     else
-      max_pool_kernel<T, INTERP, false, false><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, nullptr, (T *)out, idx, (int)n,
+      max_pool_kernel<T, INTERP, false, false><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, nullptr, (T *)out, idx, bt,
                                                               (int)planes, (int)H, (int)W, (int)K, 0);
   });
   return launch_status();
@@ -550,8 +609,8 @@ extern "C" int sph_mapped_pool_ws(const void *x, const void *map, const void *iw
       SPH_DISPATCH_GROUP(c.group_planes, return pool_groups<PG>(c, x, map, iw, out, idx, IH, IW, OH, OW, K, P, interp, st, average != 0));
     }
   }
-  return dtype == SPH_F32 ? pool<float>(x, map, iw, out, idx, B * C, IH, IW, OH * OW, K, P, interp, st, average != 0)
-                          : pool<double>(x, map, iw, out, idx, B * C, IH, IW, OH * OW, K, P, interp, st, average != 0);
+  return dtype == SPH_F32 ? pool<float>(x, map, iw, out, idx, B * C, IH, IW, OH, OW, K, P, interp, st, average != 0)
+                          : pool<double>(x, map, iw, out, idx, B * C, IH, IW, OH, OW, K, P, interp, st, average != 0);
 }
 
 extern "C" int sph_map_locality(const void *map, int64_t n, int64_t K, int *flag, void *stream) {

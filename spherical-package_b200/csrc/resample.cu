@@ -10,16 +10,19 @@ namespace sph {
 // (batch, channel) planes with the same taps.  Reference kernel:
 // ext_modules/include/cuda/resample.cuh:50-81 (one thread per (c, position), one
 // launch per image); arithmetic: common/resample.h:34-52, 85-107.
+// Bound: wavefronts of the SM's path to L1, as many per load as the lines that a warp's positions lie in (89 %).  A block's positions
+// are 16 x 16: a row of 256 tangent-image samples crosses many image rows (96 planes of 1024 x 2048 into 20 x 256 x 256: rows of 256
+// 454 us, 32 x 8 391, 16 x 16 358, 8 x 32 411).
 //
 // With `quad` (UV-map gather, common/resample.h:133-159) every plane holds NT textures of H x W and position i samples
 // texture quad[i]; an index outside [0, NT) yields zero.
 template <typename T, int INTERP, bool WEIGHTED, int PPT>
 __global__ void __launch_bounds__(256)
 resample_from_map_kernel(const T *__restrict__ x, const T *__restrict__ map, const T *__restrict__ iw,
-                         T *__restrict__ y, int n, int planes, int H, int W, int P, const int64_t *__restrict__ quad,
+                         T *__restrict__ y, BlockTile bt, int planes, int H, int W, int P, const int64_t *__restrict__ quad,
                          int NT) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const int i = bt.output(), n = bt.width * bt.height;
+  if (i < 0) return;
   const int p0 = blockIdx.y * PPT;
   const int np = min(PPT, planes - p0);
   size_t hw = (size_t)H * W;
@@ -38,6 +41,14 @@ resample_from_map_kernel(const T *__restrict__ x, const T *__restrict__ map, con
     if (dead) {
 #pragma unroll
       for (int k = 0; k < 4; k++) t.off[k] = -1;
+    }
+    if constexpr (sizeof(T) == 4) {
+      if (INTERP != SPH_NEAREST && !quad && np == PPT && __all_sync(__activemask(), square_taps(t, W))) {
+        const float *at = xp + t.off[0];
+#pragma unroll
+        for (int j = 0; j < PPT; j++, at += hw) yp[(size_t)j * n] = gather_square(at, W, t);
+        return;
+      }
     }
 #pragma unroll
     for (int j = 0; j < PPT; j++)
@@ -125,23 +136,24 @@ static int planes_per_thread(int64_t n, int64_t planes) {
 
 template <typename T, int PPT>
 static void from_map_launch(const void *x, const void *map, const void *iw, void *y, int64_t planes, int64_t H, int64_t W,
-                            int64_t n, int64_t P, int interp, cudaStream_t st, const int64_t *quad, int NT) {
-  dim3 grid(cdiv(n, 256), cdiv(planes, PPT));
+                            int64_t MH, int64_t MW, int64_t P, int interp, cudaStream_t st, const int64_t *quad, int NT) {
+  const BlockTile bt = BlockTile::make(MH, MW, 4);
+  dim3 grid(bt.blocks(), cdiv(planes, PPT));
   SPH_DISPATCH_INTERP(interp, {
     if (P > 0)
       resample_from_map_kernel<T, INTERP, true, PPT><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, (const T *)iw, (T *)y,
-                                                                           (int)n, (int)planes, (int)H, (int)W, (int)P, nullptr, 1);
+                                                                           bt, (int)planes, (int)H, (int)W, (int)P, nullptr, 1);
     else
       resample_from_map_kernel<T, INTERP, false, PPT><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, nullptr, (T *)y,
-                                                                            (int)n, (int)planes, (int)H, (int)W, 0, quad, NT);
+                                                                            bt, (int)planes, (int)H, (int)W, 0, quad, NT);
   });
 }
 
 template <typename T>
 static int from_map(const void *x, const void *map, const void *iw, void *y, int64_t planes, int64_t H, int64_t W,
-                    int64_t n, int64_t P, int interp, cudaStream_t st, const int64_t *quad = nullptr, int NT = 1) {
-  if (planes_per_thread(n, planes) == 8) from_map_launch<T, 8>(x, map, iw, y, planes, H, W, n, P, interp, st, quad, NT);
-  else from_map_launch<T, 2>(x, map, iw, y, planes, H, W, n, P, interp, st, quad, NT);
+                    int64_t MH, int64_t MW, int64_t P, int interp, cudaStream_t st, const int64_t *quad = nullptr, int NT = 1) {
+  if (planes_per_thread(MH * MW, planes) == 8) from_map_launch<T, 8>(x, map, iw, y, planes, H, W, MH, MW, P, interp, st, quad, NT);
+  else from_map_launch<T, 2>(x, map, iw, y, planes, H, W, MH, MW, P, interp, st, quad, NT);
   return launch_status();
 }
 
@@ -366,8 +378,8 @@ extern "C" int sph_resample_from_map_ws(const void *x, const void *map, const vo
       SPH_DISPATCH_GROUP(c.group_planes, return from_map_groups<PG>(c, x, map, iw, y, H, W, MH, MW, P, interp, st));
     }
   }
-  return dtype == SPH_F32 ? from_map<float>(x, map, iw, y, planes, H, W, n, P, interp, st)
-                          : from_map<double>(x, map, iw, y, planes, H, W, n, P, interp, st);
+  return dtype == SPH_F32 ? from_map<float>(x, map, iw, y, planes, H, W, MH, MW, P, interp, st)
+                          : from_map<double>(x, map, iw, y, planes, H, W, MH, MW, P, interp, st);
 }
 
 namespace {
@@ -427,8 +439,8 @@ extern "C" int sph_resample_from_uv_maps(const void *tex, const int64_t *quad_id
   if (NT * TH * TW >= lim || n * 2 >= lim || planes / 2 >= 65535) return SPH_ERR_TOO_LARGE;
   if (n == 0 || planes == 0) return SPH_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  return dtype == SPH_F32 ? from_map<float>(tex, tex_uv, nullptr, out, planes, TH, TW, n, 0, interp, st, quad_idx, (int)NT)
-                          : from_map<double>(tex, tex_uv, nullptr, out, planes, TH, TW, n, 0, interp, st, quad_idx, (int)NT);
+  return dtype == SPH_F32 ? from_map<float>(tex, tex_uv, nullptr, out, planes, TH, TW, IH, IW, 0, interp, st, quad_idx, (int)NT)
+                          : from_map<double>(tex, tex_uv, nullptr, out, planes, TH, TW, IH, IW, 0, interp, st, quad_idx, (int)NT);
 }
 
 extern "C" int sph_voting_resample_to_map(const int64_t *labels, const void *plan, int plan_dtype, int64_t *out, int64_t B,

@@ -558,18 +558,16 @@ std::vector<torch::Tensor> max_pool_impl(torch::Tensor x, torch::Tensor map, con
   // and where random reads hit L1 or L2 and cost less than the second launch: up to half a million values, and some more if a
   // plane fits L1 (random map, direct and in groups: 64 planes of 65 x 131 5.9 and 8.7 us, 128 planes 8.5 and 9.7 us, 512 planes 28
   // and 17 us; 16 planes of 144 x 288 12.6 and 9.0 us).
-  // Four taps: the groups are faster, but for a second wave of blocks that is nearly empty (four blocks of 64 outputs x 32 planes
-  // per SM), where a local map is read directly, too (3 x 3 gnomonic maps of stride 2, direct and in groups, by waves: 0.55 23 and
-  // 20 us, 0.82 28 and 25, 1.09 32 and 36, 1.28 32 and 38, 1.37 37.5 and 39.8, 1.52 37.5 and 37.9, 1.64 46 and 42, 1.92 49 and 44,
-  // 2.19 54 and 55, 2.74 69 and 60).
+  // Four taps: in place over a local map (3 x 3 gnomonic maps of stride 2, direct and in groups: 1024 planes of 256 x 512 384 and
+  // 568 us, 64 planes 39 and 42, 1024 planes of 40 x 80 22 and 25, 32 planes of 320 x 640 28 and 40), in groups over a scattered one
+  // (2912 and 557, 196 and 42, 62 and 25, 166 and 38).
   const int64_t planes = x.size(0) * x.size(1), values = planes * x.size(2) * x.size(3);
   const bool float_taps = m.P == 0 && x.scalar_type() == torch::kFloat && x.numel() > 0 && m.H * m.W > 0;
   const bool nearest = it == InterpolationType::NEAREST && float_taps && m.K <= 16;
-  const int64_t pixels = x.size(2) * x.size(3), wave = 4 * at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  const int64_t blocks = (planes + 31) / 32 * ((m.H + 7) / 8) * ((m.W + 7) / 8);
+  const int64_t pixels = x.size(2) * x.size(3);
   const bool few = nearest && (values <= ((int64_t)1 << 19) || (pixels <= ((int64_t)1 << 14) && values <= ((int64_t)5 << 18)));
-  const bool thin_wave = !nearest && float_taps && planes >= 64 && blocks > wave && 5 * blocks <= 7 * wave;
-  const bool direct = few || ((nearest || thin_wave) && locality_of(map, m.H * m.W, m.K) == Locality::Local);
+  const bool four = float_taps && it != InterpolationType::NEAREST;
+  const bool direct = few || ((nearest || four) && locality_of(map, m.H * m.W, m.K) == Locality::Local);
   const Staging sg(SPH_STAGE_POOL, direct ? 0 : planes, x.size(2) * x.size(3), m.H * m.W * m.K * std::max<int64_t>(m.P, 1) * taps_of(it), x);
   ok(sph_mapped_pool_ws(x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, out.data_ptr(), idx.data_ptr<int64_t>(),
                         x.size(0), x.size(1), x.size(2), x.size(3), m.H, m.W, m.K, m.P, 0, dtype_of(x), (int)it, sg.ptr(), sg.bytes,

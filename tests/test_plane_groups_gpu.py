@@ -135,6 +135,32 @@ def test_second_wave_of_pooling_blocks(local):
     _chosen(lambda: MappedMaxPool(9, InterpolationType.BILINEAR, return_indices=True)(x, m), 3, 1 if local else 2)
 
 
+@pytest.mark.parametrize("planes", [7, 8, 17])
+@pytest.mark.parametrize("h,w,oh,ow", [(40, 83, 40, 83), (64, 128, 33, 65), (24, 10, 12, 5), (9, 200, 9, 129)])
+@pytest.mark.parametrize("interp", [1, 2])
+def test_squares_of_pixels(planes, h, w, oh, ow, interp):
+    """Maps whose taps are mostly 2 x 2 pixels inside the image, where the kernels that read in place address them together: outputs
+    around the blocks' 64 and 16 columns, taps across every edge, infinities, and coordinates that lie at a multiple of four bytes.
+    Against the plane groups, bit for bit."""
+    from sphmap import capi
+    g = torch.Generator().manual_seed(planes)
+    at = torch.stack(torch.meshgrid(torch.arange(oh) * (h / oh), torch.arange(ow) * (w / ow), indexing="ij")[::-1], -1)
+    kernel = torch.tensor([[a, b] for b in (-1.25, 0.0, 1.5) for a in (-1.0, 0.25, 1.0)])
+    storage = torch.empty(oh * ow * 18 + 1, device="cuda")
+    m = storage[1:].view(oh, ow, 9, 2)
+    m.copy_(at[:, :, None] + kernel)
+    x = torch.randn(1, planes, h, w, generator=g)
+    x[0, 0, 3, 5], x[0, 1, 6, 7], x[0, 2, 8, 1] = float("inf"), float("-inf"), float("nan")
+    x = x.cuda()
+    ws = capi.staging(capi.STAGE_POOL, planes, h * w, ANY, x)
+    for smap in (m, m.clone()):
+        (a, ia), (b, ib) = capi.mapped_max_pool(x, smap, 9, interp), capi.mapped_max_pool(x, smap, 9, interp, ws=ws)
+        assert torch.equal(a, b) and torch.equal(ia, ib)
+        one = storage[1:1 + oh * ow * 2].view(oh, ow, 2).copy_(at) if smap is m else smap[:, :, 6].contiguous()
+        a, b = capi.resample_from_map(x, one, interp), capi.resample_from_map(x, one, interp, ws=ws)
+        assert torch.equal(a.nan_to_num(nan=7.0), b.nan_to_num(nan=7.0))
+
+
 @pytest.mark.parametrize("local", [True, False])
 def test_gather_by_locality(local):
     """Between one and eight reads a pixel: in place over a local map or one not looked at yet, in groups over a scattered one."""
