@@ -122,9 +122,10 @@ max_pool_square_kernel(const float *__restrict__ x, const float *__restrict__ ma
 }
 
 // Whether neighbouring positions of a map read neighbouring pixels: 256 pairs spread over it, slot 0; *flag = 1 if three quarters
-// of the pairs are at most 8 pixels apart in both directions, else 2.
+// of the pairs are at most 8 pixels apart in both directions, else 2.  (Multiples of the golden section of 2^32: positions at equal
+// distances would all lie in one column, and be pairs across the end of a row, where that distance is a multiple of the width.)
 __global__ void __launch_bounds__(256) map_locality_kernel(const float *__restrict__ map, long long n, int K, int *flag) {
-  const long long o = (n - 1) * (long long)threadIdx.x / 256;
+  const long long o = (long long)__umul64hi((unsigned long long)(threadIdx.x * 0x9e3779b9u) << 32, (unsigned long long)n);
   const float *a = map + 2 * (size_t)(o * K), *b = a + 2 * (o + 1 < n ? K : 0);
   const bool near = fabsf(__ldg(b) - __ldg(a)) <= 8.0f && fabsf(__ldg(b + 1) - __ldg(a + 1)) <= 8.0f;
   const int c = __syncthreads_count(near);

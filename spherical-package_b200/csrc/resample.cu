@@ -71,20 +71,53 @@ resample_from_map_kernel(const T *__restrict__ x, const T *__restrict__ map, con
   }
 }
 
+// a[j] / d for all j, rounded as a division is.  Float32: with the reciprocal r of d, rounded to nearest, q = a r is less than two units
+// off, and each step q + (a - q d) r, the remainder in one fused operation, makes an approximation within a unit the nearest one (P.
+// Markstein, IBM J. Res. Dev. 34, 1990); two steps of them, and no operation over- or underflows for divisors within 2^+-60 and values
+// that are zero or within 2^-80 and 2^60.  Others are divided.  Ten instructions per value where a division has seventeen
+// (154 planes of 974 x 1948 pixels: 472 us, 327 of them without the divisions).
+template <int N> __device__ __forceinline__ void divide_all(float (&a)[N], float d) {
+  float least = 1.0f, most = 1.0f;
+#pragma unroll
+  for (int j = 0; j < N; j++) {
+    least = fminf(least, a[j] == 0.0f ? 1.0f : fabsf(a[j]));
+    most = fmaxf(most, fabsf(a[j]));
+  }
+  if (d >= 0x1p-60f && d <= 0x1p60f && least >= 0x1p-80f && most <= 0x1p60f) {
+    const float r = 1.0f / d;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      float q = __fmul_rn(a[j], r);
+      q = fmaf(fmaf(-q, d, a[j]), r, q);
+      a[j] = fmaf(fmaf(-q, d, a[j]), r, q);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; j++) a[j] = a[j] / d;
+  }
+}
+template <int N> __device__ __forceinline__ void divide_all(double (&a)[N], double d) {
+#pragma unroll
+  for (int j = 0; j < N; j++) a[j] = a[j] / d;
+}
+
 // Adjoint as a gather through the plan.  A thread owns one destination pixel of PL planes and walks the pixel's segment:
 // an entry's source and weight are read once (the next entry's while this one's values are on their way) and serve PL
-// independent loads, products and sums.  Sums run in plan order whatever the scheduling: deterministic, with no zero-fill
+// independent loads, products and sums.  A block's pixels are 32 x 8: their entries lie in fewer lines than those of 256 pixels of
+// a row (96 planes of 20 x 256 x 256 tangent samples onto 1024 x 2048 pixels, in rows 740 us, 32 x 8 586, 16 x 16 609, 64 x 4 601, 8 x 32 713;
+// with 12 planes per thread 536, 16 542, 24 544, four 870;
+// normalised 683, 12 planes 622, 566 with five blocks per SM and divide_all).  Sums run in plan order whatever the scheduling: deterministic, with no zero-fill
 // pass and no atomics (the reference's scatter kernels use atomicAdd: ext_modules/include/cuda/resample.cuh:14-47).
 //   DIV   x[s / div] / div instead of x[s]: mapped average unpooling, whose plan runs over the flattened map slots
 //         s = o * K + k and whose slots all carry grad[o] / K (common/mapped_avg_pool.h:41-69, 109-143)
 //   NORM  the sum is divided by (sum of the segment's weights + 1e-12), i.e. scatter(x) / (scatter(1) + 1e-12), the
 //         weight-sum normalisation the reference composes in Python (layers/functional/sphere_ops.py:74-80)
 template <typename T, int PL, bool NORM, bool DIV>
-__global__ void __launch_bounds__(256)
-resample_to_map_kernel(const T *__restrict__ x, const void *__restrict__ plan_blob, T *__restrict__ out, int n_dst, int n_src,
+__global__ void __launch_bounds__(256, PL == 12 ? 5 : 1)
+resample_to_map_kernel(const T *__restrict__ x, const void *__restrict__ plan_blob, T *__restrict__ out, BlockTile bt, int n_src,
                        int planes, int div, FastDiv fd) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n_dst) return;
+  const int q = bt.output(), n_dst = bt.width * bt.height;
+  if (q < 0) return;
   bool ok;
   const PlanView<T> pv = plan_view<T>(plan_blob, n_dst, ok, DIV ? n_src * div : n_src);
   const int e0 = ok ? __ldg(pv.offsets + q) : 0, e1 = ok ? __ldg(pv.offsets + q + 1) : 0;
@@ -117,10 +150,8 @@ resample_to_map_kernel(const T *__restrict__ x, const void *__restrict__ plan_bl
     for (int j = 0; j < PL; j++) acc[j] = RN<T>::add(acc[j], RN<T>::mul(we, DIV ? v[j] / (T)div : v[j]));
     if (NORM) wsum += we;
   }
-  if (NORM && e1 > e0) {  // (an empty sum is zero already: dividing a zero takes the slow way through the divide)
-    const T den = wsum + T(1e-12);
-#pragma unroll
-    for (int j = 0; j < PL; j++) acc[j] = acc[j] / den;
+  if (NORM && e1 > e0) {  // (an empty sum is zero already)
+    divide_all(acc, wsum + T(1e-12));
   }
   T *op = out + (size_t)p0 * n_dst + q;
 #pragma unroll
@@ -157,20 +188,30 @@ static int from_map(const void *x, const void *map, const void *iw, void *y, int
   return launch_status();
 }
 
-template <typename T>
-static int to_map(const void *x, const void *plan, void *out, int64_t planes, int64_t n_src, int64_t n_dst, cudaStream_t st,
-                  int src_div = 1, bool normalize = false) {
-  constexpr int PL = 8;
-  const dim3 grid(cdiv(n_dst, 256), cdiv(planes, PL));
+template <typename T, int PL>
+static int to_map_launch(const void *x, const void *plan, void *out, int64_t planes, int64_t n_src, int64_t OH, int64_t OW, cudaStream_t st,
+                         int src_div, bool normalize) {
+  const BlockTile bt = BlockTile::make(OH, OW, 5);
+  const dim3 grid(bt.blocks(), cdiv(planes, PL));
   const FastDiv fd = FastDiv::make((unsigned)src_div);
-#define SPH_SCATTER(NORM, DIV)                                                                                                       \
-  resample_to_map_kernel<T, PL, NORM, DIV><<<grid, 256, 0, st>>>((const T *)x, plan, (T *)out, (int)n_dst, (int)n_src, (int)planes, \
+#define SPH_SCATTER(NORM, DIV)                                                                                               \
+  resample_to_map_kernel<T, PL, NORM, DIV><<<grid, 256, 0, st>>>((const T *)x, plan, (T *)out, bt, (int)n_src, (int)planes, \
                                                                  src_div, fd)
   if (src_div > 1) SPH_SCATTER(false, true);  // (never normalised)
   else if (normalize) SPH_SCATTER(true, false);
   else SPH_SCATTER(false, false);
 #undef SPH_SCATTER
   return launch_status();
+}
+
+// Planes per thread: 12 share an entry best (comment of the kernel), 8 where there are no more or where groups of 12 would have to be
+// filled up further.
+template <typename T>
+static int to_map(const void *x, const void *plan, void *out, int64_t planes, int64_t n_src, int64_t OH, int64_t OW, cudaStream_t st,
+                  int src_div = 1, bool normalize = false) {
+  if (sizeof(T) == 4 && planes > 8 && (planes + 11) / 12 * 12 <= (planes + 7) / 8 * 8)
+    return to_map_launch<T, 12>(x, plan, out, planes, n_src, OH, OW, st, src_div, normalize);
+  return to_map_launch<T, 8>(x, plan, out, planes, n_src, OH, OW, st, src_div, normalize);
 }
 
 // ---- over plane groups (plane_groups.cuh) ----------------------------------------------------------------------
@@ -225,12 +266,9 @@ struct ScatterOp {
         }
         if (!more) break;
       }
-      if (NORM) {  // (an empty sum is zero already: dividing a zero takes the slow way through the divide)
-        const float den = wsum + 1e-12f;
+      if (NORM) {
 #pragma unroll
-        for (int i = 0; i < NV; i++)
-#pragma unroll
-          for (int j = 0; j < VP; j++) acc[i].f[j] = acc[i].f[j] / den;
+        for (int i = 0; i < NV; i++) divide_all(acc[i].f, wsum + 1e-12f);
       }
     }
 #pragma unroll
@@ -398,8 +436,8 @@ int resample_to_map(const void *x, const void *plan, void *out, int64_t B, int64
       SPH_DISPATCH_GROUP(c.group_planes, return to_map_groups<PG>(c, x, plan, out, MH * MW, OH * OW, normalize, st));
     }
   }
-  return dtype == SPH_F32 ? to_map<float>(x, plan, out, planes, MH * MW, OH * OW, st, (int)K, normalize)
-                          : to_map<double>(x, plan, out, planes, MH * MW, OH * OW, st, (int)K, normalize);
+  return dtype == SPH_F32 ? to_map<float>(x, plan, out, planes, MH * MW, OH, OW, st, (int)K, normalize)
+                          : to_map<double>(x, plan, out, planes, MH * MW, OH, OW, st, (int)K, normalize);
 }
 }  // namespace
 

@@ -172,6 +172,54 @@ def test_gather_by_locality(local):
     assert torch.equal(y, capi.resample_from_map(x, m, 1))
 
 
+@pytest.mark.parametrize("planes", [8, 9, 12, 13, 16, 20, 25])
+@pytest.mark.parametrize("h,w", [(8, 33), (17, 64), (30, 5)])
+def test_scatter_in_place(planes, h, w):
+    """Threads of 8 and of 12 planes, whole and with a remainder, at the edges of blocks of 32 x 8 pixels; against the plane groups."""
+    from sphmap import capi
+    _, m, _, go = _case(planes, h, w, 2 * h, w, 1, 0, seed=5)
+    m = m[:, :, 0].contiguous()
+    plan = capi.plan_build(m, None, 2 * h * w, 1, 1, h, w)
+    ws = capi.staging(capi.STAGE_SCATTER, planes, 2 * h * w, 0, go)
+    _grouped(lambda s: capi.resample_to_map(go, plan, h, w, ws=s), ws)
+    _grouped(lambda s: capi.resample_to_map_normalized(go, plan, h, w, ws=s), ws)
+
+
+def test_normalised_scatter_divides():
+    """sum / (weights + 1e-12) with the rounding of a division, also for values that have none of the usual magnitudes."""
+    from sphmap import capi
+    h, w = 16, 40
+    _, m, iw, go = _case(9, h, w, 2 * h, w, 1, 1, seed=6)
+    m, iw = m[:, :, 0].contiguous(), iw[:, :, 0].contiguous()
+    scale = torch.tensor([1.0, 1e-38, 1e38, 1e-25, 0.0, 1e20, 3e-45, 1e3, float("inf")]).cuda()
+    go *= scale.view(1, 9, 1, 1)
+    for weights in (iw, iw * 1e-20, -iw, iw * 1e25):
+        plan = capi.plan_build(m, weights, 2 * h * w, 1, 1, h, w)
+        total = capi.resample_to_map(go, plan, h, w)
+        den = capi.resample_to_map(torch.ones_like(go[:, :1]), plan, h, w) + 1e-12
+        want = torch.where(total == 0, total, total / den)
+        for ws in (None, capi.staging(capi.STAGE_SCATTER, 9, 2 * h * w, 0, go)):
+            got = capi.resample_to_map_normalized(go, plan, h, w, ws=ws)
+            assert torch.equal(got.nan_to_num(nan=7.0), want.nan_to_num(nan=7.0))
+
+
+@pytest.mark.parametrize("local", [True, False])
+def test_scatter_by_locality(local):
+    """In place over a local map, in groups over a scattered one, one not looked at yet and one of many positions per pixel."""
+    import _spherical_distortion_ext._C as C
+    m = (_map(True, 40, 80, 0, 0, 9)[:, :, 4] if local else _map(False, 40, 80, 20, 40, 1)[:, :, 0]).contiguous()
+    x = torch.randn(2, 8, 20, 40, generator=torch.Generator().manual_seed(4)).cuda()
+    for run in (C.resample_to_map, lambda x, m, h, w, it: C.resample_to_map_normalized(x, m, None, h, w, it)):
+        C.clear_plan_cache()
+        smap = m.clone()
+        run(x, smap, 40, 80, C.InterpolationType.BILINEAR)    # (the plan, and a look at the map)
+        torch.cuda.synchronize()
+        got, n = _launches(lambda: run(x, smap, 40, 80, C.InterpolationType.BILINEAR))
+        assert n == (1 if local else 2)
+        few, n = _launches(lambda: run(x, smap, 19, 20, C.InterpolationType.BILINEAR))
+        assert n > 2
+
+
 @pytest.mark.parametrize("planes", [3, 8, 16])
 def test_scatter_with_a_plan_of_another_size_yields_zeros(planes):
     """A plan that was built for another destination, or is none, is not followed: zeros, as from the direct kernel."""
