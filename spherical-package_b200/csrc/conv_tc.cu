@@ -349,6 +349,138 @@ __device__ inline Smem carve(uint8_t *raw, const TcParams &p, bool direct) {
   return s;
 }
 
+// ---- a tile's tap table -------------------------------------------------------------------------------------------------
+// Nobody computes while the producers fill it, so what it costs is the latency of its reads: a thread reads for kFill entries at a
+// time (all of a 3 x 3 kernel's) before it decodes any.
+// (One entry after the other and so, eight images of the encoder: forward of 64 -> 128, 128 -> 256 and 256 -> 256 channels 140 and 135,
+// 240 and 236, 396 and 392 us, plan mode of the last two 419 and 413, 489 and 475; four random points, 64 -> 128 channels, 16 x 256 x 512:
+// 1345 and 1286.)
+constexpr int kFill = 3;
+
+// Entries are built in registers and stored as two 16-byte vectors (field-by-field stores at this 32-byte stride collide eight ways).
+__device__ __forceinline__ void store_four(Tap *dst, const Tap (&t)[4]) {
+  ((uint4 *)dst)[0] = make_uint4((uint32_t)t[0].off, t[0].w, (uint32_t)t[1].off, t[1].w);
+  ((uint4 *)dst)[1] = make_uint4((uint32_t)t[2].off, t[2].w, (uint32_t)t[3].off, t[3].w);
+}
+
+// Four taps of one unweighted point.
+__device__ __forceinline__ void fill_four_taps(const Gather &g, Tap *taps, int ty, int tx, int pt) {
+  const int total = g.K * kTileM, zero_off = g.SH * g.SW * g.Cp * 2;
+  for (int i0 = pt; i0 < total; i0 += kFill * kProducerThreads) {
+    float x[kFill], y[kFill];
+    bool in[kFill];
+#pragma unroll
+    for (int u = 0; u < kFill; u++) {
+      const int idx = i0 + u * kProducerThreads, pix = tile_pixel(idx % kTileM, ty, tx, kTH, g.GH, g.GW);
+      in[u] = idx < total && pix >= 0;
+      const float *m = g.map + 2 * ((size_t)max(pix, 0) * g.K + idx / kTileM);
+      x[u] = in[u] ? __ldg(m) : 0.0f;
+      y[u] = in[u] ? __ldg(m + 1) : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kFill; u++) {
+      const int idx = i0 + u * kProducerThreads;
+      if (idx >= total) break;
+      Tap t[4];
+      taps_from_xy<4>(g, x[u], y[u], t);
+      if (!in[u]) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) { t[i].off = zero_off; t[i].w = 0u; }
+      }
+      store_four(taps + (size_t)idx * 4, t);
+    }
+  }
+}
+
+// Four weighted nearest points.
+__device__ __forceinline__ void fill_four_points(const Gather &g, Tap *taps, int ty, int tx, int pt) {
+  const int total = g.K * kTileM, zero_off = g.SH * g.SW * g.Cp * 2;
+  for (int i0 = pt; i0 < total; i0 += kFill * kProducerThreads) {
+    float x[kFill][4], y[kFill][4], w[kFill][4];
+    bool in[kFill];
+#pragma unroll
+    for (int u = 0; u < kFill; u++) {
+      const int idx = i0 + u * kProducerThreads, pix = tile_pixel(idx % kTileM, ty, tx, kTH, g.GH, g.GW);
+      in[u] = idx < total && pix >= 0;
+      const size_t e = ((size_t)max(pix, 0) * g.K + idx / kTileM) * 4;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        x[u][i] = in[u] ? __ldg(g.map + 2 * (e + i)) : 0.0f;
+        y[u][i] = in[u] ? __ldg(g.map + 2 * (e + i) + 1) : 0.0f;
+        w[u][i] = in[u] ? __ldg(g.iw + e + i) : 0.0f;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kFill; u++) {
+      const int idx = i0 + u * kProducerThreads;
+      if (idx >= total) break;
+      Tap t[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        Taps<float> q;
+        decode<float, SPH_NEAREST>(x[u][i], y[u][i], g.SH, g.SW, q);
+        const bool ok = in[u] && q.off[0] >= 0;
+        t[i].off = ok ? q.off[0] * (g.Cp * 2) : zero_off;
+        t[i].w = tap_weight(ok ? w[u][i] : 0.0f);
+      }
+      store_four(taps + (size_t)idx * 4, t);
+    }
+  }
+}
+
+// The first four entries of every key of a plan; the range of the others, and four of these if they have a table.
+template <bool LEAN>
+__device__ __forceinline__ void fill_plan_taps(const TcParams &p, const Smem &sm, const PlanView<float> &pv, bool plan_ok, int npix, int pitch,
+                                               int zero_off, int ty, int tx, int pt) {
+  const Gather &g = p.g;
+  const int total = g.K * kTileM;
+  for (int i0 = pt; i0 < total; i0 += kFill * kProducerThreads) {
+    int e0[kFill], e1[kFill];
+#pragma unroll
+    for (int u = 0; u < kFill; u++) {
+      const int idx = i0 + u * kProducerThreads, pix = tile_pixel(idx % kTileM, ty, tx, kTH, g.GH, g.GW);
+      const bool in = plan_ok && idx < total && pix >= 0;
+      const int *off = pv.offsets + (in ? pix * g.K + idx / kTileM : 0);
+      e0[u] = in ? __ldg(off) : 0;
+      e1[u] = in ? __ldg(off + 1) : 0;
+    }
+    int sp[kFill][kPlanTaps];
+    float w[kFill][kPlanTaps];
+#pragma unroll
+    for (int u = 0; u < kFill; u++)
+#pragma unroll
+      for (int i = 0; i < kPlanTaps; i++) {
+        const bool in = e0[u] + i < e1[u];
+        sp[u][i] = in ? __ldg(pv.src + e0[u] + i) : -1;
+        w[u][i] = in ? __ldg(pv.w + e0[u] + i) : 0.0f;
+      }
+#pragma unroll
+    for (int u = 0; u < kFill; u++) {
+      const int idx = i0 + u * kProducerThreads;
+      if (idx >= total) break;
+      Tap t[kPlanTaps];
+#pragma unroll
+      for (int i = 0; i < kPlanTaps; i++) {
+        t[i].off = sp[u][i] >= 0 && index_ok(sp[u][i], pv.n_src) ? sp[u][i] * pitch : zero_off;
+        t[i].w = tap_weight(w[u][i]);
+      }
+      static_assert(kPlanTaps == 4, "two 16-byte stores per entry");
+      store_four(sm.taps + (size_t)idx * g.nt, t);
+      sm.rest[idx] = make_int2(e0[u] + kPlanTaps, max(e1[u] - e0[u] - kPlanTaps, 0));
+      if (LEAN && p.over && e1[u] - e0[u] > kPlanTaps) {
+        Tap *o = sm.over + (size_t)idx * 4;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const bool in = e0[u] + kPlanTaps + i < e1[u];
+          const int s = in ? __ldg(pv.src + e0[u] + kPlanTaps + i) : 0;
+          o[i].off = (in && index_ok(s, pv.n_src)) ? s * pitch : zero_off;
+          o[i].w = in && index_ok(s, pv.n_src) ? tap_weight(__ldg(pv.w + e0[u] + kPlanTaps + i)) : 0u;
+        }
+      }
+    }
+  }
+}
+
 constexpr int kRowStep = kProducerThreads / 8;  // pixel rows covered by one pass of all producer threads
 
 // One producer thread's share of a 128-pixel x 64-column tile: 16-byte vector v = pt & 7 of pixels
@@ -805,58 +937,18 @@ __global__ void __launch_bounds__(ROWS ? kRowThreads : kThreads, 1) tc_gemm_kern
       if (pt == 0) { TC_TOC(t_b0, 2); }
       if (!alive) { producer_bar(); continue; }
       TC_TIC(t_fill);
-      for (int idx = pt; idx < g.K * kTileM; idx += kProducerThreads) {
-        const int slot = idx / kTileM, pl = idx % kTileM;
-        const int pix = tile_pixel(pl, ty, tx, kTH, g.GH, g.GW);
-        Tap *dst = sm.taps + (size_t)idx * g.nt;
-        if (MODE == MODE_DIRECT) {
-          if constexpr (NT == 4) {
-            if (g.P == 0) {
-              // entry built in registers and stored as two 16-byte vectors (field-by-field stores at this
-              // 32-byte stride collide eight ways)
-              Tap t[4];
-              if (pix >= 0) {
-                const float *m = g.map + 2 * ((size_t)pix * g.K + slot);
-                taps_from_xy<4>(g, __ldg(m), __ldg(m + 1), t);
-              } else {
-#pragma unroll
-                for (int i = 0; i < 4; i++) { t[i].off = zero_off; t[i].w = 0u; }
-              }
-              ((uint4 *)dst)[0] = make_uint4((uint32_t)t[0].off, t[0].w, (uint32_t)t[1].off, t[1].w);
-              ((uint4 *)dst)[1] = make_uint4((uint32_t)t[2].off, t[2].w, (uint32_t)t[3].off, t[3].w);
-              continue;
-            }
-          }
-          if (pix >= 0) fill_taps_any(g, pix, slot, dst);
+      if constexpr (MODE == MODE_PLAN) {
+        fill_plan_taps<LEAN>(p, sm, pv, plan_ok, npix, pitch, zero_off, ty, tx, pt);
+      } else if (NT == 4 && g.P == 0) {
+        fill_four_taps(g, sm.taps, ty, tx, pt);
+      } else if (NT == 4 && g.P == 4) {
+        fill_four_points(g, sm.taps, ty, tx, pt);
+      } else {
+        for (int idx = pt; idx < g.K * kTileM; idx += kProducerThreads) {
+          const int pix = tile_pixel(idx % kTileM, ty, tx, kTH, g.GH, g.GW);
+          Tap *dst = sm.taps + (size_t)idx * g.nt;
+          if (pix >= 0) fill_taps_any(g, pix, idx / kTileM, dst);
           else fill_taps_zero(g, dst);
-        } else {
-          int e0 = 0, e1 = 0;
-          if (plan_ok && pix >= 0) {
-            e0 = __ldg(pv.offsets + pix * g.K + slot);
-            e1 = __ldg(pv.offsets + pix * g.K + slot + 1);
-          }
-          Tap t[kPlanTaps];
-#pragma unroll
-          for (int i = 0; i < kPlanTaps; i++) {
-            const bool in = e0 + i < e1;
-            const int sp = in ? __ldg(pv.src + e0 + i) : 0;
-            t[i].off = (in && index_ok(sp, pv.n_src)) ? sp * pitch : zero_off;
-            t[i].w = tap_weight(in ? __ldg(pv.w + e0 + i) : 0.0f);
-          }
-          static_assert(kPlanTaps == 4, "two 16-byte stores per entry");
-          ((uint4 *)dst)[0] = make_uint4((uint32_t)t[0].off, t[0].w, (uint32_t)t[1].off, t[1].w);
-          ((uint4 *)dst)[1] = make_uint4((uint32_t)t[2].off, t[2].w, (uint32_t)t[3].off, t[3].w);
-          sm.rest[idx] = make_int2(e0 + kPlanTaps, max(e1 - e0 - kPlanTaps, 0));
-          if (LEAN && p.over && e1 - e0 > kPlanTaps) {
-            Tap *o = sm.over + (size_t)idx * 4;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-              const bool in = e0 + kPlanTaps + i < e1;
-              const int sp = in ? __ldg(pv.src + e0 + kPlanTaps + i) : 0;
-              o[i].off = (in && index_ok(sp, pv.n_src)) ? sp * pitch : zero_off;
-              o[i].w = in && index_ok(sp, pv.n_src) ? tap_weight(__ldg(pv.w + e0 + kPlanTaps + i)) : 0u;
-            }
-          }
         }
       }
       if (tile == (int)blockIdx.x) wait_for_launcher();
