@@ -103,10 +103,63 @@ __device__ __forceinline__ int tile_pixel3(int l, int ty, int tx, int GH, int GW
   return (y < GH && x < GW) ? y * GW + x : -1;
 }
 
+// Two entries at a time: nobody computes meanwhile, and an entry's reads are two round trips to L2 (input gradient of 64 -> 128 channels,
+// 8 x 128 x 256: one at a time 555 us, two 531, three, which spill, 561; the map modes, one round trip per entry, lose by it: 330, 349
+// and 352).
+template <int SRC>
+__device__ __forceinline__ void fill_plan3(const Src3 &g, const TapTable<SRC> &t, const PlanView<float> &pv, bool plan_ok, int s0, int ns,
+                                           int ty, int tx, int pt) {
+  constexpr int U = 2, STEP = 32 * kProd;
+  const uint32_t pitch = (uint32_t)g.Cp * 4u, zero = (uint32_t)(g.SH * g.SW) * pitch;
+  const auto key = [&](int idx, bool &in) {  // (pixel, slot) of an entry as an index, 0 where there is none
+    const int slot = s0 + idx / kPix, pix = tile_pixel3(idx % kPix, ty, tx, g.GH, g.GW);
+    in = idx < ns * kPix && pix >= 0 && slot < g.K;
+    return in ? (size_t)pix * g.K + slot : (size_t)0;
+  };
+  const int total = ns * kPix;
+#pragma unroll 1
+  for (int i0 = pt; i0 < total; i0 += U * STEP) {
+    int e0[U], e1[U], sp[U][4];
+    float w[U][4];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      bool in;
+      const int *off = pv.offsets + key(i0 + u * STEP, in);
+      in = in && plan_ok;
+      e0[u] = in ? __ldg(off) : 0;
+      e1[u] = in ? __ldg(off + 1) : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const bool in = e0[u] + i < e1[u];
+        sp[u][i] = in ? __ldg(pv.src + e0[u] + i) : -1;
+        w[u][i] = in ? __ldg(pv.w + e0[u] + i) : 0.0f;
+      }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int idx = i0 + u * STEP;
+      if (idx >= ns * kPix) break;
+      uint32_t o[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const bool ok = sp[u][i] >= 0 && index_ok(sp[u][i], pv.n_src);
+        o[i] = ok ? (uint32_t)sp[u][i] * pitch : zero;
+        w[u][i] = ok ? w[u][i] : 0.0f;
+      }
+      asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(t.rest + idx * 8), "r"(min(e0[u] + 4, e1[u])), "r"(e1[u]) : "memory");
+      sts128(t.off + idx * 16, make_uint4(o[0], o[1], o[2], o[3]));
+      sts128(t.w + idx * 16, make_uint4(__float_as_uint(w[u][0]), __float_as_uint(w[u][1]), __float_as_uint(w[u][2]), __float_as_uint(w[u][3])));
+    }
+  }
+}
+
 template <int SRC>
 __device__ __forceinline__ void fill_taps3(const Src3 &g, const TapTable<SRC> &t, const PlanView<float> &pv, bool plan_ok, int s0, int ns,
                                            int ty, int tx, int pt) {
   if (SRC == SRC_SELF) return;
+  if (SRC == SRC_PLAN) return fill_plan3<SRC>(g, t, pv, plan_ok, s0, ns, ty, tx, pt);
   const uint32_t pitch = (uint32_t)g.Cp * 4u, zero = (uint32_t)(g.SH * g.SW) * pitch;
   for (int idx = pt; idx < ns * kPix; idx += 32 * kProd) {
     const int slot = s0 + idx / kPix, pix = tile_pixel3(idx % kPix, ty, tx, g.GH, g.GW);
@@ -146,22 +199,6 @@ __device__ __forceinline__ void fill_taps3(const Src3 &g, const TapTable<SRC> &t
             }
           }
         }
-      } else {
-        int e0 = 0, e1 = 0;
-        if (plan_ok && in) {
-          e0 = __ldg(pv.offsets + (size_t)pix * g.K + slot);
-          e1 = __ldg(pv.offsets + (size_t)pix * g.K + slot + 1);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-          if (e0 + i < e1) {
-            const int s = __ldg(pv.src + e0 + i);
-            if (index_ok(s, pv.n_src)) {
-              o[i] = (uint32_t)s * pitch;
-              w[i] = __ldg(pv.w + e0 + i);
-            }
-          }
-        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(t.rest + idx * 8), "r"(min(e0 + 4, e1)), "r"(e1) : "memory");
       }
       sts128(t.off + idx * 16, make_uint4(o[0], o[1], o[2], o[3]));
       sts128(t.w + idx * 16, make_uint4(__float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), __float_as_uint(w[3])));
