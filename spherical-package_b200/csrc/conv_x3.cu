@@ -18,7 +18,7 @@
 //
 // The two kernels mirror conv_tc.cu (tiles of 128 pixels, producer warps that gather, weights or gradient tile images by
 // bulk copies, one MMA thread, epilogue warps), but gather float32 values from a channels-last float32 copy of the source
-// and interpolate in float32 with the roundings of the SIMT kernels before the values are split:
+// and interpolate in float32, each tap after the first in one fused operation, before the values are split:
 //   x3_gemm_kernel   Out[b, n, pix] = sum_j Col[b, pix, j] * Wt[n, j]  (+ bias[n])     through a map, a plan, or the identity
 //   x3_dw_kernel     dW[n, j] = sum_{b, pix} G[b, n, pix] * Col[b, pix, j]
 //
@@ -210,6 +210,35 @@ __device__ __forceinline__ void fill_taps3(const Src3 &g, const TapTable<SRC> &t
 struct V8 {
   float f[8];
 };
+// Two values per instruction: four producer warps per scheduler wait for each other's and their own instructions as long as for their
+// reads (a chunk was 240 instructions per warp, issue 48 % busy).  64 -> 128 channels, 8 x 128 x 256, one value per instruction and so:
+// forward 330 and 310 us, input gradient 547 and 520, weight gradient 316 and 295.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 __device__ __forceinline__ V8 load8(const char *p) {
   V8 v;
   asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -250,18 +279,19 @@ __device__ __forceinline__ V8 item_value(const Item<SRC> &it, const TapTable<SRC
   V8 v;
   if constexpr (Item<SRC>::NT == 1) {
     v = it.q[0];
-  } else if constexpr (SRC == SRC_MAP4) {
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-      v.f[j] = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(it.w[0], it.q[0].f[j]), __fmul_rn(it.w[1], it.q[1].f[j])),
-                                   __fmul_rn(it.w[2], it.q[2].f[j])), __fmul_rn(it.w[3], it.q[3].f[j]));
   } else {
+    uint64_t w[4];
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-      v.f[j] = it.w[0] * it.q[0].f[j];
+    for (int i = 0; i < 4; i++) w[i] = pack2(it.w[i], it.w[i]);
 #pragma unroll
-      for (int i = 1; i < 4; i++) v.f[j] = fmaf(it.w[i], it.q[i].f[j], v.f[j]);
+    for (int j = 0; j < 8; j += 2) {
+      uint64_t a = mul2(w[0], pack2(it.q[0].f[j], it.q[0].f[j + 1]));
+#pragma unroll
+      for (int i = 1; i < 4; i++) a = fma2(w[i], pack2(it.q[i].f[j], it.q[i].f[j + 1]), a);
+      unpack2(a, v.f[j], v.f[j + 1]);
     }
+  }
+  if constexpr (SRC == SRC_PLAN) {
     const uint2 r = lds64(t.rest + entry * 8);
     if (r.x < r.y) {
       // Segments longer than the table: the next entry's index and weight are on their way with this one's row.  (Each entry's
@@ -278,8 +308,10 @@ __device__ __forceinline__ V8 item_value(const Item<SRC> &it, const TapTable<SRC
           s = __ldg(pv.src + e);
           w = __ldg(pv.w + e);
         }
+        const uint64_t w2 = pack2(we, we);
 #pragma unroll
-        for (int j = 0; j < 8; j++) v.f[j] = fmaf(we, x.f[j], v.f[j]);
+        for (int j = 0; j < 8; j += 2)
+          unpack2(fma2(w2, pack2(x.f[j], x.f[j + 1]), pack2(v.f[j], v.f[j + 1])), v.f[j], v.f[j + 1]);
         if (!more) break;
       }
     }
@@ -287,14 +319,17 @@ __device__ __forceinline__ V8 item_value(const Item<SRC> &it, const TapTable<SRC
   return v;
 }
 
+__device__ __forceinline__ float upper(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
 // x = h + m + l by truncation; the parts of eight values as three 16-byte vectors, stored `part` bytes apart.
 __device__ __forceinline__ void store_parts(uint32_t dst, uint32_t part, const V8 &v) {
   uint32_t h[4], m[4], l[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const float a = v.f[2 * i], b = v.f[2 * i + 1];
-    const float ra = a - __uint_as_float(__float_as_uint(a) & 0xffff0000u), rb = b - __uint_as_float(__float_as_uint(b) & 0xffff0000u);
-    const float la = ra - __uint_as_float(__float_as_uint(ra) & 0xffff0000u), lb = rb - __uint_as_float(__float_as_uint(rb) & 0xffff0000u);
+    float ra, rb, la, lb;
+    const uint64_t rest = sub2(pack2(a, b), pack2(upper(a), upper(b)));
+    unpack2(rest, ra, rb);
+    unpack2(sub2(rest, pack2(upper(ra), upper(rb))), la, lb);
     h[i] = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
     m[i] = __byte_perm(__float_as_uint(ra), __float_as_uint(rb), 0x7632);
     l[i] = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
@@ -371,6 +406,14 @@ __device__ __forceinline__ uint32_t add_small(uint32_t large, uint32_t small) {
   return __float_as_uint(__fadd_rn(__uint_as_float(large), fmaxf(__uint_as_float(small), -FLT_MAX)));
 }
 
+// r[j] += t[j], r[j + 1] += t[j + 1]
+__device__ __forceinline__ void add_pair(uint32_t (&r)[16], const uint32_t (&t)[16], int j) {
+  float a, b;
+  unpack2(add2(pack2(__uint_as_float(t[j]), __uint_as_float(t[j + 1])), pack2(__uint_as_float(r[j]), __uint_as_float(r[j + 1]))), a, b);
+  r[j] = __float_as_uint(a);
+  r[j + 1] = __float_as_uint(b);
+}
+
 // One tile's sums in an epilogue warp (lanes 32 * warp ..): every finished segment of large products is added to the running
 // sums in tensor memory; with the last one the small products join and the 16-column blocks go to `put(first column, values)`.
 // `sg` and `rn` count segments and runs over all tiles; `nc`: buffers of the small products.  False if a wait gave up.
@@ -391,7 +434,7 @@ __device__ __forceinline__ bool drain_tile(const Bars &b, uint32_t lane_addr, in
       tmem_ld_wait();
       if (s > 0) {
 #pragma unroll
-        for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(t[j]), __uint_as_float(r[j])));
+        for (int j = 0; j < 16; j += 2) add_pair(r, t, j);
       }
       if (last) {  // (the small products' last one was committed with this segment)
         float v[16];
@@ -435,7 +478,7 @@ __device__ __forceinline__ bool drain_long_tile(const Bars &b, uint32_t lane_add
           for (int j = 0; j < 16; j++) r[j] = add_small(t[j], r[j]);
         } else if (s > 0) {
 #pragma unroll
-          for (int j = 0; j < 16; j++) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(t[j]), __uint_as_float(r[j])));
+          for (int j = 0; j < 16; j += 2) add_pair(r, t, j);
         }
         tmem_st_32x16(lane_addr + kSum + c, r);
       }
