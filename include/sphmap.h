@@ -333,7 +333,8 @@ enum sph_conv_op {
   SPH_TCONV_FORWARD = 3,
   SPH_TCONV_BACKWARD_INPUT = 4,
   SPH_TCONV_BACKWARD_WEIGHT = 5,
-  SPH_CONV_BACKWARD = 6 /* sph_mapped_conv_backward_cl: input, weight and bias gradients in one call */
+  SPH_CONV_BACKWARD = 6, /* sph_mapped_conv_backward_cl: input, weight and bias gradients in one call */
+  SPH_TCONV_BACKWARD = 7 /* sph_mapped_tconv_backward */
 };
 size_t sph_conv_workspace_bytes(int op, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW,
                                 int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp,
@@ -413,9 +414,9 @@ int sph_mapped_conv_relu_backward_weight(const void *gout, const void *act_out, 
  *       NULL) the companion of x; gx (and plan) NULL: an input that takes no
  *       gradient.  Workspace: op SPH_CONV_BACKWARD.  Returns
  *       SPH_ERR_UNSUPPORTED before launching anything for shapes that do not
- *       run on tensor-core kernels (exact precision; thin layers whose
- *       tensor-core form does not apply): use the separate entry points
- *       there.
+ *       run on tensor-core kernels (thin layers whose tensor-core form does not
+ *       apply) and in exact precision, but for float32 with gx, without act_out
+ *       and with the preferred scratch: use the separate entry points there.
  *   sph_conv_companion_fill  writes the companion of an existing float32
  *       tensor (a host that calls the same layer's forward and backward can
  *       convert the input once and pass the copy to both).
@@ -466,6 +467,13 @@ int sph_mapped_tconv_backward_weight(const void *gout, const void *x, const void
                                      void *gw, void *gb, int64_t B, int64_t Cin, int64_t Cout, int64_t IH,
                                      int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype,
                                      int interp, int precision, void *ws, size_t ws_bytes, void *stream);
+
+/* All three gradients of a transposed convolution in one call: float32, exact precision, with the preferred scratch of op
+ * SPH_TCONV_BACKWARD; SPH_ERR_UNSUPPORTED, before anything is launched, otherwise (use the two entry points above). */
+int sph_mapped_tconv_backward(const void *gout, const void *x, const void *map, const void *iw, const void *weight,
+                              void *gx, void *gw, void *gb, int64_t B, int64_t Cin, int64_t Cout, int64_t IH,
+                              int64_t IW, int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp,
+                              int precision, void *ws, size_t ws_bytes, void *stream);
 
 #ifdef __cplusplus
 }

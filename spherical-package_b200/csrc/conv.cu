@@ -63,6 +63,7 @@ size_t base_workspace(int op, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, 
     case SPH_CONV_BACKWARD: if (small_ok(Cin, K, Cout, ts)) return 0; break;  // thin layers: the separate entry points
     default: break;
   }
+  if (op == SPH_TCONV_BACKWARD) return 0;  // (with the preferred scratch of float32 in the exact precision alone)
   if (op == SPH_CONV_BACKWARD)
     return precision == SPH_PRECISION_BF16 ? tc_conv_backward_workspace(B, Cin, Cout, IH, IW, OH, OW, K, P, interp) : 0;
   if (precision == SPH_PRECISION_BF16) return tc_workspace_bytes(op, B, Cin, Cout, IH, IW, OH, OW, K, P, interp);
@@ -117,7 +118,7 @@ extern "C" size_t sph_conv_workspace_preferred_bytes(int op, int64_t B, int64_t 
     const size_t more = tc_conv_backward_workspace(B, Cin, Cout, IH, IW, OH, OW, K, P, interp, true);
     return more > base ? more : base;
   }
-  const bool transposed = op == SPH_TCONV_FORWARD || op == SPH_TCONV_BACKWARD_INPUT || op == SPH_TCONV_BACKWARD_WEIGHT;
+  const bool transposed = op == SPH_TCONV_FORWARD || op == SPH_TCONV_BACKWARD_INPUT || op == SPH_TCONV_BACKWARD_WEIGHT || op == SPH_TCONV_BACKWARD;
   if (transposed ? small_ok(Cout, K, Cin, 4) : small_ok(Cin, K, Cout, 4)) return base;
   size_t x3 = 0;
   switch (op) {
@@ -127,6 +128,8 @@ extern "C" size_t sph_conv_workspace_preferred_bytes(int op, int64_t B, int64_t 
     case SPH_TCONV_FORWARD: x3 = x3_gemm_workspace(true, B, Cin, IH * IW, K, 0, 0, Cout, OH * OW); break;
     case SPH_TCONV_BACKWARD_INPUT: x3 = x3_gemm_workspace(false, B, Cout, OH * OW, K, P, interp, Cin, 0); break;
     case SPH_TCONV_BACKWARD_WEIGHT: x3 = x3_dw_workspace(B, Cout, OH * OW, K, P, interp, Cin, IH, IW); break;
+    case SPH_CONV_BACKWARD: x3 = x3_backward_workspace(false, B, Cin, Cout, IH, IW, OH, OW, K, P, interp); break;
+    case SPH_TCONV_BACKWARD: x3 = x3_backward_workspace(true, B, Cin, Cout, IH, IW, OH, OW, K, P, interp); break;
     default: break;
   }
   return x3 > base ? x3 : base;
@@ -326,6 +329,9 @@ extern "C" int sph_mapped_conv_backward_cl(const void *gout, const void *act_out
   const int rc = check_dims(d, dtype, interp, precision);
   if (rc != SPH_OK) return rc;
   if (!gout || !x || (gx && !plan) || !map || !weight || !gw || !gb || (P > 0 && !iw)) return SPH_ERR_INVALID_ARGUMENT;
+  if (precision == SPH_PRECISION_EXACT && gx && !act_out && B > 0 && dtype == SPH_F32 && !small_ok(Cin, K, Cout, 4) &&
+      split_fits(dtype, ws, ws_bytes, x3_backward_workspace(false, B, Cin, Cout, IH, IW, OH, OW, K, P, interp)))
+    return x3_backward(false, gout, x, plan, map, iw, weight, gx, gw, gb, B, Cin, Cout, IH, IW, OH, OW, K, P, interp, ws, (cudaStream_t)stream);
   if (precision != SPH_PRECISION_BF16 || B == 0) return SPH_ERR_UNSUPPORTED;
   if (tc_thin_backward_ok(Cin, K, Cout, OH * OW)) {
     const int rt = tc_thin_conv_backward(gout, act_out, x, plan, map, iw, weight, gx, gw, gb, B, Cin, Cout, IH, IW, OH, OW, K, P, interp, ws,
@@ -408,4 +414,19 @@ extern "C" int sph_mapped_tconv_backward_weight(const void *gout, const void *x,
     return x3_dw(x, gout, map, iw, Cout, OH, OW, K, P, IH, IW, interp, Cin, B, gw, Cout * K, K, 1, gb, true, ws, st);
   return SPH_BY_DTYPE(simt_dw, x, gout, map, iw, Cout, OH, OW, K, P, IH * IW, interp, Cin, B, gw, Cout * K, K, 1, gout, Cout,
                       OH * OW, gb, ws, ws_bytes, st);
+}
+
+extern "C" int sph_mapped_tconv_backward(const void *gout, const void *x, const void *map, const void *iw, const void *weight, void *gx,
+                                         void *gw, void *gb, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH,
+                                         int64_t OW, int64_t K, int64_t P, int dtype, int interp, int precision, void *ws, size_t ws_bytes,
+                                         void *stream) {
+  SPH_RANGE("sph_mapped_tconv_backward");
+  const Dims d{B, Cin, Cout, IH, IW, OH, OW, K, P};
+  const int rc = check_dims(d, dtype, interp, precision);
+  if (rc != SPH_OK) return rc;
+  if (!gout || !x || !map || !weight || !gx || !gw || !gb || (P > 0 && !iw)) return SPH_ERR_INVALID_ARGUMENT;
+  if (precision != SPH_PRECISION_EXACT || B == 0 || small_ok(Cout, K, Cin, 4) ||
+      !split_fits(dtype, ws, ws_bytes, x3_backward_workspace(true, B, Cin, Cout, IH, IW, OH, OW, K, P, interp)))
+    return SPH_ERR_UNSUPPORTED;
+  return x3_backward(true, gout, x, nullptr, map, iw, weight, gx, gw, gb, B, Cin, Cout, IH, IW, OH, OW, K, P, interp, ws, (cudaStream_t)stream);
 }

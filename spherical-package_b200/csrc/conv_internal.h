@@ -78,6 +78,12 @@ size_t x3_dw_workspace(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P,
 int x3_dw(const void *A, const void *src, const void *map, const void *iw, int64_t CH, int64_t SH, int64_t SW, int64_t K, int64_t P,
           int64_t GH, int64_t GW, int interp, int64_t M, int64_t B, void *gw, int64_t sm, int64_t sc, int64_t sk, void *gb, bool bias_of_src,
           void *ws, cudaStream_t st);
+// input, weight and bias gradients together; operands as sph_mapped_conv_backward_cl / sph_mapped_tconv_backward
+size_t x3_backward_workspace(bool transposed, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K,
+                             int64_t P, int interp);
+int x3_backward(bool transposed, const void *gout, const void *x, const void *plan, const void *map, const void *iw, const void *weight,
+                void *gx, void *gw, void *gb, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K,
+                int64_t P, int interp, void *ws, cudaStream_t st);
 int x3_wait_status(int reset);  // sticky word of a bounded wait that gave up; < 0: CUDA error
 
 template <typename T>

@@ -973,6 +973,19 @@ __global__ void __launch_bounds__(256) dw_prepare3_kernel(const Nhwc3 src, const
   else nhwc_block(src, blockIdx.x - grad.blocks, tile);
 }
 
+// The pre-pass of both in one launch (x3_backward): two gathered sides, the second one empty where both products gather from the same.
+__global__ void __launch_bounds__(256) backward_prepare3_kernel(const Nhwc3 src, const Nhwc3 src2, const Weight3 wgt, const Grad3 grad,
+                                                                int *status, int *status2) {
+  __shared__ NhwcTile tile;
+  launch_dependents();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *status = *status2 = 0;
+  int block = blockIdx.x;
+  if (block < grad.blocks) return grad_block(grad, block);
+  if ((block -= grad.blocks) < wgt.blocks) return weight_block(wgt, block);
+  if ((block -= wgt.blocks) < src.blocks) return nhwc_block(src, block, tile);
+  nhwc_block(src2, block - src.blocks, tile);
+}
+
 // The post-pass of x3_dw in one launch: gw[m, ch, k] = sum over splits, in order, of the partial sums (256 values per block, columns
 // fastest), and gb[c] = sum over `parts` of sums[part * pitch + c], one block per channel, in a fixed order.
 struct Reduce3 {
@@ -1212,45 +1225,76 @@ size_t x3_gemm_workspace(bool use_plan, int64_t B, int64_t CH, int64_t SHW, int6
   return q.ok ? 256 + q.xl_bytes + q.wp_bytes : 0;
 }
 
-int x3_gemm(bool use_plan, const void *src, const void *map, const void *iw, const void *plan, int64_t CH, int64_t SH, int64_t SW, int64_t K,
-            int64_t P, int64_t GH, int64_t GW, int interp, const void *wgt, int64_t sm, int64_t sc, int64_t sk, const void *bias, void *out,
-            int64_t Nout, int64_t B, void *ws, cudaStream_t st) {
-  const Premul3 r = use_plan ? premul3(B, CH, SH * SW, K, Nout, GH * GW) : Premul3{};
-  const int kind = r.use ? (int)SRC_SELF : source3(use_plan, P, interp);
-  const GemmPlan3 q = r.use ? r.q : gemm_plan3(kind, B, CH, SH * SW, K, Nout);
+namespace {
+
+// What x3_gemm launches: the pre-pass's operands, the product, the row gather of the multiply-first form.
+struct GemmCall3 {
+  Premul3 r;
+  GemmPlan3 q;
+  int kind;
+  Nhwc3 pre;
+  Weight3 wt;
+  Gemm3 p;
+  const void *plan, *bias;
+  void *out;
+  int64_t Nout, K, B, n_src, n_dst;
+};
+GemmCall3 gemm_call3(bool use_plan, const void *src, const void *map, const void *iw, const void *plan, int64_t CH, int64_t SH, int64_t SW,
+                     int64_t K, int64_t P, int64_t GH, int64_t GW, int interp, const void *wgt, int64_t sm, int64_t sc, int64_t sk,
+                     const void *bias, void *out, int64_t Nout, int64_t B, void *ws) {
+  GemmCall3 c{};
+  c.r = use_plan ? premul3(B, CH, SH * SW, K, Nout, GH * GW) : Premul3{};
+  c.kind = c.r.use ? (int)SRC_SELF : source3(use_plan, P, interp);
+  c.q = c.r.use ? c.r.q : gemm_plan3(c.kind, B, CH, SH * SW, K, Nout);
+  const Premul3 &r = c.r;
+  const GemmPlan3 &q = c.q;
   char *w = (char *)ws;
-  int *status = (int *)w;
   float *xl = (float *)(w + 256);
   uint16_t *wp = (uint16_t *)(w + 256 + q.xl_bytes);
   float *T = (float *)(w + 256 + q.xl_bytes + q.wp_bytes);
-  const Nhwc3 pre = nhwc3(src, xl, B, CH, q.Cp, SH * SW);
-  const Weight3 wt{(const float *)wgt, wp, (int)Nout, (int)CH, q.Cp, (int)K, q.Npb, q.nblk, q.nchunks, r.use ? r.Mp : 0,
-                   cdiv((int64_t)q.nblk * q.nchunks * q.Npb * kCols, 256), sm, sc, sk};
-  gemm_prepare3_kernel<<<(unsigned)(wt.blocks + pre.blocks), 256, 0, st>>>(pre, wt, status);
-  Gemm3 p{};
+  c.pre = nhwc3(src, xl, B, CH, q.Cp, SH * SW);
+  c.wt = Weight3{(const float *)wgt, wp, (int)Nout, (int)CH, q.Cp, (int)K, q.Npb, q.nblk, q.nchunks, r.use ? r.Mp : 0,
+                 cdiv((int64_t)q.nblk * q.nchunks * q.Npb * kCols, 256), sm, sc, sk};
+  Gemm3 &p = c.p;
   p.g = Src3{(const char *)xl, (const float *)map, (const float *)iw, plan, q.Cp, (int)SH, (int)SW, r.use ? 1 : (int)K, (int)P,
              (int)(r.use ? SH : GH), (int)(r.use ? SW : GW), interp};
   p.wp = (const __nv_bfloat16 *)wp;
   p.bias = r.use ? nullptr : (const float *)bias;
   p.out = r.use ? T : (float *)out;
-  p.status = status;
+  p.status = (int *)w;
   p.B = (int)B; p.Nout = (int)(r.use ? K * r.Mp : Nout); p.Npb = q.Npb; p.nblk = q.nblk; p.nchunks = q.nchunks;
   p.tiles_x = cdiv(p.g.GW, kTileW); p.tiles_y = cdiv(p.g.GH, kTileH); p.stages = q.stages;
-  const int64_t tiles = B * p.tiles_x * p.tiles_y * q.nblk;
-  switch (kind) {
-    case SRC_MAP1: launch_gemm3<SRC_MAP1>(p, tiles, q.smem, st); break;
-    case SRC_MAP4: launch_gemm3<SRC_MAP4>(p, tiles, q.smem, st); break;
-    case SRC_PLAN: launch_gemm3<SRC_PLAN>(p, tiles, q.smem, st); break;
-    default: launch_gemm3<SRC_SELF>(p, tiles, q.smem, st); break;
+  c.plan = plan; c.bias = bias; c.out = out;
+  c.Nout = Nout; c.K = K; c.B = B; c.n_src = SH * SW; c.n_dst = GH * GW;
+  return c;
+}
+// The product; `prepared`: launches of the pre-pass.
+int run_gemm3(const GemmCall3 &c, int prepared, cudaStream_t st) {
+  const int64_t tiles = c.B * c.p.tiles_x * c.p.tiles_y * c.q.nblk;
+  switch (c.kind) {
+    case SRC_MAP1: launch_gemm3<SRC_MAP1>(c.p, tiles, c.q.smem, st); break;
+    case SRC_MAP4: launch_gemm3<SRC_MAP4>(c.p, tiles, c.q.smem, st); break;
+    case SRC_PLAN: launch_gemm3<SRC_PLAN>(c.p, tiles, c.q.smem, st); break;
+    default: launch_gemm3<SRC_SELF>(c.p, tiles, c.q.smem, st); break;
   }
-  const int rc = launch_status(2);
-  if (rc != SPH_OK || !r.use) return rc;
-  const int vecs = r.Mp / 8, lanes = vecs >= 4 ? 4 : vecs >= 2 ? 2 : 1, nv = vecs > 4 ? 2 : 1;
-  const dim3 grid(cdiv(GH * GW, 256 / lanes), cdiv(vecs, nv * lanes), (unsigned)B);
+  const int rc = launch_status(1 + prepared);
+  if (rc != SPH_OK || !c.r.use) return rc;
+  const int vecs = c.r.Mp / 8, lanes = vecs >= 4 ? 4 : vecs >= 2 ? 2 : 1, nv = vecs > 4 ? 2 : 1;
+  const dim3 grid(cdiv(c.n_dst, 256 / lanes), cdiv(vecs, nv * lanes), (unsigned)c.B);
   const auto rows = nv == 2 ? plan_gather_rows3_kernel<2, 4>
                             : (lanes == 4 ? plan_gather_rows3_kernel<1, 4> : lanes == 2 ? plan_gather_rows3_kernel<1, 2> : plan_gather_rows3_kernel<1, 1>);
-  rows<<<grid, 256, 0, st>>>(T, plan, (const float *)bias, (float *)out, (int)K, (int)Nout, r.Mp, (int)(SH * SW), (int)(GH * GW));
+  rows<<<grid, 256, 0, st>>>(c.p.out, c.plan, (const float *)c.bias, (float *)c.out, (int)c.K, (int)c.Nout, c.r.Mp, (int)c.n_src, (int)c.n_dst);
   return launch_status();
+}
+
+}  // namespace
+
+int x3_gemm(bool use_plan, const void *src, const void *map, const void *iw, const void *plan, int64_t CH, int64_t SH, int64_t SW, int64_t K,
+            int64_t P, int64_t GH, int64_t GW, int interp, const void *wgt, int64_t sm, int64_t sc, int64_t sk, const void *bias, void *out,
+            int64_t Nout, int64_t B, void *ws, cudaStream_t st) {
+  const GemmCall3 c = gemm_call3(use_plan, src, map, iw, plan, CH, SH, SW, K, P, GH, GW, interp, wgt, sm, sc, sk, bias, out, Nout, B, ws);
+  gemm_prepare3_kernel<<<(unsigned)(c.wt.blocks + c.pre.blocks), 256, 0, st>>>(c.pre, c.wt, c.p.status);
+  return run_gemm3(c, 1, st);
 }
 
 size_t x3_dw_workspace(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int interp, int64_t M, int64_t GH, int64_t GW) {
@@ -1258,33 +1302,96 @@ size_t x3_dw_workspace(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P,
   return d.ok ? 256 + d.xl_bytes + d.gt_bytes + d.partial_bytes + d.sums_bytes : 0;
 }
 
+namespace {
+
+// What x3_dw launches.  `copy`: the gathered side's channels-last copy, if another product's pre-pass makes it.
+struct DwCall3 {
+  DwPlan3 d;
+  int kind;
+  Nhwc3 pre;
+  Grad3 grad;
+  Dw3 p;
+  Reduce3 red;
+  int channels;  // of the bias gradient
+};
+DwCall3 dw_call3(const void *A, const void *src, const void *map, const void *iw, int64_t CH, int64_t SH, int64_t SW, int64_t K, int64_t P,
+                 int64_t GH, int64_t GW, int interp, int64_t M, int64_t B, void *gw, int64_t sm, int64_t sc, int64_t sk, void *gb,
+                 bool bias_of_src, void *ws, const char *copy = nullptr) {
+  DwCall3 c{};
+  c.kind = source3(false, P, interp);
+  c.d = dw_plan3(c.kind, B, CH, SH * SW, K, M, GH, GW);
+  const DwPlan3 &d = c.d;
+  char *w = (char *)ws + 256;
+  float *xl = (float *)w;
+  if (!copy) w += d.xl_bytes;
+  uint8_t *gt = (uint8_t *)w;
+  float *partial = (float *)(w + d.gt_bytes), *sums = (float *)((char *)partial + d.partial_bytes);
+  c.pre = nhwc3(src, xl, B, CH, d.Cp, SH * SW, bias_of_src ? sums : nullptr);
+  const int tiles = (int)(B * d.tiles_x * d.tiles_y);
+  c.grad = Grad3{(const float *)A, gt, bias_of_src ? nullptr : sums, (int)M, (int)GH, (int)GW, d.tiles_x, d.tiles_y, d.mbs, tiles * d.mbs};
+  Dw3 &p = c.p;
+  p.g = Src3{copy ? copy : (const char *)xl, (const float *)map, (const float *)iw, nullptr, d.Cp, (int)SH, (int)SW, (int)K, (int)P, (int)GH,
+             (int)GW, interp};
+  p.gt = (const __nv_bfloat16 *)gt; p.partial = partial; p.status = (int *)ws;
+  p.B = (int)B; p.mbs = d.mbs; p.groups = d.groups; p.slots = d.slots; p.tiles_x = d.tiles_x; p.tiles_y = d.tiles_y;
+  p.splits = d.splits; p.stages = d.stages;
+  c.red = Reduce3{partial, sums, (float *)gw, (float *)gb, d.splits, d.mbs * 128, d.groups * kDwN, (int)M, (int)CH, d.Cp, (int)K,
+                  cdiv(M * CH * K, 256), bias_of_src ? (int)B * c.pre.px_blocks : tiles, bias_of_src ? d.Cp : d.mbs * 128, sm, sc, sk};
+  c.channels = (int)(bias_of_src ? CH : M);
+  return c;
+}
+int run_dw3(const DwCall3 &c, int prepared, cudaStream_t st) {
+  if (c.kind == SRC_MAP1) launch_dw3<SRC_MAP1>(c.p, c.d.smem, st);
+  else launch_dw3<SRC_MAP4>(c.p, c.d.smem, st);
+  dw_reduce3_kernel<<<(unsigned)(c.red.blocks + c.channels), 256, 0, st>>>(c.red);
+  return launch_status(2 + prepared);
+}
+
+}  // namespace
+
 // gw[m, ch, k] = sum A[b, m, pix] * Col[b, pix, (ch, k)], and the bias gradient gb: the sums of A's rows or (bias_of_src: a
 // transposed convolution, whose gathered side is the output's gradient) of the source's channels.
 int x3_dw(const void *A, const void *src, const void *map, const void *iw, int64_t CH, int64_t SH, int64_t SW, int64_t K, int64_t P,
           int64_t GH, int64_t GW, int interp, int64_t M, int64_t B, void *gw, int64_t sm, int64_t sc, int64_t sk, void *gb, bool bias_of_src,
           void *ws, cudaStream_t st) {
-  const int kind = source3(false, P, interp);
-  const DwPlan3 d = dw_plan3(kind, B, CH, SH * SW, K, M, GH, GW);
-  char *w = (char *)ws;
-  int *status = (int *)w;
-  float *xl = (float *)(w + 256);
-  uint8_t *gt = (uint8_t *)(w + 256 + d.xl_bytes);
-  float *partial = (float *)(w + 256 + d.xl_bytes + d.gt_bytes), *sums = (float *)((char *)partial + d.partial_bytes);
-  const Nhwc3 pre = nhwc3(src, xl, B, CH, d.Cp, SH * SW, bias_of_src ? sums : nullptr);
-  const int tiles = (int)(B * d.tiles_x * d.tiles_y);
-  const Grad3 grad{(const float *)A, gt, bias_of_src ? nullptr : sums, (int)M, (int)GH, (int)GW, d.tiles_x, d.tiles_y, d.mbs, tiles * d.mbs};
-  dw_prepare3_kernel<<<(unsigned)(grad.blocks + pre.blocks), 256, 0, st>>>(pre, grad, status);
-  Dw3 p{};
-  p.g = Src3{(const char *)xl, (const float *)map, (const float *)iw, nullptr, d.Cp, (int)SH, (int)SW, (int)K, (int)P, (int)GH, (int)GW, interp};
-  p.gt = (const __nv_bfloat16 *)gt; p.partial = partial; p.status = status;
-  p.B = (int)B; p.mbs = d.mbs; p.groups = d.groups; p.slots = d.slots; p.tiles_x = d.tiles_x; p.tiles_y = d.tiles_y;
-  p.splits = d.splits; p.stages = d.stages;
-  if (kind == SRC_MAP1) launch_dw3<SRC_MAP1>(p, d.smem, st);
-  else launch_dw3<SRC_MAP4>(p, d.smem, st);
-  const Reduce3 red{partial, sums, (float *)gw, (float *)gb, d.splits, d.mbs * 128, d.groups * kDwN, (int)M, (int)CH, d.Cp, (int)K,
-                    cdiv(M * CH * K, 256), bias_of_src ? (int)B * pre.px_blocks : tiles, bias_of_src ? d.Cp : d.mbs * 128, sm, sc, sk};
-  dw_reduce3_kernel<<<(unsigned)(red.blocks + (bias_of_src ? CH : M)), 256, 0, st>>>(red);
-  return launch_status(3);
+  const DwCall3 c = dw_call3(A, src, map, iw, CH, SH, SW, K, P, GH, GW, interp, M, B, gw, sm, sc, sk, gb, bias_of_src, ws);
+  dw_prepare3_kernel<<<(unsigned)(c.grad.blocks + c.pre.blocks), 256, 0, st>>>(c.pre, c.grad, c.p.status);
+  return run_dw3(c, 1, st);
+}
+
+// All gradients of a convolution, or of a transposed one, with one pre-pass.  Both products of a transposed convolution gather from the
+// output's gradient: its copy is made once.
+size_t x3_backward_workspace(bool transposed, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K,
+                             int64_t P, int interp) {
+  const size_t dx = transposed ? x3_gemm_workspace(false, B, Cout, OH * OW, K, P, interp, Cin, 0)
+                               : x3_gemm_workspace(true, B, Cout, OH * OW, K, 0, 0, Cin, IH * IW);
+  const size_t dw = transposed ? x3_dw_workspace(B, Cout, OH * OW, K, P, interp, Cin, IH, IW)
+                               : x3_dw_workspace(B, Cin, IH * IW, K, P, interp, Cout, OH, OW);
+  if (dx == 0 || dw == 0) return 0;
+  const size_t shared = transposed ? dw_plan3(source3(false, P, interp), B, Cout, OH * OW, K, Cin, IH, IW).xl_bytes : 0;
+  return align_up(dx, 256) + dw - shared;
+}
+
+int x3_backward(bool transposed, const void *gout, const void *x, const void *plan, const void *map, const void *iw, const void *weight,
+                void *gx, void *gw, void *gb, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K,
+                int64_t P, int interp, void *ws, cudaStream_t st) {
+  GemmCall3 dx = transposed ? gemm_call3(false, gout, map, iw, nullptr, Cout, OH, OW, K, P, IH, IW, interp, weight, Cout * K, K, 1, nullptr,
+                                         gx, Cin, B, ws)
+                            : gemm_call3(true, gout, nullptr, nullptr, plan, Cout, OH, OW, K, 0, IH, IW, 0, weight, K, Cin * K, 1, nullptr, gx,
+                                         Cin, B, ws);
+  void *ws2 = (char *)ws + align_up(transposed ? x3_gemm_workspace(false, B, Cout, OH * OW, K, P, interp, Cin, 0)
+                                               : x3_gemm_workspace(true, B, Cout, OH * OW, K, 0, 0, Cin, IH * IW), 256);
+  DwCall3 dw = transposed ? dw_call3(x, gout, map, iw, Cout, OH, OW, K, P, IH, IW, interp, Cin, B, gw, Cout * K, K, 1, gb, true, ws2,
+                                     dx.p.g.xl)
+                          : dw_call3(gout, x, map, iw, Cin, IH, IW, K, P, OH, OW, interp, Cout, B, gw, Cin * K, K, 1, gb, false, ws2);
+  if (transposed) {
+    dx.pre.sums = dw.pre.sums;
+    dw.pre.blocks = 0;
+  }
+  backward_prepare3_kernel<<<(unsigned)(dw.grad.blocks + dx.wt.blocks + dx.pre.blocks + dw.pre.blocks), 256, 0, st>>>(
+      dx.pre, dw.pre, dx.wt, dw.grad, dx.p.status, dw.p.status);
+  const int rc = run_gemm3(dx, 1, st);
+  return rc != SPH_OK ? rc : run_dw3(dw, 0, st);
 }
 
 int x3_wait_status(int reset) {

@@ -706,6 +706,17 @@ struct ConvScratch {
       buf = workspace(bytes, like);
     }
   }
+  // The preferred scratch or nothing: for an operator that others stand in for.
+  bool get_all(int op, const ConvArgs &a, const torch::Tensor &like) {
+    bytes = sph_conv_workspace_preferred_bytes(op, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec);
+    if (bytes == 0) return false;
+    try {
+      buf = workspace(bytes, like);
+      return true;
+    } catch (const c10::OutOfMemoryError &) {
+      return false;
+    }
+  }
   void *ptr() const { return buf.data_ptr(); }
 };
 
@@ -828,8 +839,21 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
       }
     }
   }
-  // The scratch of the input gradient is given back before the weight gradient's is taken.
   const void *q = iw ? iw->data_ptr() : nullptr;
+  if (a.prec == SPH_PRECISION_EXACT && need_gx && !act_out) {  // one pre-pass for both products
+    ConvScratch wsc;
+    if (wsc.get_all(SPH_CONV_BACKWARD, a, x)) {
+      const int rc = sph_mapped_conv_backward_cl(go.data_ptr(), nullptr, x.data_ptr(), nullptr, plan.data_ptr(), map.data_ptr(), q,
+                                                 weight.data_ptr(), gx.data_ptr(), gw.data_ptr(), gb.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW,
+                                                 a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec, wsc.ptr(), wsc.bytes, stream());
+      if (rc != SPH_ERR_UNSUPPORTED) {
+        ok(rc, "sph_mapped_conv_backward_cl");
+        maybe_check_device("mapped convolution");
+        return {gx, gw, gb};
+      }
+    }
+  }
+  // The scratch of the input gradient is given back before the weight gradient's is taken.
   ConvScratch wsx, wsw;
   const auto input_gradient = [&](const torch::Tensor *mask) -> int {
     if (!need_gx) return SPH_OK;
@@ -948,6 +972,17 @@ std::vector<torch::Tensor> tconv_backward_impl(torch::Tensor go, torch::Tensor m
                    (int)it, dtype_of(x) == SPH_F32 ? precision() : SPH_PRECISION_EXACT};
   torch::Tensor gx = torch::empty_like(x), gw = torch::empty_like(weight), gb = torch::empty({a.Cout}, x.options());
   ConvScratch ws;
+  if (a.prec == SPH_PRECISION_EXACT && ws.get_all(SPH_TCONV_BACKWARD, a, x)) {  // one pre-pass, and one copy of grad_output
+    const int rc = sph_mapped_tconv_backward(go.data_ptr(), x.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, weight.data_ptr(),
+                                             gx.data_ptr(), gw.data_ptr(), gb.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P,
+                                             a.dtype, a.interp, a.prec, ws.ptr(), ws.bytes, stream());
+    if (rc != SPH_ERR_UNSUPPORTED) {
+      ok(rc, "sph_mapped_tconv_backward");
+      maybe_check_device("mapped convolution");
+      return {gx, gw, gb};
+    }
+  }
+  ws = ConvScratch();
   ws.get(SPH_TCONV_BACKWARD_INPUT, a, x);
   ok(sph_mapped_tconv_backward_input(go.data_ptr(), map.data_ptr(), iw ? iw->data_ptr() : nullptr, weight.data_ptr(),
                                      gx.data_ptr(), a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp,

@@ -19,7 +19,7 @@ F32, F64 = 0, 1
 NEAREST, BILINEAR, BISPHERICAL = 0, 1, 2
 EXACT, BF16 = 0, 1
 CONV_FORWARD, CONV_BACKWARD_INPUT, CONV_BACKWARD_WEIGHT = 0, 1, 2
-CONV_BACKWARD = 6
+CONV_BACKWARD, TCONV_BACKWARD = 6, 7
 TCONV_FORWARD, TCONV_BACKWARD_INPUT, TCONV_BACKWARD_WEIGHT = 3, 4, 5
 
 SYMBOLS = [
@@ -32,7 +32,7 @@ SYMBOLS = [
     "sph_mapped_avg_unpool", "sph_resample_to_map_normalized", "sph_resample_from_uv_maps", "sph_plan_build_uv",
     "sph_voting_resample_to_map", "sph_map_locality", "sph_build_kernel_map", "sph_build_is_checked", "sph_conv_companion_bytes",
     "sph_staging_bytes", "sph_conv_workspace_preferred_bytes", "sph_resample_from_map_ws", "sph_resample_to_map_ws", "sph_mapped_pool_ws", "sph_mapped_max_unpool_ws",
-    "sph_conv_companion_channels", "sph_conv_companion_fill", "sph_trace_phases", "sph_mapped_conv_forward_cl", "sph_mapped_conv_backward_cl",
+    "sph_conv_companion_channels", "sph_conv_companion_fill", "sph_trace_phases", "sph_mapped_conv_forward_cl", "sph_mapped_conv_backward_cl", "sph_mapped_tconv_backward",
 ]
 ERR_UNSUPPORTED = 2
 
@@ -511,3 +511,20 @@ def tconv_backward_weight(go, x, smap, K, interp, iw=None, precision=EXACT):
                                              _int(int(interp)), _int(precision), _ptr(ws[0]), _sz(ws[1]), _stream()),
         "sph_mapped_tconv_backward_weight")
     return gw, gb
+
+
+def tconv_backward(go, x, smap, weight, K, interp, iw=None, ws=None):
+    """(grad_input, grad_weight, grad_bias) of float32 in the exact precision in one call.  Raises Unsupported elsewhere."""
+    B, Cin, IH, IW = x.shape
+    _, Cout, OH, OW = go.shape
+    gx, gw = torch.empty_like(x), torch.empty_like(weight)
+    gb = torch.empty(Cout, dtype=x.dtype, device=x.device)
+    if ws is None:
+        ws = conv_workspace(TCONV_BACKWARD, B, Cin, Cout, IH, IW, OH, OW, K, _P(iw), _dt(x), interp, EXACT, x, preferred=True)
+    rc = lib.sph_mapped_tconv_backward(_ptr(go), _ptr(x), _ptr(smap), _ptr(iw), _ptr(weight), _ptr(gx), _ptr(gw), _ptr(gb),
+                                       *_ints(B, Cin, Cout, IH, IW, OH, OW, K, _P(iw)), _int(_dt(x)), _int(int(interp)), _int(EXACT),
+                                       _ptr(ws[0]), _sz(ws[1]), _stream())
+    if rc == ERR_UNSUPPORTED:
+        raise Unsupported("sph_mapped_tconv_backward")
+    _ok(rc, "sph_mapped_tconv_backward")
+    return gx, gw, gb

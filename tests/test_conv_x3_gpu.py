@@ -142,3 +142,38 @@ def test_infinities_and_nans_are_those_of_float32(case, kind):
     for what, n, o in zip(("forward", "dInput", "dW", "dBias", "t forward", "t dInput", "t dW", "t dBias"), new, old):
         for which, f in (("NaN", torch.isnan), ("+inf", torch.isposinf), ("-inf", torch.isneginf)):
             assert torch.equal(f(n), f(o)), (what, which, int(f(n).sum()), int(f(o).sum()))
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_one_pre_pass_for_all_gradients(case):
+    """The combined backward, of a convolution and of a transposed one: the bits of the separate calls, one launch less; and none
+    without the scratch for it."""
+    from _gpu_impl import preferred_scratch
+    from sphmap import capi
+    B, ci, co, (H, W), (OH, OW), K, interp, P = case
+    g = torch.Generator().manual_seed(ci)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()  # noqa: E731
+    x, w, go, wt, xt, got = r(B, ci, H, W), r(co, ci, K), r(B, co, OH, OW), r(ci, co, K), r(B, ci, OH, OW), r(B, co, H, W)
+    m = (torch.rand(*((OH, OW, K, P, 2) if P else (OH, OW, K, 2)), generator=g) * torch.tensor([W + 1.0, H + 1.0]) - 1.0).cuda()
+    iw = torch.rand(OH, OW, K, P, generator=g).cuda() if P else None
+    plan = capi.plan_build(m, iw, OH * OW, K, interp, H, W)
+
+    def launches(fn):
+        before = capi.lib.sph_launch_count()
+        out = fn()
+        return out, capi.lib.sph_launch_count() - before
+
+    with preferred_scratch():
+        ref, n = launches(lambda: [capi.conv_backward_input(go, plan, w, H, W, K), *capi.conv_backward_weight(go, x, m, K, interp, iw)])
+        tref, tn = launches(lambda: [capi.tconv_backward_input(got, m, wt, K, interp, iw), *capi.tconv_backward_weight(got, xt, m, K, interp, iw)])
+        new, nn = launches(lambda: capi.conv_backward_cl(go, None, x, None, plan, m, w, K, interp, iw, capi.EXACT))
+    tnew, tnn = launches(lambda: capi.tconv_backward(got, xt, m, wt, K, interp, iw))
+    assert all(torch.equal(a, b) for a, b in zip([*new, *tnew], [*ref, *tref]))
+    assert nn == n - 1 and tnn == tn - 1
+    for call in (lambda: capi.conv_backward_cl(go, None, x, None, plan, m, w, K, interp, iw, capi.EXACT),
+                 lambda: capi.conv_backward_cl(go, go, x, None, plan, m, w, K, interp, iw, capi.EXACT),
+                 lambda: capi.tconv_backward(got, xt, m, wt, K, interp, iw, ws=capi.conv_workspace(
+                     capi.TCONV_BACKWARD, B, ci, co, OH, OW, H, W, K, P, capi.F32, interp, capi.EXACT, x))):
+        with pytest.raises(capi.Unsupported):
+            call()
+    assert capi.device_status() == 0
