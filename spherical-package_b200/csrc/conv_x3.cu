@@ -974,16 +974,28 @@ __global__ void __launch_bounds__(256) dw_prepare3_kernel(const Nhwc3 src, const
 }
 
 // The pre-pass of both in one launch (x3_backward): two gathered sides, the second one empty where both products gather from the same.
+// A convolution's products share the output's gradient, one as the gathered side, the other as tile images: their blocks take turns, in
+// proportion, so that the second read comes from L2 (8 x 128 planes of 128 x 256: 119 us one after the other, so 102; a transposed
+// convolution, which makes its images of another tensor, 41 and 45).
 __global__ void __launch_bounds__(256) backward_prepare3_kernel(const Nhwc3 src, const Nhwc3 src2, const Weight3 wgt, const Grad3 grad,
                                                                 int *status, int *status2) {
   __shared__ NhwcTile tile;
   launch_dependents();
   if (blockIdx.x == 0 && threadIdx.x == 0) *status = *status2 = 0;
+  const int both = grad.blocks + src.blocks;
   int block = blockIdx.x;
-  if (block < grad.blocks) return grad_block(grad, block);
-  if ((block -= grad.blocks) < wgt.blocks) return weight_block(wgt, block);
-  if ((block -= wgt.blocks) < src.blocks) return nhwc_block(src, block, tile);
-  nhwc_block(src2, block - src.blocks, tile);
+  if (block < both) {
+    int s = max(block - grad.blocks, 0), next = max(block + 1 - grad.blocks, 0);  // blocks of `src` before this one and the next
+    if (src.x == grad.g) {
+      s = (int)((int64_t)block * src.blocks / both);
+      next = (int)((int64_t)(block + 1) * src.blocks / both);
+    }
+    if (next > s) nhwc_block(src, s, tile);
+    else grad_block(grad, block - s);
+    return;
+  }
+  if ((block -= both) < wgt.blocks) return weight_block(wgt, block);
+  nhwc_block(src2, block - wgt.blocks, tile);
 }
 
 // The post-pass of x3_dw in one launch: gw[m, ch, k] = sum over splits, in order, of the partial sums (256 values per block, columns
