@@ -223,9 +223,10 @@ int64_t plan_cache_size() {
 }
 
 // ---- locality of sample maps ------------------------------------------------------
-// Gathers and max pooling by nearest neighbours read the planes where they lie if neighbouring outputs read neighbouring pixels,
-// and transposed groups of planes if not.  Which it is depends only on the map: a small kernel looks, the first time a map is seen,
-// and writes the answer into pinned memory; until it is there, and while a stream is captured, it is unknown.  (Both ways give the
+// Gathers, scatters and max pooling read the planes where they lie if neighbouring outputs read neighbouring pixels, and
+// transposed groups of planes if not.  Which it is depends only on the map: a small kernel looks, the first time a map is seen or,
+// with `later`, the second time (where little is won per call, a map that is used once does not pay the 4 us of a look), and writes
+// the answer into pinned memory; until it is there, and while a stream is captured, it is unknown.  (Both ways give the
 // same bits, so an answer that comes late or belongs to a map whose place was given away costs time only.)
 enum class Locality { Unknown = 0, Local = 1, Scattered = 2 };
 struct LocalityEntry {
@@ -233,20 +234,24 @@ struct LocalityEntry {
   const void *map_p;
   uint32_t map_v;
   int64_t n, K;
-  int slot;
+  int slot;  // -1: seen, not looked at
 };
 std::mutex g_locality_mu;
 constexpr int kMaxLocalities = 64;
 
-Locality locality_of(const torch::Tensor &map, int64_t n, int64_t K) {
+Locality locality_of(const torch::Tensor &map, int64_t n, int64_t K, bool later = false) {
   static auto *entries = new std::list<LocalityEntry>();
   static volatile int *flags = nullptr;
   static int next = 0;
   std::lock_guard<std::mutex> lock(g_locality_mu);
-  for (const LocalityEntry &e : *entries)
+  LocalityEntry *entry = nullptr;
+  for (LocalityEntry &e : *entries)
     if (e.map_p == map.data_ptr() && e.map_v == version_of(map) && e.n == n && e.K == K &&
-        e.map_s.lock().get() == map.storage().unsafeGetStorageImpl())
-      return (Locality)flags[e.slot];
+        e.map_s.lock().get() == map.storage().unsafeGetStorageImpl()) {
+      if (e.slot >= 0) return (Locality)flags[e.slot];
+      entry = &e;
+      break;
+    }
   const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
@@ -259,13 +264,20 @@ Locality locality_of(const torch::Tensor &map, int64_t n, int64_t K) {
     }
     flags = (volatile int *)p;
   }
+  if (entry == nullptr) {
+    entries->remove_if([](const LocalityEntry &e) { return e.map_s.expired(); });
+    if (entries->size() >= 2 * kMaxLocalities) entries->pop_back();
+    entries->push_front(LocalityEntry{c10::weak_intrusive_ptr<c10::StorageImpl>(map.storage().getWeakStorageImpl()), map.data_ptr(),
+                                      version_of(map), n, K, -1});
+    if (later) return Locality::Unknown;
+    entry = &entries->front();
+  }
   const int slot = next;
   next = (next + 1) % kMaxLocalities;
-  entries->remove_if([&](const LocalityEntry &e) { return e.slot == slot || e.map_s.expired(); });
+  entries->remove_if([&](const LocalityEntry &e) { return e.slot == slot; });
   flags[slot] = 0;
   ok(sph_map_locality(map.data_ptr(), n, K, (int *)flags + slot, st), "sph_map_locality");
-  entries->push_front(LocalityEntry{c10::weak_intrusive_ptr<c10::StorageImpl>(map.storage().getWeakStorageImpl()), map.data_ptr(),
-                                    version_of(map), n, K, slot});
+  entry->slot = slot;
   return Locality::Unknown;
 }
 
@@ -393,7 +405,7 @@ torch::Tensor resample_from_map_impl(torch::Tensor x, torch::Tensor map, const t
 int64_t scatter_group_planes(const torch::Tensor &x, const torch::Tensor &map, const MapInfo &m, int64_t oh, int64_t ow, bool normalize) {
   const int64_t planes = x.size(0) * x.size(1), n = m.H * m.W;
   const bool in_place = m.P == 0 && x.scalar_type() == torch::kFloat && planes >= (normalize ? 4 : 3) && n <= 2 * oh * ow && 8 * n >= oh * ow &&
-                        locality_of(map, n, 1) == Locality::Local;
+                        locality_of(map, n, 1, true) == Locality::Local;
   return in_place ? 0 : planes;
 }
 

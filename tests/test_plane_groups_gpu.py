@@ -212,7 +212,9 @@ def test_scatter_by_locality(local):
     for run in (C.resample_to_map, lambda x, m, h, w, it: C.resample_to_map_normalized(x, m, None, h, w, it)):
         C.clear_plan_cache()
         smap = m.clone()
-        run(x, smap, 40, 80, C.InterpolationType.BILINEAR)    # (the plan, and a look at the map)
+        run(x, smap, 40, 80, C.InterpolationType.BILINEAR)    # (the plan)
+        seen, n = _launches(lambda: run(x, smap, 40, 80, C.InterpolationType.BILINEAR))
+        assert n == 3                                         # (a look at the map)
         torch.cuda.synchronize()
         got, n = _launches(lambda: run(x, smap, 40, 80, C.InterpolationType.BILINEAR))
         assert n == (1 if local else 2)
