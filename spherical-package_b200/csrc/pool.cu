@@ -69,7 +69,7 @@ max_pool_kernel(const T *__restrict__ x, const T *__restrict__ map, const T *__r
 // Max pooling of unweighted float32 maps of four taps, the planes read where they lie: the kernel above with fewer instructions per
 // value where the taps of a warp are squares of pixels, which they are but at the image's edges, and the next slot's coordinates
 // fetched with this one's pixels.  Bound: the SM's path to L1 (two to three wavefronts per load of 32 taps two pixels apart, and what
-// it fetches from L2, 80 %) and issue (65 %).  3 x 3 gnomonic map of stride 2, 1024 planes of 256 x 512: the kernel above on blocks of
+// it fetches from L2, 87 %) and issue (73 %).  3 x 3 gnomonic map of stride 2, 1024 planes of 256 x 512: the kernel above on blocks of
 // 256 outputs of a row 547 us, over plane groups 568; on blocks of 32 x 8 447; so 407, on blocks of 64 x 4 385.  (Five blocks per SM
 // 421, six 433; sixteen planes per thread 466, four 453; three slots at a time, so that their lines are fetched once, 434: it fetches
 // a third and holds 80 registers; pairs as eight-byte loads where a warp's are aligned: 405, odd widths 463.)

@@ -74,8 +74,8 @@ resample_from_map_kernel(const T *__restrict__ x, const T *__restrict__ map, con
 // a[j] / d for all j, rounded as a division is.  Float32: with the reciprocal r of d, rounded to nearest, q = a r is less than two units
 // off, and each step q + (a - q d) r, the remainder in one fused operation, makes an approximation within a unit the nearest one (P.
 // Markstein, IBM J. Res. Dev. 34, 1990); two steps of them, and no operation over- or underflows for divisors within 2^+-60 and values
-// that are zero or within 2^-80 and 2^60.  Others are divided.  Ten instructions per value where a division has seventeen
-// (154 planes of 974 x 1948 pixels: 472 us, 327 of them without the divisions).
+// that are zero or within 2^-80 and 2^60.  Others are divided.  (154 planes of 974 x 1948
+// pixels with plain divisions: 472 us, 145 of them the divisions.)
 template <int N> __device__ __forceinline__ void divide_all(float (&a)[N], float d) {
   float least = 1.0f, most = 1.0f;
 #pragma unroll
