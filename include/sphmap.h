@@ -340,8 +340,7 @@ size_t sph_conv_workspace_bytes(int op, int64_t B, int64_t Cin, int64_t Cout, in
                                 int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp,
                                 int precision);
 /* Scratch with which the float32 operators of precision 0 run on the tensor cores (operands split into three bf16 parts
- * each: csrc/conv_x3.cu); with less, down to sph_conv_workspace_bytes(), they run on the CUDA cores.  For SPH_CONV_BACKWARD in bf16
- * precision over weighted maps: scratch with which the input gradient may multiply first (csrc/conv_tc.cu).
+ * each: csrc/conv_x3.cu); with less, down to sph_conv_workspace_bytes(), they run on the CUDA cores.
  * For everything else the two are equal. */
 size_t sph_conv_workspace_preferred_bytes(int op, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW,
                                           int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp,

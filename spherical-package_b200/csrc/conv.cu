@@ -112,12 +112,7 @@ extern "C" size_t sph_conv_workspace_preferred_bytes(int op, int64_t B, int64_t 
                                                      int64_t OW, int64_t K, int64_t P, int dtype, int interp, int precision) {
   const size_t base = sph_conv_workspace_bytes(op, B, Cin, Cout, IH, IW, OH, OW, K, P, dtype, interp, precision);
   const Dims d{B, Cin, Cout, IH, IW, OH, OW, K, P};
-  if (check_dims(d, dtype, interp, precision) != SPH_OK || dtype != SPH_F32 || B == 0) return base;
-  if (precision == SPH_PRECISION_BF16) {
-    if (op != SPH_CONV_BACKWARD || base == 0 || small_ok(Cin, K, Cout, 4)) return base;
-    const size_t more = tc_conv_backward_workspace(B, Cin, Cout, IH, IW, OH, OW, K, P, interp, true);
-    return more > base ? more : base;
-  }
+  if (check_dims(d, dtype, interp, precision) != SPH_OK || precision != SPH_PRECISION_EXACT || dtype != SPH_F32 || B == 0) return base;
   const bool transposed = op == SPH_TCONV_FORWARD || op == SPH_TCONV_BACKWARD_INPUT || op == SPH_TCONV_BACKWARD_WEIGHT || op == SPH_TCONV_BACKWARD;
   if (transposed ? small_ok(Cout, K, Cin, 4) : small_ok(Cin, K, Cout, 4)) return base;
   size_t x3 = 0;

@@ -18,14 +18,12 @@ namespace sph {
 // disappear: src_cl is the copy of the gathered tensor, out_cl (forward only) is where the epilogue also writes the
 // output in that layout (real channels, and zeros into the extra pixels; padding channels are zero-filled once by the owner).
 // a_cl (weight gradient): channels-last copy of the left operand, masked; its row sums already sit in the workspace.
-// reads (adjoints): taps of a slot of a weighted map, if the workspace has room to multiply first over such a map.
 struct Fusion {
   bool relu_out = false;
   const void *mask = nullptr;
   const void *src_cl = nullptr;
   void *out_cl = nullptr;
   const void *a_cl = nullptr;
-  int64_t reads = 0;
   bool active() const { return relu_out || mask != nullptr; }
 };
 
@@ -123,9 +121,8 @@ int tc_conv_backward_weight(const void *gout, const void *x, const void *map, co
 int tc_conv_backward(const void *gout, const void *x, const void *plan, const void *map, const void *iw, const void *weight,
                      void *gx, void *gw, void *gb, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH,
                      int64_t OW, int64_t K, int64_t P, int interp, void *ws, size_t ws_bytes, cudaStream_t st, const Fusion &fz);
-// preferred: with room for the column buffer of a weighted map's multiply-first input gradient
 size_t tc_conv_backward_workspace(int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH, int64_t OW,
-                                  int64_t K, int64_t P, int interp, bool preferred = false);
+                                  int64_t K, int64_t P, int interp);
 int padded_channels(int64_t CH);
 int tc_fill_companion(const void *x, void *x_cl, int64_t B, int64_t C, int64_t HW, cudaStream_t st);
 // Thin gathered side (channels x K <= 63) on the tensor cores, bf16 precision: see conv_tc_thin.cuh.

@@ -1951,19 +1951,12 @@ struct PremulGeometry {
   bool use;
 };
 
-// The same over a weighted map (reads > 0: taps of a slot) with at least three entries per destination pixel and slot, which the
-// gather form reads as rows of Cp channels and this one as rows of M: over a map without locality either waits for these rows,
-// and the gather form's warps wait for the longest of their pixels' segments on top (backward of four random points a slot,
-// gather and multiply-first: 64 -> 128 channels, 16 x 256 x 512, 5406 and 4845 us; 4 x 128 x 256: 64 -> 256 556 and 355, 64 -> 96
-// 342 and 300, 16 -> 32 235 and 207, 32 -> 64 274 and 271, but 64 -> 64 247 and 286).  Not where the gather form is one wave of
-// tiles (64 -> 128, 4 x 64 x 128 121 and 115 us; 16 x 24 x 48 84 and 95; 1 x 64 x 128 76 and 81).
-PremulGeometry premul_geometry(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t M, int64_t n_dst, int64_t reads = 0) {
+PremulGeometry premul_geometry(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t M, int64_t n_dst) {
   PremulGeometry q{};
   q.Mp = (int)align_up((size_t)M, 8);
   q.g = geometry(B, CH, SHW, 1, 0, SPH_NEAREST, K * q.Mp, true);
   q.t_bytes = align_up((size_t)(B * SHW) * K * q.Mp * 2, 256);
-  const bool weighted = reads * SHW >= 3 * n_dst && 2 * M <= q.g.Cp && B * n_dst > (int64_t)sm_count() * kTileM;
-  q.use = q.g.ok && (n_dst >= 3 * SHW || weighted) && q.t_bytes <= ((size_t)8 << 30) && CH >= 32;
+  q.use = q.g.ok && n_dst >= 3 * SHW && q.t_bytes <= ((size_t)8 << 30) && CH >= 32;
   return q;
 }
 
@@ -2005,7 +1998,7 @@ int tc_gemm(bool use_plan, const void *src, const void *map, const void *iw, con
             int64_t sk, const void *bias, void *out, int64_t Nout, int64_t B, void *ws, size_t ws_bytes, cudaStream_t st,
             const Fusion &fz = Fusion{}) {
   if (use_plan) {
-    const PremulGeometry q = premul_geometry(B, CH, SH * SW, K, Nout, GH * GW, fz.reads);
+    const PremulGeometry q = premul_geometry(B, CH, SH * SW, K, Nout, GH * GW);
     if (q.use) return tc_adjoint_premul(q, src, plan, CH, SH, SW, K, GH, GW, wgt, sn, sc, sk, bias, out, Nout, B, ws, ws_bytes, st, fz);
   }
   const Geometry g = geometry(B, CH, SH * SW, K, P, interp, Nout, !use_plan);
@@ -2046,9 +2039,9 @@ int tc_gemm(bool use_plan, const void *src, const void *map, const void *iw, con
 
 // n_dst > 0: plan mode with that many destination pixels (may select the multiply-first adjoint)
 size_t gemm_ws(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int interp, int64_t Nout, bool direct,
-               int64_t n_dst = 0, int64_t reads = 0) {
+               int64_t n_dst = 0) {
   if (!direct) {
-    const PremulGeometry q = premul_geometry(B, CH, SHW, K, Nout, n_dst, reads);
+    const PremulGeometry q = premul_geometry(B, CH, SHW, K, Nout, n_dst);
     if (q.use) return 256 + q.g.xh_bytes + q.g.wp_bytes + q.t_bytes;
   }
   const Geometry g = geometry(B, CH, SHW, K, P, interp, Nout, direct);
@@ -2247,16 +2240,14 @@ int tc_conv_backward_weight(const void *gout, const void *x, const void *map, co
                ws_bytes, st, fz);
 }
 
-static int64_t adjoint_reads(int64_t P, int interp) { return P * (interp == SPH_NEAREST ? 1 : 4); }
-
 // Combined backward of one convolution.  grad_output feeds two kernels, the input-gradient gather and the weight-gradient
 // MMA, from one channels-last bf16 copy and, with a fused ReLU, has to be masked for both.  One pre-pass reads it (and the
 // mask) once; the reference likewise computes all three gradients in one call
 // (ext_modules/include/layers/mapped_convolution_layer.h:89-134).  Workspace: the input-gradient part first, then
 // the weight-gradient part, each laid out as its own operator expects.
 size_t tc_conv_backward_workspace(int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH, int64_t OW,
-                                  int64_t K, int64_t P, int interp, bool preferred) {
-  const size_t a = gemm_ws(B, Cout, OH * OW, K, 0, 0, Cin, false, IH * IW, preferred ? adjoint_reads(P, interp) : 0);
+                                  int64_t K, int64_t P, int interp) {
+  const size_t a = gemm_ws(B, Cout, OH * OW, K, 0, 0, Cin, false, IH * IW);
   const DwGeometry d = dw_geometry(B, Cin, IH * IW, K, P, interp, Cout, OH, OW, Cout, OH * OW, false);
   if (a == 0 || !d.ok) return 0;
   return align_up(a, 256) + d.total();
@@ -2265,17 +2256,11 @@ size_t tc_conv_backward_workspace(int64_t B, int64_t Cin, int64_t Cout, int64_t 
 int tc_conv_backward(const void *gout, const void *x, const void *plan, const void *map, const void *iw, const void *weight,
                      void *gx, void *gw, void *gb, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH,
                      int64_t OW, int64_t K, int64_t P, int interp, void *ws, size_t ws_bytes, cudaStream_t st, const Fusion &fz) {
-  size_t dx_bytes = gemm_ws(B, Cout, OH * OW, K, 0, 0, Cin, false, IH * IW);
+  const size_t dx_bytes = gemm_ws(B, Cout, OH * OW, K, 0, 0, Cin, false, IH * IW);
   const DwGeometry d = dw_geometry(B, Cin, IH * IW, K, P, interp, Cout, OH, OW, Cout, OH * OW, false);
   if (dx_bytes == 0 || !d.ok) return SPH_ERR_UNSUPPORTED;  // one of the two runs on other kernels: use the separate entry points
   if (!ws || ws_bytes < align_up(dx_bytes, 256) + d.total()) return SPH_ERR_WORKSPACE_TOO_SMALL;
   if ((uintptr_t)ws & 255) return SPH_ERR_INVALID_ARGUMENT;
-  Fusion fx;
-  const size_t more = gemm_ws(B, Cout, OH * OW, K, 0, 0, Cin, false, IH * IW, adjoint_reads(P, interp));
-  if (more != dx_bytes && ws_bytes >= align_up(more, 256) + d.total()) {
-    fx.reads = adjoint_reads(P, interp);
-    dx_bytes = more;
-  }
   char *ws_dx = (char *)ws, *ws_dw = (char *)ws + align_up(dx_bytes, 256);
   __nv_bfloat16 *go_cl = (__nv_bfloat16 *)(ws_dx + 256);  // where tc_gemm / tc_adjoint_premul keep their source
   struct PhaseScope {  // the event list is consumed by this call, whatever its outcome
@@ -2285,6 +2270,7 @@ int tc_conv_backward(const void *gout, const void *x, const void *plan, const vo
   to_nhwc(gout, go_cl, B, Cout, d.a_pitch, OH * OW, st, fz.mask, (float *)(ws_dw + d.bias_at()), (int *)ws_dw);
   note_launches(1);
   mark_phase(1, st);
+  Fusion fx;
   fx.src_cl = go_cl;  // already masked
   int rc = SPH_OK;
   if (gx)

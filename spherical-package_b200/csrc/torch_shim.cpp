@@ -835,14 +835,15 @@ std::vector<torch::Tensor> conv_backward_impl(torch::Tensor go, torch::Tensor ma
   if (a.prec == SPH_PRECISION_BF16) {
     // all three gradients in one call: grad_output is converted (and masked) once for both of its consumers, and the
     // input's channels-last copy is used if a previous layer left one
-    if (sph_conv_workspace_bytes(SPH_CONV_BACKWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec) > 0) {
+    const size_t wbc = sph_conv_workspace_bytes(SPH_CONV_BACKWARD, a.B, a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype,
+                                                a.interp, a.prec);
+    if (wbc > 0) {
       const torch::Tensor cl = find_companion(x);
-      ConvScratch wsc;
-      wsc.get(SPH_CONV_BACKWARD, a, x);
+      torch::Tensor wsc = workspace(wbc, x);
       const int rc = sph_mapped_conv_backward_cl(go.data_ptr(), act_out ? act_out->data_ptr() : nullptr, x.data_ptr(),
                                                  cl.defined() ? cl.data_ptr() : nullptr, need_gx ? plan.data_ptr() : nullptr, map.data_ptr(), iw ? iw->data_ptr() : nullptr,
                                                  weight.data_ptr(), need_gx ? gx.data_ptr() : nullptr, gw.data_ptr(), gb.data_ptr(), a.B,
-                                                 a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec, wsc.ptr(), wsc.bytes,
+                                                 a.Cin, a.Cout, a.IH, a.IW, a.OH, a.OW, a.K, a.P, a.dtype, a.interp, a.prec, wsc.data_ptr(), wbc,
                                                  stream());
       if (rc != SPH_ERR_UNSUPPORTED) {
         ok(rc, "sph_mapped_conv_backward_cl");

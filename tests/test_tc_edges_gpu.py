@@ -52,30 +52,25 @@ def test_extra_pixels_of_an_uninitialised_copy(cin, cout, width):
     assert torch.equal(copy[:, :-1].transpose(1, 2).reshape(3, cout, 16, width), out.bfloat16())
 
 
-@pytest.mark.parametrize("cin,cout,h,w,P,first", [
-    (20, 40, 140, 141, 4, True),     # a copy of 64 channels, ragged tiles
-    (64, 96, 149, 128, 3, True),     # the fewest points, and tiles, that multiply first; a copy of 128 channels
-    (64, 96, 148, 128, 3, False),    # as many pixels as one wave of tiles holds
-    (64, 64, 149, 128, 4, False),    # rows as wide as the gather's
-    (20, 40, 140, 141, 2, False),    # two points
-])
-def test_weighted_input_gradient_multiplies_first(cin, cout, h, w, P, first):
-    """With the preferred scratch, over weighted maps of three points a slot or more; in either form against the oracle."""
+@pytest.mark.parametrize("cin,cout,h,w,P", [(20, 40, 140, 141, 4), (64, 96, 149, 128, 3)])
+def test_weighted_input_gradient_sums_in_float32(cin, cout, h, w, P):
+    """Over a weighted map as over others, the products of the output channels are summed in float32 and nothing between them and the
+    result is rounded to fewer bits: whole numbers whose operands are exact in bf16 come out exact, with either scratch."""
     from sphmap import capi
-    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
-        pytest.skip("the sizes are those of 148 SMs")
+    g = torch.Generator().manual_seed(41)
+    whole = lambda *shape: torch.randint(-7, 8, shape, generator=g).float()  # noqa: E731
     K = 2
-    x, wgt, b, m, iw, go = _case(41, 1, cin, cout, h, w, h, w, K, 0, P)
-    want = port.mapped_conv_backward(go, m, x, wgt, b, K, 0, iw)
+    x, wgt, go = whole(1, cin, h, w), whole(cout, cin, K), whole(1, cout, h, w)
+    m = torch.rand(h, w, K, P, 2, generator=g) * torch.tensor([w - 1.0, h - 1.0])
+    iw = torch.zeros(h, w, K, P)
+    iw[..., 0] = 1.0
+    want = port.mapped_conv_backward(go, m, x, wgt, torch.zeros(cout), K, 0, iw)
+    assert want[0].abs().max() > 1024     # (a bf16 holds every whole number up to 256)
     x, wgt, m, iw, go = [t.cuda() for t in (x, wgt, m, iw, go)]
     plan = capi.plan_build(m, iw, h * w, K, 0, h, w)
-    launches = []
     for preferred in (False, True):
         ws = capi.conv_workspace(capi.CONV_BACKWARD, 1, cin, cout, h, w, h, w, K, P, capi.F32, 0, capi.BF16, x, preferred=preferred)
-        before = capi.lib.sph_launch_count()
         got = capi.conv_backward_cl(go, None, x, None, plan, m, wgt, K, 0, iw, capi.BF16, ws=ws)
-        launches.append(capi.lib.sph_launch_count() - before)
-        for name, a, ref in zip(("grad_input", "grad_weight", "grad_bias"), got, want):
-            _close(a.cpu(), ref, name)
-    assert launches[1] - launches[0] == (1 if first else 0)
+        for a, ref in zip(got, want):
+            assert torch.equal(a.cpu(), ref)
     assert capi.device_status() == 0
