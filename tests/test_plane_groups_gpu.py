@@ -185,8 +185,49 @@ def test_scatter_in_place(planes, h, w):
     _grouped(lambda s: capi.resample_to_map_normalized(go, plan, h, w, ws=s), ws)
 
 
+def _two_by_two(values, weights, h, w):
+    """A map, weights and gradients with which pixel q sums weights[q] * 0 and 1 * values[:, q]."""
+    n = h * w
+    q = torch.arange(n).repeat_interleave(2)
+    m = torch.stack([q % w, q // w], -1).float().view(1, 2 * n, 1, 2)
+    iw = torch.stack([weights, torch.ones(n)], -1).view(1, 2 * n, 1)
+    go = torch.stack([torch.zeros_like(values), values], -1).view(1, -1, 1, 2 * n)
+    return m.cuda(), iw.cuda(), go.cuda()
+
+
+@pytest.mark.parametrize("kind", ["ordinary", "subnormal", "edges"])
+def test_normalised_scatter_divides_in_bounds(kind):
+    """Sums and weights between which the division goes by a reciprocal, in the kernel in place and over groups, all planes of a thread
+    within its bounds: 200,000 pairs with the quotient that IEEE division gives.  `subnormal`: divisors up to its bound, under values down
+    to 2^-80 whose quotients lie half way between two subnormal numbers, on top of one pair that a reciprocal rounds wrongly."""
+    from sphmap import capi
+    planes, h, w = 9, 160, 139
+    n = h * w
+    g = torch.Generator().manual_seed(7)
+    power = lambda lo, hi, *shape: torch.exp2(torch.randint(lo, hi + 1, shape, generator=g).float())  # noqa: E731
+    mantissa = lambda *shape: 1 + torch.rand(*shape, generator=g)  # noqa: E731
+    if kind == "ordinary":
+        values = torch.randn(planes, n, generator=g) * torch.tensor([1.0, 1e3, 1e-10, 0.0, 1e10, 1e-3, 1.0, 30.0, 1.0])[:, None]
+        weights = mantissa(n) * power(-20, 20, n)
+    elif kind == "subnormal":
+        values = 3 * (2 * torch.randint(1000, 1 << 21, (planes, n), generator=g) + 1).double() * 2.0 ** -92
+        weights = torch.full((n,), 3 * 2.0 ** 58)
+        values[:, 0], weights[0] = float.fromhex("0x1.51b5dep-79"), float.fromhex("0x1.faep+59")
+        assert torch.equal(values.float().double(), values)
+        values = values.float()
+    else:
+        values, weights = mantissa(planes, n) * power(-62, 59, planes, n), mantissa(n) * power(-40, 59, n)
+    m, iw, go = _two_by_two(values, weights, h, w)
+    plan = capi.plan_build(m, iw, 2 * n, 1, 0, h, w)
+    den = ((weights + 1.0) + torch.tensor(1e-12)).numpy()
+    want = torch.from_numpy(values.numpy() / den).view(1, planes, h, w)
+    for ws in (None, capi.staging(capi.STAGE_SCATTER, planes, 2 * n, 0, go)):
+        assert torch.equal(capi.resample_to_map_normalized(go, plan, h, w, ws=ws).cpu(), want)
+
+
 def test_normalised_scatter_divides():
-    """sum / (weights + 1e-12) with the rounding of a division, also for values that have none of the usual magnitudes."""
+    """sum / (weights + 1e-12) with the rounding of a division, also for values that have none of the usual magnitudes, which are
+    divided.  (Such a plane takes the others of its thread along.)"""
     from sphmap import capi
     h, w = 16, 40
     _, m, iw, go = _case(9, h, w, 2 * h, w, 1, 1, seed=6)
