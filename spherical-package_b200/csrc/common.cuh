@@ -274,14 +274,24 @@ struct FastDiv {
 
 inline int cdiv(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
-// Outputs (height x width) cut into tiles of 256, one per block, 2^log_tx wide or narrower where the outputs are: neighbours in both
-// directions read the same lines.
+// Outputs (height x width) cut into tiles of 256, one per block: neighbours in both directions read the same lines.
 struct BlockTile {
   int width, height, log_tx;
   FastDiv across;
-  static BlockTile make(int64_t height, int64_t width, int log_tx) {
-    while (log_tx > 2 && (1 << log_tx) >= 2 * width) log_tx--;
+  static BlockTile of(int64_t height, int64_t width, int log_tx) {
     return BlockTile{(int)width, (int)height, log_tx, FastDiv::make((unsigned)cdiv(width, 1 << log_tx))};
+  }
+  // 256 consecutive outputs, whatever their rows.
+  static BlockTile flat(int64_t outputs) { return of(1, outputs, 8); }
+  // Tiles 2^log_tx wide, or half that where they are fewer by a tenth; flat over images narrower than that half, and where even those
+  // are a quarter more than the outputs fill (and eight more: a GPU that is not full anyway gains by more blocks).  Threads without an
+  // output cost as much as others: 64 planes of one row of 65536 positions gathered in 16 x 16 tiles 71 us, flat 13; 2 x 32768 38 and 17,
+  // 5000 x 12 15.6 and 12.5; max pooling onto 33 x 66 outputs in tiles of 64 x 4 12.3 us, 32 x 8 10.0, flat 14.7.
+  static BlockTile make(int64_t height, int64_t width, int log_tx) {
+    const BlockTile wide = of(height, width, log_tx), narrow = of(height, width, log_tx - 1);
+    const BlockTile &t = 10 * (int64_t)narrow.blocks() < 9 * (int64_t)wide.blocks() ? narrow : wide;
+    const bool empty = 4 * (int64_t)t.blocks() > 5 * (int64_t)cdiv(height * width, 256) + 32;
+    return empty || 2 * width < (1 << log_tx) ? flat(height * width) : t;
   }
   unsigned blocks() const { return across.d * (unsigned)cdiv(height, 256 >> log_tx); }
   // This thread's output, or -1.

@@ -17,12 +17,16 @@ namespace sph {
 //
 // AVG = true turns the same walk into mapped average pooling: the K slot values are added in slot order and the sum
 // is divided by K (ext_modules/include/common/mapped_avg_pool.h:12-39, 71-107); idx is not written.
+//
+// Bound: latency and issue.  A block's outputs are 256 in a row: in tiles of 64 x 4, which suit the kernel below, average pooling of 64
+// planes of 320 x 641 takes 63.9 us instead of 54.6, weighted max pooling of 8 planes of 256 x 512 73 instead of 46, float64 max pooling
+// of 256 planes of 130 x 261 95 instead of 72.
 template <typename T, int INTERP, bool WEIGHTED, bool AVG>
 __global__ void __launch_bounds__(256)
 max_pool_kernel(const T *__restrict__ x, const T *__restrict__ map, const T *__restrict__ iw, T *__restrict__ out,
-                int64_t *__restrict__ idx, BlockTile bt, int planes, int H, int W, int K, int P) {
-  const int o = bt.output(), n = bt.width * bt.height;
-  if (o < 0) return;
+                int64_t *__restrict__ idx, int n, int planes, int H, int W, int K, int P) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= n) return;
   const int p0 = blockIdx.y * kPlanesPerThread;
   const int np = min(kPlanesPerThread, planes - p0);
   const size_t hw = (size_t)H * W;
@@ -521,40 +525,42 @@ static int unpool_planned(const void *g, const int64_t *idx, const void *plan, v
 template <typename T>
 static int pool(const void *x, const void *map, const void *iw, void *out, int64_t *idx, int64_t planes, int64_t H,
                 int64_t W, int64_t OH, int64_t OW, int64_t K, int64_t P, int interp, cudaStream_t st, bool avg = false) {
-  const BlockTile bt = BlockTile::make(OH, OW, 6);
+  const int n = (int)(OH * OW);
   if (avg) {
-    dim3 grid(bt.blocks(), cdiv(planes, kPlanesPerThread));
+    dim3 grid(cdiv(n, 256), cdiv(planes, kPlanesPerThread));
     SPH_DISPATCH_INTERP(interp, {
       if (P > 0)
         max_pool_kernel<T, INTERP, true, true><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, (const T *)iw, (T *)out,
-                                                                     nullptr, bt, (int)planes, (int)H, (int)W, (int)K, (int)P);
+                                                                     nullptr, n, (int)planes, (int)H, (int)W, (int)K, (int)P);
       else
         max_pool_kernel<T, INTERP, false, true><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, nullptr, (T *)out, nullptr,
-                                                                      bt, (int)planes, (int)H, (int)W, (int)K, 0);
+                                                                      n, (int)planes, (int)H, (int)W, (int)K, 0);
     });
     return launch_status();
   }
   if (interp == SPH_NEAREST && P == 0 && K <= kPoolMaxK) {
     constexpr int PPT = 4;
-    dim3 grid(cdiv(OH * OW, 256), cdiv(planes, PPT));
+    dim3 grid(cdiv(n, 256), cdiv(planes, PPT));
 #define SPH_POOL_NEAREST(KMAX) \
-    max_pool_nearest_kernel<T, PPT, KMAX><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, (T *)out, idx, (int)(OH * OW), (int)planes, (int)H, (int)W, (int)K)
+    max_pool_nearest_kernel<T, PPT, KMAX><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, (T *)out, idx, n, (int)planes, (int)H, (int)W, (int)K)
     if (K <= 4) SPH_POOL_NEAREST(4);
     else if (K <= 9) SPH_POOL_NEAREST(9);
     else SPH_POOL_NEAREST(16);
 #undef SPH_POOL_NEAREST
     return launch_status();
   }
-  dim3 grid(bt.blocks(), cdiv(planes, kPlanesPerThread));
+  dim3 grid(cdiv(n, 256), cdiv(planes, kPlanesPerThread));
   SPH_DISPATCH_INTERP(interp, {
     if (P > 0)
       max_pool_kernel<T, INTERP, true, false><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, (const T *)iw, (T *)out, idx,
-                                                             bt, (int)planes, (int)H, (int)W, (int)K, (int)P);
-    else if constexpr (sizeof(T) == 4 && INTERP != SPH_NEAREST)
-      max_pool_square_kernel<INTERP><<<grid, 256, 0, st>>>((const float *)x, (const float *)map, (float *)out, idx, bt, (int)planes, (int)H, (int)W,
+                                                             n, (int)planes, (int)H, (int)W, (int)K, (int)P);
+    else if constexpr (sizeof(T) == 4 && INTERP != SPH_NEAREST) {
+      const BlockTile sq = BlockTile::make(OH, OW, 6);
+      grid.x = sq.blocks();
+      max_pool_square_kernel<INTERP><<<grid, 256, 0, st>>>((const float *)x, (const float *)map, (float *)out, idx, sq, (int)planes, (int)H, (int)W,
                                                         (int)K);
-    else
-      max_pool_kernel<T, INTERP, false, false><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, nullptr, (T *)out, idx, bt,
+    } else
+      max_pool_kernel<T, INTERP, false, false><<<grid, 256, 0, st>>>((const T *)x, (const T *)map, nullptr, (T *)out, idx, n,
                                                               (int)planes, (int)H, (int)W, (int)K, 0);
   });
   return launch_status();

@@ -161,6 +161,24 @@ def test_squares_of_pixels(planes, h, w, oh, ow, interp):
         assert torch.equal(a.nan_to_num(nan=7.0), b.nan_to_num(nan=7.0))
 
 
+@pytest.mark.parametrize("interp", [1, 2])
+@pytest.mark.parametrize("oh,ow", [(1, 700), (700, 1), (2, 331), (331, 2), (3, 333), (9, 130), (33, 66), (4100, 3), (3, 4100)])
+def test_lists_of_positions(oh, ow, interp):
+    """Outputs of a few rows or columns, which take tiles of other shapes or none; gathers, pooling and scatters against the plane groups."""
+    from sphmap import capi
+    x, m, _, go = _case(9, 40, 83, oh, ow, 9, 0, seed=8)
+    one = m[:, :, 4].contiguous()
+    _grouped(lambda s: capi.resample_from_map(x, one, interp, ws=s), capi.staging(capi.STAGE_GATHER, 9, 40 * 83, ANY, x))
+    ws = capi.staging(capi.STAGE_POOL, 9, 40 * 83, ANY, x)
+    _grouped(lambda s: capi.mapped_max_pool(x, m, 9, interp, ws=s), ws)
+    _grouped(lambda s: capi.mapped_avg_pool(x, m, 9, interp, ws=s), ws)
+    at = torch.rand(40, 83, 2, generator=torch.Generator().manual_seed(9)).mul(torch.tensor([ow - 0.5, oh - 0.5])).cuda()
+    plan = capi.plan_build(at, None, 40 * 83, 1, interp, oh, ow)
+    ws = capi.staging(capi.STAGE_SCATTER, 9, 40 * 83, 0, x)
+    _grouped(lambda s: capi.resample_to_map(x, plan, oh, ow, ws=s), ws)
+    _grouped(lambda s: capi.resample_to_map_normalized(x, plan, oh, ow, ws=s), ws)
+
+
 @pytest.mark.parametrize("local", [True, False])
 def test_gather_by_locality(local):
     """Between one and eight reads a pixel: in place over a local map or one not looked at yet, in groups over a scattered one."""
