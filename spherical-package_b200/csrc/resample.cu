@@ -113,8 +113,11 @@ template <int N> __device__ __forceinline__ void divide_all(double (&a)[N], doub
 //         s = o * K + k and whose slots all carry grad[o] / K (common/mapped_avg_pool.h:41-69, 109-143)
 //   NORM  the sum is divided by (sum of the segment's weights + 1e-12), i.e. scatter(x) / (scatter(1) + 1e-12), the
 //         weight-sum normalisation the reference composes in Python (layers/functional/sphere_ops.py:74-80)
+// Blocks per SM that registers leave room for: six (40 registers) for plain float32 sums of eight planes, five (48) for others, four (64)
+// and three for float64.  With 48, 56 and 72 registers, a block less each, 64 planes of 321 x 641 took 34.6 us instead of 30.8, in
+// float64 56.8 instead of 51.1.
 template <typename T, int PL, bool NORM, bool DIV>
-__global__ void __launch_bounds__(256, PL == 12 ? 5 : 1)
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? (DIV ? 3 : 4) : PL == 12 || NORM || DIV ? 5 : 6)
 resample_to_map_kernel(const T *__restrict__ x, const void *__restrict__ plan_blob, T *__restrict__ out, BlockTile bt, int n_src,
                        int planes, int div, FastDiv fd) {
   const int q = bt.output(), n_dst = bt.width * bt.height;
