@@ -208,13 +208,18 @@ static int to_map_launch(const void *x, const void *plan, void *out, int64_t pla
   return launch_status();
 }
 
-// Planes per thread: 12 share an entry best (comment of the kernel), 8 where there are no more or where groups of 12 would have to be
-// filled up further.
+// Planes per thread: 12 share an entry best (comment of the kernel), 8 in float64, where there are no more, and where groups of 12 would
+// have to be filled up further.  Average unpooling, which divides each value, takes 12 only where that fills up less (3 x 3 gnomonic maps
+// of stride 2, 8 and 12 planes per thread: 12 planes of 400 x 801 53 and 32 us, 36 100 and 82, 60 148 and 132; but 24 planes of 64 x 128
+// 7.0 and 9.0, 24 of 400 x 801 53.4 and 56.9, 48 101 and 107, 96 195 and 207).
 template <typename T>
 static int to_map(const void *x, const void *plan, void *out, int64_t planes, int64_t n_src, int64_t OH, int64_t OW, cudaStream_t st,
                   int src_div = 1, bool normalize = false) {
-  if (sizeof(T) == 4 && planes > 8 && (planes + 11) / 12 * 12 <= (planes + 7) / 8 * 8)
-    return to_map_launch<T, 12>(x, plan, out, planes, n_src, OH, OW, st, src_div, normalize);
+  if constexpr (sizeof(T) == 4) {
+    const int64_t by12 = (planes + 11) / 12 * 12, by8 = (planes + 7) / 8 * 8;
+    if (planes > 8 && by12 < by8 + (src_div > 1 ? 0 : 1))
+      return to_map_launch<T, 12>(x, plan, out, planes, n_src, OH, OW, st, src_div, normalize);
+  }
   return to_map_launch<T, 8>(x, plan, out, planes, n_src, OH, OW, st, src_div, normalize);
 }
 

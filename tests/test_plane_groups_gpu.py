@@ -203,6 +203,17 @@ def test_scatter_in_place(planes, h, w):
     _grouped(lambda s: capi.resample_to_map_normalized(go, plan, h, w, ws=s), ws)
 
 
+@pytest.mark.parametrize("planes", [8, 9, 12, 13, 24, 36])
+def test_average_unpooling_by_planes(planes):
+    """Threads of 8 and of 12 planes, whole and with a remainder: every plane as if it came alone."""
+    from sphmap import capi
+    x, m, _, go = _case(planes, 17, 33, 9, 17, 9, 0, seed=10)
+    plan = capi.slot_plan_build(m, None, 9, 1, 17, 33)
+    got = capi.mapped_avg_unpool(go, plan, 17, 33, 9)
+    for j in range(planes):
+        assert torch.equal(got[:, j:j + 1], capi.mapped_avg_unpool(go[:, j:j + 1].contiguous(), plan, 17, 33, 9))
+
+
 def _two_by_two(values, weights, h, w):
     """A map, weights and gradients with which pixel q sums weights[q] * 0 and 1 * values[:, q]."""
     n = h * w
