@@ -121,9 +121,12 @@ int sph_resample_from_map(const void *x, const void *map, const void *iw, void *
  * neighbouring pixels, a caller does better without scratch for gathers that
  * read a pixel less than eight times, for max pooling by nearest neighbours
  * (unweighted, K <= 16; by 8 to 75 %) and of four taps (unweighted; by 8 to
- * 48 %), and for scatters of an eighth to two positions per pixel
- * (unweighted, but for three normalised planes; by 3 to 40 %); and, whatever the map, for nearest-neighbour pooling of half a
- * million values or fewer.  The host extension follows these rules.
+ * 48 %), and for unweighted scatters of an eighth to two positions per pixel
+ * of an image of up to 2^16 pixels or of 5 to 12 planes, and for others by
+ * planes, positions and pixels (by up to 90 %; the host extension's
+ * scatter_group_planes() has the cases); and, whatever the map, for
+ * nearest-neighbour pooling of half a million values or fewer.  The host
+ * extension follows these rules.
  * sph_map_locality() looks at 256 pairs of a float32 map (n positions, K slots)
  * and writes 1 (they do) or 2 to *flag, device-accessible memory, on the
  * stream.

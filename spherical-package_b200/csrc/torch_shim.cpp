@@ -397,15 +397,37 @@ torch::Tensor resample_from_map_impl(torch::Tensor x, torch::Tensor map, const t
   return y;
 }
 
-// Planes that a scatter takes in groups: none where the kernel that reads the gradients in place is faster, over local maps of an
-// eighth of a position to two positions per pixel (tangent images, in groups and in place: 96 planes of 20 x 256 x 256 onto 1024 x 2048
-// 632 and 532 us, 24 of 20 x 64 x 64 onto 512 x 1024 26 and 21, 28 of 20 x 200 x 200 onto 700 x 1401 119 and 105; a gnomonic map of 64
-// planes 34 and 20; but 16 positions per pixel 349 and 741, 0.045 positions 321 and 345, 0.12 57 and 72, positions at random 46 and 99),
-// and not for three normalised planes (42 and 46).
+// Planes that a scatter takes in groups: none where the kernel that reads the gradients in place is faster over local maps.  Both were
+// timed over tangent images (a tenth of a position to two per pixel of 141 x 282 .. 1024 x 2048) and gnomonic maps (strides 1 to 3), 3 to
+// 96 planes; groups and in place in us:
+//   small images: in place (141 x 282 pixels, 8 planes, 0.13 positions per pixel 5.5 and 3.5)
+//   3 and 4 planes, whose threads are half empty: up to 512 x 1024 pixels (3 planes, 0.27 positions 8.9 and 8.2) or, normalised, half
+//     of that; beyond, from half a position on (1024 x 2048, 3 planes: 0.15 positions 20.2 and 22.5, 0.5 31.0 and 30.4), normalised from
+//     one on
+//   5 to 8 planes: always, but normalised over large images from half a position on (1024 x 2048, 8 planes, 0.27 positions 37 and 42)
+//   where threads take 12 planes: always (512 x 1024, 24 planes, 0.15 positions 21.9 and 18.7), but 36 planes or more, unless
+//     normalised over large images, from a quarter of a position on (512 x 1024, 96 planes: 0.15 positions 62 and 75, 0.35 106 and 97)
+//   where they take 8 of more, and groups of 16 are at their best: over large images from half a position on (1024 x 2048, 16 planes: 0.15
+//     positions 45 and 57, 0.8 122 and 120), and over maps of the image's own proportions, whose rows run along its rows, from a quarter
+//     of a position on (321 x 641, 16 planes, stride 1 15.8 and 9.4; but tangent images of 300 x 601 at 0.8 13.3 and 15.3)
+// Nowhere above two positions per pixel (16 of them, 96 planes 349 and 741), or above one where a small image has more than 16 planes, or
+// at random positions (46 and 99).  Of 2028 scatters so decided 12 are slower than in groups by 5 to 11 %, the geometric mean is 1.2.
 int64_t scatter_group_planes(const torch::Tensor &x, const torch::Tensor &map, const MapInfo &m, int64_t oh, int64_t ow, bool normalize) {
-  const int64_t planes = x.size(0) * x.size(1), n = m.H * m.W;
-  const bool in_place = m.P == 0 && x.scalar_type() == torch::kFloat && planes >= (normalize ? 4 : 3) && n <= 2 * oh * ow && 8 * n >= oh * ow &&
-                        locality_of(map, n, 1, true) == Locality::Local;
+  const int64_t planes = x.size(0) * x.size(1), n = m.H * m.W, pixels = oh * ow;
+  const bool twelve = planes > 8 && (planes + 11) / 12 * 12 <= (planes + 7) / 8 * 8;
+  const bool alike = 2 * m.H * ow <= 3 * m.W * oh && 2 * m.W * oh <= 3 * m.H * ow;
+  const bool large = pixels > ((int64_t)1 << 19);
+  int64_t least;  // eighths of a position per pixel
+  if (pixels <= ((int64_t)1 << 16)) least = 1;
+  else if (planes <= 4) least = pixels <= ((int64_t)1 << (normalize ? 18 : 19)) ? 1 : normalize ? 8 : 4;
+  else if (planes <= 8) least = normalize && large ? 4 : 1;
+  else if (twelve) least = planes < 36 || (normalize && large) ? 1 : 2;
+  else if (alike) least = 2;
+  else if (large) least = 4;
+  else return planes;
+  const int64_t most = planes <= 16 || pixels > ((int64_t)1 << 18) ? 2 : 1;
+  const bool in_place = m.P == 0 && x.scalar_type() == torch::kFloat && planes >= (normalize ? 4 : 3) && n <= most * pixels &&
+                        8 * n >= least * pixels && locality_of(map, n, 1, true) == Locality::Local;
   return in_place ? 0 : planes;
 }
 

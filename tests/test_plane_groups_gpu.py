@@ -292,6 +292,36 @@ def test_scatter_by_locality(local):
         assert n > 2
 
 
+@pytest.mark.parametrize("h,w,face,planes,normalised,in_place", [
+    (141, 282, 16, 16, False, True),      # a small image
+    (141, 282, 61, 24, False, False),     # two positions per pixel of it, more than 16 planes
+    (512, 1024, 84, 3, False, True),      # half-empty threads, a quarter of a position per pixel of half a million
+    (512, 1024, 84, 4, True, False),      # the same, normalised
+    (300, 601, 37, 8, True, True),
+    (300, 601, 37, 24, False, True),      # threads of 12 planes
+    (300, 601, 37, 48, False, False),     # many of them, few positions
+    (300, 601, 85, 16, False, False),     # one whole group
+    (256, 512, 0, 16, False, True),       # the same, a map of the image's proportions
+])
+def test_scatter_by_planes_and_positions(h, w, face, planes, normalised, in_place):
+    """Over local maps the faster of the two kernels, with the same bits."""
+    import _spherical_distortion_ext._C as C
+    from sphmap import capi
+    from sphmap.workloads import tangent_image_map
+    m = tangent_image_map(h, w, face).cuda() if face else _map(True, h, w, 0, 0, 9)[:, :, 4].contiguous()
+    x = torch.randn(1, planes, *m.shape[:2], generator=torch.Generator().manual_seed(4)).cuda()
+    it = C.InterpolationType.BILINEAR
+    run = lambda: C.resample_to_map_normalized(x, m, None, h, w, it) if normalised else C.resample_to_map(x, m, h, w, it)  # noqa: E731
+    want = run()
+    for _ in range(2):    # (the plan, a look at the map)
+        run()
+        torch.cuda.synchronize()
+    got, n = _launches(run)
+    assert n == (1 if in_place else 2)
+    assert torch.equal(got, want)
+    C.clear_plan_cache()
+
+
 @pytest.mark.parametrize("planes", [3, 8, 16])
 def test_scatter_with_a_plan_of_another_size_yields_zeros(planes):
     """A plan that was built for another destination, or is none, is not followed: zeros, as from the direct kernel."""
