@@ -466,7 +466,7 @@ def run_pool(args, rank, local, world):
     # the scratch that the host extension brings: forward over plane groups unless the map is local, the deterministic backward always
     planes, npix, nout = x.shape[0] * x.shape[1], x.shape[2] * x.shape[3], out.shape[2] * out.shape[3]
     ws_fwd, ws_bwd = capi.staging(capi.STAGE_POOL, planes, npix, 9 * nout, x), capi.staging(capi.STAGE_ARGMAX, planes, nout, 0, x)
-    local = {id(m): capi.map_locality(m, 9) == 1}
+    in_place = {id(m): capi.map_locality(m, 9) == 1}
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
     ef = [torch.cuda.Event(enable_timing=True) for _ in range(6)]
     tf, tb, td = [], [], []
@@ -475,7 +475,7 @@ def run_pool(args, rank, local, world):
     def step():
         flush.zero_()
         ef[0].record()
-        capi.mapped_max_pool(x, m, 9, 0, None, out, idx, ws=None if local[id(m)] else ws_fwd)
+        capi.mapped_max_pool(x, m, 9, 0, None, out, idx, ws=None if in_place[id(m)] else ws_fwd)
         ef[1].record()
         flush.zero_()
         ef[2].record()
@@ -507,7 +507,7 @@ def run_pool(args, rank, local, world):
     # the same kernels on a map with locality (3x3 gnomonic, stride 2: what a pooling layer of a spherical network
     # uses), same tensor sizes: shows the kernels' bandwidth when the taps are not uniformly random
     ml = wl.gnomonic_map(x.shape[2], x.shape[3], 2).to(dev)
-    local[id(ml)] = capi.map_locality(ml, 9) == 1
+    in_place[id(ml)] = capi.map_locality(ml, 9) == 1
     tf_r, tb_r, det_ms = list(tf), list(tb), sum(td) / len(td)
     tf.clear(), tb.clear(), td.clear()
     m_random, m = m, ml
