@@ -124,15 +124,20 @@ def test_few_values_are_pooled_in_place(planes, h, w):
     _chosen(lambda: MappedMaxPool(9, InterpolationType.NEAREST, return_indices=True)(x, m), 1, 1)
 
 
+@pytest.mark.parametrize("planes,h", [(3, 40), (8, 144), (64, 40), (64, 144)])
+@pytest.mark.parametrize("interp", [1, 2])
 @pytest.mark.parametrize("local", [True, False])
-def test_second_wave_of_pooling_blocks(local):
-    """Four taps, and blocks of plane groups that fill the GPU once and a little: in place over a local map."""
-    from spherical_distortion.nn import InterpolationType, MappedMaxPool
-    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
-        pytest.skip("the size is one of 148 SMs")
-    m = _map(local, 144, 288, 72, 144, 9)
-    x = torch.randn(2, 64, 144, 288, generator=torch.Generator().manual_seed(4)).cuda()
-    _chosen(lambda: MappedMaxPool(9, InterpolationType.BILINEAR, return_indices=True)(x, m), 3, 1 if local else 2)
+def test_four_tap_pooling_by_locality(local, interp, planes, h):
+    """Four taps: in place over a local map, whatever the planes and the waves of blocks, in groups over a scattered one or one not looked
+    at yet (one launch more)."""
+    import _spherical_distortion_ext._C as C
+    from spherical_distortion.nn import MappedMaxPool
+    from sphmap import capi
+    m = _map(local, h, 2 * h, h // 2, h, 9)
+    x = torch.randn(1, planes, h, 2 * h, generator=torch.Generator().manual_seed(4)).cuda()
+    out, idx = _chosen(lambda: MappedMaxPool(9, C.InterpolationType(interp), return_indices=True)(x, m), 3, 1 if local else 2)
+    want, at = capi.mapped_max_pool(x, m, 9, interp, ws=capi.staging(capi.STAGE_POOL, planes, 2 * h * h, ANY, x))
+    assert torch.equal(out, want) and torch.equal(idx, at)
 
 
 @pytest.mark.parametrize("planes", [7, 8, 17])
