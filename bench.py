@@ -553,12 +553,16 @@ def run_pool(args, rank, local, world):
             "clocks": clocks}
 
 
-def _time_resample(capi, x, m, plan, H, W, steps, warmup, flush):
-    """(gather ms, scatter ms, launches): the gather reads the planes in place (less than one read a pixel), the scatter goes over
-    plane groups, as in the host extension."""
-    y = capi.resample_from_map(x, m, 1)
+def _time_resample(capi, x, m, H, W, steps, warmup, flush):
+    """(gather ms, scatter ms, launches) of the host extension's operators, which choose between planes in place and plane groups; it
+    knows the map after three scatters."""
+    from _spherical_distortion_ext import _C
+    bilinear = _C.InterpolationType.BILINEAR
+    y = _C.resample_from_map(x, m, bilinear)
     out = torch.empty_like(x)
-    ws = capi.staging(capi.STAGE_SCATTER, x.shape[0] * x.shape[1], m.shape[0] * m.shape[1], 0, x)
+    for _ in range(3):
+        _C.resample_to_map(y, m, H, W, bilinear)
+        torch.cuda.synchronize()
     ev = [torch.cuda.Event(enable_timing=True) for _ in range(4)]
     tg, ts = [], []
     for i in range(warmup + steps):
@@ -566,11 +570,11 @@ def _time_resample(capi, x, m, plan, H, W, steps, warmup, flush):
             l0 = capi.lib.sph_launch_count()
         flush.zero_()
         ev[0].record()
-        capi.resample_from_map(x, m, 1)
+        _C.resample_from_map(x, m, bilinear)
         ev[1].record()
         flush.zero_()
         ev[2].record()
-        capi.resample_to_map(y, plan, H, W, ws=ws)
+        _C.resample_to_map(y, m, H, W, bilinear)
         ev[3].record()
         torch.cuda.synchronize()
         if i >= warmup:
@@ -597,15 +601,14 @@ def run_resample(args, rank, local, world):
     lo, hi = shard_batch(B, rank, world)
     x, m = cfg["x"][lo:hi].to(dev), cfg["map"].to(dev)
     H, W = cfg["out_hw"]
-    plan = capi.plan_build(m, None, m.shape[0] * m.shape[1], 1, 1, H, W)
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)
-    g_ms, s_ms, launches = _time_resample(capi, x, m, plan, H, W, args.steps, args.warmup, flush)
+    g_ms, s_ms, launches = _time_resample(capi, x, m, H, W, args.steps, args.warmup, flush)
     n, C, ns = hi - lo, x.shape[1], m.shape[0] * m.shape[1]
     g_bytes, s_bytes = _resample_bytes(n, C, ns, H, W, m.numel())
     # scaled variant: 256 images, seeded the same way
     gbig = torch.Generator().manual_seed(1)
     xb = torch.rand(256 // world, C, H, W, generator=gbig).to(dev)
-    gb_ms, sb_ms, _ = _time_resample(capi, xb, m, plan, H, W, max(3, args.steps // 2), 2, flush)
+    gb_ms, sb_ms, _ = _time_resample(capi, xb, m, H, W, max(3, args.steps // 2), 2, flush)
     gb_bytes, sb_bytes = _resample_bytes(xb.shape[0], C, ns, H, W, m.numel())
     g_ms, s_ms = max_over_ranks(g_ms, world, dev), max_over_ranks(s_ms, world, dev)
     gb_ms, sb_ms = max_over_ranks(gb_ms, world, dev), max_over_ranks(sb_ms, world, dev)
