@@ -320,6 +320,7 @@ extern "C" int sph_mapped_conv_backward_cl(const void *gout, const void *act_out
                                            int64_t OH, int64_t OW, int64_t K, int64_t P, int dtype, int interp, int precision,
                                            void *ws, size_t ws_bytes, void *stream) {
   SPH_RANGE("sph_mapped_conv_backward_cl");
+  const PhaseScope phase_scope;
   const Dims d{B, Cin, Cout, IH, IW, OH, OW, K, P};
   const int rc = check_dims(d, dtype, interp, precision);
   if (rc != SPH_OK) return rc;

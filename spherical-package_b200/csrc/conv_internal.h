@@ -82,6 +82,11 @@ size_t x3_backward_workspace(bool transposed, int64_t B, int64_t Cin, int64_t Co
 int x3_backward(bool transposed, const void *gout, const void *x, const void *plan, const void *map, const void *iw, const void *weight,
                 void *gx, void *gw, void *gb, int64_t B, int64_t Cin, int64_t Cout, int64_t IH, int64_t IW, int64_t OH, int64_t OW, int64_t K,
                 int64_t P, int interp, void *ws, cudaStream_t st);
+// Tracing (sph_trace_phases): records event i of the list that the next combined backward call on this thread takes.
+void mark_phase(int i, cudaStream_t st);
+struct PhaseScope {  // of that call: the list serves it alone, whatever its outcome
+  ~PhaseScope();
+};
 int x3_wait_status(int reset);  // sticky word of a bounded wait that gave up; < 0: CUDA error
 
 template <typename T>

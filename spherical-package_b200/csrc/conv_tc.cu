@@ -2171,13 +2171,13 @@ size_t dw_ws(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int inter
 
 }  // namespace
 
-// Tracing aid (sph_trace_phases): events the next combined backward call on this thread records at its phase boundaries.
 thread_local cudaEvent_t g_phase_events[4];
 thread_local int g_phase_count = 0;
 
-static void mark_phase(int i, cudaStream_t st) {
+void mark_phase(int i, cudaStream_t st) {
   if (i < g_phase_count && g_phase_events[i] != nullptr) cudaEventRecord(g_phase_events[i], st);
 }
+PhaseScope::~PhaseScope() { g_phase_count = 0; }
 
 namespace {
 #include "conv_tc_thin.cuh"
@@ -2263,9 +2263,6 @@ int tc_conv_backward(const void *gout, const void *x, const void *plan, const vo
   if ((uintptr_t)ws & 255) return SPH_ERR_INVALID_ARGUMENT;
   char *ws_dx = (char *)ws, *ws_dw = (char *)ws + align_up(dx_bytes, 256);
   __nv_bfloat16 *go_cl = (__nv_bfloat16 *)(ws_dx + 256);  // where tc_gemm / tc_adjoint_premul keep their source
-  struct PhaseScope {  // the event list is consumed by this call, whatever its outcome
-    ~PhaseScope() { g_phase_count = 0; }
-  } phase_scope;
   mark_phase(0, st);
   to_nhwc(gout, go_cl, B, Cout, d.a_pitch, OH * OW, st, fz.mask, (float *)(ws_dw + d.bias_at()), (int *)ws_dw);
   note_launches(1);

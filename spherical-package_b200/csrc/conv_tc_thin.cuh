@@ -733,9 +733,7 @@ int tc_thin_backward(const void *gout, const void *act, const void *x, const voi
   p.total_steps = (long long)B * p.steps_per_image;
   p.do_dw = do_dw ? 1 : 0; p.do_dx = do_dx ? 1 : 0;
   p.t2_pitch = (int)thin_t2_pitch(K);
-  struct PhaseScope {  // the event list is consumed by this call, whatever its outcome
-    ~PhaseScope() { g_phase_count = 0; }
-  } phase_scope;
+  const PhaseScope phase_scope;
   mark_phase(0, st);
   if (do_dx)
     thin_wt_image_kernel<<<cdiv(128 * kChunk, 256), 256, 0, st>>>((const float *)weight, (__nv_bfloat16 *)(w8 + L.off_wt), (int)N, (int)CH,

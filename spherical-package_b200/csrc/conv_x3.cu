@@ -1400,10 +1400,16 @@ int x3_backward(bool transposed, const void *gout, const void *x, const void *pl
     dx.pre.sums = dw.pre.sums;
     dw.pre.blocks = 0;
   }
+  mark_phase(0, st);
   backward_prepare3_kernel<<<(unsigned)(dw.grad.blocks + dx.wt.blocks + dx.pre.blocks + dw.pre.blocks), 256, 0, st>>>(
       dx.pre, dw.pre, dx.wt, dw.grad, dx.p.status, dw.p.status);
-  const int rc = run_gemm3(dx, 1, st);
-  return rc != SPH_OK ? rc : run_dw3(dw, 0, st);
+  mark_phase(1, st);
+  int rc = run_gemm3(dx, 1, st);
+  if (rc != SPH_OK) return rc;
+  mark_phase(2, st);
+  rc = run_dw3(dw, 0, st);
+  mark_phase(3, st);
+  return rc;
 }
 
 int x3_wait_status(int reset) {

@@ -177,3 +177,39 @@ def test_one_pre_pass_for_all_gradients(case):
         with pytest.raises(capi.Unsupported):
             call()
     assert capi.device_status() == 0
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_phases_of_the_combined_backward(prec):
+    """sph_trace_phases: the next combined call records its events, in order, whatever the precision; the list serves one call, also
+    one that declines."""
+    from sphmap import capi
+    B, ci, co, H, W, K = 2, 32, 32, 16, 32, 9
+    g = torch.Generator().manual_seed(3)
+    r = lambda *s: torch.randn(*s, generator=g).cuda()  # noqa: E731
+    x, w, go = r(B, ci, H, W), r(co, ci, K), r(B, co, H, W)
+    m = (torch.rand(H, W, K, 2, generator=g) * torch.tensor([W - 1.0, H - 1.0])).cuda()
+    plan = capi.plan_build(m, None, H * W, K, 1, H, W)
+    ws = capi.conv_workspace(capi.CONV_BACKWARD, B, ci, co, H, W, H, W, K, 0, capi.F32, 1, prec, x, preferred=True)
+    events, begin = ([torch.cuda.Event(enable_timing=True) for _ in range(n)] for n in (4, 1))
+
+    def recorded(call):
+        """Times of the events since the start of the call; negative: not recorded by it."""
+        for e in events:
+            e.record()
+        torch.cuda._sleep(1000000)
+        begin[0].record()
+        call()
+        torch.cuda.synchronize()
+        return [begin[0].elapsed_time(e) for e in events]
+
+    call = lambda: capi.conv_backward_cl(go, None, x, None, plan, m, w, K, 1, None, prec, ws=ws)  # noqa: E731
+    recorded(call)
+    capi.trace_phases(events)
+    t = recorded(call)
+    assert t[0] >= 0 and t == sorted(t) and t[3] > t[1], t
+    assert max(recorded(call)) < 0
+    capi.trace_phases(events)
+    with pytest.raises(capi.Unsupported):
+        capi.conv_backward_cl(go.double(), None, x.double(), None, plan, m.double(), w.double(), K, 1, None, capi.EXACT, ws=ws)
+    assert max(recorded(call)) < 0
