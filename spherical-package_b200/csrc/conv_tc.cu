@@ -314,7 +314,6 @@ struct Smem {
 constexpr int kOutStageCh = 16;
 constexpr int kClStageBytes = kEpilogueWarps * 32 * kOutStageCh * 2;  // channels-last copy: [warp][2 rows][16 px][16 ch] bf16
 constexpr int kOutStageBytes = kEpilogueWarps * kOutStageCh * 32 * 4 + kClStageBytes;
-constexpr int kBiasBytes = 256 * 4;
 constexpr int kRowStage = 32 * 128;  // bf16 rows: [warp][2 buffers][32 pixels][64 columns], 128-byte swizzle
 constexpr int kRowStageBytes = kEpilogueWarps * 2 * kRowStage + 1024;
 
@@ -325,7 +324,7 @@ inline size_t gemm_smem_bytes(int stages, int Npb, int K, int nt, bool direct, b
   if (!direct) s += (size_t)K * kTileM * sizeof(int2);
   if (over) s += (size_t)K * kTileM * 4 * sizeof(Tap);
   s += 8 * (2 * stages + 4) + 16;
-  s += kOutStageBytes + 128 + kBiasBytes;
+  s += kOutStageBytes + 128 + Npb * 4;
   return s;
 }
 
@@ -1812,11 +1811,12 @@ Geometry geometry(int64_t B, int64_t CH, int64_t SHW, int64_t K, int64_t P, int 
   if ((SHW + 1) * g.Cp * 2 >= ((int64_t)1 << 31)) g.ok = false;
   g.wp_bytes = align_up((size_t)g.nblk * g.nchunks * g.Npb * kChunk * 2, 256);
   g.ok = g.ok && (size_t)K * kTileM * g.nt * sizeof(Tap) <= (size_t)kMaxTapBytes;
-  // Pipeline depth.  Shared memory and L1 share one 256 KB array whose split moves in steps; a CTA that asks for more
-  // than 196 KB leaves 28 KB of L1 for the gather instead of 60 KB, which costs more than a pipeline stage gains
-  // (layer-4 input gradient of the encoder: 3 stages at 207 KB 3.97 ms, 2 stages at 158 KB 3.77 ms).  So: as many stages
-  // as fit 196 KB, and only if two do not fit, as many as fit the whole array.
-  constexpr size_t kSoftLimit = 196 * 1024;
+  // Pipeline depth.  Shared memory and L1 share one 256 KB array whose split moves in steps; a CTA that takes more
+  // than 196 KB, one of them the system's, leaves 28 KB of L1 for the gather instead of 60 KB, which costs more than a pipeline
+  // stage gains (layer-4 input gradient of the encoder: 3 stages at 207 KB 3.97 ms, 2 stages at 158 KB 3.77 ms; plan mode of
+  // 32 -> 135 channels, 2 x 57 x 114, 4 stages: 194.2 KB 27.6 us, 195.2 KB 34.0).  So: as many stages as fit 195 KB, and only
+  // if two do not fit, as many as fit the whole array.
+  constexpr size_t kSoftLimit = 195 * 1024;
   // Plan mode: a key has about four entries on a map that neither stretches nor folds the image, but their number varies - on a
   // map without locality it is near a Poisson variable of mean four, and more than a third of the keys have five or more.
   // Entries five to eight come from a second table where two stages still fit beside it; without it each is a dependent
