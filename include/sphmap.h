@@ -26,7 +26,14 @@
  *           sph_conv_workspace_preferred_bytes() of scratch, else on the CUDA
  *           cores, as float64 always does;
  *           1: bf16 operands with fp32 accumulation on the tcgen05 tensor
- *           cores (float32 tensors only).
+ *           cores (float32 tensors only).  Gathered values are rounded
+ *           to bf16 after each tap (in thin layers once).  Adjoints of 32
+ *           channels or more onto at least three times as many pixels as
+ *           they read (input gradients through maps of stride 2,
+ *           transposed convolutions that double the resolution) and thin
+ *           layers' input gradients multiply first: their sums over the
+ *           channels are rounded to bf16 once, before the fp32 sum over
+ *           slots and taps.
  *
  * Reference interfaces are cited as file:line inside the reference project.
  */
